@@ -24,33 +24,8 @@ namespace ph {
 
 constexpr int NACC = 13;  // rho, gradh, gradsoft, divB + 9 dB/dx sums
 
-// cubic spline W and dW/dq (kernel_cubic.f90:34-50), exact rounding
-__device__ __forceinline__ void kern_exact(double q2, double q, double &w, double &g) {
-  if (q < 1.0) {
-    w = dadd(dsub(dmul(dmul(0.75, q2), q), dmul(1.5, q2)), 1.0);
-    g = dmul(q, dsub(dmul(2.25, q), 3.0));
-  } else if (q < 2.0) {
-    double t = dsub(q, 2.0);
-    w = dmul(-0.25, dmul(dmul(t, t), t));
-    g = dmul(-0.75, dmul(t, t));
-  } else {
-    w = 0.0; g = 0.0;
-  }
-}
-// get_kernel_grav1 (kernel_cubic.f90:78-99) dphidh term
-__device__ __forceinline__ double dphidh_exact(double q2, double q) {
-  if (q < 1.0) {
-    double q4 = dmul(q2, q2);
-    return dadd(dsub(dadd(dmul(dmul(-0.6, q4), q), dmul(1.5, q4)), dmul(2.0, q2)), 1.4);
-  } else if (q < 2.0) {
-    double q4 = dmul(q2, q2);
-    return dadd(dsub(dadd(dsub(dmul(dmul(0.2, q4), q), dmul(1.5, q4)), dmul(dmul(4.0, q2), q)), dmul(4.0, q2)), 1.6);
-  }
-  return 0.0;
-}
-
-// the same term in FP32 (mixed form). For 1 <= q < 2 the reference's
-// polynomial vanishes at q = 2 out of terms ~30; in t = 2 - q it is exactly
+// get_kernel_grav1 (kernel_cubic.f90:78-99) dphidh term in FP32 (mixed form).
+// For 1 <= q < 2 the reference's polynomial vanishes at q = 2 out of terms ~30; in t = 2 - q it is exactly
 // t^4 (1/2 - t/5), evaluated that way.
 __device__ __forceinline__ float dphidh_f(float q2, float q) {
   if (q < 1.0f) {
@@ -63,15 +38,22 @@ __device__ __forceinline__ float dphidh_f(float q2, float q) {
   return 0.0f;
 }
 
-// FP32 B_j rho_j per tree position for the mixed MHD sums, rho_j from h_j at
-// entry of the density call (the value the divcurlB sums read)
+// B_j rho_j per tree position for the MHD sums (FP64 rows of 4, or FP32 for
+// the mixed form), rho_j from h_j at entry of the density call (the value the
+// divcurlB sums read)
 __global__ void k_dens_bprep(Params p, int n, const int *perm, const double *Bevol, const double *hj_entry,
-                             float4 *bjf) {
+                             double *bj, float4 *bjf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double rho = rhoh(hj_entry[i], p.massoftype, p.hfact);
   const double *b = Bevol + 4 * (size_t)perm[i];
-  bjf[i] = make_float4((float)(b[0] * rho), (float)(b[1] * rho), (float)(b[2] * rho), 0.0f);
+  const double bx = dmul(b[0], rho), by = dmul(b[1], rho), bz = dmul(b[2], rho);
+  if (bjf) {
+    bjf[i] = make_float4((float)bx, (float)by, (float)bz, 0.0f);
+  } else {
+    double *o = bj + 4 * (size_t)i;
+    o[0] = bx; o[1] = by; o[2] = bz;
+  }
 }
 
 // gather per-particle tree-order inputs: h, and h into the FP32 copy (its
@@ -121,7 +103,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
     Params p, const Node *nodes, const int *leaves, const int *act, int nact, const LeafEntry *pool,
     const int *cell_off, const int *cell_nleaf, const int *cell_ntrial, const int *perm, const double *tx,
     const double *ty, const double *tz, const float4 *txf, const double *hcur, const double *Bevol,
-    const double *hj_entry, const float4 *bjf, double *psum, int64_t ps, unsigned long long *stats, double pf_hmin,
+    const double *bj64, const float4 *bjf, double *psum, int64_t ps, unsigned long long *stats, double pf_hmin,
     const unsigned char *actf, int want_hash, int *err) {
   extern __shared__ __align__(16) unsigned char dsm[];
   const int w = threadIdx.x >> 5, lane = lane_id();
@@ -148,17 +130,18 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
   const float hi21f = (float)hi21;
   const bool use_pf = hi > pf_hmin;
   const float q2lim = 4.0f * 1.001f;
-  double bxi = 0, byi = 0, bzi = 0, rhoi_b = 0;
-  float bxrf = 0.0f, byrf = 0.0f, bzrf = 0.0f;  // B_i rho_i (mixed form)
+  double bxi = 0, byi = 0, bzi = 0;             // B_i rho_i
+  float bxrf = 0.0f, byrf = 0.0f, bzrf = 0.0f;  // (mixed form)
   if (MHD) {
     const double *b = Bevol + 4 * (size_t)perm[i];
-    bxi = b[0]; byi = b[1]; bzi = b[2];
-    rhoi_b = rhoh(hi, pm, p.hfact);
-    bxrf = (float)(bxi * rhoi_b); byrf = (float)(byi * rhoi_b); bzrf = (float)(bzi * rhoi_b);
+    const double rhoi_b = rhoh(hi, pm, p.hfact);
+    bxi = dmul(b[0], rhoi_b); byi = dmul(b[1], rhoi_b); bzi = dmul(b[2], rhoi_b);
+    bxrf = (float)bxi; byrf = (float)byi; bzrf = (float)bzi;
   }
-  double acc[NACC];
-  for (int k = 0; k < NACC; ++k) acc[k] = 0.0;
-  Kahan kacc[NACC];
+  constexpr int PHI = 3;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  double accb[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  Kahan kacc[MIXED ? NACC : 1];
   const float hi1f = (float)hi1, pmf = (float)pm;
   int nn = 0;
   unsigned long long hh = 0;
@@ -227,75 +210,80 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
       }
     };
     auto body = [&](int k) {
-      const int n = base + k, j = sm.st.jidx[k];
-      const int code = sm.st.code[k];
-      const double ox = offset_of(code, 0, p.dxbound), oy = offset_of(code, 1, p.dybound),
-                   oz = offset_of(code, 2, p.dzbound);
+      // FP64 pair: separation and r^2 (6 FP64 instructions), r (5), the
+      // kernel sums (7). acc[0] = sum u s, acc[1] = sum w^2, acc[2] = sum s
+      // (combined after the loop), acc[PHI] the softening sum
+      const int j = sm.st.jidx[k];
       double dx, dy, dz;
-      if (n < CELLCACHE && code != 0) {
-        dx = dsub(xi, dadd(tx[j], ox)); dy = dsub(yi, dadd(ty[j], oy)); dz = dsub(zi, dadd(tz[j], oz));
-      } else {
-        dx = dsub(xi, tx[j]); dy = dsub(yi, ty[j]); dz = dsub(zi, tz[j]);
-      }
-      dx = wrap(dx, p.dxbound, p.hdlx, p.periodic); dy = wrap(dy, p.dybound, p.hdly, p.periodic);
-      dz = wrap(dz, p.dzbound, p.hdlz, p.periodic);
-      const double rij2 = r2_exact(dx, dy, dz);
-      const double q2i = dmul(rij2, hi21);
-      if (q2i < RADKERN2) {
-        const double rij = sqrt(rij2);
-        const double qi = dmul(rij, hi1);
-        double wab, grk;
-        kern_exact(q2i, qi, wab, grk);
-        const double dwdh = dsub(-dmul(qi, grk), dmul(3.0, wab));
-        acc[0] = dadd(acc[0], dmul(wab, pm));
-        acc[1] = dadd(acc[1], dmul(dwdh, pm));
-        if (GRAV) acc[2] = dadd(acc[2], dmul(dphidh_exact(q2i, qi), pm));
+      separation_fp64(p, xi, yi, zi, base + k, j, sm.st.code[k], tx, ty, tz, dx, dy, dz);
+      const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+      const double y = rsqrt_seed(r2), t = r2 * y;
+      const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
+      const double u = fma(-fma(t, pe, t), hi1, 2.0);
+      // the reference's test where the sign of u does not decide it
+      bool in = u_inside(u);
+      if (u_near_edge(u)) in = dmul(r2_exact(dx, dy, dz), hi21) < RADKERN2;
+      if (in) {
+        const double w = kern_w(u), u2 = u * u, s = fma(-w, w, u2);
+        acc[0] = fma(u, s, acc[0]);
+        acc[1] = fma(w, w, acc[1]);
+        acc[2] += s;
+        if (GRAV) {
+          // get_kernel_grav1 (kernel_cubic.f90:78-99): u^4 (1/2 - u/5) - w^4 (1 - 2w/5) / 16
+          const double w2 = w * w;
+          acc[PHI] = fma(u2 * u2, fma(-0.2, u, 0.5), acc[PHI]);
+          acc[PHI] = fma(w2 * w2, fma(0.025, w, -0.0625), acc[PHI]);
+        }
         ++nn;
         if (want_hash) hh += mix64((unsigned long long)perm[j] + 1ull);
-        if (MHD) {  // dens.F90:745-829 (getdB)
-          const double rij1 = ddiv(1.0, dadd(rij, EPS_D));
-          const double r1g = dmul(rij1, grk);
-          const double rux = dmul(dmul(dx, r1g), pm), ruy = dmul(dmul(dy, r1g), pm), ruz = dmul(dmul(dz, r1g), pm);
-          const double rhoj = rhoh(hj_entry[j], pm, p.hfact);
-          const double *bj = Bevol + 4 * (size_t)perm[j];
-          const double dBx = dsub(dmul(bxi, rhoi_b), dmul(bj[0], rhoj));
-          const double dBy = dsub(dmul(byi, rhoi_b), dmul(bj[1], rhoj));
-          const double dBz = dsub(dmul(bzi, rhoi_b), dmul(bj[2], rhoj));
-          acc[3] = dadd(acc[3], dadd(dadd(dmul(dBx, rux), dmul(dBy, ruy)), dmul(dBz, ruz)));
-          acc[4] = dadd(acc[4], dmul(dBx, rux)); acc[5] = dadd(acc[5], dmul(dBx, ruy)); acc[6] = dadd(acc[6], dmul(dBx, ruz));
-          acc[7] = dadd(acc[7], dmul(dBy, rux)); acc[8] = dadd(acc[8], dmul(dBy, ruy)); acc[9] = dadd(acc[9], dmul(dBy, ruz));
-          acc[10] = dadd(acc[10], dmul(dBz, rux)); acc[11] = dadd(acc[11], dmul(dBz, ruy)); acc[12] = dadd(acc[12], dmul(dBz, ruz));
+        if (MHD) {  // dens.F90:745-829 (getdB): dW/dq / r = -3/4 s / r
+          const double r1g = -0.75 * s * fma(y, pe, y);
+          const double rux = dx * r1g, ruy = dy * r1g, ruz = dz * r1g;
+          const double *bj = bj64 + 4 * (size_t)j;
+          const double dBx = bxi - bj[0], dBy = byi - bj[1], dBz = bzi - bj[2];
+          accb[0] = fma(dBx, rux, fma(dBy, ruy, fma(dBz, ruz, accb[0])));
+          accb[2] = fma(dBx, ruy, accb[2]); accb[3] = fma(dBx, ruz, accb[3]);
+          accb[4] = fma(dBy, rux, accb[4]); accb[6] = fma(dBy, ruz, accb[6]);
+          accb[7] = fma(dBz, rux, accb[7]); accb[8] = fma(dBz, ruy, accb[8]);
         }
       }
     };
     if constexpr (MIXED) queue_window(cnt, S, active_lane, il, stripe, sm.q, test, [&](int k) { body_m(load(k)); });
     else queue_window(cnt, S, active_lane, il, stripe, sm.q, test, body);
   }
-  if constexpr (MIXED) {
-    for (int k = 0; k < NACC; ++k) acc[k] = kacc[k].value();
-  }
+  // sum W m, sum (-q dW/dq - 3 W) m, sum phi m, and the dB sums m (slot 3 div
+  // B, 4..12 dB_a/dx_b, whose diagonal no output reads)
+  auto lane_sum = [&](int k) -> double {
+    if constexpr (MIXED) return kacc[k].value();
+    if (k == 0) return 0.25 * pm * (acc[0] + acc[1]);
+    if (k == 1) return 0.75 * pm * (2.0 * (acc[2] - acc[0]) - acc[1]);
+    if (k == 2) return GRAV ? pm * acc[PHI] : 0.0;
+    return MHD && k != 4 && k != 8 && k != 12 ? pm * accb[k == 3 ? 0 : k - 3] : 0.0;
+  };
+  // the slots in use: the dB sums only with MHD
+  constexpr int NA = MHD ? NACC : 3;
   // combine the stripes of each particle in stripe order (the staged window
   // is no longer needed: its shared memory holds the partial sums)
   constexpr int RW = NACC + 2;
   double *red = reinterpret_cast<double *>(&sm.st);
   __syncwarp();
-  for (int k = 0; k < NACC; ++k) red[lane * RW + k] = acc[k];
+  for (int k = 0; k < NA; ++k) red[lane * RW + k] = lane_sum(k);
   red[lane * RW + DSLOT_NN] = (double)nn;
   red[lane * RW + DSLOT_HASH] = __longlong_as_double((long long)hh);
   __syncwarp();
   if (lane < np) {
-    double r[NACC];
-    for (int k = 0; k < NACC; ++k) r[k] = 0.0;
+    double r[NA];
+    for (int k = 0; k < NA; ++k) r[k] = 0.0;
     double nni = 0.0;
     unsigned long long hhi = 0;
     for (int q = 0; q < S; ++q) {
       const double *src = red + (lane * S + q) * RW;
-      for (int k = 0; k < NACC; ++k) r[k] = dadd(r[k], src[k]);
+      for (int k = 0; k < NA; ++k) r[k] = dadd(r[k], src[k]);
       nni += src[DSLOT_NN];
       hhi += (unsigned long long)__double_as_longlong(src[DSLOT_HASH]);
     }
     const size_t ip = (size_t)(s0 + cell_pos(am, lane));
-    for (int k = 0; k < NACC; ++k) psum[k * ps + ip] = r[k];
+    for (int k = 0; k < NA; ++k) psum[k * ps + ip] = r[k];
     psum[DSLOT_NN * ps + ip] = nni;
     psum[DSLOT_HASH * ps + ip] = __longlong_as_double((long long)hhi);
   }
@@ -442,26 +430,18 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_dv(
         }
         return;
       }
-      const double ox = offset_of(code, 0, p.dxbound), oy = offset_of(code, 1, p.dybound),
-                   oz = offset_of(code, 2, p.dzbound);
       double dx, dy, dz;
-      if (n < CELLCACHE && code != 0) {
-        dx = dsub(xi, dadd(tx[j], ox)); dy = dsub(yi, dadd(ty[j], oy)); dz = dsub(zi, dadd(tz[j], oz));
-      } else {
-        dx = dsub(xi, tx[j]); dy = dsub(yi, ty[j]); dz = dsub(zi, tz[j]);
-      }
-      dx = wrap(dx, p.dxbound, p.hdlx, p.periodic); dy = wrap(dy, p.dybound, p.hdly, p.periodic);
-      dz = wrap(dz, p.dzbound, p.hdlz, p.periodic);
-      const double rij2 = r2_exact(dx, dy, dz);
-      const double q2i = dmul(rij2, hi21);
-      if (q2i < RADKERN2) {
-        const double rij = sqrt(rij2);
-        const double qi = dmul(rij, hi1);
-        double wab, grk;
-        kern_exact(q2i, qi, wab, grk);
-        const double rij1 = ddiv(1.0, dadd(rij, EPS_D));
-        const double r1g = dmul(rij1, grk);
-        const double rux = dmul(dmul(dx, r1g), pm), ruy = dmul(dmul(dy, r1g), pm), ruz = dmul(dmul(dz, r1g), pm);
+      separation_fp64(p, xi, yi, zi, n, j, code, tx, ty, tz, dx, dy, dz);
+      const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+      const double y = rsqrt_seed(r2), t = r2 * y;
+      const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
+      const double u = fma(-fma(t, pe, t), hi1, 2.0);
+      bool in = u_inside(u);
+      if (u_near_edge(u)) in = dmul(r2_exact(dx, dy, dz), hi21) < RADKERN2;
+      if (in) {
+        const double w = kern_w(u), s = fma(-w, w, u * u);
+        const double r1g = -0.75 * pm * s * fma(y, pe, y);
+        const double rux = dx * r1g, ruy = dy * r1g, ruz = dz * r1g;
         const double *vj = vf + 6 * (size_t)j;
         const double dvx = dsub(vfi[0], vj[0]), dvy = dsub(vfi[1], vj[1]), dvz = dsub(vfi[2], vj[2]);
         acc[0] = dadd(acc[0], dadd(dadd(dmul(dvx, rux), dmul(dvy, ruy)), dmul(dvz, ruz)));
@@ -744,8 +724,10 @@ int density(ph_ctx *c, int icall) {
   // the Bevol of the evaluation (Bpred in a step: derivs passes its Bevol
   // argument on to densityiterate, deriv.f90:135)
   const double *Bd = c->dens_B ? c->dens_B : c->Bevol;
-  if (p.mhd && p.precision == PH_PREC_MIXED) {
-    k_dens_bprep<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, Bd, hj_entry, c->bjf);
+  const bool dB = p.mhd;
+  if (dB) {
+    k_dens_bprep<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, Bd, hj_entry, c->jrec,
+                                                p.precision == PH_PREC_MIXED ? c->bjf : nullptr);
     count_launch(c, 1);
   }
   int nact = ncell;
@@ -805,13 +787,13 @@ int density(ph_ctx *c, int icall) {
 #define PH_DENS(X, M, G)                                                                                         \
   k_density_pairs<X, M, G><<<nblk(nact, dw), 32 * dw, smem, st>>>(                                    \
       p, c->nodes, c->leaves, act, nact, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->perm, c->tx, c->ty,  \
-      c->tz, c->txf, c->hcur, Bd, hj_entry, c->bjf, c->psum, c->cap, c->stats, pf_hmin, actf,             \
+      c->tz, c->txf, c->hcur, Bd, c->jrec, c->bjf, c->psum, c->cap, c->stats, pf_hmin, actf,             \
       c->want_diag ? 1 : 0, c->d_err)
     if (p.precision == PH_PREC_MIXED) {
-      if (p.mhd) { if (p.gravity) PH_DENS(true, true, true); else PH_DENS(true, true, false); }
+      if (dB) { if (p.gravity) PH_DENS(true, true, true); else PH_DENS(true, true, false); }
       else { if (p.gravity) PH_DENS(true, false, true); else PH_DENS(true, false, false); }
     } else {
-      if (p.mhd) { if (p.gravity) PH_DENS(false, true, true); else PH_DENS(false, true, false); }
+      if (dB) { if (p.gravity) PH_DENS(false, true, true); else PH_DENS(false, true, false); }
       else { if (p.gravity) PH_DENS(false, false, true); else PH_DENS(false, false, false); }
     }
 #undef PH_DENS

@@ -128,6 +128,28 @@ __device__ __forceinline__ void separation_mixed(const Params &p, double xi, dou
   }
 }
 
+// ------------------------------------------------------------------ FP64 separation
+// Pair separation with the reference's rounding: cached positions x_j + offset
+// for the first 1000 trial entries (dens.F90:660-669, force.F90:1258-1269),
+// else x_i - x_j and the wrap into the half box. Inside the box (nearly every
+// pair) that is three FP64 subtractions: the wrap test compares bit patterns,
+// and the offset and shift adds sit in branches of their own, since an FP64
+// instruction holds the pipe for a whole warp when one lane needs it.
+__device__ __forceinline__ void separation_fp64(const Params &p, double xi, double yi, double zi, int n, int j,
+                                                int code, const double *tx, const double *ty, const double *tz,
+                                                double &dx, double &dy, double &dz) {
+  double xj = tx[j], yj = ty[j], zj = tz[j];
+  if (code != 0 && n < CELLCACHE) {
+    xj = dadd(xj, offset_of(code, 0, p.dxbound)); yj = dadd(yj, offset_of(code, 1, p.dybound));
+    zj = dadd(zj, offset_of(code, 2, p.dzbound));
+  }
+  dx = dsub(xi, xj); dy = dsub(yi, yj); dz = dsub(zi, zj);
+  if (p.periodic && (abs_gt(dx, p.hdlx) || abs_gt(dy, p.hdly) || abs_gt(dz, p.hdlz))) {
+    dx = wrap(dx, p.dxbound, p.hdlx, true); dy = wrap(dy, p.dybound, p.hdly, true);
+    dz = wrap(dz, p.dzbound, p.hdlz, true);
+  }
+}
+
 // ------------------------------------------------------------------ active particles of a cell
 // With individual timesteps a cell's pair loops run over its active
 // particles only (dens.F90:1293-1378, force.F90 start_cell skip inactive
