@@ -724,7 +724,10 @@ int density(ph_ctx *c, int icall) {
   // the Bevol of the evaluation (Bpred in a step: derivs passes its Bevol
   // argument on to densityiterate, deriv.f90:135)
   const double *Bd = c->dens_B ? c->dens_B : c->Bevol;
-  const bool dB = p.mhd;
+  // the div B and curl B sums feed divcurlB only, which only a ph_density call
+  // returns (ideal MHD forces do not read it): the evaluations of derivs and
+  // the step take the density sums alone
+  const bool dB = p.mhd && c->want_diag;
   if (dB) {
     k_dens_bprep<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, Bd, hj_entry, c->jrec,
                                                 p.precision == PH_PREC_MIXED ? c->bjf : nullptr);
