@@ -22,46 +22,31 @@ namespace ph {
 
 constexpr int JREC = 16;   // doubles per particle, hydro record
 constexpr int JMHD = 16;   // doubles per particle, MHD record
+// The FP64 pair terms' record: every factor of a pair term that belongs to one
+// particle is formed once in the prologue (the particle mass is applied to
+// the finished sums). JR_K = -3/4 cnormk h^-4 / Omega (on s of kern_w, giving
+// grad W), JR_C = -1/(2 rho) of the viscosity, JR_AVW = alpha v_wave,
+// JR_AU = alpha_u / (2 rho) (with the sqrt(2) of the conductivity's signal
+// speed, force.F90:1605-1621), JR_AB = alpha_B / (2 rho^2)
+enum { JR_H1 = 0, JR_RHO, JR_C, JR_PRO2, JR_VW, JR_P, JR_AU, JR_K, JR_VX, JR_VY, JR_VZ, JR_U, JR_GS, JR_AB, JR_AVW,
+       JR_R21 };
+// MHD: B, psi, overcleanfac psi v_wave; B/rho in the finish's slots 10..12
+enum { JM_BX = 0, JM_BY, JM_BZ, JM_PSI, JM_CL };
 constexpr int NF = 12;     // fsum entries
 constexpr int JRECF = 16, JMHDF = 16;  // floats per particle, FP32 copies of the records (mixed form)
 
-// M4 dW/dq (kernel_cubic.f90:56-66)
-__device__ __forceinline__ double grkern(double q) {
-  if (q < 1.0) return q * (2.25 * q - 3.0);
-  if (q < 2.0) { double t = q - 2.0; return -0.75 * (t * t); }
-  return 0.0;
-}
-// kernel_softening (kernel_cubic.f90:101-120)
-__device__ __forceinline__ void kernel_softening(double q2, double q, double &pot, double &fs) {
-  if (q < 1.0) {
-    double q4 = q2 * q2;
-    pot = q4 * q / 10.0 - 3.0 * q4 / 10.0 + 2.0 * q2 / 3.0 - 7.0 / 5.0;
-    fs = q * (15.0 * q2 * q - 36.0 * q2 + 40.0) / 30.0;
-  } else if (q < 2.0) {
-    double q4 = q2 * q2, q6 = q4 * q2;
-    pot = (q * (-q4 * q + 9.0 * q4 - 30.0 * q2 * q + 40.0 * q2 - 48.0) + 2.0) / (30.0 * q);
-    fs = (-5.0 * q6 + 36.0 * q4 * q - 90.0 * q4 + 80.0 * q2 * q - 2.0) / (30.0 * q2);
-  } else {
-    pot = -1.0 / q;
-    fs = 1.0 / q2;
-  }
-}
-
-// get_stress (force.F90:2068-2168) without physical viscosity / radiation
+// get_stress (force.F90:2068-2168) without physical viscosity / radiation: P/rho^2
+// with the magnetic pressure and the wave speed (the pair terms form the
+// anisotropic stress -(B/rho)(B/rho).n from the Lorentz projections)
 __device__ __forceinline__ void get_stress(const Params &p, double pri, double cs, double rhoi, double rho1i,
-                                           double bx, double by, double bz, double &pro2, double &vwave,
-                                           double *s) {
-  const double pm = p.massoftype;
+                                           double bx, double by, double bz, double &pro2, double &vwave) {
   if (p.mhd) {
     double brx = bx * rho1i, bry = by * rho1i, brz = bz * rho1i;
     double bro2 = brx * brx + bry * bry + brz * brz;
     double va2 = bro2 * rhoi;
     vwave = sqrt(cs * cs + va2);
-    s[0] = -pm * brx * brx; s[1] = -pm * brx * bry; s[2] = -pm * brx * brz;
-    s[3] = -pm * bry * bry; s[4] = -pm * bry * brz; s[5] = -pm * brz * brz;
     pro2 = pri * rho1i * rho1i + 0.5 * bro2;
   } else {
-    for (int k = 0; k < 6; ++k) s[k] = 0.0;
     pro2 = pri * rho1i * rho1i;
     vwave = cs;
   }
@@ -156,11 +141,10 @@ __global__ void k_force_prologue_mixed(Params p, int n, const int *perm, const d
   txf[j].w = h1;
 }
 
-__global__ void k_force_prologue(Params p, int n, const int *perm, const double *tx, const double *ty,
-                                 const double *tz, const double *th, const double *vel, const double *Bv,
-                                 const float *gradh, double *eos_t, double *jrec, double *jmhd, float *jrecf,
-                                 float *jmhdf, float4 *txf, const float *alpha1, const float *ddivvdt_c,
-                                 const float *dvdx_c, float *alphaloc_t, int *err) {
+__global__ void k_force_prologue(Params p, int n, const int *perm, const double *th, const double *vel,
+                                 const double *Bv, const float *gradh, double *eos_t, double *jrec, double *jmhd,
+                                 float4 *txf, const float *alpha1, const float *ddivvdt_c, const float *dvdx_c,
+                                 float *alphaloc_t, int *err) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const double pm = p.massoftype;
@@ -184,47 +168,39 @@ __global__ void k_force_prologue(Params p, int n, const int *perm, const double 
     const double xi = xi_limiter(dvdx_c + 9 * (size_t)pid);
     alphaloc_t[j] = (float)get_alphaloc((double)ddivvdt_c[pid], cs, h, xi, p.alpha, p.alphamax);
   }
-  // j-side of compute_forces (force.F90:1428-1511)
-  const double hj1 = 1.0 / h;
-  const double hj = 1.0 / hj1;
-  const double rhoj = rhoh(hj, pm, p.hfact);
-  const double rho1j = 1.0 / rhoj;
+  // start_cell and the j-side of compute_forces (force.F90:1428-1511, 2270-2340)
+  const double h1 = 1.0 / h;
+  const double rho1 = 1.0 / rho_c;
   double bx = 0, by = 0, bz = 0;
   if (p.mhd) {
     const double *b = Bv + 4 * (size_t)pid;
     bx = b[0] * rho_c; by = b[1] * rho_c; bz = b[2] * rho_c;
   }
-  double pro2, vwave, s[6];
-  get_stress(p, P, cs, rhoj, rho1j, bx, by, bz, pro2, vwave, s);
-  const double mrhoj5 = 0.5 * pm * rho1j;
+  double pro2, vwave;
+  get_stress(p, P, cs, rho_c, rho1, bx, by, bz, pro2, vwave);
   double *r = jrec + JREC * (size_t)j;
-  r[0] = hj1; r[1] = rhoj; r[2] = rho1j; r[3] = pro2; r[4] = vwave; r[5] = P;
-  r[6] = mrhoj5 * p.alphau;
   // gradh in tree order; with individual timesteps in caller order, where
   // inactive particles keep the values of their last density solve
   const size_t g = p.ind ? (size_t)pid : (size_t)j;
-  r[7] = (double)gradh[2 * g];
-  r[8] = v[0]; r[9] = v[1]; r[10] = v[2]; r[11] = p.isothermal ? 0.0 : v[3];
-  r[12] = (double)gradh[2 * g + 1];
-  r[13] = mrhoj5 * p.alphaB * rho1j;
-  r[14] = p.nalpha > 0 ? (double)alpha1[pid] : p.alpha;  // alphaind(1,j) (force.F90:1478, 2430-2433)
-  r[15] = rho1j * rho1j;
+  const double h21 = h1 * h1;
+  r[JR_H1] = h1; r[JR_RHO] = rho_c; r[JR_C] = -0.5 * rho1; r[JR_PRO2] = pro2;
+  r[JR_VW] = vwave; r[JR_P] = P;
+  r[JR_AU] = 0.5 * rho1 * p.alphau * (p.gravity ? 1.0 : 1.4142135623730951);
+  r[JR_K] = -0.75 * CNORMK * (h21 * h21) * (double)gradh[2 * g];
+  r[JR_VX] = v[0]; r[JR_VY] = v[1]; r[JR_VZ] = v[2]; r[JR_U] = p.isothermal ? 0.0 : v[3];
+  r[JR_GS] = (double)gradh[2 * g + 1];
+  r[JR_AB] = 0.5 * p.alphaB * rho1 * rho1;
+  // alphaind(1,j) (force.F90:1478, 2430-2433)
+  r[JR_AVW] = (p.nalpha > 0 ? (double)alpha1[pid] : p.alpha) * vwave;
+  r[JR_R21] = rho1 * rho1;
   if (p.mhd) {
     double *m = jmhd + JMHD * (size_t)j;
-    m[0] = bx; m[1] = by; m[2] = bz; m[3] = Bv[4 * (size_t)pid + 3];
-    for (int k = 0; k < 6; ++k) m[4 + k] = s[k];
-    m[10] = Bv[4 * (size_t)pid]; m[11] = Bv[4 * (size_t)pid + 1]; m[12] = Bv[4 * (size_t)pid + 2];
+    const double *b = Bv + 4 * (size_t)pid;
+    m[JM_BX] = bx; m[JM_BY] = by; m[JM_BZ] = bz; m[JM_PSI] = b[3];
+    m[JM_CL] = p.overcleanfac * b[3] * vwave;
+    m[10] = b[0]; m[11] = b[1]; m[12] = b[2];
   }
-  if (jrecf) {  // FP32 copies for the mixed form (rounded on the integer pipe)
-    float *o = jrecf + JRECF * (size_t)j;
-    for (int k = 0; k < JREC; ++k) o[k] = d2f_rn(r[k]);
-    if (p.mhd) {
-      const double *m = jmhd + JMHD * (size_t)j;
-      float *q = jmhdf + JMHDF * (size_t)j;
-      for (int k = 0; k < 13; ++k) q[k] = d2f_rn(m[k]);
-    }
-  }
-  txf[j].w = (float)(1.0 / h);  // x, y, z: set by the tree build
+  txf[j].w = (float)h1;  // x, y, z: set by the tree build
 }
 
 struct ForceOut {
@@ -407,8 +383,8 @@ __global__ void __launch_bounds__(256) k_force_finish(Params p, int nt, const do
       const double *m = jmhd + JMHD * (size_t)ip;
       bx = m[10] * rho; by = m[11] * rho; bz = m[12] * rho;
       psi = m[3];
-      double pro2, s[6];
-      get_stress(p, pr, cs, rho, rho1, bx, by, bz, pro2, vwave, s);
+      double pro2;
+      get_stress(p, pr, cs, rho, rho1, bx, by, bz, pro2, vwave);
       b2 = bx * bx + by * by + bz * bz;
       const double divBsymmi = fs[7];
       double frac = 0.0;
@@ -502,9 +478,11 @@ __global__ void k_wake_apply(int nt, const int *perm, const unsigned char *wakem
 
 // the stripes of each particle summed in stripe order through shared memory
 // (the staged window's memory, no longer needed), written to psum by lanes < np
-template <bool IND, class Get>
+// (pm: the particle mass the FP64 loops leave out of their pair terms, applied
+// to every sum but d(rho)/dt's, which the finish multiplies; 1 for the mixed form)
+template <bool IND, bool SCALE, class Get>
 __device__ __forceinline__ void store_pair_sums(PairSmem &sm, int lane, int np, int S, int s0, unsigned am,
-                                                double *psum, int64_t ps, Get get) {
+                                                double *psum, int64_t ps, double pm, Get get) {
   constexpr int RW = IND ? NF + 2 : NF + 1;
   double *red = reinterpret_cast<double *>(&sm.st);
   __syncwarp();
@@ -521,7 +499,7 @@ __device__ __forceinline__ void store_pair_sums(PairSmem &sm, int lane, int np, 
       if (IND) nb = fmax(nb, src[NF + 1]);
     }
     const size_t ip = (size_t)(s0 + (IND ? cell_pos(am, lane) : lane));
-    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = fs[k];
+    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = SCALE && k != 4 ? pm * fs[k] : fs[k];
     psum[FSLOT_VSIG * ps + ip] = vsm;
     if (IND) psum[FSLOT_NBIN * ps + ip] = nb;
   }
@@ -534,55 +512,57 @@ __device__ __forceinline__ double fmax_pos(double a, double b) {
 }
 
 // ------------------------------------------------------------------ FP64 pair terms
-// The i-side quantities of the FP64 pair loop (start_cell force.F90:2270-2340
-// and compute_cell :2606-2629) for tree position i.
+// The FP64 pair loops are bound by the FP64 pipe (2 lanes per SM and clock), so
+// their cost is the number of FP64 instructions per pair. Each particle's own
+// factors come from its record, no division or library square root is left
+// (rsqrt_fast), the kernel needs no branch on q (kern_w), comparisons and
+// maxima run on the integer pipe, and the particle mass is applied to the sums.
+// i-side quantities (start_cell force.F90:2270-2340, compute_cell :2606-2629)
+// of tree position i.
 struct IFp64 {
-  double hi, hi1, hi21, rhoi, rho1i, rho21i, pri, csi;
-  double bxi, byi, bzi, psii, vxi, vyi, vzi, eni;
-  double sxx, sxy, sxz, syy, syz, szz, pro2i, vwavei;
-  double gradsofti, hfacgrkern, mrhoi5, auterm, avBterm, alphai;
-  double xi, yi, zi;
+  double h1, rho, c, pro2, vw, P, au, K, vx, vy, vz, u, gs, ab, avw, r21;
+  double bx, by, bz, cl;
+  double x, y, z;
 };
 
 template <bool MHD, bool GRAV>
 __device__ __forceinline__ IFp64 ifp64_init(const Params &p, int i, const double *tx, const double *ty,
-                                            const double *tz, const double *th, const double *jrec,
-                                            const double *jmhd, const double *eos_t) {
+                                            const double *tz, const double *jrec, const double *jmhd) {
   IFp64 I;
-  const double pm = p.massoftype;
-  I.hi = th[i];
-  I.hi1 = 1.0 / fabs(I.hi);
-  const double t3 = p.hfact * I.hi1;
-  I.rhoi = pm * (t3 * t3 * t3);
-  I.rho1i = 1.0 / I.rhoi;
-  const double *ri = jrec + JREC * (size_t)i;
-  I.pri = eos_t[2 * (size_t)i]; I.csi = eos_t[2 * (size_t)i + 1];
-  I.bxi = 0; I.byi = 0; I.bzi = 0; I.psii = 0;
+  const double *r = jrec + JREC * (size_t)i;
+  I.h1 = fabs(r[JR_H1]); I.rho = r[JR_RHO]; I.c = r[JR_C]; I.pro2 = r[JR_PRO2]; I.vw = r[JR_VW]; I.P = r[JR_P];
+  I.au = r[JR_AU]; I.K = r[JR_K]; I.vx = r[JR_VX]; I.vy = r[JR_VY]; I.vz = r[JR_VZ]; I.u = r[JR_U];
+  I.gs = GRAV ? r[JR_GS] : 0.0;
+  I.ab = r[JR_AB]; I.avw = r[JR_AVW]; I.r21 = r[JR_R21];
+  // start_cell takes 1/Omega = 1 where the stored value is not positive
+  if (!(I.K < 0.0)) { const double h21 = I.h1 * I.h1; I.K = -0.75 * CNORMK * (h21 * h21); }
+  I.bx = I.by = I.bz = I.cl = 0.0;
   if (MHD) {
-    // B_i = Bevol_i * rho_i with rho_i from rhoanddhdrho (force.F90:2309-2311)
     const double *m = jmhd + JMHD * (size_t)i;
-    I.bxi = m[10] * I.rhoi; I.byi = m[11] * I.rhoi; I.bzi = m[12] * I.rhoi;
-    I.psii = m[3];
+    I.bx = m[JM_BX]; I.by = m[JM_BY]; I.bz = m[JM_BZ]; I.cl = m[JM_CL];
   }
-  I.vxi = ri[8]; I.vyi = ri[9]; I.vzi = ri[10]; I.eni = ri[11];
-  {
-    double s[6];
-    get_stress(p, I.pri, I.csi, I.rhoi, I.rho1i, I.bxi, I.byi, I.bzi, I.pro2i, I.vwavei, s);
-    I.sxx = s[0]; I.sxy = s[1]; I.sxz = s[2]; I.syy = s[3]; I.syz = s[4]; I.szz = s[5];
-  }
-  const double gradhraw = ri[7];
-  const double gradhi = (gradhraw > 0.0) ? gradhraw : 1.0;
-  I.gradsofti = GRAV ? ri[12] : 0.0;
-  I.hi21 = I.hi1 * I.hi1;
-  const double hi41 = I.hi21 * I.hi21;
-  I.hfacgrkern = hi41 * CNORMK * gradhi;
-  I.rho21i = I.rho1i * I.rho1i;
-  I.mrhoi5 = 0.5 * pm * I.rho1i;
-  I.auterm = I.mrhoi5 * p.alphau;
-  I.avBterm = I.mrhoi5 * p.alphaB * I.rho1i;
-  I.alphai = jrec[JREC * (size_t)i + 14];
-  I.xi = tx[i]; I.yi = ty[i]; I.zi = tz[i];
+  I.x = tx[i]; I.y = ty[i]; I.z = tz[i];
   return I;
+}
+
+// largest of two signal speeds as bit patterns (the first non-negative; a
+// negative second one, whose clamp to zero changes no maximum, orders below)
+__device__ __forceinline__ long long vmax_bits(long long a, double b) { return max(a, __double_as_longlong(b)); }
+
+// softened self-gravity of one side (kernel_softening, kernel_cubic.f90:
+// 101-120), u = 2 - q inside the kernel: fs/h^2 and, with POT, pot/h. For
+// q >= 1 the reference's polynomials are expanded about q = 2,
+//   q^2 fs = 1 - u^4 (1 - 4/5 u + u^2/6),  q pot = -1 + u^5 (1/10 - u/30).
+template <bool POT>
+__device__ __forceinline__ double softened(double u, double r, double y, double h1, double &pot) {
+  if (__double2hiint(u) >= 0x3ff00000) {  // u >= 1: q <= 1
+    const double q = r * h1, q2 = q * q;
+    if (POT) pot = h1 * fma(q2, fma(q2, fma(0.1, q, -0.3), 2.0 / 3.0), -1.4);
+    return h1 * h1 * q * fma(q2, fma(0.5, q, -1.2), 4.0 / 3.0);
+  }
+  const double u2 = u * u, u4 = u2 * u2;
+  if (POT) pot = y * fma(u4 * u, fma(-1.0 / 30.0, u, 0.1), -1.0);
+  return y * y * fma(-u4, fma(u, fma(1.0 / 6.0, u, -0.8), 1.0), 1.0);
 }
 
 // j-side pair sums of the symmetric evaluation: the force components, d(rho)/dt
@@ -597,178 +577,167 @@ __device__ __forceinline__ int njs_slot(int v, bool mhd) {
   return v < 3 ? v : v + 1;  // 0,1,2 -> 0,1,2; 3.. -> 4..
 }
 
+// The plain 1/r^2 of a trial pair outside both kernels (force.F90:1991-2053).
+__device__ __forceinline__ void far_pair_fp64(double dx, double dy, double dz, double y, double (&f)[NF]) {
+  const double y3 = y * y * y;
+  f[0] = fma(-dx, y3, f[0]); f[1] = fma(-dy, y3, f[1]); f[2] = fma(-dz, y3, f[2]);
+  f[3] -= y;
+}
+
 // One trial pair (i, j) of compute_forces (force.F90:914-2060) in FP64 with the
 // reference's neighbour test and cached-position rule; n is j's position in
-// i's trial list. The i-side sums go to f / vsigmax / nbi. With SYM the pair's
-// contribution to j's own sums (j's force loop over i, the same pair term seen
-// from j) is returned in jv; it is only requested for pairs without gravity
-// and with global timesteps.
+// i's trial list. The i-side sums (without the particle mass) go to f,
+// vsigmax / nbi. With SYM the pair's contribution to j's own sums (j's force
+// loop over i, the same pair term seen from j) is returned in jv; it is only
+// requested for pairs without gravity and with global timesteps.
 template <bool MHD, bool GRAV, bool IND, bool SYM>
 __device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I, int n, int j, int code,
                                                 const double *tx, const double *ty, const double *tz,
                                                 const double *jrec, const double *jmhd,
                                                 const int8_t *ibin_old_t, unsigned char *wakemark,
-                                                double (&f)[NF], double &vsigmax, int &nbi,
+                                                double (&f)[NF], long long &vsigmax, int &nbi,
                                                 double (&jv)[NJS<MHD>::n]) {
-  const double pm = p.massoftype;
   const bool adiab = !p.isothermal;
-  const double beta = p.beta;
-  const double ox = offset_of(code, 0, p.dxbound), oy = offset_of(code, 1, p.dybound),
-               oz = offset_of(code, 2, p.dzbound);
   double dx, dy, dz;
-  if (n < CELLCACHE && code != 0) {
-    dx = dsub(I.xi, dadd(tx[j], ox)); dy = dsub(I.yi, dadd(ty[j], oy)); dz = dsub(I.zi, dadd(tz[j], oz));
-  } else {
-    dx = dsub(I.xi, tx[j]); dy = dsub(I.yi, ty[j]); dz = dsub(I.zi, tz[j]);
-  }
-  dx = wrap(dx, p.dxbound, p.hdlx, p.periodic); dy = wrap(dy, p.dybound, p.hdly, p.periodic);
-      dz = wrap(dz, p.dzbound, p.hdlz, p.periodic);
-  const double rij2 = r2_exact(dx, dy, dz);
+  separation_fp64(p, I.x, I.y, I.z, n, j, code, tx, ty, tz, dx, dy, dz);
   const double *rj = jrec + JREC * (size_t)j;
-  const double hj1 = rj[0];
-  const double q2i = dmul(rij2, I.hi21);
-  const double hj21 = dmul(hj1, hj1);
-  const double q2j = dmul(rij2, hj21);
-  const bool qi_in = q2i < RADKERN2, qj_in = q2j < RADKERN2;
-  if (qi_in || qj_in) {
-    if (IND) {  // force.F90:1346-1353: j is woken for the next step; the limiter's neighbour bin
-      wakemark[j] = 1;
-      nbi = max(nbi, (int)ibin_old_t[j]);
+  const double hj1 = rj[JR_H1];
+  // With self-gravity the direction of a neighbour pair keeps the reference's
+  // rounding (r^2 without contraction, the library's rsqrt): in solid-body
+  // rotation, where such clouds start, dv . n is zero but for rounding, and
+  // its sign switches the viscosity. The neighbours are a few per cent of the
+  // trial list there, the other pairs are far_pair_fp64's.
+  double r2, y;
+  if (GRAV) {
+    r2 = r2_exact(dx, dy, dz);
+    y = r2 > TINY_D ? rsqrt(r2) : 0.0;
+  } else {
+    r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+    y = rsqrt_fast(r2);
+  }
+  const double r = r2 * y;
+  double ui = fma(-r, I.h1, 2.0), uj = fma(-r, hj1, 2.0);
+  bool qi_in = u_inside(ui), qj_in = u_inside(uj);
+  if (u_near_edge(ui) || u_near_edge(uj)) {  // the reference's q^2 < 4
+    const double rij2 = r2_exact(dx, dy, dz);
+    qi_in = dmul(rij2, dmul(I.h1, I.h1)) < RADKERN2;
+    qj_in = dmul(rij2, dmul(hj1, hj1)) < RADKERN2;
+  }
+  if (!(qi_in || qj_in)) {
+    if (GRAV) far_pair_fp64(dx, dy, dz, y, f);
+    if (SYM) for (int v = 0; v < NJS<MHD>::n; ++v) jv[v] = 0.0;
+    return;
+  }
+  if (IND) {  // force.F90:1346-1353: j is woken for the next step; the limiter's neighbour bin
+    wakemark[j] = 1;
+    nbi = max(nbi, (int)ibin_old_t[j]);
+  }
+  ui = qi_in ? ui : 0.0; uj = qj_in ? uj : 0.0;
+  const double wi = kern_w(ui), wj = kern_w(uj);
+  const double gi = I.K * fma(-wi, wi, ui * ui), gj = rj[JR_K] * fma(-wj, wj, uj * uj);
+  double fgrav = 0.0;
+  if (GRAV) {
+    const double y2 = y * y;
+    double phii = -y, none, fgi = y2, fgj = y2;
+    if (qi_in) fgi = fma(I.gs, gi, softened<true>(ui, r, y, I.h1, phii));
+    if (qj_in) fgj = fma(rj[JR_GS], gj, softened<false>(uj, r, y, hj1, none));
+    fgrav = fgi + fgj;
+    f[3] += phii;
+  }
+  // j's terms enter i's sums when q_j < 2, or always with MHD or an energy
+  // equation (force.F90 usej); seen from j likewise
+  const bool both = MHD || (adiab && !GRAV);
+  const bool usej = both || qj_in, usei = both || qi_in;
+  const double dvx = I.vx - rj[JR_VX], dvy = I.vy - rj[JR_VY], dvz = I.vz - rj[JR_VZ];
+  double pv;  // dv . n
+  if (GRAV) {
+    const double nx = dx * y, ny = dy * y, nz = dz * y;
+    pv = dvx * nx + dvy * ny + dvz * nz;
+  } else {
+    pv = y * fma(dvz, dz, fma(dvy, dy, dvx * dx));
+  }
+  const double vwj = rj[JR_VW];
+  const double vsi = fma(-p.beta, pv, I.vw), vsj = fma(-p.beta, pv, vwj);
+  vsigmax = vmax_bits(vsigmax, vsi);
+  if (usej) vsigmax = vmax_bits(vsigmax, vsj);
+  const double pgi = pv * gi;
+  f[4] += pgi;
+  double qi = 0.0, qj = 0.0;
+  if (__double2hiint(pv) < 0) {  // approaching: artificial viscosity
+    double vai = fma(-p.beta, pv, I.avw), vaj = fma(-p.beta, pv, rj[JR_AVW]);
+    vai = __double2hiint(vai) < 0 ? 0.0 : vai; vaj = __double2hiint(vaj) < 0 ? 0.0 : vaj;
+    qi = I.c * pv * vai;
+    qj = rj[JR_C] * pv * vaj;
+    if (adiab) f[5] = fma(qi, pgi, f[5]);
+  }
+  double gp = fma(rj[JR_PRO2] + qj, gj, (I.pro2 + qi) * gi);
+  if (GRAV) gp = fma(0.5, fgrav, gp);
+  double dendiss = 0.0;
+  if (adiab && p.alphau != 0.0) {
+    // conductivity: |dv . n| with self-gravity, else sqrt(2 |dP| / (rho_i + rho_j))
+    // as sqrt(2) |dP| (|dP| (rho_i + rho_j))^(-1/2)
+    double vsu;
+    if (GRAV) vsu = fabs(pv);
+    else { const double dP = fabs(I.P - rj[JR_P]); vsu = dP * rsqrt_fast(dP * (I.rho + rj[JR_RHO])); }
+    dendiss = vsu * (I.u - rj[JR_U]) * fma(I.au, gi, rj[JR_AU] * gj);
+    f[6] += dendiss;
+  }
+  if (SYM) {
+    jv[3] = pv * gj;
+    jv[4] = adiab ? qj * jv[3] : 0.0;
+    jv[5] = -dendiss;
+    long long b = vmax_bits(0, vsj);
+    if (usei) b = vmax_bits(b, vsi);
+    jv[NJS<MHD>::n - 1] = __longlong_as_double(b);
+  }
+  if constexpr (!MHD) {
+    const double gpy = gp * y;
+    f[0] = fma(-dx, gpy, f[0]); f[1] = fma(-dy, gpy, f[1]); f[2] = fma(-dz, gpy, f[2]);
+    if (SYM) { jv[0] = dx * gpy; jv[1] = dy * gpy; jv[2] = dz * gpy; }
+  } else {
+    const double nx = dx * y, ny = dy * y, nz = dz * y;
+    const double *mj = jmhd + JMHD * (size_t)j;
+    const double bxj = mj[JM_BX], byj = mj[JM_BY], bzj = mj[JM_BZ];
+    const double dBx = I.bx - bxj, dBy = I.by - byj, dBz = I.bz - bzj;
+    const double projBj = fma(bzj, nz, fma(byj, ny, bxj * nx));
+    const double projdB = fma(dBz, nz, fma(dBy, ny, dBx * nx));
+    const double projBi = projBj + projdB;
+    f[11] = fma(-projdB, gi, f[11]);  // div B diffusion
+    const double tx_ = fma(-pv, nx, dvx), ty_ = fma(-pv, ny, dvy), tz_ = fma(-pv, nz, dvz);
+    const double vsigB = sqrt_fast(fma(tz_, tz_, fma(ty_, ty_, tx_ * tx_)));
+    const double dBdiss = vsigB * fma(I.ab, gi, rj[JR_AB] * gj);
+    const double pmi = I.r21 * gi, pmj = rj[JR_R21] * gj;
+    const double ti = pmi * projBi, tj = pmj * projBj;
+    const double f7 = ti + tj;
+    f[7] += f7;  // div B (symmetric)
+    const double dpsi = fma(pmi, I.cl, pmj * mj[JM_CL]);
+    f[8] = fma(-ti, dvx, fma(dBdiss, dBx, fma(-dpsi, nx, f[8])));
+    f[9] = fma(-ti, dvy, fma(dBdiss, dBy, fma(-dpsi, ny, f[9])));
+    f[10] = fma(-ti, dvz, fma(dBdiss, dBz, fma(-dpsi, nz, f[10])));
+    double res = 0.0;
+    if (p.iresistive_heating > 0 && adiab) {
+      res = -0.5 * fma(dBz, dBz, fma(dBy, dBy, dBx * dBx)) * dBdiss;
+      f[5] += res;
     }
-    double rij1, qi;
-    if (rij2 > TINY_D) { rij1 = rsqrt(rij2); qi = (rij2 * rij1) * I.hi1; }
-    else { rij1 = 0.0; qi = 0.0; }
-    double grkerni = 0.0, fgravi = 0.0, phii = 0.0;
-    if (qi_in) {
-      grkerni = grkern(qi) * I.hfacgrkern;
-      if (GRAV) {
-        double fmi;
-        kernel_softening(q2i, qi, phii, fmi);
-        phii = phii * I.hi1;
-        fmi = fmi * I.hi21;
-        fgravi = fmi + I.gradsofti * grkerni;
-      }
-    } else if (GRAV) {
-      phii = -rij1; fgravi = rij1 * rij1;
-    }
-    const double runix = dx * rij1, runiy = dy * rij1, runiz = dz * rij1;
-    double grkernj = 0.0, fgravj = 0.0;
-    bool usej;
-    if (qj_in) {
-      const double qj = (rij2 * rij1) * hj1;
-      grkernj = grkern(qj) * hj21 * hj21 * CNORMK * rj[7];
-      if (GRAV) {
-        double phij, fmj;
-        kernel_softening(q2j, qj, phij, fmj);
-        fgravj = fmj * hj21 + rj[12] * grkernj;
-      }
-      usej = true;
-    } else {
-      if (GRAV) fgravj = rij1 * rij1;
-      usej = false;
-    }
-    if (MHD) usej = true;
-    if (adiab && !GRAV) usej = true;
-    // seen from j, i's terms are used when q_i < 2 (or always, as usej)
-    const bool usei = qi_in || MHD || (adiab && !GRAV);
-    const double fgrav = GRAV ? 0.5 * (pm * fgravi + pm * fgravj) : 0.0;
-    const double dvx = I.vxi - rj[8], dvy = I.vyi - rj[9], dvz = I.vzi - rj[10];
-    const double projv = dvx * runix + dvy * runiy + dvz * runiz;
-    const double denij = adiab ? I.eni - rj[11] : 0.0;
-    const double vsigi = fmax(I.vwavei - beta * projv, 0.0);
-    const double vsigavi = fmax(I.alphai * I.vwavei - beta * projv, 0.0);
-    vsigmax = fmax_pos(vsigmax, vsigi);
-    double rho1j = 0, rho21j = 0, pro2j = 0, vwavej = 0, autermj = 0, avBtermj = 0, vsigavj = 0, prj = 0;
-    double vsigj = 0.0;
-    double rhoj = rj[1];
-    if (usej || SYM) {
-      rho1j = rj[2]; rho21j = rj[15]; pro2j = rj[3]; vwavej = rj[4]; prj = rj[5];
-      autermj = rj[6]; avBtermj = rj[13];
-      vsigj = fmax(vwavej - beta * projv, 0.0);
-      vsigavj = fmax(rj[14] * vwavej - beta * projv, 0.0);  // alphaj = alphaind(1,j)
-      if (usej) vsigmax = fmax_pos(vsigmax, vsigj);
-    }
-    double qrho2i = 0.0, qrho2j = 0.0;
-    if (projv < 0.0) {
-      qrho2i = -0.5 * I.rho1i * vsigavi * projv;
-      if (usej || SYM) qrho2j = -0.5 * rho1j * vsigavj * projv;
-    }
-    const double dudtdissi = pm * qrho2i * projv * grkerni;
-    const double gradpi = pm * (I.pro2i + qrho2i) * grkerni;
-    const double gradpj = usej ? pm * (pro2j + qrho2j) * grkernj : 0.0;
-    double dendiss = 0.0;
-    if (adiab) {
-      double vsigu;
-      if (GRAV) vsigu = fabs(projv);
-      else vsigu = sqrt(fabs(I.pri - prj) * (2.0 / (I.rhoi + rhoj)));
-      dendiss = vsigu * denij * (I.auterm * grkerni + autermj * grkernj);
-    }
-    double projsx = 0, projsy = 0, projsz = 0, dudtresist = 0.0;
-    if (MHD) {
-      const double *mj = jmhd + JMHD * (size_t)j;
-      const double bxj = mj[0], byj = mj[1], bzj = mj[2], psij = mj[3];
-      const double dBx = I.bxi - bxj, dBy = I.byi - byj, dBz = I.bzi - bzj;
-      const double projBi = I.bxi * runix + I.byi * runiy + I.bzi * runiz;
-      const double projBj = bxj * runix + byj * runiy + bzj * runiz;
-      const double projdB = dBx * runix + dBy * runiy + dBz * runiz;
-      const double dB2 = dBx * dBx + dBy * dBy + dBz * dBz;
-      f[11] += -pm * projdB * grkerni;  // divBdiffterm
-      const double tx_ = dvx - projv * runix, ty_ = dvy - projv * runiy, tz_ = dvz - projv * runiz;
-      const double vsigB = sqrt(tx_ * tx_ + ty_ * ty_ + tz_ * tz_);
-      const double dBdiss = (I.avBterm * grkerni + avBtermj * grkernj) * vsigB;
-      if (p.iresistive_heating > 0 && adiab) dudtresist = -0.5 * dB2 * dBdiss;
-      const double pmi = pm * I.rho21i * grkerni, pmj = pm * rho21j * grkernj;
-      const double termi = pmi * projBi;
-      const double f7 = termi + pmj * projBj;
-      f[7] += f7;  // divBsymmterm
-      const double dpsi = p.overcleanfac * (pmi * I.psii * I.vwavei + pmj * psij * vwavej);
-      f[8] += -termi * dvx + dBdiss * dBx - dpsi * runix;
-      f[9] += -termi * dvy + dBdiss * dBy - dpsi * runiy;
-      f[10] += -termi * dvz + dBdiss * dBz - dpsi * runiz;
-      projsx = (I.sxx * runix + I.sxy * runiy + I.sxz * runiz) * grkerni +
-               (mj[4] * runix + mj[5] * runiy + mj[6] * runiz) * grkernj;
-      projsy = (I.sxy * runix + I.syy * runiy + I.syz * runiz) * grkerni +
-               (mj[5] * runix + mj[7] * runiy + mj[8] * runiz) * grkernj;
-      projsz = (I.sxz * runix + I.syz * runiy + I.szz * runiz) * grkerni +
-               (mj[6] * runix + mj[8] * runiy + mj[9] * runiz) * grkernj;
-      if (SYM) {
-        // from j: r -> -r, dv -> -dv, dB -> -dB; its own term -pmj (B_j . r) dv
-        const double termj = pmj * projBj;
-        jv[6] = -f7;
-        jv[7] = -termj * dvx - dBdiss * dBx + dpsi * runix;
-        jv[8] = -termj * dvy - dBdiss * dBy + dpsi * runiy;
-        jv[9] = -termj * dvz - dBdiss * dBz + dpsi * runiz;
-        jv[10] = -pm * projdB * grkernj;
-      }
-    }
-    // the zero terms of a build without gravity or MHD are not added (x + 0 = x)
-    const double gp = GRAV ? (gradpi + gradpj) + fgrav : gradpi + gradpj;
-    double fx = -runix * gp, fy = -runiy * gp, fz = -runiz * gp;
-    if (MHD) { fx -= projsx; fy -= projsy; fz -= projsz; }
-    f[0] += fx; f[1] += fy; f[2] += fz;
-    if (GRAV) f[3] += pm * phii;
-    f[4] += projv * grkerni;
-    if (adiab) { f[5] += MHD ? dudtdissi + dudtresist : dudtdissi; f[6] += dendiss; }
+    // anisotropic stress: -(S_i.n gi + S_j.n gj) with S = -(B/rho)(B/rho), i.e.
+    // ti B_i + tj B_j
     if (SYM) {
+      const double fx = fma(ti, I.bx, fma(tj, bxj, -nx * gp)), fy = fma(ti, I.by, fma(tj, byj, -ny * gp)),
+                   fz = fma(ti, I.bz, fma(tj, bzj, -nz * gp));
+      f[0] += fx; f[1] += fy; f[2] += fz;
       jv[0] = -fx; jv[1] = -fy; jv[2] = -fz;
-      jv[3] = projv * grkernj;
-      if (adiab) {
-        const double dj = pm * qrho2j * projv * grkernj;
-        jv[4] = MHD ? dj + dudtresist : dj;
-        jv[5] = -dendiss;
-      } else {
-        jv[4] = 0.0; jv[5] = 0.0;
-      }
-      jv[NJS<MHD>::n - 1] = usei ? fmax_pos(vsigj, vsigi) : vsigj;
+      jv[4] += res;
+      // from j: r -> -r, dv -> -dv, dB -> -dB; its own term -tj dv
+      jv[6] = -f7;
+      jv[7] = fma(-tj, dvx, fma(-dBdiss, dBx, dpsi * nx));
+      jv[8] = fma(-tj, dvy, fma(-dBdiss, dBy, dpsi * ny));
+      jv[9] = fma(-tj, dvz, fma(-dBdiss, dBz, dpsi * nz));
+      jv[10] = -projdB * gj;
+    } else {
+      f[0] = fma(ti, I.bx, fma(tj, bxj, fma(-nx, gp, f[0])));
+      f[1] = fma(ti, I.by, fma(tj, byj, fma(-ny, gp, f[1])));
+      f[2] = fma(ti, I.bz, fma(tj, bzj, fma(-nz, gp, f[2])));
     }
-  } else if (GRAV) {
-    // plain 1/r^2 for trial pairs outside both kernels (force.F90:1991-2053)
-    const double rij1 = 1.0 / sqrt(rij2);
-    const double fgj = rij1 * rij1 * rij1 * pm;
-    f[0] -= dx * fgj; f[1] -= dy * fgj; f[2] -= dz * fgj;
-    f[3] += pm * (-rij1);
-  } else if (SYM) {
-    for (int v = 0; v < NJS<MHD>::n; ++v) jv[v] = 0.0;
   }
 }
 
@@ -776,8 +745,7 @@ template <bool MHD, bool GRAV, bool IND>
 __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const int *perm, const double *tx, const double *ty, const double *tz, const double *th,
-    const float4 *txf, const double *jrec, const double *jmhd, const double *eos_t, ForceOut out, double *psum,
-    int64_t ps, double pf_hmin,
+    const float4 *txf, const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin,
     const int *cells, const unsigned char *actf, const int8_t *ibin_old_t,
     unsigned char *wakemark, int *err) {
   const int w = threadIdx.x >> 5, lane = lane_id();
@@ -797,15 +765,15 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
   const bool act = lane < np * S;
   const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
   const int i = s0 + (IND ? cell_pos(am, il) : il);
-  const IFp64 I = ifp64_init<MHD, GRAV>(p, i, tx, ty, tz, th, jrec, jmhd, eos_t);
+  const IFp64 I = ifp64_init<MHD, GRAV>(p, i, tx, ty, tz, jrec, jmhd);
   const float4 xif = txf[i];
-  const float hi21f = (float)I.hi21;
-  const bool pf_i = (I.hi > pf_hmin) && !GRAV;
+  const float hi21f = xif.w * xif.w;
+  const bool pf_i = th[i] > pf_hmin;
   const float q2lim = 4.0f * 1.001f;
   const float pf_h1max = (float)(1.0 / pf_hmin);
   double f[NF];
   for (int k = 0; k < NF; ++k) f[k] = 0.0;
-  double vsigmax = 0.0;
+  long long vsigmax = 0;  // largest signal speed (bit pattern)
   int nbi = 0;  // largest ibin_old of the SPH neighbours (individual timesteps)
   const int off = cell_off[cell], nleaf = cell_nleaf[cell];
   if (lane == 0) {
@@ -830,7 +798,15 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
         if (fabsf(dzf) > 0.5f * p.dzboundf) dzf -= copysignf(p.dzboundf, dzf);
       }
       const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
-      return r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
+      const bool near = r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
+      if (!GRAV || near) return near;
+      // self-gravity: a trial pair provably outside both kernels (most of the
+      // list) takes its 1/r^2 term here, in the dense test sweep, without being
+      // queued with its record
+      double dx, dy, dz;
+      separation_fp64(p, I.x, I.y, I.z, base + k, stg.jidx[k], stg.code[k], tx, ty, tz, dx, dy, dz);
+      far_pair_fp64(dx, dy, dz, rsqrt_fast(fma(dz, dz, fma(dy, dy, dx * dx))), f);
+      return false;
     };
     auto body = [&](int k) {
       double jv[NJS<MHD>::n];
@@ -839,8 +815,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
     };
     queue_window(cnt, S, act, il, stripe, sm.q, test, body);
   }
-  store_pair_sums<IND>(sm, lane, np, S, s0, am, psum, ps, [&](int q) -> double {
-    return q < NF ? f[q] : (q == NF ? vsigmax : (double)nbi);
+  store_pair_sums<IND, true>(sm, lane, np, S, s0, am, psum, ps, p.massoftype, [&](int q) -> double {
+    return q < NF ? f[q] : (q == NF ? __longlong_as_double(vsigmax) : (double)nbi);
   });
 }
 
@@ -881,8 +857,7 @@ template <bool MHD>
 __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const double *th,
-    const float4 *txf, const double *jrec, const double *jmhd, const double *eos_t, ForceOut out, double *psum,
-    int64_t ps, double pf_hmin, const int *toff, double *jbuf, int64_t jstride, int *err) {
+    const float4 *txf, const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin, const int *toff, double *jbuf, int64_t jstride, int *err) {
   constexpr int NJ = NJS<MHD>::n;
   const unsigned FULL = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = lane_id();
@@ -895,15 +870,15 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
   const bool act = lane < np * S;
   const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
   const int i = s0 + il;
-  const IFp64 I = ifp64_init<MHD, false>(p, i, tx, ty, tz, th, jrec, jmhd, eos_t);
+  const IFp64 I = ifp64_init<MHD, false>(p, i, tx, ty, tz, jrec, jmhd);
   const float4 xif = txf[i];
-  const float hi21f = (float)I.hi21;
-  const bool pf_i = I.hi > pf_hmin;
+  const float hi21f = xif.w * xif.w;
+  const bool pf_i = th[i] > pf_hmin;
   const float q2lim = 4.0f * 1.001f;
   const float pf_h1max = (float)(1.0 / pf_hmin);
   double f[NF];
   for (int k = 0; k < NF; ++k) f[k] = 0.0;
-  double vsigmax = 0.0;
+  long long vsigmax = 0;  // largest signal speed (bit pattern)
   int nbi = 0;
   const int off = cell_off[cell], nleaf = cell_nleaf[cell];
   // the owned prefix of the list: entries starting at or after s0
@@ -1008,7 +983,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
   constexpr int RW = NF + 1;
   double *red = sm.u.red;
   __syncwarp();
-  for (int k = 0; k < RW; ++k) red[lane * RW + k] = k < NF ? f[k] : vsigmax;
+  for (int k = 0; k < RW; ++k) red[lane * RW + k] = k < NF ? f[k] : __longlong_as_double(vsigmax);
   __syncwarp();
   if (lane < np) {
     double fs[NF];
@@ -1020,7 +995,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
       vsm = fmax(vsm, src[NF]);
     }
     const size_t ip = (size_t)(s0 + lane);
-    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = fs[k];
+    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = k == 4 ? fs[k] : p.massoftype * fs[k];
     psum[FSLOT_VSIG * ps + ip] = vsm;
   }
 }
@@ -1033,7 +1008,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
 template <bool MHD>
 __global__ void k_force_gather(const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool,
                                const int *cell_off, const int *cell_nleaf, const int *cell_at, const int *toff,
-                               const double *jbuf, int64_t jstride, double *psum, int64_t ps, int *err) {
+                               const double *jbuf, int64_t jstride, double pm, double *psum, int64_t ps,
+                               int *err) {
   constexpr int NJ = NJS<MHD>::n;
   const unsigned FULL = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = lane_id();
@@ -1092,7 +1068,8 @@ __global__ void k_force_gather(const Node *nodes, const int *leaves, int ncell, 
     const int v = c / MAXCELL, t = c % MAXCELL;
     if (v < NJ && t < np) {
       double *dst = psum + (int64_t)njs_slot(v, MHD) * ps + s0 + t;
-      *dst = (v == NJ - 1) ? fmax_pos(*dst, acc[r]) : *dst + acc[r];
+      // v == 3: d(rho)/dt, without the particle mass
+      *dst = (v == NJ - 1) ? fmax_pos(*dst, acc[r]) : (v == 3 ? *dst + acc[r] : fma(pm, acc[r], *dst));
     }
   }
 }
@@ -1397,7 +1374,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed(
     // and 16 warps (4.94 -> 4.37 ms per Sedov 128^3 launch)
     queue_window(cnt, S, act, il, stripe, sm.q, test, [&](int k) { body(load(k)); });
   }
-  store_pair_sums<IND>(sm, lane, np, S, s0, am, psum, ps, [&](int q) -> double {
+  store_pair_sums<IND, false>(sm, lane, np, S, s0, am, psum, ps, 1.0, [&](int q) -> double {
     return q < NF ? f[q].value() : (q == NF ? (double)vsigmax : (double)nbi);
   });
 }
@@ -1510,9 +1487,9 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
                                                           c->jrecf, jmhdf, c->txf, c->alpha1, c->ddivvdt_c,
                                                           c->dvdx_c, c->alphaloc_t, c->d_err);
   else
-    k_force_prologue<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, c->tx, c->ty, c->tz, c->th, vel, Bv,
-                                                    p.ind ? c->gradh : c->gradh_t, eos_t, c->jrec, jmhd, nullptr,
-                                                    nullptr, c->txf, c->alpha1, c->ddivvdt_c, c->dvdx_c,
+    k_force_prologue<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, c->th, vel, Bv,
+                                                    p.ind ? c->gradh : c->gradh_t, eos_t, c->jrec, jmhd, c->txf,
+                                                    c->alpha1, c->ddivvdt_c, c->dvdx_c,
                                                     c->alphaloc_t, c->d_err);
   count_launch(c, 1);
   const int lr = force_lists(c);
@@ -1568,17 +1545,17 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
     if (p.mhd) {
       k_force_sym<true><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SymSmem<true>), st>>>(
           p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,
-          c->jrec, jmhd, eos_t, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
+          c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
       k_force_gather<true><<<nblk(nfc, 4), 128, 0, st>>>(c->nodes, c->leaves, nfc, c->pool, c->cell_off,
                                                          c->cell_nleaf, c->cell_at, c->toff, c->jbuf,
-                                                         c->jbuf_stride, c->psum, c->cap, c->d_err);
+                                                         c->jbuf_stride, p.massoftype, c->psum, c->cap, c->d_err);
     } else {
       k_force_sym<false><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SymSmem<false>), st>>>(
           p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,
-          c->jrec, jmhd, eos_t, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
+          c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
       k_force_gather<false><<<nblk(nfc, 4), 128, 0, st>>>(c->nodes, c->leaves, nfc, c->pool, c->cell_off,
                                                           c->cell_nleaf, c->cell_at, c->toff, c->jbuf,
-                                                          c->jbuf_stride, c->psum, c->cap, c->d_err);
+                                                          c->jbuf_stride, p.massoftype, c->psum, c->cap, c->d_err);
     }
     count_launch(c, 1);
   } else {
@@ -1588,7 +1565,7 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
 #define PH_FORCE_FP64_I(M, G, I)                                                                                 \
   k_force<M, G, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(PairSmem), st>>>(                    \
       p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->perm, c->tx, c->ty, c->tz, c->th,       \
-      c->txf, c->jrec, jmhd, eos_t, out, c->psum, c->cap, c->pf_hmin, cells, actf, ibo, wake, c->d_err)
+      c->txf, c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, cells, actf, ibo, wake, c->d_err)
     if (p.mhd) { if (p.gravity) PH_FORCE_FP64(true, true); else PH_FORCE_FP64(true, false); }
     else { if (p.gravity) PH_FORCE_FP64(false, true); else PH_FORCE_FP64(false, false); }
 #undef PH_FORCE_FP64
