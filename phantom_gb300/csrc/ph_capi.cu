@@ -79,7 +79,7 @@ int alloc_all(ph_ctx *c, int64_t cap) {
   c->pool_cap = (int64_t)std::max<int64_t>(65536, (int64_t)n * 48);
   r |= dalloc(c, &c->pool, (size_t)c->pool_cap);
   r |= dalloc(c, &c->pool_top, 1);
-  r |= dalloc(c, &c->txf, n);
+  r |= dalloc(c, &c->txf, n); r |= dalloc(c, &c->txl, n);
   r |= dalloc(c, &c->bjf, n);
   r |= dalloc(c, &c->jrec, 32 * n);
   r |= dalloc(c, &c->jrecf, 32 * n);

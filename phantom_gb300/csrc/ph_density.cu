@@ -56,15 +56,18 @@ __global__ void k_dens_bprep(Params p, int n, const int *perm, const double *Bev
   }
 }
 
-// gather per-particle tree-order inputs: h, and h into the FP32 copy (its
-// x, y, z are set by the tree build)
+// gather per-particle tree-order inputs: h, and for the mixed form the low
+// parts of the positions (txf holds the high parts, set by the tree build)
 __global__ void k_dens_gather(int n, const int *perm, const double *xyzh, const double *tx, const double *ty,
-                              const double *tz, double *hcur, double *hold, float4 *txf) {
+                              const double *tz, double *hcur, double *hold, const float4 *txf, float4 *txl) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double h = xyzh[4 * (size_t)perm[i] + 3];
   hcur[i] = h; hold[i] = h;
-  txf[i].w = (float)h;
+  if (txl) {
+    const float4 f = txf[i];
+    txl[i] = make_float4(d2f_rn(tx[i] - (double)f.x), d2f_rn(ty[i] - (double)f.y), d2f_rn(tz[i] - (double)f.z), 0.0f);
+  }
 }
 
 __global__ void k_dens_init_cells(int ncell, const int *leaves, const Node *nodes, double *cell_hmax,
@@ -78,7 +81,7 @@ __global__ void k_dens_init_cells(int ncell, const int *leaves, const Node *node
 
 // per-particle pair sums written by k_density_pairs (tree order, slot-major
 // with stride ps): slots 0..NACC-1 the sums, then the neighbour count and the
-// neighbour-set hash (bit pattern) of each particle, self excluded
+// neighbour-set hash (bit patterns) of each particle, self excluded
 constexpr int DSLOT_NN = NACC, DSLOT_HASH = NACC + 1;
 
 struct DensOut {
@@ -97,14 +100,18 @@ struct DensOut {
 };
 
 // get_density_sums (dens.F90:578-857) for the active cells: one warp per cell,
-// lanes (particle il, stripe), accepted pairs drained from per-particle queues.
+// the trial list swept into per-particle queues and drained with the lanes
+// dealt out by queue length (list sweep). The neighbour test is the
+// reference's: FP32 with a 1e-3 margin in r^2 rejects pairs provably outside
+// the kernel (bypassed when h is small against the coordinates), the rest is
+// decided in FP64.
 template <bool MIXED, bool MHD, bool GRAV>
 __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
     Params p, const Node *nodes, const int *leaves, const int *act, int nact, const LeafEntry *pool,
     const int *cell_off, const int *cell_nleaf, const int *cell_ntrial, const int *perm, const double *tx,
-    const double *ty, const double *tz, const float4 *txf, const double *hcur, const double *Bevol,
-    const double *bj64, const float4 *bjf, double *psum, int64_t ps, unsigned long long *stats, double pf_hmin,
-    const unsigned char *actf, int want_hash, int *err) {
+    const double *ty, const double *tz, const float4 *txf, const float4 *txl, const double *hcur, const double *Bevol,
+    const double *bj64, const float4 *bjf, double *psum, int64_t ps, unsigned long long *stats, double pf_hmin, const unsigned char *actf,
+    int want_hash, int *err) {
   extern __shared__ __align__(16) unsigned char dsm[];
   const int w = threadIdx.x >> 5, lane = lane_id();
   const int a = blockIdx.x * (blockDim.x >> 5) + w;
@@ -116,75 +123,72 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
     if (lane == 0) set_error(err, PH_ERR_TREE);
     return;
   }
-  int np;
-  const unsigned am = cell_active_mask(actf, s0, np_all, np);  // active particles (individual timesteps)
+  int np = np_all;
+  unsigned am = 0u;  // active particles (individual timesteps)
+  if (actf) am = cell_active_mask(actf, s0, np_all, np);
   if (np == 0) return;
-  const int S = 32 / np;
-  const bool active_lane = lane < np * S;
-  const int il = active_lane ? lane / S : 0, stripe = active_lane ? lane % S : 0;
-  const int i = s0 + cell_pos(am, il);
+  ListSmem &sm = reinterpret_cast<ListSmem *>(dsm)[w];
   const double pm = p.massoftype;
-  const double xi = tx[i], yi = ty[i], zi = tz[i];
-  const double hi = hcur[i], hi1 = ddiv(1.0, hi), hi21 = dmul(hi1, hi1);
-  const float4 xif = txf[i];
-  const float hi21f = (float)hi21;
-  const bool use_pf = hi > pf_hmin;
-  const float q2lim = 4.0f * 1.001f;
-  double bxi = 0, byi = 0, bzi = 0;             // B_i rho_i
-  float bxrf = 0.0f, byrf = 0.0f, bzrf = 0.0f;  // (mixed form)
-  if (MHD) {
-    const double *b = Bevol + 4 * (size_t)perm[i];
-    const double rhoi_b = rhoh(hi, pm, p.hfact);
-    bxi = dmul(b[0], rhoi_b); byi = dmul(b[1], rhoi_b); bzi = dmul(b[2], rhoi_b);
-    bxrf = (float)bxi; byrf = (float)byi; bzrf = (float)bzi;
+  const float pmf = d2f_rn(pm);
+  double h1own = 0.0;  // lane il: 1/h of particle il
+  if (lane < np) {
+    const int ip = s0 + (actf ? cell_pos(am, lane) : lane);
+    const double h = hcur[ip];
+    h1own = ddiv(1.0, h);
+    const float hf = d2f_rn(h);
+    float4 x = txf[ip];
+    x.w = MIXED || h > pf_hmin ? 4.0f * 1.001f * (hf * hf) : __int_as_float(0x7f800000);
+    sm.xi[lane] = x;
+    sm.ipos[lane] = ip;
   }
-  constexpr int PHI = 3;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  double accb[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  Kahan kacc[MIXED ? NACC : 1];
-  const float hi1f = (float)hi1, pmf = (float)pm;
-  int nn = 0;
-  unsigned long long hh = 0;
   const int off = cell_off[cell], nleaf = cell_nleaf[cell];
-  const int ntrial = cell_ntrial[cell];
   if (lane == 0) {
+    const int ntrial = cell_ntrial[cell];
     atomicAdd(&stats[9], (unsigned long long)ntrial);
     atomicAdd(&stats[11], (unsigned long long)np * (unsigned long long)ntrial);
   }
-  PairSmem &sm = reinterpret_cast<PairSmem *>(dsm)[w];
-  for (int base = 0; base < ntrial; base += STAGE) {
-    const int cnt = stage_window(p, pool, off, nleaf, ntrial, base, txf, sm.st);
-    auto test = [&](int k) -> bool {
-      if (sm.st.jidx[k] == i) return false;  // ignoreself (dens.F90:650)
-      if (!(use_pf || MIXED)) return true;
-      const float4 xj = sm.st.pos[k];
-      float dxf = xif.x - xj.x, dyf = xif.y - xj.y, dzf = xif.z - xj.z;
-      if (p.periodic) {
-        if (fabsf(dxf) > 0.5f * p.dxboundf) dxf -= copysignf(p.dxboundf, dxf);
-        if (fabsf(dyf) > 0.5f * p.dyboundf) dyf -= copysignf(p.dyboundf, dyf);
-        if (fabsf(dzf) > 0.5f * p.dzboundf) dzf -= copysignf(p.dzboundf, dzf);
-      }
-      const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
-      return r2f * hi21f < q2lim;
-    };
-    // mixed form: the pair's operands, then its body
-    struct PF { int j, code; float4 xj; double x, y, z; };
-    auto load = [&](int k) -> PF {
-      PF f;
-      f.j = sm.st.jidx[k]; f.code = sm.st.code[k]; f.xj = sm.st.pos[k];
-      f.x = tx[f.j]; f.y = ty[f.j]; f.z = tz[f.j];
-      return f;
-    };
-    auto body_m = [&](const PF &pf) {
-      const int j = pf.j;
-      {
-        // separation formed in FP64 (the periodic image chosen on the FP32
-        // copy), rounded to FP32; W, dW/dh and the sums in FP32 (Kahan)
-        const float4 xj = pf.xj;
-        float dx, dy, dz;
-        separation_mixed(p, xi, yi, zi, pf.x, pf.y, pf.z, pf.code, xif.x - xj.x, xif.y - xj.y, xif.z - xj.z, dx,
-                         dy, dz);
-        const float r2 = dx * dx + dy * dy + dz * dz;
+  const float4 cc = make_float4((float)nd.x, (float)nd.y, (float)nd.z, (float)nd.size);
+  const int qstride = LQ / np;
+  // sum slots: sum W m, sum (-q dW/dq - 3 W) m, sum phi m, with MHD the dB sums
+  // (3 div B, 4..12 dB_a/dx_b, whose diagonal no output reads), the neighbour
+  // count and the neighbour-set hash (bit patterns)
+  constexpr int NA = MHD ? NACC : 3, RW = NA + 2, NR = (RW * MAXCELL + 31) / 32, PHI = 3;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  ListPos pos;
+  __syncwarp();
+  bool more = true;
+  while (more) {
+    int myc;
+    more = sweep_list<false>(p, cc, np, pool, off, nleaf, txf, sm, qstride, pos, myc, [](float) { return 0.0f; });
+    const QueueLanes ql = balance_queues(np, myc, sm);
+    const int il = max(ql.il, 0), i = sm.ipos[il];
+    const double hi1 = __shfl_sync(0xffffffffu, h1own, il);
+    const int *qj = sm.qj + il * qstride;
+    const unsigned char *qc = sm.qc + il * qstride;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    double accb[MHD ? 9 : 1] = {};
+    Kahan kacc[MIXED ? NA : 1];
+    int nn = 0;
+    unsigned long long hh = 0;
+    // B_i rho_i with the h of this pass (B_j with h at entry of the call)
+    double bxi = 0.0, byi = 0.0, bzi = 0.0;
+    if (MHD) {
+      const double *b = Bevol + 4 * (size_t)perm[i];
+      const double rho = rhoh(hcur[i], pm, p.hfact);
+      bxi = dmul(b[0], rho); byi = dmul(b[1], rho); bzi = dmul(b[2], rho);
+    }
+    if constexpr (MIXED) {
+      const Sep2 I = sep2_init(txf, txl, i);
+      const float hi1f = d2f_rn(hi1), hi21f = d2f_rn(dmul(hi1, hi1));
+      float4 bi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (MHD) bi = make_float4((float)bxi, (float)byi, (float)bzi, 0.0f);
+      for (int m = ql.m0; m < ql.c; m += ql.step) {
+        // separation to FP32 precision of the FP64 positions; W, dW/dh and the
+        // sums in FP32 (Kahan)
+        const int j = qj[m];
+        float dx, dy, dz, r2;
+        separation_2f(p, I, j, qc[m] & 63, txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
         const float q2 = r2 * hi21f;
         if (q2 < 4.0f) {
           const float rij = sqrtf(r2), q = rij * hi1f;
@@ -196,11 +200,11 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
           if (GRAV) kacc[2].add(dphidh_f(q2, q) * pmf);
           ++nn;
           if (want_hash) hh += mix64((unsigned long long)perm[j] + 1ull);
-          if (MHD) {
+          if constexpr (MHD) {
             const float r1g = grk / (rij + 1.0e-30f);
             const float rux = dx * r1g * pmf, ruy = dy * r1g * pmf, ruz = dz * r1g * pmf;
             const float4 bj = bjf[j];
-            const float dBx = bxrf - bj.x, dBy = byrf - bj.y, dBz = bzrf - bj.z;
+            const float dBx = bi.x - bj.x, dBy = bi.y - bj.y, dBz = bi.z - bj.z;
             kacc[3].add(dBx * rux + dBy * ruy + dBz * ruz);
             kacc[4].add(dBx * rux); kacc[5].add(dBx * ruy); kacc[6].add(dBx * ruz);
             kacc[7].add(dBy * rux); kacc[8].add(dBy * ruy); kacc[9].add(dBy * ruz);
@@ -208,84 +212,72 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
           }
         }
       }
-    };
-    auto body = [&](int k) {
-      // FP64 pair: separation and r^2 (6 FP64 instructions), r (5), the
-      // kernel sums (7). acc[0] = sum u s, acc[1] = sum w^2, acc[2] = sum s
-      // (combined after the loop), acc[PHI] the softening sum
-      const int j = sm.st.jidx[k];
-      double dx, dy, dz;
-      separation_fp64(p, xi, yi, zi, base + k, j, sm.st.code[k], tx, ty, tz, dx, dy, dz);
-      const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-      const double y = rsqrt_seed(r2), t = r2 * y;
-      const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
-      const double u = fma(-fma(t, pe, t), hi1, 2.0);
-      // the reference's test where the sign of u does not decide it
-      bool in = u_inside(u);
-      if (u_near_edge(u)) in = dmul(r2_exact(dx, dy, dz), hi21) < RADKERN2;
-      if (in) {
-        const double w = kern_w(u), u2 = u * u, s = fma(-w, w, u2);
-        acc[0] = fma(u, s, acc[0]);
-        acc[1] = fma(w, w, acc[1]);
-        acc[2] += s;
-        if (GRAV) {
-          // get_kernel_grav1 (kernel_cubic.f90:78-99): u^4 (1/2 - u/5) - w^4 (1 - 2w/5) / 16
-          const double w2 = w * w;
-          acc[PHI] = fma(u2 * u2, fma(-0.2, u, 0.5), acc[PHI]);
-          acc[PHI] = fma(w2 * w2, fma(0.025, w, -0.0625), acc[PHI]);
-        }
-        ++nn;
-        if (want_hash) hh += mix64((unsigned long long)perm[j] + 1ull);
-        if (MHD) {  // dens.F90:745-829 (getdB): dW/dq / r = -3/4 s / r
-          const double r1g = -0.75 * s * fma(y, pe, y);
-          const double rux = dx * r1g, ruy = dy * r1g, ruz = dz * r1g;
-          const double *bj = bj64 + 4 * (size_t)j;
-          const double dBx = bxi - bj[0], dBy = byi - bj[1], dBz = bzi - bj[2];
-          accb[0] = fma(dBx, rux, fma(dBy, ruy, fma(dBz, ruz, accb[0])));
-          accb[2] = fma(dBx, ruy, accb[2]); accb[3] = fma(dBx, ruz, accb[3]);
-          accb[4] = fma(dBy, rux, accb[4]); accb[6] = fma(dBy, ruz, accb[6]);
-          accb[7] = fma(dBz, rux, accb[7]); accb[8] = fma(dBz, ruy, accb[8]);
+    } else {
+      const double xi = tx[i], yi = ty[i], zi = tz[i];
+      for (int m = ql.m0; m < ql.c; m += ql.step) {
+        // separation and r^2 (6 FP64 instructions), r (5), the kernel sums (7).
+        // acc[0] = sum u s, acc[1] = sum w^2, acc[2] = sum s (combined after the
+        // loop), acc[PHI] the softening sum
+        const int j = qj[m];
+        double dx, dy, dz;
+        separation_fp64(p, xi, yi, zi, j, qc[m], tx, ty, tz, dx, dy, dz);
+        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+        const double y = rsqrt_seed(r2), t = r2 * y;
+        const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
+        const double u = fma(-fma(t, pe, t), hi1, 2.0);
+        // the reference's test where the sign of u does not decide it
+        bool in = u_inside(u);
+        if (u_near_edge(u)) in = inside_exact(dx, dy, dz, hi1);
+        if (in) {
+          const double w = kern_w(u), u2 = u * u, s = fma(-w, w, u2);
+          acc[0] = fma(u, s, acc[0]);
+          acc[1] = fma(w, w, acc[1]);
+          acc[2] += s;
+          if (GRAV) {
+            // get_kernel_grav1 (kernel_cubic.f90:78-99): u^4 (1/2 - u/5) - w^4 (1 - 2w/5) / 16
+            const double w2 = w * w;
+            acc[PHI] = fma(u2 * u2, fma(-0.2, u, 0.5), acc[PHI]);
+            acc[PHI] = fma(w2 * w2, fma(0.025, w, -0.0625), acc[PHI]);
+          }
+          ++nn;
+          if (want_hash) hh += mix64((unsigned long long)perm[j] + 1ull);
+          if constexpr (MHD) {  // dens.F90:745-829 (getdB): dW/dq / r = -3/4 s / r
+            const double r1g = -0.75 * s * fma(y, pe, y);
+            const double rux = dx * r1g, ruy = dy * r1g, ruz = dz * r1g;
+            const double *bj = bj64 + 4 * (size_t)j;
+            const double dBx = bxi - bj[0], dBy = byi - bj[1], dBz = bzi - bj[2];
+            accb[0] = fma(dBx, rux, fma(dBy, ruy, fma(dBz, ruz, accb[0])));
+            accb[2] = fma(dBx, ruy, accb[2]); accb[3] = fma(dBx, ruz, accb[3]);
+            accb[4] = fma(dBy, rux, accb[4]); accb[6] = fma(dBy, ruz, accb[6]);
+            accb[7] = fma(dBz, rux, accb[7]); accb[8] = fma(dBz, ruy, accb[8]);
+          }
         }
       }
-    };
-    if constexpr (MIXED) queue_window(cnt, S, active_lane, il, stripe, sm.q, test, [&](int k) { body_m(load(k)); });
-    else queue_window(cnt, S, active_lane, il, stripe, sm.q, test, body);
-  }
-  // sum W m, sum (-q dW/dq - 3 W) m, sum phi m, and the dB sums m (slot 3 div
-  // B, 4..12 dB_a/dx_b, whose diagonal no output reads)
-  auto lane_sum = [&](int k) -> double {
-    if constexpr (MIXED) return kacc[k].value();
-    if (k == 0) return 0.25 * pm * (acc[0] + acc[1]);
-    if (k == 1) return 0.75 * pm * (2.0 * (acc[2] - acc[0]) - acc[1]);
-    if (k == 2) return GRAV ? pm * acc[PHI] : 0.0;
-    return MHD && k != 4 && k != 8 && k != 12 ? pm * accb[k == 3 ? 0 : k - 3] : 0.0;
-  };
-  // the slots in use: the dB sums only with MHD
-  constexpr int NA = MHD ? NACC : 3;
-  // combine the stripes of each particle in stripe order (the staged window
-  // is no longer needed: its shared memory holds the partial sums)
-  constexpr int RW = NACC + 2;
-  double *red = reinterpret_cast<double *>(&sm.st);
-  __syncwarp();
-  for (int k = 0; k < NA; ++k) red[lane * RW + k] = lane_sum(k);
-  red[lane * RW + DSLOT_NN] = (double)nn;
-  red[lane * RW + DSLOT_HASH] = __longlong_as_double((long long)hh);
-  __syncwarp();
-  if (lane < np) {
-    double r[NA];
-    for (int k = 0; k < NA; ++k) r[k] = 0.0;
-    double nni = 0.0;
-    unsigned long long hhi = 0;
-    for (int q = 0; q < S; ++q) {
-      const double *src = red + (lane * S + q) * RW;
-      for (int k = 0; k < NA; ++k) r[k] = dadd(r[k], src[k]);
-      nni += src[DSLOT_NN];
-      hhi += (unsigned long long)__double_as_longlong(src[DSLOT_HASH]);
     }
-    const size_t ip = (size_t)(s0 + cell_pos(am, lane));
-    for (int k = 0; k < NA; ++k) psum[k * ps + ip] = r[k];
-    psum[DSLOT_NN * ps + ip] = nni;
-    psum[DSLOT_HASH * ps + ip] = __longlong_as_double((long long)hhi);
+    flush_lanes<RW>(np, sm, tot,
+        [&](int k) -> double {
+          if (k == NA) return __longlong_as_double((long long)nn);
+          if (k == NA + 1) return __longlong_as_double((long long)hh);
+          if constexpr (MIXED) return kacc[k].value();
+          else {
+            if (k == 0) return 0.25 * pm * (acc[0] + acc[1]);
+            if (k == 1) return 0.75 * pm * (2.0 * (acc[2] - acc[0]) - acc[1]);
+            if (k == 2) return GRAV ? pm * acc[PHI] : 0.0;
+            return MHD && k != 4 && k != 8 && k != 12 ? pm * accb[k == 3 ? 0 : k - 3] : 0.0;
+          }
+        },
+        [](int k, double s, double v) -> double {
+          if (k >= NA) return __longlong_as_double(__double_as_longlong(s) + __double_as_longlong(v));
+          return dadd(s, v);
+        });
+  }
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane + 32 * r;
+    if (idx < RW * np) {
+      const int k = idx / np;
+      const int slot = k < NA ? k : (k == NA ? DSLOT_NN : DSLOT_HASH);
+      psum[slot * ps + sm.ipos[idx - k * np]] = tot[r];
+    }
   }
 }
 
@@ -431,13 +423,13 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_dv(
         return;
       }
       double dx, dy, dz;
-      separation_fp64(p, xi, yi, zi, n, j, code, tx, ty, tz, dx, dy, dz);
+      separation_fp64(p, xi, yi, zi, j, code | (n < CELLCACHE ? QC_CACHED : 0), tx, ty, tz, dx, dy, dz);
       const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
       const double y = rsqrt_seed(r2), t = r2 * y;
       const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
       const double u = fma(-fma(t, pe, t), hi1, 2.0);
       bool in = u_inside(u);
-      if (u_near_edge(u)) in = dmul(r2_exact(dx, dy, dz), hi21) < RADKERN2;
+      if (u_near_edge(u)) in = inside_exact(dx, dy, dz, hi1);
       if (in) {
         const double w = kern_w(u), s = fma(-w, w, u * u);
         const double r1g = -0.75 * pm * s * fma(y, pe, y);
@@ -668,7 +660,7 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
         db[2] = (float)(dmul(-dsub(r6, r10), term));
         db[3] = (float)(dmul(-dsub(r7, r5), term));
       }
-      const int nni = (int)psum[DSLOT_NN * ps + ip] + 1;  // + self
+      const int nni = (int)__double_as_longlong(psum[DSLOT_NN * ps + ip]) + 1;  // + self
       if (out.diag) {
         out.nneigh[pid] = nni;
         out.nhash[pid] = (uint64_t)__double_as_longlong(psum[DSLOT_HASH * ps + ip]);
@@ -713,7 +705,8 @@ int density(ph_ctx *c, int icall) {
   cudaStream_t st = c->stream;
   const int nt = (int)c->ntree, ncell = c->nleaves;
   const Params p = c->dp;
-  k_dens_gather<<<nblk(nt, 256), 256, 0, st>>>(nt, c->perm, c->xyzh, c->tx, c->ty, c->tz, c->hcur, c->hold, c->txf);
+  k_dens_gather<<<nblk(nt, 256), 256, 0, st>>>(nt, c->perm, c->xyzh, c->tx, c->ty, c->tz, c->hcur, c->hold, c->txf,
+                                              p.precision == PH_PREC_MIXED ? c->txl : nullptr);
   k_dens_init_cells<<<nblk(ncell, 256), 256, 0, st>>>(ncell, c->leaves, c->nodes, c->cell_hmax, c->cell_nits, c->act_a);
   cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), st);
   cudaMemsetAsync(c->red, 0, 8 * sizeof(double), st);
@@ -751,9 +744,9 @@ int density(ph_ctx *c, int icall) {
               c->want_diag ? 1 : 0, getdv ? c->dvterm_t : nullptr, c->red + 2, c->stats};
   double pf_hmin = c->pf_hmin;
   const int dw = c->dens_warps, ww = c->walk_warps;
-  const int smem = dw * (int)sizeof(PairSmem);
+  const int smem = dw * (int)sizeof(ListSmem);
   if (!(c->attr_done & 1u)) {
-    const int smax = MAX_WARPS * (int)sizeof(PairSmem);
+    const int smax = MAX_WARPS * (int)sizeof(ListSmem);
     cudaFuncSetAttribute(k_density_pairs<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
     cudaFuncSetAttribute(k_density_pairs<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
     cudaFuncSetAttribute(k_density_pairs<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
@@ -790,7 +783,7 @@ int density(ph_ctx *c, int icall) {
 #define PH_DENS(X, M, G)                                                                                         \
   k_density_pairs<X, M, G><<<nblk(nact, dw), 32 * dw, smem, st>>>(                                    \
       p, c->nodes, c->leaves, act, nact, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->perm, c->tx, c->ty,  \
-      c->tz, c->txf, c->hcur, Bd, c->jrec, c->bjf, c->psum, c->cap, c->stats, pf_hmin, actf,             \
+      c->tz, c->txf, c->txl, c->hcur, Bd, c->jrec, c->bjf, c->psum, c->cap, c->stats, pf_hmin, actf,             \
       c->want_diag ? 1 : 0, c->d_err)
     if (p.precision == PH_PREC_MIXED) {
       if (dB) { if (p.gravity) PH_DENS(true, true, true); else PH_DENS(true, true, false); }

@@ -599,7 +599,7 @@ __device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I,
                                                 double (&jv)[NJS<MHD>::n]) {
   const bool adiab = !p.isothermal;
   double dx, dy, dz;
-  separation_fp64(p, I.x, I.y, I.z, n, j, code, tx, ty, tz, dx, dy, dz);
+  separation_fp64(p, I.x, I.y, I.z, j, code | (n < CELLCACHE ? QC_CACHED : 0), tx, ty, tz, dx, dy, dz);
   const double *rj = jrec + JREC * (size_t)j;
   const double hj1 = rj[JR_H1];
   // With self-gravity the direction of a neighbour pair keeps the reference's
@@ -619,9 +619,8 @@ __device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I,
   double ui = fma(-r, I.h1, 2.0), uj = fma(-r, hj1, 2.0);
   bool qi_in = u_inside(ui), qj_in = u_inside(uj);
   if (u_near_edge(ui) || u_near_edge(uj)) {  // the reference's q^2 < 4
-    const double rij2 = r2_exact(dx, dy, dz);
-    qi_in = dmul(rij2, dmul(I.h1, I.h1)) < RADKERN2;
-    qj_in = dmul(rij2, dmul(hj1, hj1)) < RADKERN2;
+    qi_in = inside_exact(dx, dy, dz, I.h1);
+    qj_in = inside_exact(dx, dy, dz, hj1);
   }
   if (!(qi_in || qj_in)) {
     if (GRAV) far_pair_fp64(dx, dy, dz, y, f);
@@ -804,7 +803,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
       // list) takes its 1/r^2 term here, in the dense test sweep, without being
       // queued with its record
       double dx, dy, dz;
-      separation_fp64(p, I.x, I.y, I.z, base + k, stg.jidx[k], stg.code[k], tx, ty, tz, dx, dy, dz);
+      separation_fp64(p, I.x, I.y, I.z, stg.jidx[k], stg.code[k] | (base + k < CELLCACHE ? QC_CACHED : 0), tx, ty, tz,
+                      dx, dy, dz);
       far_pair_fp64(dx, dy, dz, rsqrt_fast(fma(dz, dz, fma(dy, dy, dx * dx))), f);
       return false;
     };

@@ -211,7 +211,8 @@ struct ph_ctx {
   // force state (tree order)
   double *jrec = nullptr;    // per tree position j-side record (force prologue)
   float *jrecf = nullptr;    // FP32 copy of the j records (mixed precision form)
-  float4 *txf = nullptr;     // float x,y,z,h for the FP32 prefilter
+  float4 *txf = nullptr;     // float x,y,z (high parts of tx, ty, tz); w: 1/h for the force
+  float4 *txl = nullptr;     // low parts: tx - (double)txf.x, ... (mixed form)
   float4 *bjf = nullptr;     // FP32 B rho per tree position (mixed MHD density)
   double pf_hmin = 0.0;      // below this h the FP32 prefilter is bypassed
   double *red = nullptr;     // reductions: dtcourant, dtforce, rhomax, ...

@@ -135,11 +135,14 @@ __device__ __forceinline__ void separation_mixed(const Params &p, double xi, dou
 // pair) that is three FP64 subtractions: the wrap test compares bit patterns,
 // and the offset and shift adds sit in branches of their own, since an FP64
 // instruction holds the pipe for a whole warp when one lane needs it.
-__device__ __forceinline__ void separation_fp64(const Params &p, double xi, double yi, double zi, int n, int j,
-                                                int code, const double *tx, const double *ty, const double *tz,
+// code: the leaf's periodic offset, with QC_CACHED where the reference uses its
+// cached position
+constexpr int QC_CACHED = 64;
+__device__ __forceinline__ void separation_fp64(const Params &p, double xi, double yi, double zi, int j, int code,
+                                                const double *tx, const double *ty, const double *tz,
                                                 double &dx, double &dy, double &dz) {
   double xj = tx[j], yj = ty[j], zj = tz[j];
-  if (code != 0 && n < CELLCACHE) {
+  if (code > QC_CACHED) {
     xj = dadd(xj, offset_of(code, 0, p.dxbound)); yj = dadd(yj, offset_of(code, 1, p.dybound));
     zj = dadd(zj, offset_of(code, 2, p.dzbound));
   }
@@ -147,6 +150,66 @@ __device__ __forceinline__ void separation_fp64(const Params &p, double xi, doub
   if (p.periodic && (abs_gt(dx, p.hdlx) || abs_gt(dy, p.hdly) || abs_gt(dz, p.hdlz))) {
     dx = wrap(dx, p.dxbound, p.hdlx, true); dy = wrap(dy, p.dybound, p.hdly, true);
     dz = wrap(dz, p.dzbound, p.hdlz, true);
+  }
+}
+
+// the reference's neighbour test r^2 h^-2 < 4 with its rounding. Out of line:
+// inlined, the compiler evaluates its six FP64 instructions for every pair
+// instead of branching around them
+static __device__ __noinline__ bool inside_exact(double dx, double dy, double dz, double h1) {
+  return dmul(r2_exact(dx, dy, dz), dmul(h1, h1)) < RADKERN2;
+}
+
+// The same separation without the FP64 pipe: each coordinate is kept as two
+// floats, x = hi + lo to 2^-49 of |x| (txf, txl), and hi_i - hi_j with its exact
+// rounding error (Knuth's two-sum) plus lo_i - lo_j gives x_i - x_j rounded to
+// FP32. That costs eight FP32 additions per axis, where the FP64 subtraction
+// held the FP64 pipe (45-49 % of the mixed pair kernels' time) and its rounding
+// to FP32 took ten integer instructions. What the two floats leave out, 2^-49
+// |x|, stays below 2^-29 of r for r > 2^-20 |x|; closer pairs, and pairs across
+// a periodic image, take the FP64 separation (out of line).
+struct Sep2 {
+  float4 h, l;   // particle i
+  float guard;   // smallest r^2 the two floats serve
+  int i;
+};
+__device__ __forceinline__ Sep2 sep2_init(const float4 *__restrict__ txf, const float4 *__restrict__ txl, int i) {
+  Sep2 s;
+  s.h = txf[i]; s.l = txl[i]; s.i = i;
+  const float m = 9.5367431640625e-07f * fmaxf(fmaxf(fabsf(s.h.x), fabsf(s.h.y)), fabsf(s.h.z));
+  s.guard = m * m;
+  return s;
+}
+__device__ __forceinline__ float diff2(float ah, float al, float bh, float bl) {
+  const float s = __fsub_rn(ah, bh), t = __fsub_rn(s, ah);
+  const float e = __fsub_rn(__fsub_rn(ah, __fsub_rn(s, t)), __fadd_rn(bh, t));
+  return __fadd_rn(s, __fadd_rn(e, __fsub_rn(al, bl)));
+}
+static __device__ __noinline__ float3 separation_image(const double *tx, const double *ty, const double *tz, int i, int j,
+                                                int mx, int my, int mz, double Lx, double Ly, double Lz) {
+  return make_float3(d2f_rn((tx[i] - tx[j]) - shift_len(mx, Lx)), d2f_rn((ty[i] - ty[j]) - shift_len(my, Ly)),
+                     d2f_rn((tz[i] - tz[j]) - shift_len(mz, Lz)));
+}
+__device__ __forceinline__ void separation_2f(const Params &p, const Sep2 &I, int j, int code, const float4 &jh,
+                                              const float4 &jl, const double *tx, const double *ty, const double *tz,
+                                              float &dx, float &dy, float &dz, float &r2) {
+  int mx = 0, my = 0, mz = 0;
+  if (p.periodic) {
+    const float ux = I.h.x - (jh.x + offset_of_f(code, 0, p.dxboundf)),
+                uy = I.h.y - (jh.y + offset_of_f(code, 1, p.dyboundf)),
+                uz = I.h.z - (jh.z + offset_of_f(code, 2, p.dzboundf));
+    mx = image_shift(code, 0, fabsf(ux) > 0.5f * p.dxboundf, ux);
+    my = image_shift(code, 1, fabsf(uy) > 0.5f * p.dyboundf, uy);
+    mz = image_shift(code, 2, fabsf(uz) > 0.5f * p.dzboundf, uz);
+  }
+  dx = diff2(I.h.x, I.l.x, jh.x, jl.x);
+  dy = diff2(I.h.y, I.l.y, jh.y, jl.y);
+  dz = diff2(I.h.z, I.l.z, jh.z, jl.z);
+  r2 = dx * dx + dy * dy + dz * dz;
+  if ((mx | my | mz) != 0 || r2 < I.guard) {
+    const float3 d = separation_image(tx, ty, tz, I.i, j, mx, my, mz, p.dxbound, p.dybound, p.dzbound);
+    dx = d.x; dy = d.y; dz = d.z;
+    r2 = dx * dx + dy * dy + dz * dz;
   }
 }
 
@@ -208,6 +271,202 @@ __device__ __forceinline__ void queue_window(int cnt, int S, bool act, int il, i
       qn = 0;
     }
   }
+}
+
+// ------------------------------------------------------------------ list sweep
+// Trial list -> per-particle pair queues -> balanced drain, by one warp.
+//
+// The sweep: batches of 32 leaf entries are expanded into shared memory (tree
+// index and offset code per trial particle); each lane then takes one trial
+// particle (its FP32 position in registers, loaded one chunk ahead) and the
+// warp tests it against the cell's particles one after the other, their FP32
+// positions broadcast from shared memory. One ballot per particle gives the
+// accepted lanes their queue slots. Per 32 tests that is about 17 instructions,
+// where testing with a lane per (particle, stripe) took about 45 (a shared
+// position load, the periodic wrap, two ballots and queue bounds each).
+// Whether a chunk needs the periodic wrap at all is decided once per chunk.
+//
+// The drain: queues are emptied when one is nearly full or the list ends,
+// normally once per cell. The lanes are dealt out so that the particle with
+// most pairs per lane has as few as possible (balance_queues); with a fixed
+// 32/np lanes per particle the longest queue set the pace and a fifth (density)
+// to two fifths (symmetric force) of the lane slots were idle.
+constexpr int LW = 32 * MAXCELL;  // trial particles of a batch
+constexpr int LQ = 1280;          // queue slots per warp, dealt out evenly to the cell's particles
+
+struct __align__(16) ListSmem {
+  int qj[LQ];             // accepted trial particle (or its index in the batch)
+  unsigned char qc[LQ];   // offset code, bit 6: the reference uses its cached position
+  float4 xi[MAXCELL];     // cell particles: x, y, z, acceptance r^2
+  int ipos[MAXCELL];      // their tree positions
+  int j[LW];
+  unsigned char code[LW];
+  unsigned char own[32];  // drain: lane -> particle
+  unsigned char first[MAXCELL], lanes[MAXCELL];
+};
+struct ListPos {  // the sweep's place in the list
+  int e0 = 0, nbase = 0, cnt = 0, k0 = 0;
+};
+
+// expand the 32 leaf entries from e0 on; returns the number of trial particles
+__device__ __forceinline__ int expand_batch(const LeafEntry *__restrict__ pool, int off, int nleaf, int e0,
+                                            ListSmem &sm) {
+  const int e = e0 + lane_id();
+  LeafEntry le{0, 0};
+  if (e < nleaf) le = pool[off + e];
+  const int jc = le.cc & 255, code = le.cc >> 8;
+  int x = jc;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane_id() >= o) x += y;
+  }
+  const int k = x - jc;
+  for (int t = 0; t < jc; ++t) { sm.j[k + t] = le.start + t; sm.code[k + t] = (unsigned char)code; }
+  return __shfl_sync(0xffffffffu, x, 31);
+}
+
+// Sweep on from `pos` until the list ends (returns false) or a queue is nearly
+// full (true: drain, then call again). sm.xi / sm.ipos describe the np cell
+// particles; ew(w) is the acceptance r^2 of a trial particle with txf.w = w;
+// myc receives lane il's count for particle il. With AFTER only trial
+// particles after the cell particle in tree order are accepted, and the queue
+// holds batch indices (the list must end with its batch: drain per batch).
+template <bool AFTER, class EW>
+__device__ __forceinline__ bool sweep_list(const Params &p, float4 cc, int np, const LeafEntry *__restrict__ pool,
+                                           int off, int nleaf, const float4 *__restrict__ txf, ListSmem &sm,
+                                           int qstride, ListPos &pos, int &myc, EW ew) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  const float hx = 0.4995f * p.dxboundf - cc.w, hy = 0.4995f * p.dyboundf - cc.w, hz = 0.4995f * p.dzboundf - cc.w;
+  int qn[MAXCELL];
+#pragma unroll
+  for (int il = 0; il < MAXCELL; ++il) qn[il] = 0;
+  myc = 0;
+  int j = -1;
+  float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  bool fresh = true;  // the chunk at k0 is not loaded yet
+  while (true) {
+    if (pos.k0 >= pos.cnt) {
+      pos.nbase += pos.cnt;
+      if (pos.e0 >= nleaf || (AFTER && pos.cnt > 0)) { pos.k0 = pos.cnt = 0; return pos.e0 < nleaf; }
+      __syncwarp();
+      pos.cnt = expand_batch(pool, off, nleaf, pos.e0, sm);
+      pos.e0 += 32;
+      pos.k0 = 0;
+      fresh = true;
+      __syncwarp();
+    }
+    const int k = pos.k0 + lane;
+    if (fresh) {
+      j = k < pos.cnt ? sm.j[k] : -1;
+      if (j >= 0) e = txf[j];
+      fresh = false;
+    }
+    const int jc = j;
+    float4 x = e;
+    const int code = jc >= 0 ? sm.code[k] : 0;
+    j = k + 32 < pos.cnt ? sm.j[k + 32] : -1;
+    if (j >= 0) e = txf[j];
+    bool wr = false;
+    if (p.periodic) {
+      if (code != 0) {
+        x.x += offset_of_f(code, 0, p.dxboundf); x.y += offset_of_f(code, 1, p.dyboundf);
+        x.z += offset_of_f(code, 2, p.dzboundf);
+      }
+      wr = __any_sync(FULL, jc >= 0 && (fabsf(cc.x - x.x) > hx || fabsf(cc.y - x.y) > hy || fabsf(cc.z - x.z) > hz));
+    }
+    const float w = ew(x.w);
+    const int val = AFTER ? k : jc;
+    const unsigned char flag =
+        (unsigned char)(code != 0 ? code | (pos.nbase + k < CELLCACHE ? QC_CACHED : 0) : 0);
+    int mx = 0;
+#pragma unroll
+    for (int il = 0; il < MAXCELL; ++il) {
+      if (il >= np) break;
+      const float4 xi = sm.xi[il];
+      float dx = xi.x - x.x, dy = xi.y - x.y, dz = xi.z - x.z;
+      if (wr) {
+        if (fabsf(dx) > 0.5f * p.dxboundf) dx -= copysignf(p.dxboundf, dx);
+        if (fabsf(dy) > 0.5f * p.dyboundf) dy -= copysignf(p.dyboundf, dy);
+        if (fabsf(dz) > 0.5f * p.dzboundf) dz -= copysignf(p.dzboundf, dz);
+      }
+      const int ip = sm.ipos[il];
+      const bool ok = dx * dx + dy * dy + dz * dz < fmaxf(xi.w, w) && (AFTER ? jc > ip : (jc >= 0 && jc != ip));
+      const unsigned b = __ballot_sync(FULL, ok);
+      if (ok) {
+        const int q = il * qstride + qn[il] + __popc(b & lt);
+        sm.qj[q] = val;
+        if (!AFTER) sm.qc[q] = flag; else sm.code[k] = flag;
+      }
+      qn[il] += __popc(b);
+      if (lane == il) myc += __popc(b);
+      mx = max(mx, qn[il]);
+    }
+    pos.k0 += 32;
+    if (mx > qstride - 32) return true;
+  }
+}
+
+// Deal the 32 lanes out to the particles' queues (lane il < np holds its
+// count c): the smallest number s of pairs per lane for which sum ceil(c/s)
+// fits, from 32 s >= sum c up. Each lane gets its particle (il, -1: none), its
+// first queue entry, the step and the count.
+struct QueueLanes { int il, m0, step, c; };
+__device__ __forceinline__ QueueLanes balance_queues(int np, int c, ListSmem &sm) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = lane_id();
+  if (lane >= np) c = 0;
+  int s = max(1, (warp_sum_int(c) + 31) >> 5), need, tot;
+  while (true) {
+    need = (c + s - 1) / s;
+    tot = warp_sum_int(need);
+    if (tot <= 32) break;
+    ++s;
+  }
+  int x = need;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(FULL, x, o);
+    if (lane >= o) x += y;
+  }
+  x -= need;
+  for (int t = 0; t < need; ++t) sm.own[x + t] = (unsigned char)lane;
+  if (lane < np) { sm.first[lane] = (unsigned char)x; sm.lanes[lane] = (unsigned char)need; }
+  __syncwarp();
+  QueueLanes a;
+  a.il = lane < tot ? (int)sm.own[lane] : -1;
+  const int src = max(a.il, 0);
+  a.m0 = lane - __shfl_sync(FULL, x, src);
+  a.step = __shfl_sync(FULL, need, src);
+  a.c = a.il >= 0 ? __shfl_sync(FULL, c, src) : (__shfl_sync(FULL, c, src), 0);
+  return a;
+}
+
+// Sum RW values of every lane into per-(value, particle) totals: total idx =
+// value * np + particle lives in tot[idx / 32] of lane idx % 32. The lane
+// values pass through shared memory (the queues' space: all lanes are done
+// with them) and are added in lane order, so totals are deterministic.
+template <int RW, int NR, class Get, class Add>
+__device__ __forceinline__ void flush_lanes(int np, ListSmem &sm, double (&tot)[NR], Get get, Add add) {
+  static_assert(32 * RW * sizeof(double) <= sizeof(int) * LQ + LQ, "lane sums staged in the queues' space");
+  static_assert(RW * MAXCELL <= 32 * NR, "totals per lane");
+  double *red = reinterpret_cast<double *>(sm.qj);
+  const int lane = lane_id();
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < RW; ++k) red[lane * RW + k] = get(k);
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane + 32 * r;
+    if (idx < RW * np) {
+      const int k = idx / np, il = idx - k * np;
+      const double *src = red + (int)sm.first[il] * RW + k;
+      const int nl = sm.lanes[il];
+      for (int q = 0; q < nl; ++q) tot[r] = add(k, tot[r], src[q * RW]);
+    }
+  }
+  __syncwarp();
 }
 
 // The walking cell: position, size and search radius (exact and FP32).

@@ -87,3 +87,27 @@ def test_density_sums(case):
     if case == "gravity":
         gs = m * dphidh(q).sum(1) / hl ** 2 * dh
         assert np.abs(d["gradh"][:, 1] - gs).max() < 2.0 ** -22 * np.abs(gs).max()
+
+
+@pytest.mark.parametrize("gap", [1e-4, 3e-6, 2e-7, 1e-9, 1e-13])
+@pytest.mark.parametrize("shift", [0.0, 0.49])
+def test_mixed_separation_of_close_pairs(gap, shift):
+    """Precision form: pairs far closer than the coordinates' FP32 rounding, in
+    the box and across its face, keep the direction and size of their FP64
+    separation: one derivs against the plain form, within the form's 1e-5."""
+    cfg, x, v, B = setups.hydro_lattice(12, jitter=0.1, seed=6)
+    rng = np.random.default_rng(7)
+    pick = rng.choice(len(x), 40, replace=False)
+    d = rng.standard_normal((20, 3))
+    x[pick[20:], :3] = x[pick[:20], :3] + gap * d / np.linalg.norm(d, axis=1)[:, None]
+    x[:, :3] = np.mod(x[:, :3] + shift, 1.0)
+    out = []
+    for prec in (capi.PH_PREC_FP64, capi.PH_PREC_MIXED):
+        ctx = capi.Context(dict(cfg, tolh=1e-7), precision=prec)
+        ctx.upload(x, v, B)
+        ctx.build_tree()
+        h = ctx.densityiterate(1)["xyzh"][:, 3]
+        out.append((h, ctx.force(1, 0.0)["fxyzu"]))
+    assert np.abs(out[1][0] / out[0][0] - 1).max() < 1e-6
+    for c in (slice(0, 3), 3):
+        assert np.abs(out[1][1][:, c] - out[0][1][:, c]).max() < 1e-5 * np.abs(out[0][1][:, c]).max()
