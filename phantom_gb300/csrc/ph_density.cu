@@ -157,10 +157,11 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
   for (int r = 0; r < NR; ++r) tot[r] = 0.0;
   ListPos pos;
   __syncwarp();
+  static_assert(32 * RW <= LQ / 2, "lane sums staged in the queues' space");
   bool more = true;
   while (more) {
     int myc;
-    more = sweep_list<false>(p, cc, np, pool, off, nleaf, txf, sm, qstride, pos, myc, [](float) { return 0.0f; });
+    more = SWEEP_END != sweep_list<false, 32>(p, cc, np, pool, off, nleaf, txf, sm, qstride, pos, myc, [](float) { return 0.0f; });
     const QueueLanes ql = balance_queues(np, myc, sm);
     const int il = max(ql.il, 0), i = sm.ipos[il];
     const double hi1 = __shfl_sync(0xffffffffu, h1own, il);
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
         }
       }
     }
-    flush_lanes<RW>(np, sm, tot,
+    flush_lanes<RW>(np, sm, sm.red, tot,
         [&](int k) -> double {
           if (k == NA) return __longlong_as_double((long long)nn);
           if (k == NA + 1) return __longlong_as_double((long long)hh);

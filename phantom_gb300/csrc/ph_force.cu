@@ -22,18 +22,19 @@ namespace ph {
 
 constexpr int JREC = 16;   // doubles per particle, hydro record
 constexpr int JMHD = 16;   // doubles per particle, MHD record
-// The FP64 pair terms' record: every factor of a pair term that belongs to one
+// The pair terms' record: every factor of a pair term that belongs to one
 // particle is formed once in the prologue (the particle mass is applied to
 // the finished sums). JR_K = -3/4 cnormk h^-4 / Omega (on s of kern_w, giving
-// grad W), JR_C = -1/(2 rho) of the viscosity, JR_AVW = alpha v_wave,
-// JR_AU = alpha_u / (2 rho) (with the sqrt(2) of the conductivity's signal
+// grad W; without the -3/4 in the mixed form, whose kernel is grkernf),
+// JR_C = -1/(2 rho) of the viscosity, JR_AVW = alpha v_wave, JR_AU =
+// alpha_u / (2 rho) (FP64: with the sqrt(2) of the conductivity's signal
 // speed, force.F90:1605-1621), JR_AB = alpha_B / (2 rho^2)
 enum { JR_H1 = 0, JR_RHO, JR_C, JR_PRO2, JR_VW, JR_P, JR_AU, JR_K, JR_VX, JR_VY, JR_VZ, JR_U, JR_GS, JR_AB, JR_AVW,
        JR_R21 };
 // MHD: B, psi, overcleanfac psi v_wave; B/rho in the finish's slots 10..12
 enum { JM_BX = 0, JM_BY, JM_BZ, JM_PSI, JM_CL };
 constexpr int NF = 12;     // fsum entries
-constexpr int JRECF = 16, JMHDF = 16;  // floats per particle, FP32 copies of the records (mixed form)
+constexpr int JRECF = 16, JMHDF = 8;  // floats per particle, FP32 records of the mixed form
 
 // get_stress (force.F90:2068-2168) without physical viscosity / radiation: P/rho^2
 // with the magnetic pressure and the wave speed (the pair terms form the
@@ -121,22 +122,20 @@ __global__ void k_force_prologue_mixed(Params p, int n, const int *perm, const d
     vwave = sqrtf(cs * cs + bro2 * rho);
     pro2 += 0.5f * bro2;
     q[0] = brx * rho; q[1] = bry * rho; q[2] = brz * rho; q[3] = d2f_rn(b[3]);
-    q[4] = -pmf * brx * brx; q[5] = -pmf * brx * bry; q[6] = -pmf * brx * brz;
-    q[7] = -pmf * bry * bry; q[8] = -pmf * bry * brz; q[9] = -pmf * brz * brz;
-    q[10] = brx; q[11] = bry; q[12] = brz;
+    q[JM_CL] = d2f_rn(p.overcleanfac) * q[3] * vwave;
     double *m = jmhd + JMHD * (size_t)j;  // the finish's B/rho and psi
     m[3] = b[3]; m[10] = b[0]; m[11] = b[1]; m[12] = b[2];
   }
   const size_t g = p.ind ? (size_t)pid : (size_t)j;
-  const float mrho5 = 0.5f * pmf * rho1;
   float *o = jrecf + JRECF * (size_t)j;
-  o[0] = h1; o[1] = rho; o[2] = rho1; o[3] = pro2; o[4] = vwave; o[5] = P;
-  o[6] = mrho5 * d2f_rn(p.alphau); o[7] = gradh[2 * g];
-  o[8] = d2f_rn(v[0]); o[9] = d2f_rn(v[1]); o[10] = d2f_rn(v[2]); o[11] = u;
-  o[12] = gradh[2 * g + 1];
-  o[13] = mrho5 * d2f_rn(p.alphaB) * rho1;
-  o[14] = p.nalpha > 0 ? alpha1[pid] : d2f_rn(p.alpha);
-  o[15] = rho1 * rho1;
+  o[JR_H1] = h1; o[JR_RHO] = rho; o[JR_C] = -0.5f * rho1; o[JR_PRO2] = pro2; o[JR_VW] = vwave; o[JR_P] = P;
+  o[JR_AU] = 0.5f * rho1 * d2f_rn(p.alphau);
+  o[JR_K] = (h1 * h1) * (h1 * h1) * (float)CNORMK * gradh[2 * g];  // on dW/dq (grkernf)
+  o[JR_VX] = d2f_rn(v[0]); o[JR_VY] = d2f_rn(v[1]); o[JR_VZ] = d2f_rn(v[2]); o[JR_U] = u;
+  o[JR_GS] = gradh[2 * g + 1];
+  o[JR_AB] = 0.5f * d2f_rn(p.alphaB) * (rho1 * rho1);
+  o[JR_AVW] = (p.nalpha > 0 ? alpha1[pid] : d2f_rn(p.alpha)) * vwave;
+  o[JR_R21] = rho1 * rho1;
   jrec[JREC * (size_t)j + 11] = p.isothermal ? 0.0 : v[3];  // the finish's u
   txf[j].w = h1;
 }
@@ -297,7 +296,9 @@ __global__ void __launch_bounds__(256) k_force_finish(Params p, int nt, const do
   const double pm = p.massoftype;
   const bool adiab = !p.isothermal;
   double fs[NF];
-  for (int k = 0; k < NF; ++k) fs[k] = psum[k * ps + ip];
+  // the slots the pair kernels wrote (3: potential, 7..11: MHD)
+  for (int k = 0; k < NF; ++k)
+    fs[k] = (k == 3 ? p.gravity : (k < 7 || p.mhd)) ? psum[k * ps + ip] : 0.0;
   const double vsm = psum[FSLOT_VSIG * ps + ip];
   const int pid = perm[ip];
   const double h = th[ip];
@@ -478,9 +479,9 @@ __global__ void k_wake_apply(int nt, const int *perm, const unsigned char *wakem
 
 // the stripes of each particle summed in stripe order through shared memory
 // (the staged window's memory, no longer needed), written to psum by lanes < np
-// (pm: the particle mass the FP64 loops leave out of their pair terms, applied
-// to every sum but d(rho)/dt's, which the finish multiplies; 1 for the mixed form)
-template <bool IND, bool SCALE, class Get>
+// (pm: the particle mass, left out of the pair terms, applied to every sum but
+// d(rho)/dt's, which the finish multiplies)
+template <bool IND, class Get>
 __device__ __forceinline__ void store_pair_sums(PairSmem &sm, int lane, int np, int S, int s0, unsigned am,
                                                 double *psum, int64_t ps, double pm, Get get) {
   constexpr int RW = IND ? NF + 2 : NF + 1;
@@ -499,7 +500,7 @@ __device__ __forceinline__ void store_pair_sums(PairSmem &sm, int lane, int np, 
       if (IND) nb = fmax(nb, src[NF + 1]);
     }
     const size_t ip = (size_t)(s0 + (IND ? cell_pos(am, lane) : lane));
-    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = SCALE && k != 4 ? pm * fs[k] : fs[k];
+    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = k != 4 ? pm * fs[k] : fs[k];
     psum[FSLOT_VSIG * ps + ip] = vsm;
     if (IND) psum[FSLOT_NBIN * ps + ip] = nb;
   }
@@ -585,13 +586,13 @@ __device__ __forceinline__ void far_pair_fp64(double dx, double dy, double dz, d
 }
 
 // One trial pair (i, j) of compute_forces (force.F90:914-2060) in FP64 with the
-// reference's neighbour test and cached-position rule; n is j's position in
-// i's trial list. The i-side sums (without the particle mass) go to f,
+// reference's neighbour test and cached-position rule (code, as separation_fp64
+// takes it). The i-side sums (without the particle mass) go to f,
 // vsigmax / nbi. With SYM the pair's contribution to j's own sums (j's force
 // loop over i, the same pair term seen from j) is returned in jv; it is only
 // requested for pairs without gravity and with global timesteps.
 template <bool MHD, bool GRAV, bool IND, bool SYM>
-__device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I, int n, int j, int code,
+__device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I, int j, int code,
                                                 const double *tx, const double *ty, const double *tz,
                                                 const double *jrec, const double *jmhd,
                                                 const int8_t *ibin_old_t, unsigned char *wakemark,
@@ -599,7 +600,7 @@ __device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I,
                                                 double (&jv)[NJS<MHD>::n]) {
   const bool adiab = !p.isothermal;
   double dx, dy, dz;
-  separation_fp64(p, I.x, I.y, I.z, j, code | (n < CELLCACHE ? QC_CACHED : 0), tx, ty, tz, dx, dy, dz);
+  separation_fp64(p, I.x, I.y, I.z, j, code, tx, ty, tz, dx, dy, dz);
   const double *rj = jrec + JREC * (size_t)j;
   const double hj1 = rj[JR_H1];
   // With self-gravity the direction of a neighbour pair keeps the reference's
@@ -740,13 +741,114 @@ __device__ __forceinline__ void force_pair_fp64(const Params &p, const IFp64 &I,
   }
 }
 
-template <bool MHD, bool GRAV, bool IND>
+// Start of the per-side pair kernels: the cell of a warp, its active particles
+// (IND: individual timesteps, inactive ones keep their forces) and the trial
+// statistics. Returns false where the warp has nothing to do.
+struct PairCell {
+  int cell, s0, np, off, nleaf;
+  unsigned am;
+  float4 cc;  // centre, size
+};
+template <bool IND>
+__device__ __forceinline__ bool pair_cell(PairCell &c, const Node *nodes, const int *leaves, int ncell,
+                                          const int *cells, const int *cell_off, const int *cell_nleaf,
+                                          const unsigned char *actf, const ForceOut &out, int *err) {
+  const int a = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = lane_id();
+  if (a >= ncell) return false;
+  c.cell = cells ? cells[a] : a;
+  const Node nd = nodes[leaves[c.cell]];
+  c.np = nd.count; c.s0 = nd.start; c.am = 0u;
+  if (c.np < 1 || c.np > MAXCELL) { if (lane == 0) set_error(err, PH_ERR_TREE); return false; }
+  if (IND) c.am = cell_active_mask(actf, c.s0, nd.count, c.np);
+  if (c.np == 0) return false;
+  c.off = cell_off[c.cell]; c.nleaf = cell_nleaf[c.cell];
+  c.cc = make_float4((float)nd.x, (float)nd.y, (float)nd.z, (float)nd.size);
+  if (lane == 0) {
+    atomicAdd(&out.stats[8], (unsigned long long)out.cell_ntrial[c.cell]);
+    atomicAdd(&out.stats[10], (unsigned long long)c.np * (unsigned long long)out.cell_ntrial[c.cell]);
+  }
+  return true;
+}
+
+// totals of a cell -> psum: value k of particle il at idx = k np + il; the
+// particle mass, left out of the pair terms, applied to every sum but
+// d(rho)/dt's (which the finish multiplies) and the maxima
+template <bool MHD, int NR>
+__device__ __forceinline__ void store_totals(const ListBase &sm, int nv, int np, double pm, const double (&tot)[NR],
+                                             double *psum, int64_t ps) {
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane_id() + 32 * r;
+    if (idx < nv * np) {
+      const int k = idx / np, slot = k < NJS<MHD>::n ? njs_slot(k, MHD) : FSLOT_NBIN;
+      psum[slot * ps + sm.ipos[idx - k * np]] = slot == 4 || slot >= NF ? tot[r] : pm * tot[r];
+    }
+  }
+}
+
+// FP64 pairs from each side, without self-gravity: individual timesteps, and
+// global ones when the symmetric loop is switched off
+template <bool MHD, bool IND>
 __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
-    const int *cell_nleaf, const int *perm, const double *tx, const double *ty, const double *tz, const double *th,
-    const float4 *txf, const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin,
-    const int *cells, const unsigned char *actf, const int8_t *ibin_old_t,
-    unsigned char *wakemark, int *err) {
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const double *th, const float4 *txf,
+    const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin, const int *cells,
+    const unsigned char *actf, const int8_t *ibin_old_t, unsigned char *wakemark, int *err) {
+  constexpr int NV = NJS<MHD>::n + (IND ? 1 : 0), NR = (NV * MAXCELL + 31) / 32, VS = NJS<MHD>::n - 1;
+  PairCell c;
+  if (!pair_cell<IND>(c, nodes, leaves, ncell, cells, cell_off, cell_nleaf, actf, out, err)) return;
+  extern __shared__ __align__(16) unsigned char dsm[];
+  ListSmem &sm = reinterpret_cast<ListSmem *>(dsm)[threadIdx.x >> 5];
+  const int lane = lane_id(), np = c.np;
+  const float q2lim = 4.0f * 1.001f, INF = __int_as_float(0x7f800000);
+  const float pf_hf = __double2float_ru(pf_hmin);
+  auto accept = [&](float h) { return h > pf_hf ? q2lim * (h * h) : INF; };
+  if (lane < np) {
+    const int ip = c.s0 + (IND ? cell_pos(c.am, lane) : lane);
+    float4 x = txf[ip];
+    x.w = accept(d2f_rn(th[ip]));
+    sm.xi[lane] = x;
+    sm.ipos[lane] = ip;
+  }
+  const int qstride = LQ / np;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  ListPos pos;
+  __syncwarp();
+  bool more = true;
+  while (more) {
+    int myc;
+    more = SWEEP_END != sweep_list<false, 32>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
+                                              [&](float h1) { return accept(__frcp_rn(h1)); });
+    const QueueLanes ql = balance_queues(np, myc, sm);
+    const int il = max(ql.il, 0);
+    const IFp64 I = ifp64_init<MHD, false>(p, sm.ipos[il], tx, ty, tz, jrec, jmhd);
+    double f[NF];
+    for (int k = 0; k < NF; ++k) f[k] = 0.0;
+    long long vsigmax = 0;  // largest signal speed (bit pattern)
+    int nbi = 0;            // largest ibin_old of the SPH neighbours (individual timesteps)
+    double jv[NJS<MHD>::n];
+    for (int m = ql.m0; m < ql.c; m += ql.step)
+      force_pair_fp64<MHD, false, IND, false>(p, I, sm.qj[il * qstride + m], sm.qc[il * qstride + m], tx, ty, tz, jrec,
+                                              jmhd, ibin_old_t, wakemark, f, vsigmax, nbi, jv);
+    static_assert(32 * NV <= LQ / 2, "lane sums staged in the queues' space");
+    flush_lanes<NV>(np, sm, sm.red, tot,
+        [&](int k) -> double {
+          return k < VS ? f[njs_slot(k, MHD)] : (k == VS ? __longlong_as_double(vsigmax) : (double)nbi);
+        },
+        [](int k, double s, double v) -> double { return k < VS ? s + v : fmax_pos(s, v); });
+  }
+  store_totals<MHD>(sm, NV, np, p.massoftype, tot, psum, ps);
+}
+
+// FP64 pairs with self-gravity. The trial lists are long (thousands of
+// particles at theta 0.5) and nearly all of it is far pairs, evaluated where
+// they are tested: a lane per (particle, stripe) keeps their sums in registers.
+template <bool MHD, bool IND>
+__global__ void __launch_bounds__(32 * MAX_WARPS) k_force_grav(
+    Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const double *th, const float4 *txf,
+    const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin, const int *cells,
+    const unsigned char *actf, const int8_t *ibin_old_t, unsigned char *wakemark, int *err) {
   const int w = threadIdx.x >> 5, lane = lane_id();
   const int a = blockIdx.x * (blockDim.x >> 5) + w;
   if (a >= ncell) return;
@@ -764,7 +866,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
   const bool act = lane < np * S;
   const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
   const int i = s0 + (IND ? cell_pos(am, il) : il);
-  const IFp64 I = ifp64_init<MHD, GRAV>(p, i, tx, ty, tz, jrec, jmhd);
+  const IFp64 I = ifp64_init<MHD, true>(p, i, tx, ty, tz, jrec, jmhd);
   const float4 xif = txf[i];
   const float hi21f = xif.w * xif.w;
   const bool pf_i = th[i] > pf_hmin;
@@ -798,7 +900,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
       }
       const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
       const bool near = r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
-      if (!GRAV || near) return near;
+      if (near) return true;
       // self-gravity: a trial pair provably outside both kernels (most of the
       // list) takes its 1/r^2 term here, in the dense test sweep, without being
       // queued with its record
@@ -810,12 +912,12 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
     };
     auto body = [&](int k) {
       double jv[NJS<MHD>::n];
-      force_pair_fp64<MHD, GRAV, IND, false>(p, I, base + k, stg.jidx[k], stg.code[k], tx, ty, tz, jrec, jmhd,
-                                             ibin_old_t, wakemark, f, vsigmax, nbi, jv);
+      force_pair_fp64<MHD, true, IND, false>(p, I, stg.jidx[k], stg.code[k] | (base + k < CELLCACHE ? QC_CACHED : 0), tx,
+                                             ty, tz, jrec, jmhd, ibin_old_t, wakemark, f, vsigmax, nbi, jv);
     };
     queue_window(cnt, S, act, il, stripe, sm.q, test, body);
   }
-  store_pair_sums<IND, true>(sm, lane, np, S, s0, am, psum, ps, p.massoftype, [&](int q) -> double {
+  store_pair_sums<IND>(sm, lane, np, S, s0, am, psum, ps, p.massoftype, [&](int q) -> double {
     return q < NF ? f[q] : (q == NF ? __longlong_as_double(vsigmax) : (double)nbi);
   });
 }
@@ -842,44 +944,52 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
 // neighbour tests are those of force_pair_fp64 (the reference's rounding and
 // cached-position rule from the evaluating cell's list); seen from j they differ
 // from the reference's own evaluation by rounding only.
-constexpr int STAGE_S = 128;
-template <bool MHD>
-struct SymSmem {
-  union {
-    StageN<STAGE_S> st;
-    double red[32 * (NF + 1)];
-  } u;
-  PairQ q;
-  double js[NJS<MHD>::n][STAGE_S];
+//
+// Work: the list sweep per batch of SYM_BL leaf entries (ph_walk.cuh), each
+// batch drained with the lanes dealt out by queue length. The j-side array of a
+// batch (NJ values of up to SYM_BL leaves) bounds the warps per SM: 24 entries
+// hold the owned half of most lists (37 entries at hfact 1.2) in one batch and
+// leave room for 11 warps at the reference's leaf size. One warp per block: the
+// SM's shared memory then fills in the smallest steps (measured per launch at
+// 64^3, hydro / MHD: 1, 2, 4 warps per block 1.88 / 3.66, 1.95 / 3.98, 2.20 /
+// 5.48 ms; batches of 16 entries 1.96 / 3.72 ms at one warp; the
+// lane-per-stripe loop before this one 2.45 / 4.46 ms).
+constexpr int SYM_BL = 24;
+struct SymSmem : ListSmemK {
+  // js[NJ][jw] doubles follow, jw = SYM_BL x leaf size
+  __device__ __forceinline__ double *js() { return reinterpret_cast<double *>(this + 1); }
 };
+template <bool MHD>
+__host__ __device__ constexpr int sym_smem_bytes(int minpart) {
+  return (int)sizeof(SymSmem) + 8 * NJS<MHD>::n * SYM_BL * minpart;
+}
 
 template <bool MHD>
-__global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
+__global__ void __launch_bounds__(32) k_force_sym(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const double *th,
-    const float4 *txf, const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin, const int *toff, double *jbuf, int64_t jstride, int *err) {
+    const float4 *txf, const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin,
+    const int *toff, double *jbuf, int64_t jstride, int *err) {
   constexpr int NJ = NJS<MHD>::n;
   const unsigned FULL = 0xffffffffu;
-  const int w = threadIdx.x >> 5, lane = lane_id();
-  const int cell = blockIdx.x * (blockDim.x >> 5) + w;
+  const int lane = lane_id(), cell = blockIdx.x;
   if (cell >= ncell) return;
   const Node nd = nodes[leaves[cell]];
   const int np = nd.count, s0 = nd.start;
-  if (np < 1 || np > MAXCELL) { if (lane == 0) set_error(err, PH_ERR_TREE); return; }
-  const int S = 32 / np;
-  const bool act = lane < np * S;
-  const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
-  const int i = s0 + il;
-  const IFp64 I = ifp64_init<MHD, false>(p, i, tx, ty, tz, jrec, jmhd);
-  const float4 xif = txf[i];
-  const float hi21f = xif.w * xif.w;
-  const bool pf_i = th[i] > pf_hmin;
-  const float q2lim = 4.0f * 1.001f;
-  const float pf_h1max = (float)(1.0 / pf_hmin);
-  double f[NF];
-  for (int k = 0; k < NF; ++k) f[k] = 0.0;
-  long long vsigmax = 0;  // largest signal speed (bit pattern)
-  int nbi = 0;
+  if (np < 1 || np > MAXCELL || np > p.minpart) { if (lane == 0) set_error(err, PH_ERR_TREE); return; }
+  extern __shared__ __align__(16) unsigned char dsm[];
+  SymSmem &sm = *reinterpret_cast<SymSmem *>(dsm);
+  double *js = sm.js();
+  const int jw = SYM_BL * p.minpart;
+  const float q2lim = 4.0f * 1.001f, INF = __int_as_float(0x7f800000);
+  const float pf_hf = __double2float_ru(pf_hmin);
+  if (lane < np) {
+    float4 x = txf[s0 + lane];
+    const float hf = d2f_rn(th[s0 + lane]);
+    x.w = hf > pf_hf ? q2lim * (hf * hf) : INF;
+    sm.xi[lane] = x;
+    sm.ipos[lane] = s0 + lane;
+  }
   const int off = cell_off[cell], nleaf = cell_nleaf[cell];
   // the owned prefix of the list: entries starting at or after s0
   int nown = 0, town = 0;
@@ -897,107 +1007,82 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_sym(
     atomicAdd(&out.stats[10], (unsigned long long)np * (unsigned long long)town);
   }
   const int64_t tb = (int64_t)toff[off];  // flattened trial index of the list's first entry
-  extern __shared__ __align__(16) unsigned char dsm[];
-  SymSmem<MHD> &sm = reinterpret_cast<SymSmem<MHD> *>(dsm)[w];
-  StageN<STAGE_S> &stg = sm.u.st;
-  const unsigned gmask = !act ? 0u : (S >= 32 ? FULL : (((1u << S) - 1u) << (il * S)));
+  const float4 cc = make_float4((float)nd.x, (float)nd.y, (float)nd.z, (float)nd.size);
+  const int qstride = LQ / np;
   const unsigned lt = (1u << lane) - 1u;
-  for (int base = 0; base < town; base += STAGE_S) {
-    const int cnt = stage_window_n<STAGE_S>(p, pool, off, nown, town, base, txf, stg);
-    for (int q = lane; q < NJ * STAGE_S; q += 32) (&sm.js[0][0])[q] = 0.0;
+  // totals per (value, particle): f[0..2], f[4..6], with MHD f[7..11], the signal speed
+  constexpr int NR = (NJ * MAXCELL + 31) / 32;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  for (int q = lane; q < NJ * jw; q += 32) js[q] = 0.0;
+  ListPos pos;
+  while (true) {
     __syncwarp();
-    auto test = [&](int k) -> bool {
-      const int j = stg.jidx[k];
-      if (j <= i && j >= s0) return false;  // own leaf: each pair once (j > i); the self pair never
-      if (!pf_i) return true;
-      const float4 xj = stg.pos[k];
-      if (xj.w >= pf_h1max) return true;
-      float dxf = xif.x - xj.x, dyf = xif.y - xj.y, dzf = xif.z - xj.z;
-      if (p.periodic) {
-        if (fabsf(dxf) > 0.5f * p.dxboundf) dxf -= copysignf(p.dxboundf, dxf);
-        if (fabsf(dyf) > 0.5f * p.dyboundf) dyf -= copysignf(p.dyboundf, dyf);
-        if (fabsf(dzf) > 0.5f * p.dzboundf) dzf -= copysignf(p.dzboundf, dzf);
-      }
-      const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
-      return r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
-    };
-    // the test sweep and per-particle queues of queue_window; the drain runs
-    // in warp-uniform steps so that lanes holding the same j can be combined
-    const int nr = (cnt + S - 1) / S;
-    int qn = 0;
-    for (int r = 0; r < nr; ++r) {
-      const int k = r * S + stripe;
-      const bool ok = act && k < cnt && test(k);
-      const unsigned b = __ballot_sync(FULL, ok);
-      if (ok) sm.q.k[il][qn + __popc(b & gmask & lt)] = (unsigned short)k;
-      qn += __popc(b & gmask);
-      if (r == nr - 1 || (int)__reduce_max_sync(FULL, (unsigned)qn) > QCAP - S) {
-        __syncwarp();
-        const int nst = (act && qn > stripe) ? (qn - stripe + S - 1) / S : 0;
-        const int nstmax = (int)__reduce_max_sync(FULL, (unsigned)nst);
-        // the particles of a cell accept nearly the same j in nearly the same
-        // order, so aligned queues would put the same j in many lanes at once;
-        // each particle starts at its own rotation of its queue instead
-        const int rot = act && qn > 0 ? (il * qn) / np : 0;
-        for (int t = 0; t < nstmax; ++t) {
-          int m = stripe + t * S + rot;
-          if (m >= qn) m -= qn;
-          const bool valid = t < nst;
-          const int kk = valid ? (int)sm.q.k[il][m] : -1;
-          double jv[NJ];
-          for (int v = 0; v < NJ; ++v) jv[v] = 0.0;
-          if (valid)
-            force_pair_fp64<MHD, false, false, true>(p, I, base + kk, stg.jidx[kk], stg.code[kk], tx, ty, tz, jrec,
-                                                     jmhd, nullptr, nullptr, f, vsigmax, nbi, jv);
-          // lanes holding the same j: the lowest adds the others' values in
-          // lane order, then adds the group's sum to j's window slot
-          const unsigned g = __match_any_sync(FULL, valid ? kk : -1 - lane);
-          const int gs = __popc(g);
-          const int gmax = (int)__reduce_max_sync(FULL, (unsigned)gs);
-          const bool lead = valid && (g & lt) == 0u;
-          for (int u = 1; u < gmax; ++u) {
-            const int src = u < gs ? (int)__fns(g, 0, u + 1) : lane;
-            for (int v = 0; v < NJ - 1; ++v) {
-              const double y = __shfl_sync(FULL, jv[v], src);
-              if (lead && u < gs) jv[v] += y;
-            }
-            const double y = __shfl_sync(FULL, jv[NJ - 1], src);
-            if (lead && u < gs) jv[NJ - 1] = fmax_pos(jv[NJ - 1], y);
-          }
-          if (lead) {
-            for (int v = 0; v < NJ - 1; ++v) sm.js[v][kk] += jv[v];
-            sm.js[NJ - 1][kk] = fmax_pos(sm.js[NJ - 1][kk], jv[NJ - 1]);
-          }
-          __syncwarp();
+    int myc;
+    const int st = sweep_list<true, SYM_BL>(p, cc, np, pool, off, nown, txf, sm, qstride, pos, myc, [&](float h1) {
+      const float hj = __frcp_rn(h1);
+      return hj > pf_hf ? q2lim * (hj * hj) : INF;
+    });
+    if (st == SWEEP_END) break;
+    const QueueLanes ql = balance_queues(np, myc, sm);
+    const int il = max(ql.il, 0);
+    const IFp64 I = ifp64_init<MHD, false>(p, s0 + il, tx, ty, tz, jrec, jmhd);
+    double f[NF];
+    for (int k = 0; k < NF; ++k) f[k] = 0.0;
+    long long vsigmax = 0;  // largest signal speed (bit pattern)
+    int nbi = 0;
+    const unsigned short *qj = sm.qj + il * qstride;
+    const int nst = ql.c > ql.m0 ? (ql.c - ql.m0 + ql.step - 1) / ql.step : 0;
+    const int nstmax = (int)__reduce_max_sync(FULL, (unsigned)nst);
+    // the particles of a cell accept nearly the same j in nearly the same
+    // order, so aligned queues would put the same j in many lanes at once;
+    // each particle starts at its own rotation of its queue instead
+    const int rot = ql.c > 0 ? (il * ql.c) / np : 0;
+    for (int t = 0; t < nstmax; ++t) {
+      const bool valid = t < nst;
+      int m = ql.m0 + t * ql.step + rot;
+      if (m >= ql.c) m -= ql.c;
+      const int kk = valid ? (int)qj[m] : -1;
+      double jv[NJ];
+      for (int v = 0; v < NJ; ++v) jv[v] = 0.0;
+      if (valid)
+        force_pair_fp64<MHD, false, false, true>(p, I, sm.j[kk], sm.code[kk], tx, ty, tz, jrec, jmhd, nullptr, nullptr,
+                                                 f, vsigmax, nbi, jv);
+      // lanes holding the same j: the lowest adds the others' values in
+      // lane order, then adds the group's sum to j's batch slot
+      const unsigned g = __match_any_sync(FULL, valid ? kk : -1 - lane);
+      const int gs = __popc(g);
+      const int gmax = (int)__reduce_max_sync(FULL, (unsigned)gs);
+      const bool lead = valid && (g & lt) == 0u;
+      for (int u = 1; u < gmax; ++u) {
+        const int src = u < gs ? (int)__fns(g, 0, u + 1) : lane;
+        for (int v = 0; v < NJ - 1; ++v) {
+          const double y = __shfl_sync(FULL, jv[v], src);
+          if (lead && u < gs) jv[v] += y;
         }
-        qn = 0;
+        const double y = __shfl_sync(FULL, jv[NJ - 1], src);
+        if (lead && u < gs) jv[NJ - 1] = fmax_pos(jv[NJ - 1], y);
       }
+      if (lead) {
+        for (int v = 0; v < NJ - 1; ++v) js[v * jw + kk] += jv[v];
+        js[(NJ - 1) * jw + kk] = fmax_pos(js[(NJ - 1) * jw + kk], jv[NJ - 1]);
+      }
+      __syncwarp();
     }
-    __syncwarp();
-    // this window's j-side sums -> jbuf (value-major, flattened trial index)
-    for (int v = 0; v < NJ; ++v)
-      for (int k = lane; k < cnt; k += 32) jbuf[(int64_t)v * jstride + tb + base + k] = sm.js[v][k];
-    __syncwarp();
+    // j-side sums of a finished batch -> jbuf (value-major, flattened trial index)
+    if (st == SWEEP_BATCH)
+      for (int v = 0; v < NJ; ++v)
+        for (int k = lane; k < pos.cnt; k += 32) jbuf[(int64_t)v * jstride + tb + pos.nbase + k] = js[v * jw + k];
+    static_assert(NJ <= 12, "lane sums staged in the queues' space");
+    flush_lanes<NJ>(np, sm, sm.red, tot,
+        [&](int k) -> double {
+          return k == NJ - 1 ? __longlong_as_double(vsigmax) : f[njs_slot(k, MHD)];
+        },
+        [](int k, double s, double v) -> double { return k == NJ - 1 ? fmax_pos(s, v) : s + v; });
+    if (st == SWEEP_BATCH)
+      for (int q = lane; q < NJ * jw; q += 32) js[q] = 0.0;
   }
-  // the stripes of each particle in stripe order (store_pair_sums)
-  constexpr int RW = NF + 1;
-  double *red = sm.u.red;
-  __syncwarp();
-  for (int k = 0; k < RW; ++k) red[lane * RW + k] = k < NF ? f[k] : __longlong_as_double(vsigmax);
-  __syncwarp();
-  if (lane < np) {
-    double fs[NF];
-    for (int k = 0; k < NF; ++k) fs[k] = 0.0;
-    double vsm = 0.0;
-    for (int q = 0; q < S; ++q) {
-      const double *src = red + (lane * S + q) * RW;
-      for (int k = 0; k < NF; ++k) fs[k] += src[k];
-      vsm = fmax(vsm, src[NF]);
-    }
-    const size_t ip = (size_t)(s0 + lane);
-    for (int k = 0; k < NF; ++k) psum[k * ps + ip] = k == 4 ? fs[k] : p.massoftype * fs[k];
-    psum[FSLOT_VSIG * ps + ip] = vsm;
-  }
+  store_totals<MHD>(sm, NJ, np, p.massoftype, tot, psum, ps);
 }
 
 // Per leaf cell B: add to its particles' pair sums the j-side contributions
@@ -1153,228 +1238,233 @@ __device__ __forceinline__ void kernel_softeningf(float q2, float q, float &pot,
 }
 
 
+// The i-side quantities of the mixed pair loop for tree position i (its FP32
+// record, positions as two floats).
+template <bool MHD>
+struct IMix {
+  float h1, rho, c, pro2, vw, P, au, K, vx, vy, vz, u, gs, ab, avw, r21;
+  float bx, by, bz, cl;
+  Sep2 s;
+};
+template <bool MHD>
+__device__ __forceinline__ IMix<MHD> imix_init(int i, const float4 *txf, const float4 *txl, const float *jrecf,
+                                               const float *jmhdf) {
+  IMix<MHD> I;
+  const float4 *r4 = reinterpret_cast<const float4 *>(jrecf + JRECF * (size_t)i);
+  const float4 a = r4[0], b = r4[1], c = r4[2], d = r4[3];
+  I.h1 = a.x; I.rho = a.y; I.c = a.z; I.pro2 = a.w; I.vw = b.x; I.P = b.y; I.au = b.z; I.K = b.w;
+  I.vx = c.x; I.vy = c.y; I.vz = c.z; I.u = c.w; I.gs = d.x; I.ab = d.y; I.avw = d.z; I.r21 = d.w;
+  // start_cell takes 1/Omega = 1 where the stored value is not positive
+  if (!(I.K > 0.0f)) I.K = (I.h1 * I.h1) * (I.h1 * I.h1) * (float)CNORMK;
+  I.bx = I.by = I.bz = I.cl = 0.0f;
+  if (MHD) {
+    const float *m = jmhdf + JMHDF * (size_t)i;
+    I.bx = m[JM_BX]; I.by = m[JM_BY]; I.bz = m[JM_BZ]; I.cl = m[JM_CL];
+  }
+  I.s = sep2_init(txf, txl, i);
+  return I;
+}
+
+// the plain 1/r^2 of a trial pair outside both kernels (force.F90:1991-2053)
+__device__ __forceinline__ void far_pair_mixed(float dx, float dy, float dz, float r2, Kahan (&f)[NF]) {
+  const float y = rsqrt_nr(r2), y3 = y * y * y;
+  f[0].add(-dx * y3); f[1].add(-dy * y3); f[2].add(-dz * y3);
+  f[3].add(-y);
+}
+
+// One trial pair of compute_forces (force.F90:914-2060) in FP32 (sums without
+// the particle mass)
 template <bool MHD, bool GRAV, bool IND>
+__device__ __forceinline__ void force_pair_mixed(const Params &p, const IMix<MHD> &I, int j, int code,
+                                                 const float4 *txf, const float4 *txl, const double *tx,
+                                                 const double *ty, const double *tz, const float *jrecf,
+                                                 const float *jmhdf, const int8_t *ibin_old_t,
+                                                 unsigned char *wakemark, Kahan (&f)[NF], float &vsigmax, int &nbi) {
+  const bool adiab = !p.isothermal;
+  const float beta = (float)p.beta;
+  const float4 *r4 = reinterpret_cast<const float4 *>(jrecf + JRECF * (size_t)j);
+  const float4 ra = r4[0], rb = r4[1], rc = r4[2], rd = r4[3];
+  float dx, dy, dz, rij2;
+  separation_2f(p, I.s, j, code, txf[j], txl[j], tx, ty, tz, dx, dy, dz, rij2);
+  const float hj1 = ra.x;
+  const float q2i = rij2 * (I.h1 * I.h1), q2j = rij2 * (hj1 * hj1);
+  const bool qi_in = q2i < 4.0f, qj_in = q2j < 4.0f;
+  if (!(qi_in || qj_in)) {
+    if (GRAV) far_pair_mixed(dx, dy, dz, rij2, f);
+    return;
+  }
+  if (IND) {  // force.F90:1346-1353: j is woken for the next step; the limiter's neighbour bin
+    wakemark[j] = 1;
+    nbi = max(nbi, (int)ibin_old_t[j]);
+  }
+  // coincident particles: no direction, rij1 = 0 (force.F90:1293-1298)
+  const float rij1 = rij2 > TINY_F ? rsqrt_nr(rij2) : 0.0f;
+  const float rij = rij2 * rij1;
+  const float qi = rij * I.h1, qj = rij * hj1;
+  const float gi = qi_in ? grkernf(qi) * I.K : 0.0f, gj = qj_in ? grkernf(qj) * rb.w : 0.0f;
+  float fgrav = 0.0f;
+  if (GRAV) {
+    const float y2 = rij1 * rij1;
+    float phii = -rij1, fgi = y2, fgj = y2;
+    if (qi_in) {
+      float fmi;
+      kernel_softeningf(q2i, qi, phii, fmi);
+      phii *= I.h1;
+      fgi = fmi * (I.h1 * I.h1) + I.gs * gi;
+    }
+    if (qj_in) {
+      float phij, fmj;
+      kernel_softeningf(q2j, qj, phij, fmj);
+      fgj = fmj * (hj1 * hj1) + rd.x * gj;
+    }
+    fgrav = 0.5f * (fgi + fgj);
+    f[3].add(phii);
+  }
+  const float nx = dx * rij1, ny = dy * rij1, nz = dz * rij1;
+  // j's terms enter when q_j < 2, or always with MHD or an energy equation
+  const bool usej = MHD || (adiab && !GRAV) || qj_in;
+  const float dvx = I.vx - rc.x, dvy = I.vy - rc.y, dvz = I.vz - rc.z;
+  const float pv = dvx * nx + dvy * ny + dvz * nz;
+  vsigmax = fmaxf(vsigmax, I.vw - beta * pv);  // starts at 0
+  if (usej) vsigmax = fmaxf(vsigmax, rb.x - beta * pv);
+  float qri = 0.0f, qrj = 0.0f;
+  if (pv < 0.0f) {
+    qri = I.c * fmaxf(I.avw - beta * pv, 0.0f) * pv;
+    if (usej) qrj = ra.z * fmaxf(rd.z - beta * pv, 0.0f) * pv;
+    if (adiab) f[5].add(qri * pv * gi);
+  }
+  const float gradp = (I.pro2 + qri) * gi + (usej ? (ra.w + qrj) * gj : 0.0f) + fgrav;
+  if (adiab) {
+    const float vsigu = GRAV ? fabsf(pv) : sqrt_nr(fabsf(I.P - rb.y) * __fdividef(2.0f, I.rho + ra.y));
+    f[6].add(vsigu * (I.u - rc.w) * (I.au * gi + (usej ? rb.z * gj : 0.0f)));
+  }
+  float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+  if (MHD) {
+    const float4 mj = *reinterpret_cast<const float4 *>(jmhdf + JMHDF * (size_t)j);
+    const float clj = jmhdf[JMHDF * (size_t)j + JM_CL];
+    const float dBx = I.bx - mj.x, dBy = I.by - mj.y, dBz = I.bz - mj.z;
+    const float projBi = I.bx * nx + I.by * ny + I.bz * nz;
+    const float projBj = mj.x * nx + mj.y * ny + mj.z * nz;
+    const float projdB = dBx * nx + dBy * ny + dBz * nz;
+    f[11].add(-projdB * gi);
+    const float tx_ = dvx - pv * nx, ty_ = dvy - pv * ny, tz_ = dvz - pv * nz;
+    const float vsigB = sqrt_nr(tx_ * tx_ + ty_ * ty_ + tz_ * tz_);
+    const float dBdiss = (I.ab * gi + rd.y * gj) * vsigB;
+    if (p.iresistive_heating > 0 && adiab) f[5].add(-0.5f * (dBx * dBx + dBy * dBy + dBz * dBz) * dBdiss);
+    const float pmi = I.r21 * gi, pmj = rd.w * gj;
+    const float ti = pmi * projBi, tj = pmj * projBj;
+    f[7].add(ti + tj);
+    const float dpsi = pmi * I.cl + pmj * clj;
+    f[8].add(-ti * dvx + dBdiss * dBx - dpsi * nx);
+    f[9].add(-ti * dvy + dBdiss * dBy - dpsi * ny);
+    f[10].add(-ti * dvz + dBdiss * dBz - dpsi * nz);
+    // anisotropic stress: -(S_i.n gi + S_j.n gj) with S = -(B/rho)(B/rho)
+    sx = ti * I.bx + tj * mj.x; sy = ti * I.by + tj * mj.y; sz = ti * I.bz + tj * mj.z;
+  }
+  f[0].add(MHD ? sx - nx * gradp : -nx * gradp);
+  f[1].add(MHD ? sy - ny * gradp : -ny * gradp);
+  f[2].add(MHD ? sz - nz * gradp : -nz * gradp);
+  f[4].add(pv * gi);
+}
+
+template <bool MHD, bool IND>
 __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
-    const int *cell_nleaf, const int *perm, const double *tx, const double *ty, const double *tz, const double *th,
-    const float4 *txf, const double *jrec, const double *jmhd, const float *jrecf, const float *jmhdf,
-    const double *eos_t, ForceOut out, double *psum, int64_t ps, const int *cells, const unsigned char *actf, const int8_t *ibin_old_t,
-    unsigned char *wakemark, int *err) {
-  const int w = threadIdx.x >> 5, lane = lane_id();
-  const int a = blockIdx.x * (blockDim.x >> 5) + w;
-  if (a >= ncell) return;
-  const int cell = cells ? cells[a] : a;  // individual timesteps: the cells holding active particles
-  const Node nd = nodes[leaves[cell]];
-  const int np_all = nd.count, s0 = nd.start;
-  if (np_all < 1 || np_all > MAXCELL) { if (lane == 0) set_error(err, PH_ERR_TREE); return; }
-  // individual timesteps (IND): the cell's active particles take the lanes;
-  // inactive ones keep their forces
-  int np = np_all;
-  unsigned am = 0u;
-  if (IND) am = cell_active_mask(actf, s0, np_all, np);
-  if (np == 0) return;
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
+    const float *jrecf, const float *jmhdf, ForceOut out, double *psum, int64_t ps, const int *cells,
+    const unsigned char *actf, const int8_t *ibin_old_t, unsigned char *wakemark, int *err) {
+  constexpr int NV = NJS<MHD>::n + (IND ? 1 : 0), NR = (NV * MAXCELL + 31) / 32, VS = NJS<MHD>::n - 1;
+  PairCell c;
+  if (!pair_cell<IND>(c, nodes, leaves, ncell, cells, cell_off, cell_nleaf, actf, out, err)) return;
+  extern __shared__ __align__(16) unsigned char dsm[];
+  ListSmem &sm = reinterpret_cast<ListSmem *>(dsm)[threadIdx.x >> 5];
+  const int lane = lane_id(), np = c.np;
+  const float q2lim = 4.0f * 1.001f;
+  if (lane < np) {
+    const int ip = c.s0 + (IND ? cell_pos(c.am, lane) : lane);
+    float4 x = txf[ip];
+    x.w = __fdividef(q2lim, x.w * x.w);
+    sm.xi[lane] = x;
+    sm.ipos[lane] = ip;
+  }
+  const int qstride = LQ / np;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  ListPos pos;
+  __syncwarp();
+  bool more = true;
+  while (more) {
+    int myc;
+    more = SWEEP_END != sweep_list<false, 32>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
+                                              [&](float h1) { return __fdividef(q2lim, h1 * h1); });
+    const QueueLanes ql = balance_queues(np, myc, sm);
+    const int il = max(ql.il, 0);
+    const IMix<MHD> I = imix_init<MHD>(sm.ipos[il], txf, txl, jrecf, jmhdf);
+    Kahan f[NF];
+    float vsigmax = 0.0f;
+    int nbi = 0;
+    for (int m = ql.m0; m < ql.c; m += ql.step)
+      force_pair_mixed<MHD, false, IND>(p, I, sm.qj[il * qstride + m], sm.qc[il * qstride + m] & 63, txf, txl, tx, ty,
+                                        tz, jrecf, jmhdf, ibin_old_t, wakemark, f, vsigmax, nbi);
+    static_assert(32 * NV <= LQ / 2, "lane sums staged in the queues' space");
+    flush_lanes<NV>(np, sm, sm.red, tot,
+        [&](int k) -> double { return k < VS ? f[njs_slot(k, MHD)].value() : (k == VS ? (double)vsigmax : (double)nbi); },
+        [](int k, double s, double v) -> double { return k < VS ? s + v : fmax_pos(s, v); });
+  }
+  store_totals<MHD>(sm, NV, np, p.massoftype, tot, psum, ps);
+}
+
+// Self-gravity: as k_force_grav, far pairs evaluated where they are tested.
+template <bool MHD, bool IND>
+__global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed_grav(
+    Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
+    const float *jrecf, const float *jmhdf, ForceOut out, double *psum, int64_t ps, const int *cells,
+    const unsigned char *actf, const int8_t *ibin_old_t, unsigned char *wakemark, int *err) {
+  PairCell c;
+  if (!pair_cell<IND>(c, nodes, leaves, ncell, cells, cell_off, cell_nleaf, actf, out, err)) return;
+  const int lane = lane_id(), np = c.np;
   const int S = 32 / np;
   const bool act = lane < np * S;
   const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
-  const int i = s0 + (IND ? cell_pos(am, il) : il);
-  const float pmf = (float)p.massoftype;
-  const bool adiab = !p.isothermal;
-  // i-side from the FP32 particle record (its density is rhoh(1/(1/h)) rather
-  // than rhoanddhdrho's m (hfact/h)^3: a last-ulp difference in FP64, nil in FP32)
-  const float *ri = jrecf + JRECF * (size_t)i;
-  const float hi1f = ri[0], hi21f = hi1f * hi1f;
-  const float gradhi = (ri[7] > 0.0f) ? ri[7] : 1.0f;
-  const float hfacgrkern = hi21f * hi21f * (float)CNORMK * gradhi;
-  const float gradsofti = GRAV ? ri[12] : 0.0f;
-  const float rhoif = ri[1], rho1if = ri[2], rho21i = ri[15], pro2if = ri[3], vwaveif = ri[4], prif = ri[5];
-  const float auterm = ri[6], avBterm = ri[13];
-  const float alphai = ri[14], beta = (float)p.beta, ocf = (float)p.overcleanfac;
-  const float vxi = ri[8], vyi = ri[9], vzi = ri[10], eni = ri[11];
-  float bxif = 0, byif = 0, bzif = 0, psiif = 0, sx[6] = {0, 0, 0, 0, 0, 0};
-  if (MHD) {
-    const float *mi = jmhdf + JMHDF * (size_t)i;
-    bxif = mi[0]; byif = mi[1]; bzif = mi[2]; psiif = mi[3];
-    for (int k = 0; k < 6; ++k) sx[k] = mi[4 + k];
-  }
-  const double xi = tx[i], yi = ty[i], zi = tz[i];
-  const float4 xif = txf[i];
-  const bool pf_i = !GRAV;
+  const int i = c.s0 + (IND ? cell_pos(c.am, il) : il);
+  const IMix<MHD> I = imix_init<MHD>(i, txf, txl, jrecf, jmhdf);
+  const float hi21f = I.h1 * I.h1;
   const float q2lim = 4.0f * 1.001f;
   const float hLx = 0.5f * p.dxboundf, hLy = 0.5f * p.dyboundf, hLz = 0.5f * p.dzboundf;
   Kahan f[NF];
   float vsigmax = 0.0f;
   int nbi = 0;
-  const int off = cell_off[cell], nleaf = cell_nleaf[cell];
-  if (lane == 0) {
-    atomicAdd(&out.stats[8], (unsigned long long)out.cell_ntrial[cell]);
-    atomicAdd(&out.stats[10], (unsigned long long)np * (unsigned long long)out.cell_ntrial[cell]);
-  }
-  const int ntrial = out.cell_ntrial[cell];
+  const int ntrial = out.cell_ntrial[c.cell];
   extern __shared__ __align__(16) unsigned char dsm[];
-  PairSmem &sm = reinterpret_cast<PairSmem *>(dsm)[w];
+  PairSmem &sm = reinterpret_cast<PairSmem *>(dsm)[threadIdx.x >> 5];
   Stage &stg = sm.st;
   for (int base = 0; base < ntrial; base += STAGE) {
-    const int cnt = stage_window(p, pool, off, nleaf, ntrial, base, txf, stg);
+    const int cnt = stage_window(p, pool, c.off, c.nleaf, ntrial, base, txf, stg);
     auto test = [&](int k) -> bool {
-      if (stg.jidx[k] == i) return false;
-      if (!pf_i && !GRAV) return true;
+      const int j = stg.jidx[k];
+      if (j == i) return false;
       const float4 xj = stg.pos[k];  // x, y, z (+ offset), 1/h
-      const float ux = xif.x - xj.x, uy = xif.y - xj.y, uz = xif.z - xj.z;
-      float dxf = ux, dyf = uy, dzf = uz;
+      float dxf = I.s.h.x - xj.x, dyf = I.s.h.y - xj.y, dzf = I.s.h.z - xj.z;
       if (p.periodic) {
         if (fabsf(dxf) > hLx) dxf -= copysignf(p.dxboundf, dxf);
         if (fabsf(dyf) > hLy) dyf -= copysignf(p.dyboundf, dyf);
         if (fabsf(dzf) > hLz) dzf -= copysignf(p.dzboundf, dzf);
       }
       const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
-      const bool near = r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
-      if (!GRAV || near) return near;
-      // self-gravity: a trial pair provably outside both kernels takes only
-      // the 1/r^2 term (force.F90:1991-2053, the body's else branch), formed
-      // here from the FP64 separation without queueing the pair
-      const int j = stg.jidx[k];
-      float dx, dy, dz;
-      separation_mixed(p, xi, yi, zi, tx[j], ty[j], tz[j], stg.code[k], ux, uy, uz, dx, dy, dz);
-      const float rij1 = rsqrt_nr(dx * dx + dy * dy + dz * dz);
-      const float fgj = rij1 * rij1 * rij1 * pmf;
-      f[0].add(-dx * fgj); f[1].add(-dy * fgj); f[2].add(-dz * fgj);
-      f[3].add(-pmf * rij1);
+      if (r2f * fminf(hi21f, xj.w * xj.w) < q2lim) return true;
+      const int code = stg.code[k];
+      float dx, dy, dz, r2;
+      separation_2f(p, I.s, j, code, code == 0 ? xj : txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
+      far_pair_mixed(dx, dy, dz, r2, f);
       return false;
     };
-    struct PF { int j, code; float4 xj; double x, y, z; float4 r0, r1, r2, r3; };
-    auto load = [&](int k) -> PF {
-      PF f;
-      f.j = stg.jidx[k]; f.code = stg.code[k]; f.xj = stg.pos[k];
-      f.x = tx[f.j]; f.y = ty[f.j]; f.z = tz[f.j];
-      const float4 *r4 = reinterpret_cast<const float4 *>(jrecf + JRECF * (size_t)f.j);
-      f.r0 = r4[0]; f.r1 = r4[1]; f.r2 = r4[2]; f.r3 = r4[3];
-      return f;
-    };
-    auto body = [&](const PF &pf) {
-      const int j = pf.j;
-      const float4 xj = pf.xj;
-      float dx, dy, dz;
-      separation_mixed(p, xi, yi, zi, pf.x, pf.y, pf.z, pf.code, xif.x - xj.x, xif.y - xj.y, xif.z - xj.z, dx,
-                       dy, dz);
-      const float rij2 = dx * dx + dy * dy + dz * dz;
-      const float rj[JRECF] = {pf.r0.x, pf.r0.y, pf.r0.z, pf.r0.w, pf.r1.x, pf.r1.y, pf.r1.z, pf.r1.w,
-                               pf.r2.x, pf.r2.y, pf.r2.z, pf.r2.w, pf.r3.x, pf.r3.y, pf.r3.z, pf.r3.w};
-      const float hj1 = rj[0];
-      const float hj21 = hj1 * hj1;
-      const float q2i = rij2 * hi21f, q2j = rij2 * hj21;
-      const bool qi_in = q2i < 4.0f, qj_in = q2j < 4.0f;
-      if (qi_in || qj_in) {
-        if (IND) {  // force.F90:1346-1353: j is woken for the next step; the limiter's neighbour bin
-          wakemark[j] = 1;
-          nbi = max(nbi, (int)ibin_old_t[j]);
-        }
-        // coincident particles: no direction, rij1 = 0 (force.F90:1293-1298)
-        const float rij1 = rij2 > TINY_F ? rsqrt_nr(rij2) : 0.0f;
-        const float rij = rij2 * rij1;
-        const float qi = rij * hi1f;
-        float grkerni = 0.0f, fgravi = 0.0f, phii = 0.0f;
-        if (qi_in) {
-          grkerni = grkernf(qi) * hfacgrkern;
-          if (GRAV) {
-            float fmi;
-            kernel_softeningf(q2i, qi, phii, fmi);
-            phii *= hi1f;
-            fgravi = fmi * hi21f + gradsofti * grkerni;
-          }
-        } else if (GRAV) {
-          phii = -rij1; fgravi = rij1 * rij1;
-        }
-        const float runix = dx * rij1, runiy = dy * rij1, runiz = dz * rij1;
-        float grkernj = 0.0f, fgravj = 0.0f;
-        bool usej;
-        if (qj_in) {
-          const float qj = rij * hj1;
-          grkernj = grkernf(qj) * (hj21 * hj21 * (float)CNORMK) * rj[7];
-          if (GRAV) {
-            float phij, fmj;
-            kernel_softeningf(q2j, qj, phij, fmj);
-            fgravj = fmj * hj21 + rj[12] * grkernj;
-          }
-          usej = true;
-        } else {
-          if (GRAV) fgravj = rij1 * rij1;
-          usej = false;
-        }
-        if (MHD) usej = true;
-        if (adiab && !GRAV) usej = true;
-        const float fgrav = 0.5f * pmf * (fgravi + fgravj);
-        const float dvx = vxi - rj[8], dvy = vyi - rj[9], dvz = vzi - rj[10];
-        const float projv = dvx * runix + dvy * runiy + dvz * runiz;
-        const float denij = adiab ? eni - rj[11] : 0.0f;
-        vsigmax = fmaxf(vsigmax, fmaxf(vwaveif - beta * projv, 0.0f));
-        const float vsigavi = fmaxf(alphai * vwaveif - beta * projv, 0.0f);
-        float rho1j = 0, rho21j = 0, pro2j = 0, vwavej = 0, autermj = 0, avBtermj = 0, vsigavj = 0, prj = 0;
-        const float rhoj = rj[1];
-        if (usej) {
-          rho1j = rj[2]; rho21j = rj[15]; pro2j = rj[3]; vwavej = rj[4]; prj = rj[5];
-          autermj = rj[6]; avBtermj = rj[13];
-          vsigmax = fmaxf(vsigmax, fmaxf(vwavej - beta * projv, 0.0f));
-          vsigavj = fmaxf(rj[14] * vwavej - beta * projv, 0.0f);  // alphaj = alphaind(1,j)
-        }
-        float qrho2i = 0.0f, qrho2j = 0.0f;
-        if (projv < 0.0f) {
-          qrho2i = -0.5f * rho1if * vsigavi * projv;
-          if (usej) qrho2j = -0.5f * rho1j * vsigavj * projv;
-        }
-        const float gradpi = pmf * (pro2if + qrho2i) * grkerni;
-        const float gradpj = usej ? pmf * (pro2j + qrho2j) * grkernj : 0.0f;
-        if (adiab) {
-          const float vsigu = GRAV ? fabsf(projv) : sqrtf(fabsf(prif - prj) * __fdividef(2.0f, rhoif + rhoj));
-          f[5].add(pmf * qrho2i * projv * grkerni);
-          f[6].add(vsigu * denij * (auterm * grkerni + autermj * grkernj));
-        }
-        float projsx = 0, projsy = 0, projsz = 0;
-        if (MHD) {
-          const float *mj = jmhdf + JMHDF * (size_t)j;
-          const float bxj = mj[0], byj = mj[1], bzj = mj[2], psij = mj[3];
-          const float dBx = bxif - bxj, dBy = byif - byj, dBz = bzif - bzj;
-          const float projBi = bxif * runix + byif * runiy + bzif * runiz;
-          const float projBj = bxj * runix + byj * runiy + bzj * runiz;
-          const float projdB = dBx * runix + dBy * runiy + dBz * runiz;
-          const float dB2 = dBx * dBx + dBy * dBy + dBz * dBz;
-          f[11].add(-pmf * projdB * grkerni);
-          const float tx_ = dvx - projv * runix, ty_ = dvy - projv * runiy, tz_ = dvz - projv * runiz;
-          const float vsigB = sqrtf(tx_ * tx_ + ty_ * ty_ + tz_ * tz_);
-          const float dBdiss = (avBterm * grkerni + avBtermj * grkernj) * vsigB;
-          if (p.iresistive_heating > 0 && adiab) f[5].add(-0.5f * dB2 * dBdiss);
-          const float pmi = pmf * rho21i * grkerni, pmj = pmf * rho21j * grkernj;
-          const float termi = pmi * projBi;
-          f[7].add(termi + pmj * projBj);
-          const float dpsi = ocf * (pmi * psiif * vwaveif + pmj * psij * vwavej);
-          f[8].add(-termi * dvx + dBdiss * dBx - dpsi * runix);
-          f[9].add(-termi * dvy + dBdiss * dBy - dpsi * runiy);
-          f[10].add(-termi * dvz + dBdiss * dBz - dpsi * runiz);
-          projsx = (sx[0] * runix + sx[1] * runiy + sx[2] * runiz) * grkerni +
-                   (mj[4] * runix + mj[5] * runiy + mj[6] * runiz) * grkernj;
-          projsy = (sx[1] * runix + sx[3] * runiy + sx[4] * runiz) * grkerni +
-                   (mj[5] * runix + mj[7] * runiy + mj[8] * runiz) * grkernj;
-          projsz = (sx[2] * runix + sx[4] * runiy + sx[5] * runiz) * grkerni +
-                   (mj[6] * runix + mj[8] * runiy + mj[9] * runiz) * grkernj;
-        }
-        const float gradp = gradpi + gradpj + fgrav;
-        f[0].add(-runix * gradp - projsx);
-        f[1].add(-runiy * gradp - projsy);
-        f[2].add(-runiz * gradp - projsz);
-        if (GRAV) f[3].add(pmf * phii);
-        f[4].add(projv * grkerni);
-      } else if (GRAV) {
-        const float rij1 = rsqrt_nr(rij2);
-        const float fgj = rij1 * rij1 * rij1 * pmf;
-        f[0].add(-dx * fgj); f[1].add(-dy * fgj); f[2].add(-dz * fgj);
-        f[3].add(-pmf * rij1);
-      }
-    };
-    // operands loaded right before their pair: at 96 registers 20 warps per SM
-    // hide the load latency better than a one-pair prefetch at 113 registers
-    // and 16 warps (4.94 -> 4.37 ms per Sedov 128^3 launch)
-    queue_window(cnt, S, act, il, stripe, sm.q, test, [&](int k) { body(load(k)); });
+    queue_window(cnt, S, act, il, stripe, sm.q, test, [&](int k) {
+      force_pair_mixed<MHD, true, IND>(p, I, stg.jidx[k], stg.code[k], txf, txl, tx, ty, tz, jrecf, jmhdf, ibin_old_t,
+                                       wakemark, f, vsigmax, nbi);
+    });
   }
-  store_pair_sums<IND, false>(sm, lane, np, S, s0, am, psum, ps, 1.0, [&](int q) -> double {
+  store_pair_sums<IND>(sm, lane, np, S, c.s0, c.am, psum, ps, p.massoftype, [&](int q) -> double {
     return q < NF ? f[q].value() : (q == NF ? (double)vsigmax : (double)nbi);
   });
 }
@@ -1498,19 +1588,18 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   cudaMemcpyAsync(c->red, init, 2 * sizeof(double), cudaMemcpyHostToDevice, st);
   ForceOut out{c->fxyzu, c->dBevol, c->divcurlv, c->divBsymm, c->poten, c->red, c->stats, c->cell_ntrial};
   if (!(c->attr_done & 2u)) {
-    const int bytes = MAX_WARPS * (int)sizeof(PairSmem);
-#define PH_FORCE_ATTR(K, M, G, I) cudaFuncSetAttribute(K<M, G, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)
-#define PH_FORCE_ATTR4(K, I) \
-    PH_FORCE_ATTR(K, false, false, I); PH_FORCE_ATTR(K, true, false, I); PH_FORCE_ATTR(K, false, true, I); \
-    PH_FORCE_ATTR(K, true, true, I)
-    PH_FORCE_ATTR4(k_force_mixed, false); PH_FORCE_ATTR4(k_force_mixed, true);
-    PH_FORCE_ATTR4(k_force, false); PH_FORCE_ATTR4(k_force, true);
-#undef PH_FORCE_ATTR4
+    const int lb = MAX_WARPS * (int)sizeof(ListSmem), pb = MAX_WARPS * (int)sizeof(PairSmem);
+#define PH_FORCE_ATTR(M, I)                                                                                  \
+  cudaFuncSetAttribute(k_force_mixed<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);                \
+  cudaFuncSetAttribute(k_force<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);                      \
+  cudaFuncSetAttribute(k_force_mixed_grav<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb);           \
+  cudaFuncSetAttribute(k_force_grav<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb)
+    PH_FORCE_ATTR(false, false); PH_FORCE_ATTR(true, false); PH_FORCE_ATTR(false, true); PH_FORCE_ATTR(true, true);
 #undef PH_FORCE_ATTR
     cudaFuncSetAttribute(k_force_sym<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         MAX_WARPS * (int)sizeof(SymSmem<false>));
+                         sym_smem_bytes<false>(MAXCELL));
     cudaFuncSetAttribute(k_force_sym<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         MAX_WARPS * (int)sizeof(SymSmem<true>));
+                         sym_smem_bytes<true>(MAXCELL));
     c->attr_done |= 2u;
   }
   const int fw = c->force_warps;
@@ -1530,27 +1619,31 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
     cudaEventRecord(c->evk[0], st);
   } else if (mixed) {
     cudaEventRecord(c->evk[0], st);
-#define PH_FORCE_MIXED(M, G)                                                                                     \
-  do { if (ind) PH_FORCE_MIXED_I(M, G, true); else PH_FORCE_MIXED_I(M, G, false); } while (0)
-#define PH_FORCE_MIXED_I(M, G, I)                                                                                \
-  k_force_mixed<M, G, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(PairSmem), st>>>(              \
-      p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->perm, c->tx, c->ty, c->tz, c->th,       \
-      c->txf, c->jrec, jmhd, c->jrecf, jmhdf, eos_t, out, c->psum, c->cap, cells, actf, ibo, wake, c->d_err)
-    if (p.mhd) { if (p.gravity) PH_FORCE_MIXED(true, true); else PH_FORCE_MIXED(true, false); }
-    else { if (p.gravity) PH_FORCE_MIXED(false, true); else PH_FORCE_MIXED(false, false); }
+#define PH_FORCE_MIXED(K, M, I, SM)                                                                            \
+  K<M, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SM), st>>>(                                                    \
+      p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl,   \
+      c->jrecf, jmhdf, out, c->psum, c->cap, cells, actf, ibo, wake, c->d_err)
+#define PH_FORCE_MIXED_I(K, M, SM) do { if (ind) PH_FORCE_MIXED(K, M, true, SM); else PH_FORCE_MIXED(K, M, false, SM); } while (0)
+    if (p.gravity) {
+      if (p.mhd) PH_FORCE_MIXED_I(k_force_mixed_grav, true, PairSmem);
+      else PH_FORCE_MIXED_I(k_force_mixed_grav, false, PairSmem);
+    } else {
+      if (p.mhd) PH_FORCE_MIXED_I(k_force_mixed, true, ListSmem);
+      else PH_FORCE_MIXED_I(k_force_mixed, false, ListSmem);
+    }
 #undef PH_FORCE_MIXED
 #undef PH_FORCE_MIXED_I
   } else if (use_sym(c)) {
     cudaEventRecord(c->evk[0], st);
     if (p.mhd) {
-      k_force_sym<true><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SymSmem<true>), st>>>(
+      k_force_sym<true><<<nfc, 32, sym_smem_bytes<true>(p.minpart), st>>>(
           p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,
           c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
       k_force_gather<true><<<nblk(nfc, 4), 128, 0, st>>>(c->nodes, c->leaves, nfc, c->pool, c->cell_off,
                                                          c->cell_nleaf, c->cell_at, c->toff, c->jbuf,
                                                          c->jbuf_stride, p.massoftype, c->psum, c->cap, c->d_err);
     } else {
-      k_force_sym<false><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SymSmem<false>), st>>>(
+      k_force_sym<false><<<nfc, 32, sym_smem_bytes<false>(p.minpart), st>>>(
           p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,
           c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
       k_force_gather<false><<<nblk(nfc, 4), 128, 0, st>>>(c->nodes, c->leaves, nfc, c->pool, c->cell_off,
@@ -1560,14 +1653,18 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
     count_launch(c, 1);
   } else {
     cudaEventRecord(c->evk[0], st);
-#define PH_FORCE_FP64(M, G)                                                                                      \
-  do { if (ind) PH_FORCE_FP64_I(M, G, true); else PH_FORCE_FP64_I(M, G, false); } while (0)
-#define PH_FORCE_FP64_I(M, G, I)                                                                                 \
-  k_force<M, G, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(PairSmem), st>>>(                    \
-      p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->perm, c->tx, c->ty, c->tz, c->th,       \
-      c->txf, c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, cells, actf, ibo, wake, c->d_err)
-    if (p.mhd) { if (p.gravity) PH_FORCE_FP64(true, true); else PH_FORCE_FP64(true, false); }
-    else { if (p.gravity) PH_FORCE_FP64(false, true); else PH_FORCE_FP64(false, false); }
+#define PH_FORCE_FP64_I(K, M, I, SM)                                                                           \
+  K<M, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SM), st>>>(                                                    \
+      p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,    \
+      c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, cells, actf, ibo, wake, c->d_err)
+#define PH_FORCE_FP64(K, M, SM) do { if (ind) PH_FORCE_FP64_I(K, M, true, SM); else PH_FORCE_FP64_I(K, M, false, SM); } while (0)
+    if (p.gravity) {
+      if (p.mhd) PH_FORCE_FP64(k_force_grav, true, PairSmem);
+      else PH_FORCE_FP64(k_force_grav, false, PairSmem);
+    } else {
+      if (p.mhd) PH_FORCE_FP64(k_force, true, ListSmem);
+      else PH_FORCE_FP64(k_force, false, ListSmem);
+    }
 #undef PH_FORCE_FP64
 #undef PH_FORCE_FP64_I
   }

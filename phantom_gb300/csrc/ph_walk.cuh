@@ -276,7 +276,7 @@ __device__ __forceinline__ void queue_window(int cnt, int S, bool act, int il, i
 // ------------------------------------------------------------------ list sweep
 // Trial list -> per-particle pair queues -> balanced drain, by one warp.
 //
-// The sweep: batches of 32 leaf entries are expanded into shared memory (tree
+// The sweep: batches of (at most) 32 leaf entries are expanded into shared memory (tree
 // index and offset code per trial particle); each lane then takes one trial
 // particle (its FP32 position in registers, loaded one chunk ahead) and the
 // warp tests it against the cell's particles one after the other, their FP32
@@ -294,26 +294,42 @@ __device__ __forceinline__ void queue_window(int cnt, int S, bool act, int il, i
 constexpr int LW = 32 * MAXCELL;  // trial particles of a batch
 constexpr int LQ = 1280;          // queue slots per warp, dealt out evenly to the cell's particles
 
-struct __align__(16) ListSmem {
-  int qj[LQ];             // accepted trial particle (or its index in the batch)
-  unsigned char qc[LQ];   // offset code, bit 6: the reference uses its cached position
+struct __align__(16) ListBase {
   float4 xi[MAXCELL];     // cell particles: x, y, z, acceptance r^2
   int ipos[MAXCELL];      // their tree positions
-  int j[LW];
+  int j[LW];              // the batch
   unsigned char code[LW];
   unsigned char own[32];  // drain: lane -> particle
   unsigned char first[MAXCELL], lanes[MAXCELL];
 };
-struct ListPos {  // the sweep's place in the list
-  int e0 = 0, nbase = 0, cnt = 0, k0 = 0;
+struct ListSmem : ListBase {
+  union {
+    int qj[LQ];           // accepted trial particle
+    double red[LQ / 2];   // lane sums of the flush
+  };
+  unsigned char qc[LQ];   // its offset code, QC_CACHED where the reference uses its cached position
+};
+// queue of batch indices (code[] then holds the flagged codes)
+struct ListSmemK : ListBase {
+  union {
+    unsigned short qj[LQ];
+    double red[32 * 12];
+  };
 };
 
-// expand the 32 leaf entries from e0 on; returns the number of trial particles
+struct ListPos {  // the sweep's place in the list
+  int e0 = 0, nbase = 0, cnt = 0, k0 = 0;
+  bool open = false;
+};
+enum { SWEEP_END = 0, SWEEP_FULL = 1, SWEEP_BATCH = 2 };
+
+// expand the BL leaf entries from e0 on; returns the number of trial particles
+template <int BL>
 __device__ __forceinline__ int expand_batch(const LeafEntry *__restrict__ pool, int off, int nleaf, int e0,
-                                            ListSmem &sm) {
+                                            ListBase &sm) {
   const int e = e0 + lane_id();
   LeafEntry le{0, 0};
-  if (e < nleaf) le = pool[off + e];
+  if (lane_id() < BL && e < nleaf) le = pool[off + e];
   const int jc = le.cc & 255, code = le.cc >> 8;
   int x = jc;
   for (int o = 1; o < 32; o <<= 1) {
@@ -325,16 +341,18 @@ __device__ __forceinline__ int expand_batch(const LeafEntry *__restrict__ pool, 
   return __shfl_sync(0xffffffffu, x, 31);
 }
 
-// Sweep on from `pos` until the list ends (returns false) or a queue is nearly
-// full (true: drain, then call again). sm.xi / sm.ipos describe the np cell
+// Sweep on from `pos` until the list ends (SWEEP_END) or a queue is nearly full
+// (SWEEP_FULL: drain, then call again). sm.xi / sm.ipos describe the np cell
 // particles; ew(w) is the acceptance r^2 of a trial particle with txf.w = w;
 // myc receives lane il's count for particle il. With AFTER only trial
-// particles after the cell particle in tree order are accepted, and the queue
-// holds batch indices (the list must end with its batch: drain per batch).
-template <bool AFTER, class EW>
-__device__ __forceinline__ bool sweep_list(const Params &p, float4 cc, int np, const LeafEntry *__restrict__ pool,
-                                           int off, int nleaf, const float4 *__restrict__ txf, ListSmem &sm,
-                                           int qstride, ListPos &pos, int &myc, EW ew) {
+// particles after the cell particle in tree order are accepted, the queue
+// holds batch indices, and the sweep also returns at the end of every batch
+// (SWEEP_BATCH: drain; trial particles [nbase, nbase + cnt) of the list are
+// done); SWEEP_END then leaves nothing to drain. BL: leaf entries per batch.
+template <bool AFTER, int BL, class Smem, class EW>
+__device__ __forceinline__ int sweep_list(const Params &p, float4 cc, int np, const LeafEntry *__restrict__ pool,
+                                          int off, int nleaf, const float4 *__restrict__ txf, Smem &sm, int qstride,
+                                          ListPos &pos, int &myc, EW ew) {
   const unsigned FULL = 0xffffffffu;
   const int lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
@@ -348,12 +366,14 @@ __device__ __forceinline__ bool sweep_list(const Params &p, float4 cc, int np, c
   bool fresh = true;  // the chunk at k0 is not loaded yet
   while (true) {
     if (pos.k0 >= pos.cnt) {
+      if (AFTER && pos.open) { pos.open = false; return SWEEP_BATCH; }
       pos.nbase += pos.cnt;
-      if (pos.e0 >= nleaf || (AFTER && pos.cnt > 0)) { pos.k0 = pos.cnt = 0; return pos.e0 < nleaf; }
+      if (pos.e0 >= nleaf) { pos.k0 = pos.cnt = 0; return SWEEP_END; }
       __syncwarp();
-      pos.cnt = expand_batch(pool, off, nleaf, pos.e0, sm);
-      pos.e0 += 32;
+      pos.cnt = expand_batch<BL>(pool, off, nleaf, pos.e0, sm);
+      pos.e0 += BL;
       pos.k0 = 0;
+      pos.open = true;
       fresh = true;
       __syncwarp();
     }
@@ -377,7 +397,6 @@ __device__ __forceinline__ bool sweep_list(const Params &p, float4 cc, int np, c
       wr = __any_sync(FULL, jc >= 0 && (fabsf(cc.x - x.x) > hx || fabsf(cc.y - x.y) > hy || fabsf(cc.z - x.z) > hz));
     }
     const float w = ew(x.w);
-    const int val = AFTER ? k : jc;
     const unsigned char flag =
         (unsigned char)(code != 0 ? code | (pos.nbase + k < CELLCACHE ? QC_CACHED : 0) : 0);
     int mx = 0;
@@ -396,15 +415,15 @@ __device__ __forceinline__ bool sweep_list(const Params &p, float4 cc, int np, c
       const unsigned b = __ballot_sync(FULL, ok);
       if (ok) {
         const int q = il * qstride + qn[il] + __popc(b & lt);
-        sm.qj[q] = val;
-        if (!AFTER) sm.qc[q] = flag; else sm.code[k] = flag;
+        if constexpr (AFTER) { sm.qj[q] = (unsigned short)k; sm.code[k] = flag; }
+        else { sm.qj[q] = jc; sm.qc[q] = flag; }
       }
       qn[il] += __popc(b);
       if (lane == il) myc += __popc(b);
       mx = max(mx, qn[il]);
     }
     pos.k0 += 32;
-    if (mx > qstride - 32) return true;
+    if (mx > qstride - 32) return SWEEP_FULL;
   }
 }
 
@@ -413,7 +432,7 @@ __device__ __forceinline__ bool sweep_list(const Params &p, float4 cc, int np, c
 // fits, from 32 s >= sum c up. Each lane gets its particle (il, -1: none), its
 // first queue entry, the step and the count.
 struct QueueLanes { int il, m0, step, c; };
-__device__ __forceinline__ QueueLanes balance_queues(int np, int c, ListSmem &sm) {
+__device__ __forceinline__ QueueLanes balance_queues(int np, int c, ListBase &sm) {
   const unsigned FULL = 0xffffffffu;
   const int lane = lane_id();
   if (lane >= np) c = 0;
@@ -444,13 +463,13 @@ __device__ __forceinline__ QueueLanes balance_queues(int np, int c, ListSmem &sm
 
 // Sum RW values of every lane into per-(value, particle) totals: total idx =
 // value * np + particle lives in tot[idx / 32] of lane idx % 32. The lane
-// values pass through shared memory (the queues' space: all lanes are done
-// with them) and are added in lane order, so totals are deterministic.
+// values pass through shared memory at red (32 RW doubles, free when every lane
+// is done with the queues) and are added in lane order, so totals are
+// deterministic.
 template <int RW, int NR, class Get, class Add>
-__device__ __forceinline__ void flush_lanes(int np, ListSmem &sm, double (&tot)[NR], Get get, Add add) {
-  static_assert(32 * RW * sizeof(double) <= sizeof(int) * LQ + LQ, "lane sums staged in the queues' space");
+__device__ __forceinline__ void flush_lanes(int np, const ListBase &sm, double *red, double (&tot)[NR], Get get,
+                                            Add add) {
   static_assert(RW * MAXCELL <= 32 * NR, "totals per lane");
-  double *red = reinterpret_cast<double *>(sm.qj);
   const int lane = lane_id();
   __syncwarp();
 #pragma unroll
