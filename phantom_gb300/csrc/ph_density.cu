@@ -104,9 +104,10 @@ struct DensOut {
 // dealt out by queue length (list sweep). The neighbour test is the
 // reference's: FP32 with a 1e-3 margin in r^2 rejects pairs provably outside
 // the kernel (bypassed when h is small against the coordinates), the rest is
-// decided in FP64.
+// decided in FP64. 28 warps per SM (the dB sums aside): Sedov 100^3, mixed, the
+// passes 7.9 -> 7.0 ms against the unbounded allocation's 24.
 template <bool MIXED, bool MHD, bool GRAV>
-__global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
+__global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 4 : 7) k_density_pairs(
     Params p, const Node *nodes, const int *leaves, const int *act, int nact, const LeafEntry *pool,
     const int *cell_off, const int *cell_nleaf, const int *cell_ntrial, const int *perm, const double *tx,
     const double *ty, const double *tz, const float4 *txf, const float4 *txl, const double *hcur, const double *Bevol,
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_pairs(
   bool more = true;
   while (more) {
     int myc;
-    more = SWEEP_END != sweep_list<false, 32>(p, cc, np, pool, off, nleaf, txf, sm, qstride, pos, myc, [](float) { return 0.0f; });
+    more = SWEEP_END != sweep_list<false>(p, cc, np, pool, off, nleaf, txf, sm, qstride, pos, myc, [](float) { return 0.0f; });
     const QueueLanes ql = balance_queues(np, myc, sm);
     const int il = max(ql.il, 0), i = sm.ipos[il];
     const double hi1 = __shfl_sync(0xffffffffu, h1own, il);

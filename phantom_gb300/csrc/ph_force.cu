@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force(
   bool more = true;
   while (more) {
     int myc;
-    more = SWEEP_END != sweep_list<false, 32>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
+    more = SWEEP_END != sweep_list<false>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
                                               [&](float h1) { return accept(__frcp_rn(h1)); });
     const QueueLanes ql = balance_queues(np, myc, sm);
     const int il = max(ql.il, 0);
@@ -945,23 +945,22 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_grav(
 // cached-position rule from the evaluating cell's list); seen from j they differ
 // from the reference's own evaluation by rounding only.
 //
-// Work: the list sweep per batch of SYM_BL leaf entries (ph_walk.cuh), each
+// Work: the list sweep per batch of BATCH leaf entries (ph_walk.cuh), each
 // batch drained with the lanes dealt out by queue length. The j-side array of a
-// batch (NJ values of up to SYM_BL leaves) bounds the warps per SM: 24 entries
+// batch (NJ values of up to BATCH leaves) bounds the warps per SM: 24 entries
 // hold the owned half of most lists (37 entries at hfact 1.2) in one batch and
 // leave room for 11 warps at the reference's leaf size. One warp per block: the
 // SM's shared memory then fills in the smallest steps (measured per launch at
 // 64^3, hydro / MHD: 1, 2, 4 warps per block 1.88 / 3.66, 1.95 / 3.98, 2.20 /
 // 5.48 ms; batches of 16 entries 1.96 / 3.72 ms at one warp; the
 // lane-per-stripe loop before this one 2.45 / 4.46 ms).
-constexpr int SYM_BL = 24;
 struct SymSmem : ListSmemK {
-  // js[NJ][jw] doubles follow, jw = SYM_BL x leaf size
+  // js[NJ][jw] doubles follow, jw = BATCH x leaf size
   __device__ __forceinline__ double *js() { return reinterpret_cast<double *>(this + 1); }
 };
 template <bool MHD>
 __host__ __device__ constexpr int sym_smem_bytes(int minpart) {
-  return (int)sizeof(SymSmem) + 8 * NJS<MHD>::n * SYM_BL * minpart;
+  return (int)sizeof(SymSmem) + 8 * NJS<MHD>::n * BATCH * minpart;
 }
 
 template <bool MHD>
@@ -980,7 +979,7 @@ __global__ void __launch_bounds__(32) k_force_sym(
   extern __shared__ __align__(16) unsigned char dsm[];
   SymSmem &sm = *reinterpret_cast<SymSmem *>(dsm);
   double *js = sm.js();
-  const int jw = SYM_BL * p.minpart;
+  const int jw = BATCH * p.minpart;
   const float q2lim = 4.0f * 1.001f, INF = __int_as_float(0x7f800000);
   const float pf_hf = __double2float_ru(pf_hmin);
   if (lane < np) {
@@ -1019,7 +1018,7 @@ __global__ void __launch_bounds__(32) k_force_sym(
   while (true) {
     __syncwarp();
     int myc;
-    const int st = sweep_list<true, SYM_BL>(p, cc, np, pool, off, nown, txf, sm, qstride, pos, myc, [&](float h1) {
+    const int st = sweep_list<true>(p, cc, np, pool, off, nown, txf, sm, qstride, pos, myc, [&](float h1) {
       const float hj = __frcp_rn(h1);
       return hj > pf_hf ? q2lim * (hj * hj) : INF;
     });
@@ -1367,8 +1366,12 @@ __device__ __forceinline__ void force_pair_mixed(const Params &p, const IMix<MHD
   f[4].add(pv * gi);
 }
 
+// 24 warps per SM (MHD 20) hide the pair's dependency chain best: at 64^3 the
+// register allocation left alone (108 registers, 16 warps) takes 0.513 ms (MHD
+// 0.75), this bound 0.47 (0.62), one more block 0.49 (0.70); self-gravity at
+// 300001 particles 2.77 -> 2.39 ms.
 template <bool MHD, bool IND>
-__global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed(
+__global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
     const float *jrecf, const float *jmhdf, ForceOut out, double *psum, int64_t ps, const int *cells,
@@ -1395,7 +1398,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed(
   bool more = true;
   while (more) {
     int myc;
-    more = SWEEP_END != sweep_list<false, 32>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
+    more = SWEEP_END != sweep_list<false>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
                                               [&](float h1) { return __fdividef(q2lim, h1 * h1); });
     const QueueLanes ql = balance_queues(np, myc, sm);
     const int il = max(ql.il, 0);
@@ -1416,7 +1419,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed(
 
 // Self-gravity: as k_force_grav, far pairs evaluated where they are tested.
 template <bool MHD, bool IND>
-__global__ void __launch_bounds__(32 * MAX_WARPS) k_force_mixed_grav(
+__global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed_grav(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
     const float *jrecf, const float *jmhdf, ForceOut out, double *psum, int64_t ps, const int *cells,

@@ -90,7 +90,7 @@ struct ph_ctx {
   // bit 0 density pair kernels, bit 1 force pair kernels, bit 2 adjoint
   unsigned attr_done = 0;
   // warps (leaf cells) per block of the pair and walk kernels (ph_autotune)
-  int dens_warps = 4, force_warps = 4, walk_warps = 2;
+  int dens_warps = 2, force_warps = 2, walk_warps = 2;
   double tune_ms_before = 0.0, tune_ms_after = 0.0;  // last ph_autotune
 
   // caller-order particle state (reference layout)

@@ -185,29 +185,33 @@ __device__ __forceinline__ float diff2(float ah, float al, float bh, float bl) {
   const float e = __fsub_rn(__fsub_rn(ah, __fsub_rn(s, t)), __fadd_rn(bh, t));
   return __fadd_rn(s, __fadd_rn(e, __fsub_rn(al, bl)));
 }
-static __device__ __noinline__ float3 separation_image(const double *tx, const double *ty, const double *tz, int i, int j,
-                                                int mx, int my, int mz, double Lx, double Ly, double Lz) {
+// FP64 separation with the pair's periodic image (the leaf's offset code, then
+// the wrap of what is left), rounded to FP32; u: the unshifted FP32 separation
+static __device__ __noinline__ float3 separation_image(const double *tx, const double *ty, const double *tz, int i,
+                                                       int j, int code, float ux, float uy, float uz, double Lx,
+                                                       double Ly, double Lz) {
+  const float fx = (float)Lx, fy = (float)Ly, fz = (float)Lz;
+  ux -= offset_of_f(code, 0, fx); uy -= offset_of_f(code, 1, fy); uz -= offset_of_f(code, 2, fz);
+  const int mx = image_shift(code, 0, fabsf(ux) > 0.5f * fx, ux), my = image_shift(code, 1, fabsf(uy) > 0.5f * fy, uy),
+            mz = image_shift(code, 2, fabsf(uz) > 0.5f * fz, uz);
   return make_float3(d2f_rn((tx[i] - tx[j]) - shift_len(mx, Lx)), d2f_rn((ty[i] - ty[j]) - shift_len(my, Ly)),
                      d2f_rn((tz[i] - tz[j]) - shift_len(mz, Lz)));
 }
 __device__ __forceinline__ void separation_2f(const Params &p, const Sep2 &I, int j, int code, const float4 &jh,
                                               const float4 &jl, const double *tx, const double *ty, const double *tz,
                                               float &dx, float &dy, float &dz, float &r2) {
-  int mx = 0, my = 0, mz = 0;
-  if (p.periodic) {
-    const float ux = I.h.x - (jh.x + offset_of_f(code, 0, p.dxboundf)),
-                uy = I.h.y - (jh.y + offset_of_f(code, 1, p.dyboundf)),
-                uz = I.h.z - (jh.z + offset_of_f(code, 2, p.dzboundf));
-    mx = image_shift(code, 0, fabsf(ux) > 0.5f * p.dxboundf, ux);
-    my = image_shift(code, 1, fabsf(uy) > 0.5f * p.dyboundf, uy);
-    mz = image_shift(code, 2, fabsf(uz) > 0.5f * p.dzboundf, uz);
-  }
   dx = diff2(I.h.x, I.l.x, jh.x, jl.x);
   dy = diff2(I.h.y, I.l.y, jh.y, jl.y);
   dz = diff2(I.h.z, I.l.z, jh.z, jl.z);
   r2 = dx * dx + dy * dy + dz * dz;
-  if ((mx | my | mz) != 0 || r2 < I.guard) {
-    const float3 d = separation_image(tx, ty, tz, I.i, j, mx, my, mz, p.dxbound, p.dybound, p.dzbound);
+  bool rare = r2 < I.guard;
+  if (p.periodic)
+    rare = rare || code != 0 || fabsf(dx) > 0.5f * p.dxboundf || fabsf(dy) > 0.5f * p.dyboundf ||
+           fabsf(dz) > 0.5f * p.dzboundf;
+  if (rare) {
+    const bool per = p.periodic != 0;
+    const double Lx = per ? p.dxbound : 1.0e300, Ly = per ? p.dybound : 1.0e300, Lz = per ? p.dzbound : 1.0e300;
+    const float3 d = separation_image(tx, ty, tz, I.i, j, code, dx, dy, dz, Lx, Ly, Lz);
     dx = d.x; dy = d.y; dz = d.z;
     r2 = dx * dx + dy * dy + dz * dz;
   }
@@ -276,7 +280,7 @@ __device__ __forceinline__ void queue_window(int cnt, int S, bool act, int il, i
 // ------------------------------------------------------------------ list sweep
 // Trial list -> per-particle pair queues -> balanced drain, by one warp.
 //
-// The sweep: batches of (at most) 32 leaf entries are expanded into shared memory (tree
+// The sweep: batches of BATCH leaf entries are expanded into shared memory (tree
 // index and offset code per trial particle); each lane then takes one trial
 // particle (its FP32 position in registers, loaded one chunk ahead) and the
 // warp tests it against the cell's particles one after the other, their FP32
@@ -291,8 +295,9 @@ __device__ __forceinline__ void queue_window(int cnt, int S, bool act, int il, i
 // most pairs per lane has as few as possible (balance_queues); with a fixed
 // 32/np lanes per particle the longest queue set the pace and a fifth (density)
 // to two fifths (symmetric force) of the lane slots were idle.
-constexpr int LW = 32 * MAXCELL;  // trial particles of a batch
-constexpr int LQ = 1280;          // queue slots per warp, dealt out evenly to the cell's particles
+constexpr int BATCH = 24;             // leaf entries of a batch
+constexpr int LW = BATCH * MAXCELL;   // trial particles of a batch
+constexpr int LQ = 1024;              // queue slots per warp, dealt out evenly to the cell's particles
 
 struct __align__(16) ListBase {
   float4 xi[MAXCELL];     // cell particles: x, y, z, acceptance r^2
@@ -323,13 +328,12 @@ struct ListPos {  // the sweep's place in the list
 };
 enum { SWEEP_END = 0, SWEEP_FULL = 1, SWEEP_BATCH = 2 };
 
-// expand the BL leaf entries from e0 on; returns the number of trial particles
-template <int BL>
+// expand the BATCH leaf entries from e0 on; returns the number of trial particles
 __device__ __forceinline__ int expand_batch(const LeafEntry *__restrict__ pool, int off, int nleaf, int e0,
                                             ListBase &sm) {
   const int e = e0 + lane_id();
   LeafEntry le{0, 0};
-  if (lane_id() < BL && e < nleaf) le = pool[off + e];
+  if (lane_id() < BATCH && e < nleaf) le = pool[off + e];
   const int jc = le.cc & 255, code = le.cc >> 8;
   int x = jc;
   for (int o = 1; o < 32; o <<= 1) {
@@ -348,8 +352,8 @@ __device__ __forceinline__ int expand_batch(const LeafEntry *__restrict__ pool, 
 // particles after the cell particle in tree order are accepted, the queue
 // holds batch indices, and the sweep also returns at the end of every batch
 // (SWEEP_BATCH: drain; trial particles [nbase, nbase + cnt) of the list are
-// done); SWEEP_END then leaves nothing to drain. BL: leaf entries per batch.
-template <bool AFTER, int BL, class Smem, class EW>
+// done); SWEEP_END then leaves nothing to drain.
+template <bool AFTER, class Smem, class EW>
 __device__ __forceinline__ int sweep_list(const Params &p, float4 cc, int np, const LeafEntry *__restrict__ pool,
                                           int off, int nleaf, const float4 *__restrict__ txf, Smem &sm, int qstride,
                                           ListPos &pos, int &myc, EW ew) {
@@ -357,21 +361,23 @@ __device__ __forceinline__ int sweep_list(const Params &p, float4 cc, int np, co
   const int lane = lane_id();
   const unsigned lt = (1u << lane) - 1u;
   const float hx = 0.4995f * p.dxboundf - cc.w, hy = 0.4995f * p.dyboundf - cc.w, hz = 0.4995f * p.dzboundf - cc.w;
-  int qn[MAXCELL];
+  int qn[MAXCELL];  // next free slot of each particle's queue
 #pragma unroll
-  for (int il = 0; il < MAXCELL; ++il) qn[il] = 0;
+  for (int il = 0; il < MAXCELL; ++il) qn[il] = il * qstride;
+  const int ipf = sm.ipos[0], ipl = sm.ipos[np - 1];  // ascending
   myc = 0;
   int j = -1;
   float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   bool fresh = true;  // the chunk at k0 is not loaded yet
+  int state;
   while (true) {
     if (pos.k0 >= pos.cnt) {
-      if (AFTER && pos.open) { pos.open = false; return SWEEP_BATCH; }
+      if (AFTER && pos.open) { pos.open = false; state = SWEEP_BATCH; break; }
       pos.nbase += pos.cnt;
-      if (pos.e0 >= nleaf) { pos.k0 = pos.cnt = 0; return SWEEP_END; }
+      if (pos.e0 >= nleaf) { pos.k0 = pos.cnt = 0; state = SWEEP_END; break; }
       __syncwarp();
-      pos.cnt = expand_batch<BL>(pool, off, nleaf, pos.e0, sm);
-      pos.e0 += BL;
+      pos.cnt = expand_batch(pool, off, nleaf, pos.e0, sm);
+      pos.e0 += BATCH;
       pos.k0 = 0;
       pos.open = true;
       fresh = true;
@@ -397,9 +403,14 @@ __device__ __forceinline__ int sweep_list(const Params &p, float4 cc, int np, co
       wr = __any_sync(FULL, jc >= 0 && (fabsf(cc.x - x.x) > hx || fabsf(cc.y - x.y) > hy || fabsf(cc.z - x.z) > hz));
     }
     const float w = ew(x.w);
+    if (jc < 0) x.x = __int_as_float(0x7f800000);  // past the end: r^2 infinite, never accepted
+    // chunks that hold the cell's own particles: no pair with itself (AFTER: or
+    // with an earlier one)
+    const bool own = __any_sync(FULL, jc >= ipf && jc <= ipl);
     const unsigned char flag =
         (unsigned char)(code != 0 ? code | (pos.nbase + k < CELLCACHE ? QC_CACHED : 0) : 0);
-    int mx = 0;
+    if (AFTER && jc >= 0) sm.code[k] = flag;
+    int left = qstride;
 #pragma unroll
     for (int il = 0; il < MAXCELL; ++il) {
       if (il >= np) break;
@@ -410,21 +421,28 @@ __device__ __forceinline__ int sweep_list(const Params &p, float4 cc, int np, co
         if (fabsf(dy) > 0.5f * p.dyboundf) dy -= copysignf(p.dyboundf, dy);
         if (fabsf(dz) > 0.5f * p.dzboundf) dz -= copysignf(p.dzboundf, dz);
       }
-      const int ip = sm.ipos[il];
-      const bool ok = dx * dx + dy * dy + dz * dz < fmaxf(xi.w, w) && (AFTER ? jc > ip : (jc >= 0 && jc != ip));
+      bool ok = dx * dx + dy * dy + dz * dz < fmaxf(xi.w, w);
+      if (own) {
+        const int ip = sm.ipos[il];
+        ok = ok && (AFTER ? jc > ip : jc != ip);
+      }
       const unsigned b = __ballot_sync(FULL, ok);
       if (ok) {
-        const int q = il * qstride + qn[il] + __popc(b & lt);
-        if constexpr (AFTER) { sm.qj[q] = (unsigned short)k; sm.code[k] = flag; }
+        const int q = qn[il] + __popc(b & lt);
+        if constexpr (AFTER) { sm.qj[q] = (unsigned short)k; }
         else { sm.qj[q] = jc; sm.qc[q] = flag; }
       }
       qn[il] += __popc(b);
-      if (lane == il) myc += __popc(b);
-      mx = max(mx, qn[il]);
+      left = min(left, (il + 1) * qstride - qn[il]);
     }
     pos.k0 += 32;
-    if (mx > qstride - 32) return SWEEP_FULL;
+    if (left < 32) { state = SWEEP_FULL; break; }
   }
+#pragma unroll
+  for (int il = 0; il < MAXCELL; ++il)
+    if (lane == il) myc = qn[il] - il * qstride;
+  if (lane >= np) myc = 0;
+  return state;
 }
 
 // Deal the 32 lanes out to the particles' queues (lane il < np holds its
