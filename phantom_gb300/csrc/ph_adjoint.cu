@@ -181,13 +181,12 @@ struct Bar {
 // kap is the receiver's cotangent of its divB sum (from the div B
 // subtraction in the finish); c also holds o . d(B_a/rho_a)/dt, the div B
 // diffusion and drho/dt sums weighted by k11 and k4, and the resistive
-// heating. Accumulates the cotangents of side a (KEEP_A) or side b into g,
-// or with BOTH those of a into g and those of b into *gb, and returns dc/dd
-// in (gdx, gdy, gdz).
-template <typename T, bool KEEP_A, bool IND, bool BOTH = false>
+// heating. Accumulates the cotangents of side a (KEEP_A) or side b into g and
+// returns dc/dd in (gdx, gdy, gdz).
+template <typename T, bool KEEP_A, bool IND>
 __device__ __forceinline__ void pair_rev(const AdjConst<T> &k, T dx, T dy, T dz, T dvx, T dvy,
                                          T dvz, const Side<T> &a, const Side<T> &b, const Wt<T> &wt,
-                                         Bar<T> &g, T &gdx, T &gdy, T &gdz, Bar<T> *gb = nullptr) {
+                                         Bar<T> &g, T &gdx, T &gdy, T &gdz) {
   const T wx = wt.wx, wy = wt.wy, wz = wt.wz, s = wt.s, kap = wt.kap;
   const T r2 = dx * dx + dy * dy + dz * dz;
   const T r = sqrt(r2), rinv = inv_sep(r2, r);
@@ -428,8 +427,7 @@ __device__ __forceinline__ void pair_rev(const AdjConst<T> &k, T dx, T dy, T dz,
     if (k.grav) gbb.gs += gsb_b;
     if (IND) gbb.psi += psib_b;
   };
-  if (BOTH) { add_a(g); add_b(*gb); }
-  else if (KEEP_A) add_a(g);
+  if (KEEP_A) add_a(g);
   else add_b(g);
 }
 
@@ -469,12 +467,17 @@ __device__ __forceinline__ double sep_t<double>(double d) { return d; }
 template <>
 __device__ __forceinline__ float sep_t<float>(double d) { return d2f_rn(d); }
 
+template <typename T>
+__device__ __forceinline__ void hydro_record(const Params &p, const double *r, T *o);
+constexpr int HREC = 32;  // values per particle of the hydro record (hydro passes below)
+
 // per-particle record: primitives of the force (cons2prim, eos.f90:184-237,
 // rho = rhoh(h)), the velocities the force was evaluated with, and the
 // cotangents w (accelerations) and s (du/dt) gathered to tree order
 __global__ void k_adj_prologue(Params p, int n, const int *perm, const double *th, const double *gradh64,
                                const double *gsoft64, const double *vel, const double *Bevol, const double *w4,
-                               const double *wB4, const float *alpha1, double *adj, float *adjf, float4 *txf) {
+                               const double *wB4, const float *alpha1, double *adj, float *adjf, double *hrec, float *hrecf,
+                               float4 *txf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int pid = perm[i];
@@ -533,6 +536,8 @@ __global__ void k_adj_prologue(Params p, int n, const int *perm, const double *t
     }
   }
   txf[i].w = (float)(1.0 / h);
+  if (hrec) hydro_record(p, r, hrec + HREC * (size_t)i);
+  if (hrecf) hydro_record(p, r, hrecf + HREC * (size_t)i);
   if (adjf) {  // FP32 copy of the record for the precision form's pair passes
     float *q = adjf + ADJREC * (size_t)i;
     for (int k = 0; k < AR_NSLOTS; ++k) q[k] = (float)r[k];
@@ -648,370 +653,403 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS) k_adj_pairs(Params p, AdjConst
   }
 }
 
-// ------------------------------------------------------------------ symmetric pass 1 (FP64 hydro)
-// Pass 1 with every unordered pair evaluated once, by the rule of the
-// symmetric FP64 force loop: cell A takes the owned prefix of its trial list
-// (entries starting at or after its first particle) and, in its own leaf, the
-// pairs j > i; every pair within either kernel lies in both cells' lists.
-// Both ordered terms of a pair (c_ij with i's cotangents, c_ji with j's) are
-// reversed once with both sides kept: two reverse terms per pair instead of
-// the four of k_adj_pairs. i's cotangents stay in the lane; j's NJA values
-// are combined in a per-window array of the warp (lanes holding the same j
-// add in lane order) written to jbuf at j's flattened trial index, and
-// k_adj_gather adds them to j's sums in the order of j's own list.
-constexpr int NJA = 15;  // j side: d-gradient (3), v (3), h, G, rho1, pro2, cs, P, rho, u, d2 rho/dh2
-constexpr int STAGE_A = 128;
-__device__ __forceinline__ int nja_slot(int v) {
-  return v < 3 ? PA_X + v : (v < 6 ? PA_VX + (v - 3) : (v == 14 ? PA_D2 : PA_H + (v - 6)));
-}
-static_assert(PA_H + 7 == PA_U && PA_D2 == PA_U + 1, "j-side slots h..u follow each other");
-struct SymAdjSmem {
-  union {
-    StageN<STAGE_A> st;
-    double red[32 * NADJ];
-  } u;
-  PairQ q;
-  double js[NJA][STAGE_A];
+// ------------------------------------------------------------------ hydro passes
+// Hydro contexts (no MHD, no self-gravity) take a joint reverse of a pair: its
+// whole contribution to L, C = c_ij + c_ji, is one scalar,
+//   C / m = A G + pv (T_i g_i + T_j g_j) + (s_i - s_j) vsu (u_i - u_j) E,
+//   A = -(w_i - w_j) . n,   G = X_i g_i + X_j g_j,   X = P/rho^2 + q,
+//   T = s ([pdV] P/rho^2 + [shock] q),   E = au_i g_i + au_j g_j,
+// (g the kernel gradient with 1/Omega, q the viscosity, pv = dv . n, vsu the
+// conductivity's signal speed), so one reverse with the difference of the
+// cotangents replaces the two of pair_rev, and the derivatives with respect to
+// a particle's rho, P, P/rho^2 and c_s are folded into its h and u with
+// factors from its record. Per unordered pair that is about 175 FP64
+// instructions where the two reverses took 700 (with a dozen divisions and
+// square roots); the passes are bound by the FP64 pipe.
+// A particle's 10 values: position gradient (3), velocity gradient (3), h, 1/Omega
+// (times 1/Omega), u, and the bracket of d^2 rho/dh^2, all without the
+// particle mass; k_adj_gather or the store of the precision form scales them.
+constexpr int NJA = 10;
+enum {
+  HR_H1 = 0, HR_KG, HR_KW, HR_RHO, HR_PRO2, HR_AVW, HR_C, HR_P, HR_U, HR_AU, HR_S, HR_WX, HR_WY, HR_WZ, HR_VX, HR_VY,
+  HR_VZ, HR_KRP, HR_KUP, HR_KRPP, HR_KUPP, HR_KRC, HR_KRA, HR_KUC, HR_KH, HR_A3, HR_B1, HR_N
+};
+static_assert(HR_N <= HREC, "hydro record slots");
+
+// kernel shape factors: HR_KG multiplies hs1 to g, HR_KW hs2 to dg/dr. FP64: hs1
+// = s of kern_w (HR_KG with -3/4); FP32: dW/dq (s would cancel at small q)
+template <typename T>
+__host__ __device__ constexpr T hs1_fac() { return sizeof(T) == 8 ? T(-0.75) : T(1.0); }
+
+struct HConst {
+  double beta;
+  bool cond, pdv, shock;
 };
 
-__global__ void __launch_bounds__(32 * ADJ_WARPS) k_adj_pairs_sym(
-    Params p, AdjConst<double> kc, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool,
-    const int *cell_off, const int *cell_nleaf, const double *tx, const double *ty, const double *tz,
-    const float4 *txf, const double *adj, double *psum, int64_t ps, double pf_hmin, const int *toff, double *jbuf,
-    int64_t jstride, int *err) {
-  const unsigned FULL = 0xffffffffu;
-  const int w = threadIdx.x >> 5, lane = lane_id();
-  const int cell = blockIdx.x * ADJ_WARPS + w;
-  if (cell >= ncell) return;
+// the record of tree position i from its adjoint record
+template <typename T>
+__device__ __forceinline__ void hydro_record(const Params &p, const double *r, T *o) {
+  const double h1 = r[AR_H1], rho = r[AR_RHO], rho1 = r[AR_RHO1], cs = r[AR_CS0], u = r[AR_U];
+  const double h4 = CNORMK * (h1 * h1) * (h1 * h1);
+  const double gm1 = p.ieos == 1 ? 0.0 : ((p.gamma > 1.0001) ? p.gamma - 1.0 : 2.0 / 3.0);
+  const double pon = p.ieos == 1 ? p.polyk : gm1 * u;
+  const double au = 0.5 * p.alphau * rho1;
+  const double v[HR_A3] = {h1, (double)hs1_fac<T>() * h4 * r[AR_G], 1.5 * h4 * h1 * r[AR_G], rho, r[AR_PRO2],
+                           r[AR_ALPHA] * cs, -0.5 * rho1, r[AR_P], u, au, r[AR_S], r[AR_WX], r[AR_WY], r[AR_WZ],
+                           r[AR_VX], r[AR_VY], r[AR_VZ], -r[AR_PRO2] * rho1, gm1 * rho1, pon, gm1 * rho,
+                           0.5 * rho1 * rho1, -au * rho1, cs > 0.0 ? r[AR_ALPHA] * p.gamma * gm1 / (2.0 * cs) : 0.0,
+                           -3.0 * rho * h1};
+  for (int k = 0; k < HR_A3; ++k) o[k] = (T)v[k];
+  if (p.ieos == 1) o[HR_KUC] = T(0.0);
+}
+
+__device__ __forceinline__ double inv_r(double r2) { return rsqrt_fast(r2); }
+__device__ __forceinline__ float inv_r(float r2) { return r2 > TINY_F ? rsqrt_nr(r2) : 0.0f; }
+__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt_fast(x); }
+__device__ __forceinline__ float rsqrt_t(float x) { return x >= TINY_F ? rsqrt_nr(x) : 0.0f; }
+
+// kernel shape at r h1: q, hs1, hs2 = w''/1.5 and the bracket 12 w + 8 q w' + q^2 w''
+__device__ __forceinline__ void hshape(double r, double h1, double &q, double &hs1, double &hs2, double &d2) {
+  double u = fma(-r, h1, 2.0);
+  u = u_inside(u) ? u : 0.0;
+  const double w = kern_w(u);
+  q = 2.0 - u;
+  hs1 = fma(-w, w, u * u);
+  hs2 = fma(-2.0, w, u);
+  // u (6 + u (10.5 u - 18)) - w/2 (6 + w (10.5 w - 18))
+  d2 = fma(u, fma(u, fma(10.5, u, -18.0), 6.0), -0.5 * w * fma(w, fma(10.5, w, -18.0), 6.0));
+}
+__device__ __forceinline__ void hshape(float r, float h1, float &q, float &hs1, float &hs2, float &d2) {
+  q = r * h1;
+  if (q < 1.0f) {
+    hs1 = q * (2.25f * q - 3.0f);
+    hs2 = 3.0f * q - 2.0f;
+    d2 = 12.0f + q * q * (31.5f * q - 45.0f);
+  } else {
+    const float t = fmaxf(2.0f - q, 0.0f);
+    hs1 = -0.75f * t * t;
+    hs2 = t;
+    d2 = t * (6.0f + t * (10.5f * t - 18.0f));
+  }
+}
+
+// Reverse of C: the gradient gd with respect to d = x_i - x_j and gv to dv =
+// v_i - v_j, and (h, 1/Omega, u, bracket) of both sides. a, b: hydro records.
+template <typename T>
+__device__ __forceinline__ void hydro_pair_rev(const HConst &k, T dx, T dy, T dz, T r2, const T *a, const T *b, T (&gd)[3],
+                                               T (&gv)[3], T (&oa)[4], T (&ob)[4]) {
+  const T beta = (T)k.beta;
+  const T y = inv_r(r2), r = r2 * y;
+  T qa_, s1a, s2a, d2a, qb_, s1b, s2b, d2b;
+  hshape(r, a[HR_H1], qa_, s1a, s2a, d2a);
+  hshape(r, b[HR_H1], qb_, s1b, s2b, d2b);
+  const T ga = a[HR_KG] * s1a, gb = b[HR_KG] * s1b;
+  const T dvx = a[HR_VX] - b[HR_VX], dvy = a[HR_VY] - b[HR_VY], dvz = a[HR_VZ] - b[HR_VZ];
+  const T pv = y * (dvx * dx + dvy * dy + dvz * dz);
+  const T wx = a[HR_WX] - b[HR_WX], wy = a[HR_WY] - b[HR_WY], wz = a[HR_WZ] - b[HR_WZ];
+  const T A = -y * (wx * dx + wy * dy + wz * dz);
+  const T sa = a[HR_S], sb = b[HR_S];
+  const bool neg = pv < T(0.0);
+  T va = T(0.0), vb = T(0.0), cpa = T(0.0), cpb = T(0.0), qa = T(0.0), qb = T(0.0);
+  if (neg) {
+    const T bp = beta * pv;
+    va = a[HR_AVW] - bp; vb = b[HR_AVW] - bp;
+    va = va > T(0.0) ? va : T(0.0); vb = vb > T(0.0) ? vb : T(0.0);
+    cpa = a[HR_C] * pv; cpb = b[HR_C] * pv;
+    qa = cpa * va; qb = cpb * vb;
+  }
+  const T Xa = a[HR_PRO2] + qa, Xb = b[HR_PRO2] + qb;
+  const T Ta = sa * (k.pdv ? (k.shock ? Xa : a[HR_PRO2]) : (k.shock ? qa : T(0.0)));
+  const T Tb = sb * (k.pdv ? (k.shock ? Xb : b[HR_PRO2]) : (k.shock ? qb : T(0.0)));
+  T pvb = Ta * ga + Tb * gb;
+  T gab = A * Xa + pv * Ta, gbb = A * Xb + pv * Tb;
+  const T Asa = A + sa * pv, Asb = A + sb * pv;
+  const T pa = ga * (k.pdv ? Asa : A), pb = gb * (k.pdv ? Asb : A);
+  T Ra = pa * a[HR_KRP], Rb = pb * b[HR_KRP], Ua = pa * a[HR_KUP], Ub = pb * b[HR_KUP];
+  if (neg) {
+    const T ea = k.shock == k.pdv ? pa : ga * (k.shock ? Asa : A), eb = k.shock == k.pdv ? pb : gb * (k.shock ? Asb : A);
+    const T vab = va > T(0.0) ? ea * cpa : T(0.0), vbb = vb > T(0.0) ? eb * cpb : T(0.0);
+    const T fa = ea * va, fb = eb * vb;
+    pvb += fa * a[HR_C] + fb * b[HR_C] - beta * (vab + vbb);
+    Ra += (fa * pv) * a[HR_KRC]; Rb += (fb * pv) * b[HR_KRC];
+    Ua += vab * a[HR_KUC]; Ub += vbb * b[HR_KUC];
+  }
+  if (k.cond) {
+    // vsu = sqrt(2 |dP| / rs) = sqrt(2) |dP| yc, yc = (|dP| rs)^(-1/2), rs = rho_i + rho_j
+    const T dP = a[HR_P] - b[HR_P], dPa = fabs(dP);
+    const T yc = rsqrt_t(dPa * (a[HR_RHO] + b[HR_RHO]));
+    const T vsu = T(1.4142135623730951) * dPa * yc;
+    const T Sd = sa - sb, Du = a[HR_U] - b[HR_U];
+    const T SD = Sd * Du, cu = SD * vsu;
+    const T E = a[HR_AU] * ga + b[HR_AU] * gb;
+    gab += cu * a[HR_AU]; gbb += cu * b[HR_AU];
+    const T du = Sd * vsu * E;
+    const T vsb = SD * E;
+    const T Pb_ = vsb * yc * (dP > T(0.0) ? T(0.70710678118654752) : T(-0.70710678118654752));
+    const T rX = T(-0.5) * vsb * vsu * (yc * yc) * dPa;
+    Ra += (cu * ga) * a[HR_KRA] + Pb_ * a[HR_KRPP] + rX;
+    Rb += (cu * gb) * b[HR_KRA] - Pb_ * b[HR_KRPP] + rX;
+    Ua += Pb_ * a[HR_KUPP] + du;
+    Ub -= Pb_ * b[HR_KUPP] + du;
+  }
+  const T Gs = Xa * ga + Xb * gb;
+  const T nbx = pvb * dvx - Gs * wx, nby = pvb * dvy - Gs * wy, nbz = pvb * dvz - Gs * wz;
+  const T nn = y * (nbx * dx + nby * dy + nbz * dz);
+  const T za = gab * a[HR_KW] * s2a, zb = gbb * b[HR_KW] * s2b;
+  const T c = y * ((za + zb) - nn * y);
+  gd[0] = nbx * y + dx * c; gd[1] = nby * y + dy * c; gd[2] = nbz * y + dz * c;
+  const T pvy = pvb * y;
+  gv[0] = pvy * dx; gv[1] = pvy * dy; gv[2] = pvy * dz;
+  oa[1] = gab * ga; ob[1] = gbb * gb;
+  oa[0] = Ra * a[HR_KH] - (za * qa_ + T(4.0) * a[HR_H1] * oa[1]);
+  ob[0] = Rb * b[HR_KH] - (zb * qb_ + T(4.0) * b[HR_H1] * ob[1]);
+  oa[2] = Ua; ob[2] = Ub;
+  oa[3] = d2a; ob[3] = d2b;
+}
+
+__host__ __device__ __forceinline__ int nja_slot(int v) {
+  return v < 3 ? PA_X + v : (v < 6 ? PA_VX + (v - 3) : (v == 6 ? PA_H : (v == 7 ? PA_G : (v == 8 ? PA_U : PA_D2))));
+}
+// a summed value in the units of the pass-1 slots
+__device__ __forceinline__ double nja_scaled(int v, double s, double m, double h1, double G) {
+  if (v == 7) return m * s / G;
+  if (v == 9) return m * CNORMK * (h1 * h1) * (h1 * h1) * h1 * s;
+  return m * s;
+}
+// the pass-1 slots the hydro record has folded into h and u
+__device__ __forceinline__ void nja_zero(double *psum, int64_t ps, size_t ip) {
+  psum[PA_RHO1 * ps + ip] = 0.0; psum[PA_PRO2 * ps + ip] = 0.0; psum[PA_CS * ps + ip] = 0.0;
+  psum[PA_P * ps + ip] = 0.0; psum[PA_RHO * ps + ip] = 0.0;
+}
+
+// acceptance and cell set-up of the hydro passes (txf.w = 1/h)
+struct AdjCell { int np, s0, off, nleaf; float4 cc; };
+__device__ __forceinline__ bool adj_cell(AdjCell &c, int cell, int ncell, const Node *nodes, const int *leaves,
+                                         const int *cell_off, const int *cell_nleaf, const float4 *txf, float pf_hf,
+                                         ListBase &sm, int *err) {
+  if (cell >= ncell) return false;
   const Node nd = nodes[leaves[cell]];
-  const int np = nd.count, s0 = nd.start;
-  if (np < 1 || np > MAXCELL) { if (lane == 0) set_error(err, PH_ERR_TREE); return; }
-  const int S = 32 / np;
-  const bool act = lane < np * S;
-  const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
-  const int i = s0 + il;
-  const double *ri = adj + ADJREC * (size_t)i;
-  const Side<double> si = load_side(ri);
-  const Wt<double> wti = load_wt(ri);
-  const double xi = tx[i], yi = ty[i], zi = tz[i];
-  const double vxi = ri[AR_VX], vyi = ri[AR_VY], vzi = ri[AR_VZ];
-  const float4 xif = txf[i];
-  const float hi21f = xif.w * xif.w;
-  const bool pf_i = ri[AR_H] > pf_hmin;
-  const float pf_h1max = (float)(1.0 / pf_hmin);
-  const float q2lim = 4.0f * 1.001f;
-  const double mcn = kc.m * kc.cn;
-  const double h51i = si.h1 * si.h1 * si.h1 * si.h1 * si.h1;
-  double gx = 0.0, gy = 0.0, gz = 0.0, d2 = 0.0;
-  Bar<double> gi;
-  const int off = cell_off[cell], nleaf = cell_nleaf[cell];
-  int nown = 0, town = 0;
-  for (int e0 = 0; e0 < nleaf; e0 += 32) {
-    const int e = e0 + lane;
-    LeafEntry le{0, 0};
-    if (e < nleaf) le = pool[off + e];
-    const bool own = e < nleaf && le.start >= s0;
-    nown += __popc(__ballot_sync(FULL, own));
-    town += warp_sum_int(own ? (le.cc & 255) : 0);
-    if (!__all_sync(FULL, e >= nleaf || own)) break;
+  c.np = nd.count; c.s0 = nd.start;
+  if (c.np < 1 || c.np > MAXCELL) { if (lane_id() == 0) set_error(err, PH_ERR_TREE); return false; }
+  c.off = cell_off[cell]; c.nleaf = cell_nleaf[cell];
+  c.cc = make_float4((float)nd.x, (float)nd.y, (float)nd.z, (float)nd.size);
+  if (lane_id() < c.np) {
+    float4 x = txf[c.s0 + lane_id()];
+    const float h = __frcp_rn(x.w);
+    x.w = h > pf_hf ? 4.0f * 1.001f * (h * h) : __int_as_float(0x7f800000);
+    sm.xi[lane_id()] = x;
+    sm.ipos[lane_id()] = c.s0 + lane_id();
   }
-  const int64_t tb = (int64_t)toff[off];
+  return true;
+}
+__device__ __forceinline__ float adj_accept(float h1, float pf_hf) {
+  const float h = __frcp_rn(h1);
+  return h > pf_hf ? 4.0f * 1.001f * (h * h) : __int_as_float(0x7f800000);
+}
+
+// Pass 1, FP64: every unordered pair once (sym_pairs); j's values go through
+// jbuf and k_adj_gather.
+__global__ void __launch_bounds__(32) k_adj_pairs_sym(
+    Params p, HConst kc, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const double *hrec,
+    double *psum, int64_t ps, double pf_hmin, const int *toff, double *jbuf, int64_t jstride, int *err) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  SymAdjSmem &sm = reinterpret_cast<SymAdjSmem *>(dsm)[w];
-  StageN<STAGE_A> &stg = sm.u.st;
-  const unsigned gmask = !act ? 0u : (S >= 32 ? FULL : (((1u << S) - 1u) << (il * S)));
-  const unsigned lt = (1u << lane) - 1u;
-  for (int base = 0; base < town; base += STAGE_A) {
-    const int cnt = stage_window_n<STAGE_A>(p, pool, off, nown, town, base, txf, stg);
-    for (int q = lane; q < NJA * STAGE_A; q += 32) (&sm.js[0][0])[q] = 0.0;
-    __syncwarp();
-    auto test = [&](int k) -> bool {
-      const int j = stg.jidx[k];
-      if (j <= i && j >= s0) return false;  // own leaf: each pair once (j > i); the self pair never
-      if (!pf_i) return true;
-      const float4 xj = stg.pos[k];
-      if (xj.w >= pf_h1max) return true;
-      float dxf = xif.x - xj.x, dyf = xif.y - xj.y, dzf = xif.z - xj.z;
-      if (p.periodic) {
-        if (fabsf(dxf) > 0.5f * p.dxboundf) dxf -= copysignf(p.dxboundf, dxf);
-        if (fabsf(dyf) > 0.5f * p.dyboundf) dyf -= copysignf(p.dyboundf, dyf);
-        if (fabsf(dzf) > 0.5f * p.dzboundf) dzf -= copysignf(p.dzboundf, dzf);
+  ListSmemK &sm = *reinterpret_cast<ListSmemK *>(dsm);
+  const float pf_hf = __double2float_ru(pf_hmin);
+  AdjCell c;
+  if (!adj_cell(c, blockIdx.x, ncell, nodes, leaves, cell_off, cell_nleaf, txf, pf_hf, sm, err)) return;
+  if (c.np > p.minpart) { if (lane_id() == 0) set_error(err, PH_ERR_TREE); return; }
+  int nown, town;
+  owned_prefix(pool, c.off, c.nleaf, c.s0, nown, town);
+  constexpr int NR = (NJA * MAXCELL + 31) / 32;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  double a[HR_A3], xi = 0.0, yi = 0.0, zi = 0.0, f[NJA];
+  sym_pairs<NJA, false>(p, c.cc, c.np, pool, c.off, nown, txf, sm, (int64_t)toff[c.off], jbuf, jstride, tot,
+      [&](float h1) { return adj_accept(h1, pf_hf); },
+      [&](int il) {
+        const int i = c.s0 + il;
+        for (int k = 0; k < HR_A3; ++k) a[k] = hrec[HREC * (size_t)i + k];
+        xi = tx[i]; yi = ty[i]; zi = tz[i];
+        for (int k = 0; k < NJA; ++k) f[k] = 0.0;
+      },
+      [&](int j, int code, double (&jv)[NJA]) {
+        double dx, dy, dz, gd[3], gv[3], oa[4], ob[4];
+        separation_fp64(p, xi, yi, zi, j, code, tx, ty, tz, dx, dy, dz);
+        hydro_pair_rev<double>(kc, dx, dy, dz, fma(dz, dz, fma(dy, dy, dx * dx)), a, hrec + HREC * (size_t)j, gd, gv, oa,
+                               ob);
+        for (int k = 0; k < 3; ++k) { f[k] += gd[k]; f[3 + k] += gv[k]; jv[k] = -gd[k]; jv[3 + k] = -gv[k]; }
+        for (int k = 0; k < 4; ++k) { f[6 + k] += oa[k]; jv[6 + k] = ob[k]; }
+      },
+      [&](int k) -> double { return f[k]; });
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane_id() + 32 * r;
+    if (idx < NJA * c.np) { const int k = idx / c.np; psum[nja_slot(k) * ps + c.s0 + (idx - k * c.np)] = tot[r]; }
+  }
+}
+
+// Pass 1, precision form: each pair from both sides, i's values kept (FP32
+// terms, compensated sums).
+__global__ void __launch_bounds__(32 * ADJ_WARPS, 4) k_adj_pairs_hydro(
+    Params p, HConst kc, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
+    const float *hrec, const double *adj, double *psum, int64_t ps, double pf_hmin, int *err) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const int w = threadIdx.x >> 5;
+  ListSmem &sm = reinterpret_cast<ListSmem *>(dsm)[w];
+  const float pf_hf = __double2float_ru(pf_hmin);
+  AdjCell c;
+  if (!adj_cell(c, blockIdx.x * ADJ_WARPS + w, ncell, nodes, leaves, cell_off, cell_nleaf, txf, pf_hf, sm, err)) return;
+  constexpr int NR = (NJA * MAXCELL + 31) / 32;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  const int qstride = LQ / c.np;
+  ListPos pos;
+  __syncwarp();
+  bool more = true;
+  while (more) {
+    int myc;
+    more = SWEEP_END != sweep_list<false>(p, c.cc, c.np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
+                                          [&](float h1) { return adj_accept(h1, pf_hf); });
+    const QueueLanes ql = balance_queues(c.np, myc, sm);
+    const int il = max(ql.il, 0), i = c.s0 + il;
+    float a[HR_A3];
+    for (int k = 0; k < HR_A3; ++k) a[k] = hrec[HREC * (size_t)i + k];
+    const Sep2 I = sep2_init(txf, txl, i);
+    Kahan f[NJA];
+    for (int m = ql.m0; m < ql.c; m += ql.step) {
+      const int j = sm.qj[il * qstride + m];
+      float dx, dy, dz, r2, gd[3], gv[3], oa[4], ob[4], b[HR_A3];
+      separation_2f(p, I, j, sm.qc[il * qstride + m] & 63, txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
+      const float4 *b4 = reinterpret_cast<const float4 *>(hrec + HREC * (size_t)j);
+#pragma unroll
+      for (int k = 0; k < (HR_A3 + 3) / 4; ++k) {
+        const float4 v = b4[k];
+        b[4 * k] = v.x;
+        if (4 * k + 1 < HR_A3) b[4 * k + 1] = v.y;
+        if (4 * k + 2 < HR_A3) b[4 * k + 2] = v.z;
+        if (4 * k + 3 < HR_A3) b[4 * k + 3] = v.w;
       }
-      const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
-      return r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
-    };
-    const int nr = (cnt + S - 1) / S;
-    int qn = 0;
-    for (int r = 0; r < nr; ++r) {
-      const int k = r * S + stripe;
-      const bool ok = act && k < cnt && test(k);
-      const unsigned b = __ballot_sync(FULL, ok);
-      if (ok) sm.q.k[il][qn + __popc(b & gmask & lt)] = (unsigned short)k;
-      qn += __popc(b & gmask);
-      if (r == nr - 1 || (int)__reduce_max_sync(FULL, (unsigned)qn) > QCAP - S) {
-        __syncwarp();
-        const int nst = (act && qn > stripe) ? (qn - stripe + S - 1) / S : 0;
-        const int nstmax = (int)__reduce_max_sync(FULL, (unsigned)nst);
-        // each particle starts at its own rotation of its queue (the cell's
-        // particles accept nearly the same j in nearly the same order)
-        const int rot = act && qn > 0 ? (il * qn) / np : 0;
-        for (int t = 0; t < nstmax; ++t) {
-          int m = stripe + t * S + rot;
-          if (m >= qn) m -= qn;
-          const bool valid = t < nst;
-          const int kk = valid ? (int)sm.q.k[il][m] : -1;
-          double jv[NJA];
-          for (int v = 0; v < NJA; ++v) jv[v] = 0.0;
-          if (valid) {
-            const int j = stg.jidx[kk], code = stg.code[kk];
-            double dx = xi - (tx[j] + offset_of(code, 0, p.dxbound));
-            double dy = yi - (ty[j] + offset_of(code, 1, p.dybound));
-            double dz = zi - (tz[j] + offset_of(code, 2, p.dzbound));
-            dx = wrap(dx, p.dxbound, p.hdlx, p.periodic); dy = wrap(dy, p.dybound, p.hdly, p.periodic);
-            dz = wrap(dz, p.dzbound, p.hdlz, p.periodic);
-            const double *rj = adj + ADJREC * (size_t)j;
-            const Side<double> sj = load_side(rj);
-            const double dvx = vxi - rj[AR_VX], dvy = vyi - rj[AR_VY], dvz = vzi - rj[AR_VZ];
-            Bar<double> gj;
-            double ax, ay, az;
-            // i receives from j (i's cotangents) ...
-            pair_rev<double, true, false, true>(kc, dx, dy, dz, dvx, dvy, dvz, si, sj, wti, gi, ax, ay, az, &gj);
-            gx += ax; gy += ay; gz += az;
-            double jgx = -ax, jgy = -ay, jgz = -az;
-            // ... and j receives from i (j's cotangents); d -> -d
-            pair_rev<double, true, false, true>(kc, -dx, -dy, -dz, -dvx, -dvy, -dvz, sj, si, load_wt(rj), gj, ax, ay,
-                                                az, &gi);
-            jgx += ax; jgy += ay; jgz += az;
-            gx -= ax; gy -= ay; gz -= az;
-            // d^2 rho / dh^2 of both (m cn h^-5 (12 w + 8 q w' + q^2 w''))
-            const double r = sqrt(dx * dx + dy * dy + dz * dz);
-            double w0, w1, w2;
-            const double qi = r * si.h1, qj = r * sj.h1;
-            if (qi < 2.0) { wshape(qi, w0, w1, w2); d2 += mcn * h51i * (12.0 * w0 + 8.0 * qi * w1 + qi * qi * w2); }
-            double jd2 = 0.0;
-            if (qj < 2.0) {
-              const double h5 = sj.h1 * sj.h1 * sj.h1 * sj.h1 * sj.h1;
-              wshape(qj, w0, w1, w2);
-              jd2 = mcn * h5 * (12.0 * w0 + 8.0 * qj * w1 + qj * qj * w2);
-            }
-            jv[0] = jgx; jv[1] = jgy; jv[2] = jgz;
-            jv[3] = gj.vx.value(); jv[4] = gj.vy.value(); jv[5] = gj.vz.value();
-            jv[6] = gj.h.value(); jv[7] = gj.G.value(); jv[8] = gj.rho1.value(); jv[9] = gj.pro2.value();
-            jv[10] = gj.cs.value(); jv[11] = gj.P.value(); jv[12] = gj.rho.value(); jv[13] = gj.u.value();
-            jv[14] = jd2;
-          }
-          // lanes holding the same j: the lowest adds the others' values in
-          // lane order, then adds the group's sum to j's window slot
-          const unsigned g = __match_any_sync(FULL, valid ? kk : -1 - lane);
-          const int gsz = __popc(g);
-          const int gmax = (int)__reduce_max_sync(FULL, (unsigned)gsz);
-          const bool lead = valid && (g & lt) == 0u;
-          for (int u = 1; u < gmax; ++u) {
-            const int src = u < gsz ? (int)__fns(g, 0, u + 1) : lane;
-            for (int v = 0; v < NJA; ++v) {
-              const double y = __shfl_sync(FULL, jv[v], src);
-              if (lead && u < gsz) jv[v] += y;
-            }
-          }
-          if (lead)
-            for (int v = 0; v < NJA; ++v) sm.js[v][kk] += jv[v];
-          __syncwarp();
-        }
-        qn = 0;
-      }
+      hydro_pair_rev<float>(kc, dx, dy, dz, r2, a, b, gd, gv, oa, ob);
+      for (int k = 0; k < 3; ++k) { f[k].add(gd[k]); f[3 + k].add(gv[k]); }
+      for (int k = 0; k < 4; ++k) f[6 + k].add(oa[k]);
     }
-    __syncwarp();
-    for (int v = 0; v < NJA; ++v)
-      for (int k = lane; k < cnt; k += 32) jbuf[(int64_t)v * jstride + tb + base + k] = sm.js[v][k];
-    __syncwarp();
+    flush_lanes<NJA>(c.np, sm, sm.red, tot, [&](int k) -> double { return f[k].value(); },
+                     [](int, double s, double v) -> double { return s + v; });
   }
-  // the stripes of each particle summed in order (the pass-1 slots; the
-  // physics this pass covers leaves the MHD and gravity slots zero)
-  double *red = sm.u.red;
-  __syncwarp();
-  for (int k = 0; k < NADJ; ++k) {
-    double v = 0.0;
-    if (k < 3) v = k == 0 ? gx : (k == 1 ? gy : gz);
-    else if (k == PA_VX) v = gi.vx.value();
-    else if (k == PA_VY) v = gi.vy.value();
-    else if (k == PA_VZ) v = gi.vz.value();
-    else if (k == PA_H) v = gi.h.value();
-    else if (k == PA_G) v = gi.G.value();
-    else if (k == PA_RHO1) v = gi.rho1.value();
-    else if (k == PA_PRO2) v = gi.pro2.value();
-    else if (k == PA_CS) v = gi.cs.value();
-    else if (k == PA_P) v = gi.P.value();
-    else if (k == PA_RHO) v = gi.rho.value();
-    else if (k == PA_U) v = gi.u.value();
-    else if (k == PA_D2) v = d2;
-    red[lane * NADJ + k] = v;
-  }
-  __syncwarp();
-  if (lane < np) {
-    const size_t ip = (size_t)(s0 + lane);
-    for (int k = 0; k < NADJ; ++k) {
-      double t = 0.0;
-      for (int q = 0; q < S; ++q) t += red[(lane * S + q) * NADJ + k];
-      psum[k * ps + ip] = t;
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane_id() + 32 * r;
+    if (idx < NJA * c.np) {
+      const int k = idx / c.np;
+      const size_t ip = (size_t)(c.s0 + (idx - k * c.np));
+      const double *rec = adj + ADJREC * ip;
+      psum[nja_slot(k) * ps + ip] = nja_scaled(k, tot[r], p.massoftype, rec[AR_H1], rec[AR_G]);
+      if (k == 0) nja_zero(psum, ps, ip);
     }
   }
 }
 
-// Pass 2 on the symmetric lists (FP64 hydro): the pair coefficient
-// m/r [A_i dW(r,h_i)/dr + B_i d2W(r,h_i)/dhdr + A_j dW(r,h_j)/dr + B_j d2W(r,h_j)/dhdr]
-// is symmetric in i and j, so an owned pair adds coef d to i and -coef d to
-// j (d = x_i - x_j); j's three values go through jbuf and k_adj_gather as in
-// pass 1 (NJ = 3 slots: the position gradient)
-struct SymDensSmem {
-  union {
-    StageN<STAGE_A> st;
-    double red[32 * 3];
-  } u;
-  PairQ q;
-  double js[3][STAGE_A];
-};
+// Pass 2 of hydro contexts: the pair coefficient
+//   m/r [A_i dW(r,h_i)/dr + B_i d2W(r,h_i)/dhdr + A_j dW(r,h_j)/dr + B_j d2W(r,h_j)/dhdr]
+// is symmetric in i and j. With A3 and B1 of the record it is hs1 A3 + q hs2 B1
+// of both sides over r.
+template <typename T>
+__device__ __forceinline__ T hydro_dens_coef(T r2, const T *a, const T *b) {
+  const T y = inv_r(r2), r = r2 * y;
+  T qa, s1a, s2a, qb, s1b, s2b, d2;
+  hshape(r, a[0], qa, s1a, s2a, d2);
+  hshape(r, b[0], qb, s1b, s2b, d2);
+  return y * ((s1a * a[1] + (qa * s2a) * a[2]) + (s1b * b[1] + (qb * s2b) * b[2]));
+}
 
-__global__ void __launch_bounds__(32 * ADJ_WARPS) k_adj_dens_sym(
+__global__ void __launch_bounds__(32) k_adj_dens_sym(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
-    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf,
-    const double *adj, double *psum, int64_t ps, double pf_hmin, const int *toff, double *jbuf, int64_t jstride,
-    int *err) {
-  const unsigned FULL = 0xffffffffu;
-  const int w = threadIdx.x >> 5, lane = lane_id();
-  const int cell = blockIdx.x * ADJ_WARPS + w;
-  if (cell >= ncell) return;
-  const Node nd = nodes[leaves[cell]];
-  const int np = nd.count, s0 = nd.start;
-  if (np < 1 || np > MAXCELL) { if (lane == 0) set_error(err, PH_ERR_TREE); return; }
-  const int S = 32 / np;
-  const bool act = lane < np * S;
-  const int il = act ? lane / S : 0, stripe = act ? lane % S : 0;
-  const int i = s0 + il;
-  const double *ri = adj + ADJREC * (size_t)i;
-  const double pm = p.massoftype;
-  const double xi = tx[i], yi = ty[i], zi = tz[i];
-  const double h1i = ri[AR_H1], Ai = ri[AR_A], Bi = ri[AR_B];
-  const double h4i = CNORMK * h1i * h1i * h1i * h1i, h5i = h4i * h1i;
-  const float4 xif = txf[i];
-  const float hi21f = xif.w * xif.w;
-  const bool pf_i = ri[AR_H] > pf_hmin;
-  const float pf_h1max = (float)(1.0 / pf_hmin);
-  const float q2lim = 4.0f * 1.001f;
-  double gx = 0.0, gy = 0.0, gz = 0.0;
-  const int off = cell_off[cell], nleaf = cell_nleaf[cell];
-  int nown = 0, town = 0;
-  for (int e0 = 0; e0 < nleaf; e0 += 32) {
-    const int e = e0 + lane;
-    LeafEntry le{0, 0};
-    if (e < nleaf) le = pool[off + e];
-    const bool own = e < nleaf && le.start >= s0;
-    nown += __popc(__ballot_sync(FULL, own));
-    town += warp_sum_int(own ? (le.cc & 255) : 0);
-    if (!__all_sync(FULL, e >= nleaf || own)) break;
-  }
-  const int64_t tb = (int64_t)toff[off];
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const double *hrec,
+    double *psum, int64_t ps, double pf_hmin, const int *toff, double *jbuf, int64_t jstride, int *err) {
   extern __shared__ __align__(16) unsigned char dsm[];
-  SymDensSmem &sm = reinterpret_cast<SymDensSmem *>(dsm)[w];
-  StageN<STAGE_A> &stg = sm.u.st;
-  const unsigned gmask = !act ? 0u : (S >= 32 ? FULL : (((1u << S) - 1u) << (il * S)));
-  const unsigned lt = (1u << lane) - 1u;
-  for (int base = 0; base < town; base += STAGE_A) {
-    const int cnt = stage_window_n<STAGE_A>(p, pool, off, nown, town, base, txf, stg);
-    for (int q = lane; q < 3 * STAGE_A; q += 32) (&sm.js[0][0])[q] = 0.0;
-    __syncwarp();
-    auto test = [&](int k) -> bool {
-      const int j = stg.jidx[k];
-      if (j <= i && j >= s0) return false;
-      if (!pf_i) return true;
-      const float4 xj = stg.pos[k];
-      if (xj.w >= pf_h1max) return true;
-      float dxf = xif.x - xj.x, dyf = xif.y - xj.y, dzf = xif.z - xj.z;
-      if (p.periodic) {
-        if (fabsf(dxf) > 0.5f * p.dxboundf) dxf -= copysignf(p.dxboundf, dxf);
-        if (fabsf(dyf) > 0.5f * p.dyboundf) dyf -= copysignf(p.dyboundf, dyf);
-        if (fabsf(dzf) > 0.5f * p.dzboundf) dzf -= copysignf(p.dzboundf, dzf);
-      }
-      const float r2f = dxf * dxf + dyf * dyf + dzf * dzf;
-      return r2f * fminf(hi21f, xj.w * xj.w) < q2lim;
-    };
-    const int nr = (cnt + S - 1) / S;
-    int qn = 0;
-    for (int r = 0; r < nr; ++r) {
-      const int k = r * S + stripe;
-      const bool ok = act && k < cnt && test(k);
-      const unsigned b = __ballot_sync(FULL, ok);
-      if (ok) sm.q.k[il][qn + __popc(b & gmask & lt)] = (unsigned short)k;
-      qn += __popc(b & gmask);
-      if (r == nr - 1 || (int)__reduce_max_sync(FULL, (unsigned)qn) > QCAP - S) {
-        __syncwarp();
-        const int nst = (act && qn > stripe) ? (qn - stripe + S - 1) / S : 0;
-        const int nstmax = (int)__reduce_max_sync(FULL, (unsigned)nst);
-        const int rot = act && qn > 0 ? (il * qn) / np : 0;
-        for (int t = 0; t < nstmax; ++t) {
-          int m = stripe + t * S + rot;
-          if (m >= qn) m -= qn;
-          const bool valid = t < nst;
-          const int kk = valid ? (int)sm.q.k[il][m] : -1;
-          double jv0 = 0.0, jv1 = 0.0, jv2 = 0.0;
-          if (valid) {
-            const int j = stg.jidx[kk], code = stg.code[kk];
-            double dx = xi - (tx[j] + offset_of(code, 0, p.dxbound));
-            double dy = yi - (ty[j] + offset_of(code, 1, p.dybound));
-            double dz = zi - (tz[j] + offset_of(code, 2, p.dzbound));
-            dx = wrap(dx, p.dxbound, p.hdlx, p.periodic); dy = wrap(dy, p.dybound, p.hdly, p.periodic);
-            dz = wrap(dz, p.dzbound, p.hdlz, p.periodic);
-            const double r2 = dx * dx + dy * dy + dz * dz, r = sqrt(r2), rinv = inv_sep(r2, r);
-            const double *rj = adj + ADJREC * (size_t)j;
-            double coef = 0.0, w0, w1, w2;
-            const double qi = r * h1i;
-            if (qi < 2.0) {
-              wshape(qi, w0, w1, w2);
-              coef += Ai * h4i * w1 + Bi * h5i * (-4.0 * w1 - qi * w2);
-            }
-            const double h1j = rj[AR_H1];
-            const double qj = r * h1j;
-            if (qj < 2.0) {
-              wshape(qj, w0, w1, w2);
-              const double h4j = CNORMK * h1j * h1j * h1j * h1j;
-              coef += rj[AR_A] * h4j * w1 + rj[AR_B] * h4j * h1j * (-4.0 * w1 - qj * w2);
-            }
-            coef *= pm * rinv;
-            gx += coef * dx; gy += coef * dy; gz += coef * dz;
-            jv0 = -coef * dx; jv1 = -coef * dy; jv2 = -coef * dz;
-          }
-          const unsigned g = __match_any_sync(FULL, valid ? kk : -1 - lane);
-          const int gsz = __popc(g);
-          const int gmax = (int)__reduce_max_sync(FULL, (unsigned)gsz);
-          const bool lead = valid && (g & lt) == 0u;
-          for (int u = 1; u < gmax; ++u) {
-            const int src = u < gsz ? (int)__fns(g, 0, u + 1) : lane;
-            const double y0 = __shfl_sync(FULL, jv0, src), y1 = __shfl_sync(FULL, jv1, src),
-                         y2 = __shfl_sync(FULL, jv2, src);
-            if (lead && u < gsz) { jv0 += y0; jv1 += y1; jv2 += y2; }
-          }
-          if (lead) { sm.js[0][kk] += jv0; sm.js[1][kk] += jv1; sm.js[2][kk] += jv2; }
-          __syncwarp();
-        }
-        qn = 0;
-      }
-    }
-    __syncwarp();
-    for (int v = 0; v < 3; ++v)
-      for (int k = lane; k < cnt; k += 32) jbuf[(int64_t)v * jstride + tb + base + k] = sm.js[v][k];
-    __syncwarp();
+  ListSmemK &sm = *reinterpret_cast<ListSmemK *>(dsm);
+  const float pf_hf = __double2float_ru(pf_hmin);
+  AdjCell c;
+  if (!adj_cell(c, blockIdx.x, ncell, nodes, leaves, cell_off, cell_nleaf, txf, pf_hf, sm, err)) return;
+  if (c.np > p.minpart) { if (lane_id() == 0) set_error(err, PH_ERR_TREE); return; }
+  int nown, town;
+  owned_prefix(pool, c.off, c.nleaf, c.s0, nown, town);
+  constexpr int NR = (3 * MAXCELL + 31) / 32;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  double a[3], xi = 0.0, yi = 0.0, zi = 0.0, f[3];
+  auto load = [&](int i, double (&o)[3]) {
+    const double *r = hrec + HREC * (size_t)i;
+    o[0] = r[HR_H1]; o[1] = r[HR_A3]; o[2] = r[HR_B1];
+  };
+  sym_pairs<3, false>(p, c.cc, c.np, pool, c.off, nown, txf, sm, (int64_t)toff[c.off], jbuf, jstride, tot,
+      [&](float h1) { return adj_accept(h1, pf_hf); },
+      [&](int il) {
+        const int i = c.s0 + il;
+        load(i, a);
+        xi = tx[i]; yi = ty[i]; zi = tz[i];
+        for (int k = 0; k < 3; ++k) f[k] = 0.0;
+      },
+      [&](int j, int code, double (&jv)[3]) {
+        double dx, dy, dz, b[3];
+        load(j, b);
+        separation_fp64(p, xi, yi, zi, j, code, tx, ty, tz, dx, dy, dz);
+        const double co = hydro_dens_coef<double>(fma(dz, dz, fma(dy, dy, dx * dx)), a, b);
+        f[0] = fma(co, dx, f[0]); f[1] = fma(co, dy, f[1]); f[2] = fma(co, dz, f[2]);
+        jv[0] = -co * dx; jv[1] = -co * dy; jv[2] = -co * dz;
+      },
+      [&](int k) -> double { return f[k]; });
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane_id() + 32 * r;
+    if (idx < 3 * c.np) { const int k = idx / c.np; psum[k * ps + c.s0 + (idx - k * c.np)] = tot[r]; }
   }
-  double *red = sm.u.red;
+}
+
+__global__ void __launch_bounds__(32 * ADJ_WARPS, 6) k_adj_dens_hydro(
+    Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
+    const float *hrec, double *psum, int64_t ps, double pf_hmin, int *err) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const int w = threadIdx.x >> 5;
+  ListSmem &sm = reinterpret_cast<ListSmem *>(dsm)[w];
+  const float pf_hf = __double2float_ru(pf_hmin);
+  AdjCell c;
+  if (!adj_cell(c, blockIdx.x * ADJ_WARPS + w, ncell, nodes, leaves, cell_off, cell_nleaf, txf, pf_hf, sm, err)) return;
+  constexpr int NR = (3 * MAXCELL + 31) / 32;
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  const int qstride = LQ / c.np;
+  ListPos pos;
   __syncwarp();
-  red[lane * 3] = gx; red[lane * 3 + 1] = gy; red[lane * 3 + 2] = gz;
-  __syncwarp();
-  if (lane < np) {
-    double t0 = 0, t1 = 0, t2 = 0;
-    for (int q = 0; q < S; ++q) {
-      const double *src = red + (lane * S + q) * 3;
-      t0 += src[0]; t1 += src[1]; t2 += src[2];
+  bool more = true;
+  while (more) {
+    int myc;
+    more = SWEEP_END != sweep_list<false>(p, c.cc, c.np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
+                                          [&](float h1) { return adj_accept(h1, pf_hf); });
+    const QueueLanes ql = balance_queues(c.np, myc, sm);
+    const int il = max(ql.il, 0), i = c.s0 + il;
+    auto load = [&](int n, float (&o)[3]) {
+      const float *r = hrec + HREC * (size_t)n;
+      o[0] = r[HR_H1]; o[1] = r[HR_A3]; o[2] = r[HR_B1];
+    };
+    float a[3];
+    load(i, a);
+    const Sep2 I = sep2_init(txf, txl, i);
+    Kahan f[3];
+    for (int m = ql.m0; m < ql.c; m += ql.step) {
+      const int j = sm.qj[il * qstride + m];
+      float dx, dy, dz, r2, b[3];
+      load(j, b);
+      separation_2f(p, I, j, sm.qc[il * qstride + m] & 63, txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
+      const float co = hydro_dens_coef<float>(r2, a, b);
+      f[0].add(co * dx); f[1].add(co * dy); f[2].add(co * dz);
     }
-    const size_t ip = (size_t)(s0 + lane);
-    psum[ip] = t0; psum[ps + ip] = t1; psum[2 * ps + ip] = t2;
+    flush_lanes<3>(c.np, sm, sm.red, tot, [&](int k) -> double { return f[k].value(); },
+                   [](int, double s, double v) -> double { return s + v; });
+  }
+  for (int r = 0; r < NR; ++r) {
+    const int idx = lane_id() + 32 * r;
+    if (idx < 3 * c.np) { const int k = idx / c.np; psum[k * ps + c.s0 + (idx - k * c.np)] = tot[r]; }
   }
 }
 
@@ -1022,7 +1060,8 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS) k_adj_dens_sym(
 template <int NJ>
 __global__ void k_adj_gather(const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool,
                              const int *cell_off, const int *cell_nleaf, const int *cell_at, const int *toff,
-                             const double *jbuf, int64_t jstride, double *psum, int64_t ps) {
+                             const double *jbuf, int64_t jstride, const double *adj, double pm, double *psum,
+                             int64_t ps) {
   const unsigned FULL = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = lane_id();
   const int cell = blockIdx.x * (blockDim.x >> 5) + w;
@@ -1071,12 +1110,23 @@ __global__ void k_adj_gather(const Node *nodes, const int *leaves, int ncell, co
   for (int r = 0; r < NC; ++r) {
     const int c = lane + 32 * r;
     const int v = c / MAXCELL, t = c % MAXCELL;
-    if (v < NJ && t < np) psum[(int64_t)nja_slot(v) * ps + s0 + t] += acc[r];
+    if (v < NJ && t < np) {
+      const size_t ip = (size_t)(s0 + t);
+      double *dst = psum + (int64_t)(NJ == NJA ? nja_slot(v) : v) * ps + ip;
+      if (NJ == NJA) {
+        const double *rec = adj + ADJREC * ip;
+        *dst = nja_scaled(v, *dst + acc[r], pm, rec[AR_H1], rec[AR_G]);
+        if (v == 0) nja_zero(psum, ps, ip);
+      } else {
+        *dst += acc[r];
+      }
+    }
   }
 }
 
 // chain rule per particle and the implicit-solve coefficients
-__global__ void k_adj_coef(Params p, int n, const double *psum, int64_t ps, double *adj, float *adjf) {
+__global__ void k_adj_coef(Params p, int n, const double *psum, int64_t ps, double *adj, float *adjf, double *hrec,
+                           float *hrecf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double *r = adj + ADJREC * (size_t)i;
@@ -1161,6 +1211,10 @@ __global__ void k_adj_coef(Params p, int n, const double *psum, int64_t ps, doub
   const double H = h_b + G_b * dG_dh;
   r[AR_A] = H * dhdrho * G;
   r[AR_B] = G_b * G * G * dhdrho;
+  // pass 2 of hydro contexts: A h^-4 w' + B h^-5 (-4 w' - q w'') on hs1 and q hs2
+  const double h4 = pm * CNORMK * (h1 * h1) * (h1 * h1), b5 = r[AR_B] * h4 * h1, a4 = r[AR_A] * h4 - 4.0 * b5;
+  if (hrec) { double *o = hrec + HREC * (size_t)i; o[HR_A3] = hs1_fac<double>() * a4; o[HR_B1] = -1.5 * b5; }
+  if (hrecf) { float *o = hrecf + HREC * (size_t)i; o[HR_A3] = (float)a4; o[HR_B1] = (float)(-1.5 * b5); }
   if (adjf) {
     float *q = adjf + ADJREC * (size_t)i;
     q[AR_A] = (float)r[AR_A]; q[AR_B] = (float)r[AR_B]; q[AR_C] = (float)C;
@@ -1320,78 +1374,83 @@ int adjoint_dev(ph_ctx *c, const double *w_dev, const double *wB_dev, double *gx
   cudaMemcpyAsync(c->psum, w_dev, sizeof(double) * n4, cudaMemcpyDeviceToDevice, st);
   if (wB) cudaMemcpyAsync(c->psum + n4, wB_dev, sizeof(double) * n4, cudaMemcpyDeviceToDevice, st);
   const bool mixed = p.precision == PH_PREC_MIXED;
+  // hydro contexts: the joint pair reverse, from its own records (in the force
+  // records' space, which the next force call rebuilds); FP64 on the symmetric
+  // force lists, each pair once
+  const bool hydro = !p.mhd && !p.gravity;
+  const bool sym = hydro && !mixed && c->force_sym && c->toff && c->sym_total > 0;
+  double *hrec = sym ? c->jrec : nullptr;
+  float *hrecf = hydro && mixed ? c->jrecf : nullptr;
   k_adj_prologue<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, c->th, c->gradh64, c->gsoft64, c->vxyzu, c->Bevol,
-                                                c->psum, wB ? c->psum + n4 : nullptr,
-                                                c->alpha1, c->adj, mixed ? c->adjf : nullptr, c->txf);
-  const int smem = ADJ_WARPS * (int)sizeof(PairSmem);
+                                                c->psum, wB ? c->psum + n4 : nullptr, c->alpha1, c->adj,
+                                                mixed && !hydro ? c->adjf : nullptr, hrec, hrecf, c->txf);
+  const int smem = ADJ_WARPS * (int)sizeof(PairSmem), lsmem = ADJ_WARPS * (int)sizeof(ListSmem);
   if (!(c->attr_done & 4u)) {
-    cudaFuncSetAttribute(k_adj_pairs<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_adj_pairs<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_adj_dens<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_adj_pairs<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_adj_pairs<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_adj_pairs_sym, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         ADJ_WARPS * (int)sizeof(SymAdjSmem));
-    cudaFuncSetAttribute(k_adj_dens<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaFuncSetAttribute(k_adj_pairs<double, false>, at, smem);
+    cudaFuncSetAttribute(k_adj_pairs<double, true>, at, smem);
+    cudaFuncSetAttribute(k_adj_dens<double>, at, smem);
+    cudaFuncSetAttribute(k_adj_pairs<float, false>, at, smem);
+    cudaFuncSetAttribute(k_adj_pairs<float, true>, at, smem);
+    cudaFuncSetAttribute(k_adj_dens<float>, at, smem);
+    cudaFuncSetAttribute(k_adj_pairs_sym, at, sym_smem_bytes<NJA>(MAXCELL));
+    cudaFuncSetAttribute(k_adj_dens_sym, at, sym_smem_bytes<3>(MAXCELL));
+    cudaFuncSetAttribute(k_adj_pairs_hydro, at, lsmem);
+    cudaFuncSetAttribute(k_adj_dens_hydro, at, lsmem);
     c->attr_done |= 4u;
   }
   cudaEventRecord(c->evk[0], st);
-  if (mixed) {
-    AdjConst<float> kc;
-    kc.m = (float)p.massoftype; kc.alpha = (float)p.alpha; kc.beta = (float)p.beta; kc.alphau = (float)p.alphau;
-    kc.cn = (float)CNORMK;
-    kc.adiab = !p.isothermal; kc.pdv = p.ipdv_heating > 0; kc.shock = p.ishock_heating > 0; kc.mhd = p.mhd != 0;
-    kc.grav = p.gravity != 0;
-    kc.alphaB = (float)p.alphaB; kc.oc = (float)p.overcleanfac;
-    kc.resist = p.mhd && p.iresistive_heating > 0 && !p.isothermal;
-    kc.induct = p.mhd && (wB || kc.resist);
-    (kc.induct ? k_adj_pairs<float, true> : k_adj_pairs<float, false>)<<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS,
-                                                                        smem, st>>>(
-        p, kc, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->tx, c->ty,
-        c->tz, c->txf, c->adjf, c->psum, c->cap, c->pf_hmin, c->d_err);
-    k_adj_coef<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->psum, c->cap, c->adj, c->adjf);
-    k_adj_dens<float><<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS, smem, st>>>(
-        p, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->tx, c->ty, c->tz,
-        c->txf, c->adjf, c->psum, c->cap, c->pf_hmin, c->d_err);
-  } else {
-    AdjConst<double> kc;
-    kc.m = p.massoftype; kc.alpha = p.alpha; kc.beta = p.beta; kc.alphau = p.alphau; kc.cn = CNORMK;
-    kc.adiab = !p.isothermal; kc.pdv = p.ipdv_heating > 0; kc.shock = p.ishock_heating > 0; kc.mhd = p.mhd != 0;
-    kc.grav = p.gravity != 0;
-    kc.alphaB = p.alphaB; kc.oc = p.overcleanfac;
-    kc.resist = p.mhd && p.iresistive_heating > 0 && !p.isothermal;
-    kc.induct = p.mhd && (wB || kc.resist);
-    // FP64 hydro on the symmetric force lists: each pair once (k_adj_pairs_sym)
-    const bool sym = !p.mhd && !p.gravity && c->force_sym && c->toff && c->sym_total > 0;
-    if (sym) {
-      if (alloc_sym(c, c->sym_total, NJA) != 0) return PH_ERR_CUDA;
-      k_adj_pairs_sym<<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS, ADJ_WARPS * (int)sizeof(SymAdjSmem), st>>>(
-          p, kc, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf,
-          c->adj, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
-      k_adj_gather<NJA><<<nblk(ncell, 4), 128, 0, st>>>(c->nodes, c->leaves, ncell, c->pool, c->cell_off,
-                                                        c->cell_nleaf, c->cell_at, c->toff, c->jbuf,
-                                                        c->jbuf_stride, c->psum, c->cap);
-      count_launch(c, 1);
-    } else {
-      (kc.induct ? k_adj_pairs<double, true> : k_adj_pairs<double, false>)<<<nblk(ncell, ADJ_WARPS),
-                                                                            32 * ADJ_WARPS, smem, st>>>(
-          p, kc, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->tx, c->ty,
-          c->tz, c->txf, c->adj, c->psum, c->cap, c->pf_hmin, c->d_err);
-    }
-    k_adj_coef<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->psum, c->cap, c->adj, nullptr);
-    if (sym) {
-      k_adj_dens_sym<<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS, ADJ_WARPS * (int)sizeof(SymDensSmem), st>>>(
-          p, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->adj,
-          c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
-      k_adj_gather<3><<<nblk(ncell, 4), 128, 0, st>>>(c->nodes, c->leaves, ncell, c->pool, c->cell_off,
+  const HConst hc{p.beta, !p.isothermal && p.alphau != 0.0, p.ipdv_heating > 0, p.ishock_heating > 0};
+  if (hydro && mixed) {
+    k_adj_pairs_hydro<<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS, lsmem, st>>>(
+        p, hc, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl,
+        hrecf, c->adj, c->psum, c->cap, c->pf_hmin, c->d_err);
+    k_adj_coef<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->psum, c->cap, c->adj, nullptr, nullptr, hrecf);
+    k_adj_dens_hydro<<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS, lsmem, st>>>(
+        p, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl, hrecf,
+        c->psum, c->cap, c->pf_hmin, c->d_err);
+  } else if (sym) {
+    if (alloc_sym(c, c->sym_total, NJA) != 0) return PH_ERR_CUDA;
+    k_adj_pairs_sym<<<ncell, 32, sym_smem_bytes<NJA>(p.minpart), st>>>(
+        p, hc, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, hrec,
+        c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
+    k_adj_gather<NJA><<<nblk(ncell, 4), 128, 0, st>>>(c->nodes, c->leaves, ncell, c->pool, c->cell_off,
                                                       c->cell_nleaf, c->cell_at, c->toff, c->jbuf, c->jbuf_stride,
-                                                      c->psum, c->cap);
-      count_launch(c, 1);
-    } else {
-      k_adj_dens<double><<<nblk(ncell, ADJ_WARPS), 32 * ADJ_WARPS, smem, st>>>(
-          p, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->tx, c->ty, c->tz,
-          c->txf, c->adj, c->psum, c->cap, c->pf_hmin, c->d_err);
-    }
+                                                      c->adj, p.massoftype, c->psum, c->cap);
+    k_adj_coef<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->psum, c->cap, c->adj, nullptr, hrec, nullptr);
+    k_adj_dens_sym<<<ncell, 32, sym_smem_bytes<3>(p.minpart), st>>>(
+        p, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, hrec, c->psum,
+        c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
+    k_adj_gather<3><<<nblk(ncell, 4), 128, 0, st>>>(c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf,
+                                                    c->cell_at, c->toff, c->jbuf, c->jbuf_stride, c->adj,
+                                                    p.massoftype, c->psum, c->cap);
+    count_launch(c, 2);
+  } else {
+    auto consts = [&](auto &kc) {
+      using T = decltype(kc.m);
+      kc.m = (T)p.massoftype; kc.alpha = (T)p.alpha; kc.beta = (T)p.beta; kc.alphau = (T)p.alphau; kc.cn = (T)CNORMK;
+      kc.adiab = !p.isothermal; kc.pdv = p.ipdv_heating > 0; kc.shock = p.ishock_heating > 0; kc.mhd = p.mhd != 0;
+      kc.grav = p.gravity != 0;
+      kc.alphaB = (T)p.alphaB; kc.oc = (T)p.overcleanfac;
+      kc.resist = p.mhd && p.iresistive_heating > 0 && !p.isothermal;
+      kc.induct = p.mhd && (wB || kc.resist);
+    };
+    const int nb = nblk(ncell, ADJ_WARPS), nthr = 32 * ADJ_WARPS;
+#define PH_ADJ(T, REC, RECF)                                                                                      \
+  do {                                                                                                            \
+    AdjConst<T> kc;                                                                                               \
+    consts(kc);                                                                                                   \
+    (kc.induct ? k_adj_pairs<T, true> : k_adj_pairs<T, false>)<<<nb, nthr, smem, st>>>(                           \
+        p, kc, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->tx, c->ty,     \
+        c->tz, c->txf, REC, c->psum, c->cap, c->pf_hmin, c->d_err);                                               \
+    k_adj_coef<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->psum, c->cap, c->adj, RECF, nullptr, nullptr);            \
+    k_adj_dens<T><<<nb, nthr, smem, st>>>(p, c->nodes, c->leaves, ncell, c->pool, c->cell_off, c->cell_nleaf,     \
+                                          c->cell_ntrial, c->tx, c->ty, c->tz, c->txf, REC, c->psum, c->cap,      \
+                                          c->pf_hmin, c->d_err);                                                  \
+  } while (0)
+    if (mixed) PH_ADJ(float, c->adjf, c->adjf);
+    else PH_ADJ(double, c->adj, nullptr);
+#undef PH_ADJ
   }
   // self-gravity: the far field's share of the position gradients (slots 3..5)
   if (p.gravity) gravity_adjoint_far(c, c->adj + AR_WX, ADJREC, c->psum + 3 * c->cap, c->cap);

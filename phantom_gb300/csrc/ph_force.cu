@@ -506,12 +506,6 @@ __device__ __forceinline__ void store_pair_sums(PairSmem &sm, int lane, int np, 
   }
 }
 
-// max of two non-negative doubles on the integer pipe (signal speeds: the
-// FP64 max would occupy the scarce FP64 pipe)
-__device__ __forceinline__ double fmax_pos(double a, double b) {
-  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
-}
-
 // ------------------------------------------------------------------ FP64 pair terms
 // The FP64 pair loops are bound by the FP64 pipe (2 lanes per SM and clock), so
 // their cost is the number of FP64 instructions per pair. Each particle's own
@@ -944,143 +938,57 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_force_grav(
 // neighbour tests are those of force_pair_fp64 (the reference's rounding and
 // cached-position rule from the evaluating cell's list); seen from j they differ
 // from the reference's own evaluation by rounding only.
-//
-// Work: the list sweep per batch of BATCH leaf entries (ph_walk.cuh), each
-// batch drained with the lanes dealt out by queue length. The j-side array of a
-// batch (NJ values of up to BATCH leaves) bounds the warps per SM: 24 entries
-// hold the owned half of most lists (37 entries at hfact 1.2) in one batch and
-// leave room for 11 warps at the reference's leaf size. One warp per block: the
-// SM's shared memory then fills in the smallest steps (measured per launch at
-// 64^3, hydro / MHD: 1, 2, 4 warps per block 1.88 / 3.66, 1.95 / 3.98, 2.20 /
-// 5.48 ms; batches of 16 entries 1.96 / 3.72 ms at one warp; the
-// lane-per-stripe loop before this one 2.45 / 4.46 ms).
-struct SymSmem : ListSmemK {
-  // js[NJ][jw] doubles follow, jw = BATCH x leaf size
-  __device__ __forceinline__ double *js() { return reinterpret_cast<double *>(this + 1); }
-};
-template <bool MHD>
-__host__ __device__ constexpr int sym_smem_bytes(int minpart) {
-  return (int)sizeof(SymSmem) + 8 * NJS<MHD>::n * BATCH * minpart;
-}
-
+// (Work decomposition: sym_pairs in ph_walk.cuh. Per launch at 64^3 1.73 ms,
+// against 2.45 for a lane per particle and stripe.)
 template <bool MHD>
 __global__ void __launch_bounds__(32) k_force_sym(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const double *th,
     const float4 *txf, const double *jrec, const double *jmhd, ForceOut out, double *psum, int64_t ps, double pf_hmin,
     const int *toff, double *jbuf, int64_t jstride, int *err) {
-  constexpr int NJ = NJS<MHD>::n;
-  const unsigned FULL = 0xffffffffu;
+  constexpr int NJ = NJS<MHD>::n, NR = (NJ * MAXCELL + 31) / 32;
   const int lane = lane_id(), cell = blockIdx.x;
   if (cell >= ncell) return;
   const Node nd = nodes[leaves[cell]];
   const int np = nd.count, s0 = nd.start;
   if (np < 1 || np > MAXCELL || np > p.minpart) { if (lane == 0) set_error(err, PH_ERR_TREE); return; }
   extern __shared__ __align__(16) unsigned char dsm[];
-  SymSmem &sm = *reinterpret_cast<SymSmem *>(dsm);
-  double *js = sm.js();
-  const int jw = BATCH * p.minpart;
+  ListSmemK &sm = *reinterpret_cast<ListSmemK *>(dsm);
   const float q2lim = 4.0f * 1.001f, INF = __int_as_float(0x7f800000);
   const float pf_hf = __double2float_ru(pf_hmin);
+  auto accept = [&](float h) { return h > pf_hf ? q2lim * (h * h) : INF; };
   if (lane < np) {
     float4 x = txf[s0 + lane];
-    const float hf = d2f_rn(th[s0 + lane]);
-    x.w = hf > pf_hf ? q2lim * (hf * hf) : INF;
+    x.w = accept(d2f_rn(th[s0 + lane]));
     sm.xi[lane] = x;
     sm.ipos[lane] = s0 + lane;
   }
-  const int off = cell_off[cell], nleaf = cell_nleaf[cell];
-  // the owned prefix of the list: entries starting at or after s0
-  int nown = 0, town = 0;
-  for (int e0 = 0; e0 < nleaf; e0 += 32) {
-    const int e = e0 + lane;
-    LeafEntry le{0, 0};
-    if (e < nleaf) le = pool[off + e];
-    const bool own = e < nleaf && le.start >= s0;
-    nown += __popc(__ballot_sync(FULL, own));
-    town += warp_sum_int(own ? (le.cc & 255) : 0);
-    if (!__all_sync(FULL, e >= nleaf || own)) break;
-  }
+  const int off = cell_off[cell];
+  int nown, town;
+  owned_prefix(pool, off, cell_nleaf[cell], s0, nown, town);
   if (lane == 0) {
     atomicAdd(&out.stats[8], (unsigned long long)out.cell_ntrial[cell]);
     atomicAdd(&out.stats[10], (unsigned long long)np * (unsigned long long)town);
   }
-  const int64_t tb = (int64_t)toff[off];  // flattened trial index of the list's first entry
   const float4 cc = make_float4((float)nd.x, (float)nd.y, (float)nd.z, (float)nd.size);
-  const int qstride = LQ / np;
-  const unsigned lt = (1u << lane) - 1u;
-  // totals per (value, particle): f[0..2], f[4..6], with MHD f[7..11], the signal speed
-  constexpr int NR = (NJ * MAXCELL + 31) / 32;
   double tot[NR];
   for (int r = 0; r < NR; ++r) tot[r] = 0.0;
-  for (int q = lane; q < NJ * jw; q += 32) js[q] = 0.0;
-  ListPos pos;
-  while (true) {
-    __syncwarp();
-    int myc;
-    const int st = sweep_list<true>(p, cc, np, pool, off, nown, txf, sm, qstride, pos, myc, [&](float h1) {
-      const float hj = __frcp_rn(h1);
-      return hj > pf_hf ? q2lim * (hj * hj) : INF;
-    });
-    if (st == SWEEP_END) break;
-    const QueueLanes ql = balance_queues(np, myc, sm);
-    const int il = max(ql.il, 0);
-    const IFp64 I = ifp64_init<MHD, false>(p, s0 + il, tx, ty, tz, jrec, jmhd);
-    double f[NF];
-    for (int k = 0; k < NF; ++k) f[k] = 0.0;
-    long long vsigmax = 0;  // largest signal speed (bit pattern)
-    int nbi = 0;
-    const unsigned short *qj = sm.qj + il * qstride;
-    const int nst = ql.c > ql.m0 ? (ql.c - ql.m0 + ql.step - 1) / ql.step : 0;
-    const int nstmax = (int)__reduce_max_sync(FULL, (unsigned)nst);
-    // the particles of a cell accept nearly the same j in nearly the same
-    // order, so aligned queues would put the same j in many lanes at once;
-    // each particle starts at its own rotation of its queue instead
-    const int rot = ql.c > 0 ? (il * ql.c) / np : 0;
-    for (int t = 0; t < nstmax; ++t) {
-      const bool valid = t < nst;
-      int m = ql.m0 + t * ql.step + rot;
-      if (m >= ql.c) m -= ql.c;
-      const int kk = valid ? (int)qj[m] : -1;
-      double jv[NJ];
-      for (int v = 0; v < NJ; ++v) jv[v] = 0.0;
-      if (valid)
-        force_pair_fp64<MHD, false, false, true>(p, I, sm.j[kk], sm.code[kk], tx, ty, tz, jrec, jmhd, nullptr, nullptr,
-                                                 f, vsigmax, nbi, jv);
-      // lanes holding the same j: the lowest adds the others' values in
-      // lane order, then adds the group's sum to j's batch slot
-      const unsigned g = __match_any_sync(FULL, valid ? kk : -1 - lane);
-      const int gs = __popc(g);
-      const int gmax = (int)__reduce_max_sync(FULL, (unsigned)gs);
-      const bool lead = valid && (g & lt) == 0u;
-      for (int u = 1; u < gmax; ++u) {
-        const int src = u < gs ? (int)__fns(g, 0, u + 1) : lane;
-        for (int v = 0; v < NJ - 1; ++v) {
-          const double y = __shfl_sync(FULL, jv[v], src);
-          if (lead && u < gs) jv[v] += y;
-        }
-        const double y = __shfl_sync(FULL, jv[NJ - 1], src);
-        if (lead && u < gs) jv[NJ - 1] = fmax_pos(jv[NJ - 1], y);
-      }
-      if (lead) {
-        for (int v = 0; v < NJ - 1; ++v) js[v * jw + kk] += jv[v];
-        js[(NJ - 1) * jw + kk] = fmax_pos(js[(NJ - 1) * jw + kk], jv[NJ - 1]);
-      }
-      __syncwarp();
-    }
-    // j-side sums of a finished batch -> jbuf (value-major, flattened trial index)
-    if (st == SWEEP_BATCH)
-      for (int v = 0; v < NJ; ++v)
-        for (int k = lane; k < pos.cnt; k += 32) jbuf[(int64_t)v * jstride + tb + pos.nbase + k] = js[v * jw + k];
-    static_assert(NJ <= 12, "lane sums staged in the queues' space");
-    flush_lanes<NJ>(np, sm, sm.red, tot,
-        [&](int k) -> double {
-          return k == NJ - 1 ? __longlong_as_double(vsigmax) : f[njs_slot(k, MHD)];
-        },
-        [](int k, double s, double v) -> double { return k == NJ - 1 ? fmax_pos(s, v) : s + v; });
-    if (st == SWEEP_BATCH)
-      for (int q = lane; q < NJ * jw; q += 32) js[q] = 0.0;
-  }
+  IFp64 I;
+  double f[NF];
+  long long vsigmax = 0;  // largest signal speed (bit pattern)
+  int nbi = 0;
+  sym_pairs<NJ, true>(p, cc, np, pool, off, nown, txf, sm, (int64_t)toff[off], jbuf, jstride, tot,
+      [&](float h1) { return accept(__frcp_rn(h1)); },
+      [&](int il) {
+        I = ifp64_init<MHD, false>(p, s0 + il, tx, ty, tz, jrec, jmhd);
+        for (int k = 0; k < NF; ++k) f[k] = 0.0;
+        vsigmax = 0;
+      },
+      [&](int j, int code, double (&jv)[NJ]) {
+        force_pair_fp64<MHD, false, false, true>(p, I, j, code, tx, ty, tz, jrec, jmhd, nullptr, nullptr, f, vsigmax,
+                                                 nbi, jv);
+      },
+      [&](int k) -> double { return k == NJ - 1 ? __longlong_as_double(vsigmax) : f[njs_slot(k, MHD)]; });
   store_totals<MHD>(sm, NJ, np, p.massoftype, tot, psum, ps);
 }
 
@@ -1600,9 +1508,9 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
     PH_FORCE_ATTR(false, false); PH_FORCE_ATTR(true, false); PH_FORCE_ATTR(false, true); PH_FORCE_ATTR(true, true);
 #undef PH_FORCE_ATTR
     cudaFuncSetAttribute(k_force_sym<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         sym_smem_bytes<false>(MAXCELL));
+                         sym_smem_bytes<NJS<false>::n>(MAXCELL));
     cudaFuncSetAttribute(k_force_sym<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         sym_smem_bytes<true>(MAXCELL));
+                         sym_smem_bytes<NJS<true>::n>(MAXCELL));
     c->attr_done |= 2u;
   }
   const int fw = c->force_warps;
@@ -1639,14 +1547,14 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   } else if (use_sym(c)) {
     cudaEventRecord(c->evk[0], st);
     if (p.mhd) {
-      k_force_sym<true><<<nfc, 32, sym_smem_bytes<true>(p.minpart), st>>>(
+      k_force_sym<true><<<nfc, 32, sym_smem_bytes<NJS<true>::n>(p.minpart), st>>>(
           p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,
           c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
       k_force_gather<true><<<nblk(nfc, 4), 128, 0, st>>>(c->nodes, c->leaves, nfc, c->pool, c->cell_off,
                                                          c->cell_nleaf, c->cell_at, c->toff, c->jbuf,
                                                          c->jbuf_stride, p.massoftype, c->psum, c->cap, c->d_err);
     } else {
-      k_force_sym<false><<<nfc, 32, sym_smem_bytes<false>(p.minpart), st>>>(
+      k_force_sym<false><<<nfc, 32, sym_smem_bytes<NJS<false>::n>(p.minpart), st>>>(
           p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->th, c->txf,
           c->jrec, jmhd, out, c->psum, c->cap, c->pf_hmin, c->toff, c->jbuf, c->jbuf_stride, c->d_err);
       k_force_gather<false><<<nblk(nfc, 4), 128, 0, st>>>(c->nodes, c->leaves, nfc, c->pool, c->cell_off,

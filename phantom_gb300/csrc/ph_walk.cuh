@@ -506,6 +506,118 @@ __device__ __forceinline__ void flush_lanes(int np, const ListBase &sm, double *
   __syncwarp();
 }
 
+// ------------------------------------------------------------------ symmetric pair passes
+// Skeleton of the passes that evaluate every unordered neighbour pair once
+// (force, adjoint). Cell A owns the entries of its trial list that start at or
+// after its own leaf (a prefix: the list is in decreasing order of first
+// particle) and, in its own leaf, the pairs j > i. Each owned batch is swept
+// and drained; a pair's NJ values for j go to a per-batch array in shared
+// memory and from there to jbuf at j's flattened trial index, its values for i
+// stay in the lane (begin/body/get) until the drain's end.
+//
+// The j-side array of a batch (NJ values of up to BATCH leaves) bounds the warps
+// per SM: 24 entries hold the owned half of most lists (37 entries at hfact
+// 1.2) in one batch and leave room for 11 warps of the force pass at the
+// reference's leaf size. One warp per block: the SM's shared memory then fills
+// in the smallest steps (force per launch at 64^3, hydro / MHD: 1, 2, 4 warps
+// per block 1.88 / 3.66, 1.95 / 3.98, 2.20 / 5.48 ms; batches of 16 entries 1.96
+// / 3.72 ms at one warp).
+template <int NJ>
+__host__ __device__ constexpr int sym_smem_bytes(int minpart) {
+  return (int)sizeof(ListSmemK) + 8 * NJ * BATCH * minpart;
+}
+// max of two non-negative doubles on the integer pipe (signal speeds: the
+// FP64 max would occupy the scarce FP64 pipe)
+__device__ __forceinline__ double fmax_pos(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+
+// the owned prefix of a cell's list: entries and trial particles
+__device__ __forceinline__ void owned_prefix(const LeafEntry *__restrict__ pool, int off, int nleaf, int s0, int &nown,
+                                             int &town) {
+  const unsigned FULL = 0xffffffffu;
+  nown = 0; town = 0;
+  for (int e0 = 0; e0 < nleaf; e0 += 32) {
+    const int e = e0 + lane_id();
+    LeafEntry le{0, 0};
+    if (e < nleaf) le = pool[off + e];
+    const bool own = e < nleaf && le.start >= s0;
+    nown += __popc(__ballot_sync(FULL, own));
+    town += warp_sum_int(own ? (le.cc & 255) : 0);
+    if (!__all_sync(FULL, e >= nleaf || own)) break;
+  }
+}
+
+// VMAX: value NJ-1 is a maximum (of non-negative doubles), the others sums.
+// begin(il): the lane's particle; body(j, code, jv): one pair; get(v): the
+// lane's i-side value; tot: totals per (value, particle) as flush_lanes.
+template <int NJ, bool VMAX, int NR, class EW, class Begin, class Body, class Get>
+__device__ __forceinline__ void sym_pairs(const Params &p, float4 cc, int np, const LeafEntry *__restrict__ pool,
+                                          int off, int nown, const float4 *__restrict__ txf, ListSmemK &sm, int64_t tb,
+                                          double *jbuf, int64_t jstride, double (&tot)[NR], EW ew, Begin begin,
+                                          Body body, Get get) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  double *js = reinterpret_cast<double *>(&sm + 1);
+  const int jw = BATCH * p.minpart, qstride = LQ / np;
+  for (int q = lane; q < NJ * jw; q += 32) js[q] = 0.0;
+  ListPos pos;
+  while (true) {
+    __syncwarp();
+    int myc;
+    const int st = sweep_list<true>(p, cc, np, pool, off, nown, txf, sm, qstride, pos, myc, ew);
+    if (st == SWEEP_END) break;
+    const QueueLanes ql = balance_queues(np, myc, sm);
+    const int il = max(ql.il, 0);
+    begin(il);
+    const unsigned short *qj = sm.qj + il * qstride;
+    const int nst = ql.c > ql.m0 ? (ql.c - ql.m0 + ql.step - 1) / ql.step : 0;
+    const int nstmax = (int)__reduce_max_sync(FULL, (unsigned)nst);
+    // the particles of a cell accept nearly the same j in nearly the same
+    // order, so aligned queues would put the same j in many lanes at once;
+    // each particle starts at its own rotation of its queue instead
+    const int rot = ql.c > 0 ? (il * ql.c) / np : 0;
+    for (int t = 0; t < nstmax; ++t) {
+      const bool valid = t < nst;
+      int m = ql.m0 + t * ql.step + rot;
+      if (m >= ql.c) m -= ql.c;
+      const int kk = valid ? (int)qj[m] : -1;
+      double jv[NJ];
+      for (int v = 0; v < NJ; ++v) jv[v] = 0.0;
+      if (valid) body(sm.j[kk], (int)sm.code[kk], jv);
+      // lanes holding the same j: the lowest adds the others' values in
+      // lane order, then adds the group's sum to j's batch slot
+      const unsigned g = __match_any_sync(FULL, valid ? kk : -1 - lane);
+      const int gs = __popc(g);
+      const int gmax = (int)__reduce_max_sync(FULL, (unsigned)gs);
+      const bool lead = valid && (g & lt) == 0u;
+      for (int u = 1; u < gmax; ++u) {
+        const int src = u < gs ? (int)__fns(g, 0, u + 1) : lane;
+        for (int v = 0; v < NJ; ++v) {
+          const double y = __shfl_sync(FULL, jv[v], src);
+          if (lead && u < gs) jv[v] = VMAX && v == NJ - 1 ? fmax_pos(jv[v], y) : jv[v] + y;
+        }
+      }
+      if (lead)
+        for (int v = 0; v < NJ; ++v)
+          js[v * jw + kk] = VMAX && v == NJ - 1 ? fmax_pos(js[v * jw + kk], jv[v]) : js[v * jw + kk] + jv[v];
+      __syncwarp();
+    }
+    // j-side sums of a finished batch -> jbuf (value-major, flattened trial index)
+    if (st == SWEEP_BATCH) {
+      for (int v = 0; v < NJ; ++v)
+        for (int k = lane; k < pos.cnt; k += 32) {
+          jbuf[(int64_t)v * jstride + tb + pos.nbase + k] = js[v * jw + k];
+          js[v * jw + k] = 0.0;
+        }
+    }
+    static_assert(NJ <= 12, "lane sums staged in the queues' space");
+    flush_lanes<NJ>(np, sm, sm.red, tot, get,
+        [](int k, double s, double v) -> double { return VMAX && k == NJ - 1 ? fmax_pos(s, v) : s + v; });
+  }
+}
+
 // The walking cell: position, size and search radius (exact and FP32).
 struct WalkCell {
   double xp, yp, zp, xsizei, rcuti;
