@@ -1377,7 +1377,7 @@ int adjoint_dev(ph_ctx *c, const double *w_dev, const double *wB_dev, double *gx
   // hydro contexts: the joint pair reverse, from its own records (in the force
   // records' space, which the next force call rebuilds); FP64 on the symmetric
   // force lists, each pair once
-  const bool hydro = !p.mhd && !p.gravity;
+  const bool hydro = !p.mhd && !p.gravity && !c->keep_order;
   const bool sym = hydro && !mixed && c->force_sym && c->toff && c->sym_total > 0;
   double *hrec = sym ? c->jrec : nullptr;
   float *hrecf = hydro && mixed ? c->jrecf : nullptr;

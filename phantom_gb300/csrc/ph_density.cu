@@ -787,7 +787,9 @@ int density(ph_ctx *c, int icall) {
       p, c->nodes, c->leaves, act, nact, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->perm, c->tx, c->ty,  \
       c->tz, c->txf, c->txl, c->hcur, Bd, c->jrec, c->bjf, c->psum, c->cap, c->stats, pf_hmin, actf,             \
       c->want_diag ? 1 : 0, c->d_err)
-    if (p.precision == PH_PREC_MIXED) {
+    if (c->keep_order) {
+      ro_density(c, act, nact);
+    } else if (p.precision == PH_PREC_MIXED) {
       if (dB) { if (p.gravity) PH_DENS(true, true, true); else PH_DENS(true, true, false); }
       else { if (p.gravity) PH_DENS(true, false, true); else PH_DENS(true, false, false); }
     } else {

@@ -1482,7 +1482,9 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   double *jmhd = c->jrec + JREC * (size_t)c->cap;
   const bool mixed = p.precision == PH_PREC_MIXED;
   float *jmhdf = c->jrecf + JRECF * (size_t)c->cap;
-  if (mixed)
+  if (c->keep_order)
+    ro_force_prologue(c, vel);
+  else if (mixed)
     k_force_prologue_mixed<<<nblk(nt, 256), 256, 0, st>>>(p, nt, c->perm, c->th, vel, Bv,
                                                           p.ind ? c->gradh : c->gradh_t, eos_t, c->jrec, jmhd,
                                                           c->jrecf, jmhdf, c->txf, c->alpha1, c->ddivvdt_c,
@@ -1528,6 +1530,9 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   }
   if (nfc == 0) {
     cudaEventRecord(c->evk[0], st);
+  } else if (c->keep_order) {
+    cudaEventRecord(c->evk[0], st);
+    ro_force(c);
   } else if (mixed) {
     cudaEventRecord(c->evk[0], st);
 #define PH_FORCE_MIXED(K, M, I, SM)                                                                            \

@@ -49,6 +49,10 @@ int get_nodes(ph_ctx *c, int64_t *nnodes, int32_t *range, double *xcen, double *
 int ref_ncells(ph_ctx *c, int64_t *ncells);
 int density(ph_ctx *c, int icall);
 int force_dev(ph_ctx *c, const double *vel, const double *Bv);
+// hydro evaluations of the precision form's rollouts (ph_rollout_pairs.cu)
+void ro_density(ph_ctx *c, const int *act, int nact);
+void ro_force_prologue(ph_ctx *c, const double *vel);
+void ro_force(ph_ctx *c);
 int derivs_dev(ph_ctx *c, int icall, const double *vel, const double *Bv, double *dtnew);
 int force_lists(ph_ctx *c);
 // symmetric FP64 pair loop: cell_at / cell_tbase (per position / cell), the
@@ -87,7 +91,8 @@ struct ph_ctx {
   int64_t launches = 0;
   bool have_tree = false, have_density = false, have_force = false, have_force_lists = false;
   // kernel attributes (dynamic shared memory) set on this context's device:
-  // bit 0 density pair kernels, bit 1 force pair kernels, bit 2 adjoint
+  // bit 0 density pair kernels, bit 1 force pair kernels, bit 2 adjoint, bit 3
+  // rollout pair kernels
   unsigned attr_done = 0;
   // warps (leaf cells) per block of the pair and walk kernels (ph_autotune)
   int dens_warps = 2, force_warps = 2, walk_warps = 2;
@@ -199,6 +204,9 @@ struct ph_ctx {
   int64_t jbuf_stride = 0, jbuf_bytes = 0;
   int64_t sym_total = 0;  // owned trial entries of the current lists (jbuf rows in use)
 
+  // within a precision-form hydro rollout: evaluations keep the pair order of
+  // ph_rollout_pairs.cu
+  bool keep_order = false;
   double *ro_buf = nullptr;  // rollout adjoint buffer (ph_rollout_adjoint)
   size_t ro_cap = 0;
 

@@ -233,6 +233,13 @@ int ph_rollout_adjoint_full(ph_ctx *c, int32_t nsteps, const double *dts, int32_
     part = wBd + 4 * n;
   }
   double *res = part + 2 * RO_RED_BLOCKS;
+  // precision-form hydro: the evaluations of the rollout keep their pair order
+  // and arithmetic (ph_rollout_pairs.cu)
+  struct KeepOrder {
+    ph_ctx *c;
+    KeepOrder(ph_ctx *cc, bool on) : c(cc) { c->keep_order = on; }
+    ~KeepOrder() { c->keep_order = false; }
+  } keep(c, p.precision == PH_PREC_MIXED && !mhd && !p.gravity);
   cudaStream_t st = c->stream;
   cudaMemsetAsync(c->d_err, 0, sizeof(int), st);
   reset_timers(c);
