@@ -17,6 +17,8 @@
 // only discards pairs that are provably outside the kernel, and every other
 // pair is tested in FP64 with the reference's rounding (no FMA contraction,
 // cached positions x_j + offset for the first 1000 trial entries).
+#include <type_traits>
+
 #include "ph_internal.h"
 #include "ph_walk.cuh"
 
@@ -345,11 +347,11 @@ __device__ void dv_from_sums(const double *rs, double term, double &divv, double
 }
 
 template <bool MIXED>
-__global__ void __launch_bounds__(32 * MAX_WARPS) k_density_dv(
+__global__ void __launch_bounds__(32 * MAX_WARPS, 4) k_density_dv(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
-    const int *cell_nleaf, const int *cell_ntrial, const int *perm, const double *tx, const double *ty,
-    const double *tz, const float4 *txf, const double *hcur, const double *vf, const float *vff,
-    double *dvsum, int64_t ps, double pf_hmin, const int *cells, const unsigned char *actf) {
+    const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
+    const double *hcur, const double *vf, const float *vff, double *dvsum, int64_t ps, double pf_hmin,
+    const int *cells, const unsigned char *actf) {
   extern __shared__ __align__(16) unsigned char dsm[];
   const int w = threadIdx.x >> 5, lane = lane_id();
   const int a = blockIdx.x * (blockDim.x >> 5) + w;
@@ -358,60 +360,67 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_dv(
   const Node nd = nodes[leaves[cell]];
   const int np_all = nd.count, s0 = nd.start;
   if (np_all < 1 || np_all > MAXCELL) return;  // reported by k_density_pairs
-  int np;
-  const unsigned am = cell_active_mask(actf, s0, np_all, np);
+  int np = np_all;
+  unsigned am = 0u;
+  if (actf) am = cell_active_mask(actf, s0, np_all, np);
   if (np == 0) return;
-  const int S = 32 / np;
-  const bool active_lane = lane < np * S;
-  const int il = active_lane ? lane / S : 0, stripe = active_lane ? lane % S : 0;
-  const int i = s0 + cell_pos(am, il);
+  ListSmem &sm = reinterpret_cast<ListSmem *>(dsm)[w];
   const double pm = p.massoftype;
-  const double xi = tx[i], yi = ty[i], zi = tz[i];
-  const double hi = hcur[i], hi1 = ddiv(1.0, hi), hi21 = dmul(hi1, hi1);
-  const float4 xif = txf[i];
-  const float hi21f = (float)hi21, hi1f = (float)hi1, pmf = (float)pm;
-  const bool use_pf = hi > pf_hmin;
-  const float q2lim = 4.0f * 1.001f;
-  const double *vfi = vf + 6 * (size_t)i;
-  double acc[NDV];
-  for (int k = 0; k < NDV; ++k) acc[k] = 0.0;
-  Kahan kacc[MIXED ? NDV : 1];
-  float vfif[6];
-  if (MIXED) for (int k = 0; k < 6; ++k) vfif[k] = vff[6 * (size_t)i + k];
-  const int off = cell_off[cell], nleaf = cell_nleaf[cell], ntrial = cell_ntrial[cell];
-  PairSmem &sm = reinterpret_cast<PairSmem *>(dsm)[w];
-  for (int base = 0; base < ntrial; base += STAGE) {
-    const int cnt = stage_window(p, pool, off, nleaf, ntrial, base, txf, sm.st);
-    auto test = [&](int k) -> bool {
-      if (sm.st.jidx[k] == i) return false;  // ignoreself
-      if (!(use_pf || MIXED)) return true;
-      const float4 xj = sm.st.pos[k];
-      float dxf = xif.x - xj.x, dyf = xif.y - xj.y, dzf = xif.z - xj.z;
-      if (p.periodic) {
-        if (fabsf(dxf) > 0.5f * p.dxboundf) dxf -= copysignf(p.dxboundf, dxf);
-        if (fabsf(dyf) > 0.5f * p.dyboundf) dyf -= copysignf(p.dyboundf, dyf);
-        if (fabsf(dzf) > 0.5f * p.dzboundf) dzf -= copysignf(p.dzboundf, dzf);
-      }
-      return (dxf * dxf + dyf * dyf + dzf * dzf) * hi21f < q2lim;
-    };
-    auto body = [&](int k) {
-      const int n = base + k, j = sm.st.jidx[k];
-      const int code = sm.st.code[k];
-      if constexpr (MIXED) {
-        const float4 xj = sm.st.pos[k];
-        float dx, dy, dz;
-        separation_mixed(p, xi, yi, zi, tx[j], ty[j], tz[j], code, xif.x - xj.x, xif.y - xj.y, xif.z - xj.z, dx, dy,
-                         dz);
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        const float q2 = r2 * hi21f;
-        if (q2 < 4.0f) {
-          const float rij = sqrtf(r2), q = rij * hi1f;
+  const float pmf = d2f_rn(pm);
+  double h1own = 0.0;  // lane il: 1/h of particle il
+  if (lane < np) {
+    const int ip = s0 + (actf ? cell_pos(am, lane) : lane);
+    const double h = hcur[ip];
+    h1own = rcp_fast(h);
+    const float hf = d2f_rn(h);
+    float4 x = txf[ip];
+    x.w = MIXED || h > pf_hmin ? 4.0f * 1.001f * (hf * hf) : __int_as_float(0x7f800000);
+    sm.xi[lane] = x;
+    sm.ipos[lane] = ip;
+  }
+  const float4 cc = make_float4((float)nd.x, (float)nd.y, (float)nd.z, (float)nd.size);
+  const int off = cell_off[cell], nleaf = cell_nleaf[cell], qstride = LQ / np;
+  // totals per (sum, particle): FP32 in the mixed form (each lane's compensated
+  // sum read out, the lanes added in FP32), FP64 in two halves otherwise
+  using T = typename std::conditional<MIXED, float, double>::type;
+  constexpr int RA = MIXED ? NDV : 13, RB = MIXED ? 1 : NDV - RA;
+  constexpr int NRA = (RA * MAXCELL + 31) / 32, NRB = (RB * MAXCELL + 31) / 32;
+  static_assert(32 * RA * sizeof(T) <= sizeof(sm.qj), "lane sums staged in the queues' space");
+  T ta[NRA], tb[NRB];
+  for (int r = 0; r < NRA; ++r) ta[r] = T(0.0);
+  for (int r = 0; r < NRB; ++r) tb[r] = T(0.0);
+  ListPos pos;
+  __syncwarp();
+  bool more = true;
+  while (more) {
+    int myc;
+    more = SWEEP_END != sweep_list<false>(p, cc, np, pool, off, nleaf, txf, sm, qstride, pos, myc,
+                                          [](float) { return 0.0f; });
+    const QueueLanes ql = balance_queues(np, myc, sm);
+    const int il = max(ql.il, 0), i = sm.ipos[il];
+    const double hi1 = __shfl_sync(0xffffffffu, h1own, il);
+    const int *qj = sm.qj + il * qstride;
+    const unsigned char *qc = sm.qc + il * qstride;
+    const auto sum = [](int, T s, T v) -> T { return s + v; };
+    if constexpr (MIXED) {
+      const Sep2 I = sep2_init(txf, txl, i);
+      const float hi1f = d2f_rn(hi1), hi21f = d2f_rn(hi1 * hi1);
+      float vi[6];
+      for (int k = 0; k < 6; ++k) vi[k] = vff[6 * (size_t)i + k];
+      Kahan kacc[NDV];
+      for (int m = ql.m0; m < ql.c; m += ql.step) {
+        const int j = qj[m];
+        float dx, dy, dz, r2;
+        separation_2f(p, I, j, qc[m] & 63, txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
+        if (r2 * hi21f < 4.0f) {
+          const float rij = sqrt_nr(r2), q = rij * hi1f;
           const float grk = q < 1.0f ? q * (2.25f * q - 3.0f) : -0.75f * (q - 2.0f) * (q - 2.0f);
-          const float r1g = grk / (rij + 1.0e-30f);
+          const float r1g = __fdividef(grk, rij + 1.0e-30f);
           const float rux = dx * r1g * pmf, ruy = dy * r1g * pmf, ruz = dz * r1g * pmf;
-          const float *vj = vff + 6 * (size_t)j;
-          const float dvx = vfif[0] - vj[0], dvy = vfif[1] - vj[1], dvz = vfif[2] - vj[2];
-          const float dax = vfif[3] - vj[3], day = vfif[4] - vj[4], daz = vfif[5] - vj[5];
+          const float2 *v2 = reinterpret_cast<const float2 *>(vff + 6 * (size_t)j);
+          const float2 va = v2[0], vb = v2[1], vc = v2[2];
+          const float dvx = vi[0] - va.x, dvy = vi[1] - va.y, dvz = vi[2] - vb.x;
+          const float dax = vi[3] - vb.y, day = vi[4] - vc.x, daz = vi[5] - vc.y;
           kacc[0].add(dvx * rux + dvy * ruy + dvz * ruz);
           kacc[1].add(dvx * rux); kacc[2].add(dvx * ruy); kacc[3].add(dvx * ruz);
           kacc[4].add(dvy * rux); kacc[5].add(dvy * ruy); kacc[6].add(dvy * ruz);
@@ -422,61 +431,52 @@ __global__ void __launch_bounds__(32 * MAX_WARPS) k_density_dv(
           kacc[19].add(-dx * rux); kacc[20].add(-dx * ruy); kacc[21].add(-dx * ruz);
           kacc[22].add(-dy * ruy); kacc[23].add(-dy * ruz); kacc[24].add(-dz * ruz);
         }
-        return;
       }
-      double dx, dy, dz;
-      separation_fp64(p, xi, yi, zi, j, code | (n < CELLCACHE ? QC_CACHED : 0), tx, ty, tz, dx, dy, dz);
-      const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-      const double y = rsqrt_seed(r2), t = r2 * y;
-      const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
-      const double u = fma(-fma(t, pe, t), hi1, 2.0);
-      bool in = u_inside(u);
-      if (u_near_edge(u)) in = inside_exact(dx, dy, dz, hi1);
-      if (in) {
-        const double w = kern_w(u), s = fma(-w, w, u * u);
-        const double r1g = -0.75 * pm * s * fma(y, pe, y);
-        const double rux = dx * r1g, ruy = dy * r1g, ruz = dz * r1g;
-        const double *vj = vf + 6 * (size_t)j;
-        const double dvx = dsub(vfi[0], vj[0]), dvy = dsub(vfi[1], vj[1]), dvz = dsub(vfi[2], vj[2]);
-        acc[0] = dadd(acc[0], dadd(dadd(dmul(dvx, rux), dmul(dvy, ruy)), dmul(dvz, ruz)));
-        acc[1] = dadd(acc[1], dmul(dvx, rux)); acc[2] = dadd(acc[2], dmul(dvx, ruy)); acc[3] = dadd(acc[3], dmul(dvx, ruz));
-        acc[4] = dadd(acc[4], dmul(dvy, rux)); acc[5] = dadd(acc[5], dmul(dvy, ruy)); acc[6] = dadd(acc[6], dmul(dvy, ruz));
-        acc[7] = dadd(acc[7], dmul(dvz, rux)); acc[8] = dadd(acc[8], dmul(dvz, ruy)); acc[9] = dadd(acc[9], dmul(dvz, ruz));
-        const double dax = dsub(vfi[3], vj[3]), day = dsub(vfi[4], vj[4]), daz = dsub(vfi[5], vj[5]);
-        acc[10] = dadd(acc[10], dmul(dax, rux)); acc[11] = dadd(acc[11], dmul(dax, ruy)); acc[12] = dadd(acc[12], dmul(dax, ruz));
-        acc[13] = dadd(acc[13], dmul(day, rux)); acc[14] = dadd(acc[14], dmul(day, ruy)); acc[15] = dadd(acc[15], dmul(day, ruz));
-        acc[16] = dadd(acc[16], dmul(daz, rux)); acc[17] = dadd(acc[17], dmul(daz, ruy)); acc[18] = dadd(acc[18], dmul(daz, ruz));
-        acc[19] = dsub(acc[19], dmul(dx, rux)); acc[20] = dsub(acc[20], dmul(dx, ruy)); acc[21] = dsub(acc[21], dmul(dx, ruz));
-        acc[22] = dsub(acc[22], dmul(dy, ruy)); acc[23] = dsub(acc[23], dmul(dy, ruz)); acc[24] = dsub(acc[24], dmul(dz, ruz));
+      flush_lanes<RA>(np, sm, reinterpret_cast<float *>(sm.qj), ta,
+                      [&](int k) -> float { return __fsub_rn(kacc[k].s, kacc[k].c); }, sum);
+    } else {
+      const double xi = tx[i], yi = ty[i], zi = tz[i];
+      const double *vfi = vf + 6 * (size_t)i;
+      double acc[NDV];
+      for (int k = 0; k < NDV; ++k) acc[k] = 0.0;
+      for (int m = ql.m0; m < ql.c; m += ql.step) {
+        const int j = qj[m];
+        double dx, dy, dz;
+        separation_fp64(p, xi, yi, zi, j, qc[m], tx, ty, tz, dx, dy, dz);
+        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+        const double y = rsqrt_seed(r2), t = r2 * y;
+        const double e = fma(-t, y, 1.0), pe = fma(0.375, e, 0.5) * e;
+        const double u = fma(-fma(t, pe, t), hi1, 2.0);
+        bool in = u_inside(u);
+        if (u_near_edge(u)) in = inside_exact(dx, dy, dz, hi1);
+        if (in) {
+          const double w = kern_w(u), s = fma(-w, w, u * u);
+          const double r1g = -0.75 * pm * s * fma(y, pe, y);
+          const double ru[3] = {dx * r1g, dy * r1g, dz * r1g};
+          const double *vj = vf + 6 * (size_t)j;
+          double d[6];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) d[k] = vfi[k] - vj[k];
+          acc[0] = fma(d[0], ru[0], fma(d[1], ru[1], fma(d[2], ru[2], acc[0])));
+#pragma unroll
+          for (int k = 0; k < 6; ++k)
+            for (int b = 0; b < 3; ++b) acc[1 + 3 * k + b] = fma(d[k], ru[b], acc[1 + 3 * k + b]);
+          acc[19] = fma(-dx, ru[0], acc[19]); acc[20] = fma(-dx, ru[1], acc[20]); acc[21] = fma(-dx, ru[2], acc[21]);
+          acc[22] = fma(-dy, ru[1], acc[22]); acc[23] = fma(-dy, ru[2], acc[23]); acc[24] = fma(-dz, ru[2], acc[24]);
+        }
       }
-    };
-    queue_window(cnt, S, active_lane, il, stripe, sm.q, test, body);
+      flush_lanes<RA>(np, sm, sm.red, ta, [&](int k) -> double { return acc[k]; }, sum);
+      flush_lanes<RB>(np, sm, sm.red, tb, [&](int k) -> double { return acc[RA + k]; }, sum);
+    }
   }
-  // stripes of each particle in stripe order (the whole per-warp scratch):
-  // FP64 in the FP64 form; in the mixed form each stripe's compensated sum
-  // is read out and the stripes added in FP32
-  double *red = reinterpret_cast<double *>(&sm);
-  float *redf = reinterpret_cast<float *>(&sm);
-  static_assert(32 * NDV * sizeof(double) <= sizeof(PairSmem), "dv reduction scratch");
-  __syncwarp();
-  if constexpr (MIXED) {
-    for (int k = 0; k < NDV; ++k) redf[lane * NDV + k] = __fsub_rn(kacc[k].s, kacc[k].c);
-  } else {
-    for (int k = 0; k < NDV; ++k) red[lane * NDV + k] = acc[k];
+  for (int r = 0; r < NRA; ++r) {
+    const int idx = lane + 32 * r;
+    if (idx < RA * np) { const int k = idx / np; dvsum[k * ps + sm.ipos[idx - k * np]] = (double)ta[r]; }
   }
-  __syncwarp();
-  if (lane < np) {
-    const size_t ip = (size_t)(s0 + cell_pos(am, lane));
-    for (int k = 0; k < NDV; ++k) {
-      if constexpr (MIXED) {
-        float r = 0.0f;
-        for (int q = 0; q < S; ++q) r += redf[(lane * S + q) * NDV + k];
-        dvsum[k * ps + ip] = (double)r;
-      } else {
-        double r = 0.0;
-        for (int q = 0; q < S; ++q) r = dadd(r, red[(lane * S + q) * NDV + k]);
-        dvsum[k * ps + ip] = r;
-      }
+  if constexpr (!MIXED) {
+    for (int r = 0; r < NRB; ++r) {
+      const int idx = lane + 32 * r;
+      if (idx < RB * np) { const int k = idx / np; dvsum[(RA + k) * ps + sm.ipos[idx - k * np]] = tb[r]; }
     }
   }
 }
@@ -507,26 +507,30 @@ __global__ void k_dv_finish(int n, const double *dvsum, int64_t ps, const double
 }
 
 // Newton-Raphson update of one particle from its sums (finish_rhosum
-// dens.F90:1486-1500, finish_cell dens.F90:1425-1462)
+// dens.F90:1486-1500, finish_cell dens.F90:1425-1462). FP64 throughout, without
+// its divisions: 1/h by rcp_fast, rho(h) = m (hfact/h)^3, dh/drho = -h^4 /
+// (3 m hfact^3), the convergence test multiplied out. The FP64 pipe bounds the
+// finish; per pass over 2M particles 0.96 -> 0.37 ms.
 struct DensNR {
-  double rhoi, gradhi, dhdrhoi, omegai, hmine;
+  double rhoi, dhdrhoi, omega1, hmine;  // omega1 = 1/Omega
   bool conv;
 };
 __device__ __forceinline__ DensNR dens_nr(const Params &p, double r0, double r1, double hme, double h_old) {
   const double pm = p.massoftype;
   DensNR o;
-  const double h1 = ddiv(1.0, hme), h21 = dmul(h1, h1), h31 = dmul(h1, h21), h41 = dmul(h21, h21);
-  o.rhoi = dmul(dmul(CNORMK, dadd(r0, dmul(1.0, pm))), h31);
-  o.gradhi = dmul(dmul(CNORMK, dadd(r1, dmul(-3.0, pm))), h41);
-  o.dhdrhoi = dhdrho(hme, pm, p.hfact);
-  o.omegai = dsub(1.0, dmul(o.dhdrhoi, o.gradhi));
-  const double rhohi = rhoh(hme, pm, p.hfact);
-  const double func = dsub(rhohi, o.rhoi);
-  const double dfdh1 = (o.omegai > TINY_D) ? ddiv(o.dhdrhoi, o.omegai) : ddiv(o.dhdrhoi, fabs(dadd(o.omegai, EPS_D)));
-  double hnew = dsub(hme, dmul(func, dfdh1));
-  if (hnew > dmul(1.2, hme)) hnew = dmul(1.2, hme);
-  else if (hnew < dmul(0.8, hme)) hnew = dmul(0.8, hme);
-  o.conv = (ddiv(fabs(dsub(hnew, hme)), h_old) < p.tolh) && o.omegai > 0.0 && hme > 0.0;
+  const double h1 = rcp_fast(hme), h21 = h1 * h1, ch21 = CNORMK * h21;
+  o.rhoi = (r0 + pm) * (ch21 * h1);
+  const double gradhi = fma(-3.0, pm, r1) * (ch21 * h21);
+  const double h2 = hme * hme, mh3 = pm * (p.hfact * p.hfact * p.hfact);
+  o.dhdrhoi = -(h2 * h2) * p.dhdrho1;
+  const double omegai = fma(-o.dhdrhoi, gradhi, 1.0);
+  const double func = fma(mh3, h21 * h1, -o.rhoi);  // rho(h) - rho
+  o.omega1 = rcp_fast(omegai);
+  const double dfdh1 = o.dhdrhoi * (omegai > TINY_D ? o.omega1 : rcp_fast(fabs(omegai + EPS_D)));
+  double hnew = fma(-func, dfdh1, hme);
+  if (hnew > 1.2 * hme) hnew = 1.2 * hme;
+  else if (hnew < 0.8 * hme) hnew = 0.8 * hme;
+  o.conv = fabs(hnew - hme) < p.tolh * h_old && omegai > 0.0 && hme > 0.0;
   o.hmine = o.conv ? hme : hnew;
   return o;
 }
@@ -575,7 +579,7 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
   double hm = mine ? o.hmine : 0.0;
   for (int m = 1; m < FIN_SEG; m <<= 1) {
     conv &= __shfl_xor_sync(FULL, conv, m);
-    hm = fmax(hm, __shfl_xor_sync(FULL, hm, m));
+    hm = fmax_pos(hm, __shfl_xor_sync(FULL, hm, m));
   }
   if (icall == 0) conv = 1;
   const double hmax_new = dmul(1.01, hm);
@@ -626,9 +630,8 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
     if (mine && hme >= 0.0) {
       const int ntry = cell_ntrial[cell];
       const int pid = perm[ip];
-      const double h1 = ddiv(1.0, hme), h21 = dmul(h1, h1), h41 = dmul(h21, h21);
-      const double grad = ddiv(1.0, o.omegai);
-      const double hfin = hrho(o.rhoi, pm, p.hfact);
+      const double grad = o.omega1;
+      const double hfin = p.hfact * cbrt_fast(pm * rcp_fast(o.rhoi));  // hrho (part.F90:845-850)
       out.xyzh[4 * (size_t)pid + 3] = hfin;
       out.th[ip] = hfin;
       if (hfin < 0.0) set_error(err, PH_ERR_NEG_H);
@@ -636,8 +639,8 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
       out.gradh64[ip] = grad;
       float gsf = 0.0f;
       if (p.gravity) {
-        double gs = dmul(dadd(psum[2 * ps + ip], dmul(DPHIDH0, pm)), h21);
-        gs = dmul(gs, o.dhdrhoi);
+        const double h1 = rcp_fast(hme);
+        const double gs = fma(DPHIDH0, pm, psum[2 * ps + ip]) * (h1 * h1) * o.dhdrhoi;
         gsf = (float)gs;
         out.gsoft64[ip] = gs;
       }
@@ -648,7 +651,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
         if (p.gravity || p.ind) out.gradh[2 * (size_t)pid + 1] = gsf;
       }
       rhoi_max = o.rhoi;
-      const double term = dmul(dmul(dmul(CNORMK, (double)gradf), ddiv(1.0, o.rhoi)), h41);
+      double term = 0.0;
+      if (out.dvterm || out.diag) {
+        const double h1 = ddiv(1.0, hme), h21 = dmul(h1, h1), h41 = dmul(h21, h21);
+        term = dmul(dmul(dmul(CNORMK, (double)gradf), ddiv(1.0, o.rhoi)), h41);
+      }
       if (out.dvterm) out.dvterm[ip] = term;
       // getdv is .false. under CONST_AV (dens.F90:1638-1640)
       if (out.diag) out.divcurlv[pid] = -(float)(0.0 * term);
@@ -678,7 +685,7 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
     for (int k = 0; k < 5; ++k) sv[k] += __shfl_xor_sync(FULL, sv[k], m);
     for (int k = 0; k < 2; ++k) mx[k] = max(mx[k], __shfl_xor_sync(FULL, mx[k], m));
   }
-  rhoi_max = warp_max(rhoi_max);
+  for (int m = 16; m > 0; m >>= 1) rhoi_max = fmax_pos(rhoi_max, __shfl_xor_sync(FULL, rhoi_max, m));
   if (lane == 0) {
     if (sv[3]) {
       atomicAdd(&bst[0], sv[0]); atomicAdd(&bst[1], sv[1]); atomicMax(&bst[2], mx[0]);
@@ -818,17 +825,17 @@ int density(ph_ctx *c, int icall) {
     k_dv_gather<<<nblk(nt, 256), 256, 0, st>>>(nt, c->perm, vel, c->fxyzu, c->jrec, mixed ? c->jrecf : nullptr);
     if (!c->dvsum && alloc_dvsum(c) != 0) return PH_ERR_CUDA;
     const int dw = c->dens_warps;
-    const int smem = dw * (int)sizeof(PairSmem);
+    const int smem = dw * (int)sizeof(ListSmem);
     const int *dv_cells = p.ind ? c->cell_act : nullptr;
     const int ndv = p.ind ? c->ncell_act : ncell;
     if (mixed)
       k_density_dv<true><<<nblk(ndv, dw), 32 * dw, smem, st>>>(
-          p, c->nodes, c->leaves, ndv, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->perm, c->tx, c->ty,
-          c->tz, c->txf, c->hcur, c->jrec, c->jrecf, c->dvsum, c->cap, pf_hmin, dv_cells, actf);
+          p, c->nodes, c->leaves, ndv, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl, c->hcur,
+          c->jrec, c->jrecf, c->dvsum, c->cap, pf_hmin, dv_cells, actf);
     else
       k_density_dv<false><<<nblk(ndv, dw), 32 * dw, smem, st>>>(
-          p, c->nodes, c->leaves, ndv, c->pool, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->perm, c->tx, c->ty,
-          c->tz, c->txf, c->hcur, c->jrec, nullptr, c->dvsum, c->cap, pf_hmin, dv_cells, actf);
+          p, c->nodes, c->leaves, ndv, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl, c->hcur,
+          c->jrec, nullptr, c->dvsum, c->cap, pf_hmin, dv_cells, actf);
     if (p.curlv && alloc_curlv(c) != 0) return PH_ERR_CUDA;
     k_dv_finish<<<nblk(nt, 256), 256, 0, st>>>(nt, c->dvsum, c->cap, c->dvterm_t, c->perm, c->ddivvdt_c, c->dvdx_c,
                                                 c->divcurlv, p.curlv ? c->curl3 : nullptr, c->want_diag ? 1 : 0,

@@ -484,9 +484,8 @@ __device__ __forceinline__ QueueLanes balance_queues(int np, int c, ListBase &sm
 // values pass through shared memory at red (32 RW doubles, free when every lane
 // is done with the queues) and are added in lane order, so totals are
 // deterministic.
-template <int RW, int NR, class Get, class Add>
-__device__ __forceinline__ void flush_lanes(int np, const ListBase &sm, double *red, double (&tot)[NR], Get get,
-                                            Add add) {
+template <int RW, int NR, class T, class Get, class Add>
+__device__ __forceinline__ void flush_lanes(int np, const ListBase &sm, T *red, T (&tot)[NR], Get get, Add add) {
   static_assert(RW * MAXCELL <= 32 * NR, "totals per lane");
   const int lane = lane_id();
   __syncwarp();
@@ -498,7 +497,7 @@ __device__ __forceinline__ void flush_lanes(int np, const ListBase &sm, double *
     const int idx = lane + 32 * r;
     if (idx < RW * np) {
       const int k = idx / np, il = idx - k * np;
-      const double *src = red + (int)sm.first[il] * RW + k;
+      const T *src = red + (int)sm.first[il] * RW + k;
       const int nl = sm.lanes[il];
       for (int q = 0; q < nl; ++q) tot[r] = add(k, tot[r], src[q * RW]);
     }
