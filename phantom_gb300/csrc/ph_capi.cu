@@ -61,7 +61,7 @@ int alloc_all(ph_ctx *c, int64_t cap) {
   // a generation holds the children of nodes of more than minpart particles
   // (sized for the smallest accepted leaf size)
   c->gen_cap = (int)(2 * (n / (MINPART_LO + 1)) + 2 * (size_t)c->lvl_cap + 64);
-  r |= dalloc(c, &c->gen_a, (size_t)c->gen_cap); r |= dalloc(c, &c->gen_b, (size_t)c->gen_cap);
+  r |= dalloc(c, &c->gen_a, (size_t)c->gen_cap);
   r |= dalloc(c, &c->mtab, (size_t)SMALL + 1);
   r |= dalloc(c, &c->gen_com, 4 * (size_t)c->gen_cap);
   r |= dalloc(c, &c->lvl_bb_a, 6 * (size_t)c->lvl_cap); r |= dalloc(c, &c->lvl_bb_b, 6 * (size_t)c->lvl_cap);

@@ -9,7 +9,7 @@
 
 namespace ph {
 
-constexpr int SMALL = 2048;  // nodes with <= SMALL particles are built by the generation kernels
+constexpr int SMALL = 2048;  // subtrees of <= SMALL particles are built by one block each
 constexpr int CHUNK = 2048;  // elements per block in the large-node level kernels
 constexpr int PSUM = 24;     // per-particle pair-sum slots (density, force and adjoint pair kernels)
 constexpr int LENFG = 20;    // gravity far-field coefficients per node (kdtree.F90 lenfgrav)
@@ -92,7 +92,7 @@ struct ph_ctx {
   bool have_tree = false, have_density = false, have_force = false, have_force_lists = false;
   // kernel attributes (dynamic shared memory) set on this context's device:
   // bit 0 density pair kernels, bit 1 force pair kernels, bit 2 adjoint, bit 3
-  // rollout pair kernels
+  // rollout pair kernels, bit 4 subtrees
   unsigned attr_done = 0;
   // warps (leaf cells) per block of the pair and walk kernels (ph_autotune)
   int dens_warps = 2, force_warps = 2, walk_warps = 2;
@@ -166,7 +166,7 @@ struct ph_ctx {
   // level-build scratch
   int *lvl_a = nullptr, *lvl_b = nullptr;
   double *lvl_bb_a = nullptr, *lvl_bb_b = nullptr;
-  ph::GenEntry *gen_a = nullptr, *gen_b = nullptr;  // small-node generation lists
+  ph::GenEntry *gen_a = nullptr;  // subtree roots; node lists of the refit
   double *gen_com = nullptr;  // per generation entry: centre of mass and hmax
   double *mtab = nullptr;    // mtab[k]: sequential sum of k particle masses, k <= SMALL
   double mtab_pm = -1.0;     // the particle mass mtab was built for

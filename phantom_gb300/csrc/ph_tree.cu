@@ -5,8 +5,8 @@
 // reference's treecache/inodeparts (kdtree.F90:429-456), with an FP32 copy of
 // the positions (txf) that moves with them. Nodes larger than SMALL particles
 // are built level by level with multi-block kernels (chunk partials, then one
-// warp per node to combine them); nodes of at most SMALL particles are then
-// built generation by generation (k_small_com, k_small_split).
+// warp per node to combine them); the subtrees of nodes of at most SMALL
+// particles are then built in shared memory, one block each (k_subtree).
 //
 // Parity notes: the two-pointer partition of sort_particles_in_cell pairs the
 // k-th misplaced element of the left region (left to right) with the k-th
@@ -642,31 +642,42 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) k_big_fin5(const int *lvl, int
 }
 
 // ------------------------------------------------------------------ small nodes
-// Nodes of at most SMALL particles are built generation by generation, the
-// children of one generation forming the next, with what construct_node does
-// for each (kdtree.F90:639-896). FP64 work on this GPU is expensive (one warp
-// instruction per ~17 SM cycles whatever the active lanes, 68-cycle dependent
-// latency), so only the reference's sequential centre-of-mass sums (the
-// pivot, hence the partition, depends on their rounding) are FP64 chains, one
-// lane per node; the quadrupoles, which no tree decision reads, are parallel
-// FP64 sums; everything else is integer or FP32, with exact FP64 only where
-// an FP32 bound cannot decide:
+// Nodes of at most SMALL particles (the level kernels' last children, or the
+// root) are roots of independent subtrees. k_subtree builds each whole subtree
+// in one block, its positions in shared memory, generation by generation (the
+// children of one generation form the next), with what construct_node does
+// for each node (kdtree.F90:639-896). Two launches, a host round trip and a
+// pass over global memory per generation made up 1.6 ms of a 2M-particle build
+// and nearly all of a 2000-particle one.
+//
+// FP64 work on this GPU is expensive (one warp instruction per ~17 SM cycles
+// whatever the active lanes, 68-cycle dependent latency), so:
+// * centre of mass: the reference's sequential FP64 sum, whose rounding decides
+//   the pivot and hence the partition, evaluated 32 terms at a time in integer
+//   arithmetic (warp_seq_sum) or, for short nodes, by one lane per node and axis;
 // * node mass: the sequential sum of n particle masses, from a table;
 // * hmax, child bounding boxes and the pivot test: order-preserving integer
 //   keys of the FP64 values (exact);
 // * size: max of the exact FP64 r^2 over the particles that FP32 bounds
-//   cannot exclude from being the maximum.
-// Node ids in this part do not depend on the order of the generation list: a
-// right child is the only right child starting at its first particle s (id
-// subbase + 2 s + 1), a left child the only left child ending at its last
-// particle e (id subbase + 2 e).
-__global__ void k_mass_table(double pm, double *mtab) {
-  double sm = 0.0;
-  mtab[0] = 0.0;
-  for (int k = 1; k <= SMALL; ++k) { sm = dadd(sm, pm); mtab[k] = sm; }
+//   cannot exclude from being the maximum;
+// * the quadrupoles, which no tree decision reads, are parallel FP64 sums.
+// Node ids do not depend on the order of the generation list: a right child is
+// the only right child starting at its first particle s (id subbase + 2 s + 1),
+// a left child the only left child ending at its last particle e (id subbase +
+// 2 e).
+// Sequential sums of k equal particle masses (node masses, chunk partials):
+// 2048 dependent additions, 105 us for one GPU lane, 2 us for the host, with
+// the same IEEE rounding.
+static void mass_table(ph_ctx *c, double pm) {
+  if (c->mtab_pm == pm) return;
+  std::vector<double> t((size_t)SMALL + 1, 0.0);
+  for (int k = 1; k <= SMALL; ++k) t[(size_t)k] = t[(size_t)k - 1] + pm;
+  cudaMemcpyAsync(c->mtab, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice, c->stream);
+  cudaStreamSynchronize(c->stream);
+  c->mtab_pm = pm;
 }
 
-// K1 of a generation: centre of mass of the nodes, one lane per node and
+// Centre of mass of a list of nodes (revtree), one lane per node and
 // axis, each lane running the reference's sequential FP64 sum of one
 // coordinate over its node. The chains are latency bound (68 cycles per
 // dependent FP64 add) and the early generations hold few nodes, so the three
@@ -730,24 +741,95 @@ __global__ void __launch_bounds__(32) k_small_com(Params p, const GenEntry *cur,
   if (valid) com[4 * (size_t)g + axis] = acc;
 }
 
-__device__ __forceinline__ long long warp_min_ll(long long v) {
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 __device__ __forceinline__ long long warp_max_ll(long long v) {
   for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 
-// K2 of a generation: a segment of SEG lanes per node (32 / SEG nodes per
-// warp), lanes over its particles (coalesced): size, hmax, the count on the
-// pivot's left, both sides' bounding boxes, the partition and the node
-// record; the children go to the next generation. Segment reductions are
-// xor butterflies inside the segment; the partition's ballots run a
-// warp-uniform number of rounds. Slots in the next generation and the node
-// list are taken with one atomic per warp. maxcnt receives the largest child
-// count (the next generation's segment width).
-constexpr int SPLIT_WARPS = 4;
+// s = x_0 + x_1 + ... in the reference's order and rounding (every partial sum
+// rounded to nearest even), 32 terms at a time. While the running sum stays in
+// one binade, with ulp u, it is an integer S times u, and adding x gives S +
+// floor(x/u) + r with r = 1 where the fraction of x/u is above 1/2, or is 1/2
+// and S + floor(x/u) is odd. So apart from ties the increments are integers
+// that do not depend on S and add in any order; a tie needs the parity of the
+// sum before it, which is even right after another tie and otherwise follows
+// from the parities of the increments in between. A term that takes the sum out
+// of its binade is added on its own; a chunk that keeps changing binade (a node
+// across a coordinate's zero) is added term by term. 2048 terms of one sign take
+// 73 rounds instead of 2048 dependent additions of 68 cycles. x_k = fac A[ix[k]].
+__device__ __forceinline__ double warp_seq_sum(const double *A, const unsigned short *ix, int n, double fac,
+                                               bool fac1) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  constexpr long long HID = 1ll << 52, MANT = HID - 1, TOP = 1ll << 53;
+  double s = 0.0;
+  for (int base = 0; base < n; base += 32) {
+    const int cnt = min(32, n - base);
+    double x = lane < cnt ? A[ix[base + lane]] : 0.0;
+    if (!fac1) x = dmul(fac, x);
+    const long long xb = __double_as_longlong(x);
+    const int exf = (int)(xb >> 52) & 0x7ff, ex = max(exf, 1);
+    const long long mx = (xb & MANT) | (exf ? HID : 0ll);
+    int k = 0, tries = 0;  // k: next term to add
+    while (k < cnt) {
+      const long long sb = __double_as_longlong(s);
+      const int es = (int)(sb >> 52) & 0x7ff;
+      if (es == 0 || es == 0x7ff || tries >= 4) {
+        const int stop = tries >= 4 ? cnt : k + 1;
+        for (; k < stop; ++k) s = dadd(s, __shfl_sync(FULL, x, k));
+        continue;
+      }
+      ++tries;
+      const long long S0 = (sb & MANT) | HID;
+      const bool in = lane >= k && lane < cnt, bad = in && ex > es;
+      const int t = min(max(es - ex, 0), 62);  // x = mx u / 2^t
+      const long long v = !in || bad ? 0ll : ((xb ^ sb) < 0 ? -mx : mx);
+      const long long f = v >> t, rem = v & ((1ll << t) - 1), half = t > 0 ? 1ll << (t - 1) : 0ll;
+      const bool tie = t > 0 && rem == half && v != 0;
+      long long d = f + (t > 0 && rem > half ? 1 : 0);
+      const unsigned T = __ballot_sync(FULL, tie), D = __ballot_sync(FULL, (d & 1) != 0);
+      if (tie) {
+        const unsigned prev = T & lt;
+        unsigned odd = D & lt;
+        if (prev) odd &= ~((2u << (31 - __clz(prev))) - 1u);
+        const long long par = (__popc(odd) + (prev ? 0 : (int)(S0 & 1))) & 1;
+        d = f + ((par + f) & 1);
+      }
+      const long long sign = sb & (long long)0xfff0000000000000ull;  // sign and exponent
+      if (!__any_sync(FULL, v < 0 || bad)) {
+        // all increments >= 0: the sum stays in the binade if its end does
+        const unsigned lo = __reduce_add_sync(FULL, (unsigned)d & 0x1fffffu),
+                       mi = __reduce_add_sync(FULL, (unsigned)(d >> 21) & 0x1fffffu),
+                       hi = __reduce_add_sync(FULL, (unsigned)(d >> 42));
+        const long long R = S0 + (long long)lo + ((long long)mi << 21) + ((long long)hi << 42);
+        if (R < TOP) {
+          s = __longlong_as_double(sign | (R & MANT));
+          k = cnt;
+          continue;
+        }
+      }
+      long long R = d;
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(FULL, R, o);
+        if (lane >= o) R += y;
+      }
+      R += S0;
+      const unsigned fail = __ballot_sync(FULL, in && (bad || !(R > HID && R < TOP)));
+      const int first = fail ? __ffs(fail) - 1 : cnt;
+      if (first > k) {
+        const long long q = __shfl_sync(FULL, R, first - 1);
+        s = __longlong_as_double(sign | (q & MANT));
+        k = first;
+      }
+      if (k < cnt) {
+        s = dadd(s, __shfl_sync(FULL, x, k));
+        ++k;
+      }
+    }
+  }
+  return s;
+}
 
 template <int SEG>
 __device__ __forceinline__ long long seg_min_ll(long long v) {
@@ -765,214 +847,325 @@ __device__ __forceinline__ int seg_sum_int(int v) {
   return v;
 }
 
+// a subtree in shared memory: original positions (FP64 and the FP32 copies of
+// the bounds), the permutation ix, the partition's pair positions, and the two
+// generation lists (first particle, count, flags: split axis in bits 0-1, bit
+// 2 a right child, bit 3 the subtree's root; parent id)
+constexpr int SUB_THREADS = 512, SUB_WARPS = SUB_THREADS / 32;
+constexpr int SUB_SEQ = 64;  // nodes up to this size: one lane per chain
+struct SubList { unsigned short *st, *ct; unsigned char *fl; int *par; };
+struct Sub {
+  double *X, *Y, *Z, *com;
+  float *XF, *YF, *ZF;
+  unsigned short *ix, *pr;
+  SubList cur, next;
+};
+__host__ __device__ __forceinline__ int sub_cap(int minpart) { return 2 * (SMALL / (minpart + 1)) + 4; }
+__host__ __device__ __forceinline__ size_t sub_smem(int minpart) {
+  return (size_t)SMALL * (3 * 8 + 3 * 4 + 2 * 2) + (size_t)sub_cap(minpart) * (3 * 8 + 2 * (4 + 2 + 2 + 1)) + 64;
+}
+
+// global arrays the subtree kernel reads and writes
+struct SubOut {
+  Node *nodes;
+  NodeF *nodesf;
+  double *nmass, *nquads;
+  int *leaf_at, *node_list, *node_count;
+};
+
+// longest bounding-box extent (kdtree.F90:800-816)
+__device__ __forceinline__ int split_axis(double e0, double e1, double e2) {
+  int ax = 0;
+  double em = e0;
+  if (e1 > em) { ax = 1; em = e1; }
+  if (e2 > em) ax = 2;
+  return ax;
+}
+
+// One generation's nodes, a segment of SEG lanes per node (32 / SEG nodes per
+// warp): size, hmax, the count on the pivot's left, both sides' bounding
+// boxes, the partition and the node record; the children go to the next list.
+// Segment reductions are xor butterflies inside the segment; the partition's
+// ballots run a warp-uniform number of rounds.
 template <int SEG>
-__global__ void __launch_bounds__(32 * SPLIT_WARPS) k_small_split(
-    Params p, const GenEntry *cur, int ncur, const double *com, GenEntry *next, int *nnext, int next_cap,
-    const double *mtab, Node *nodes, double *nmass, double *nquads, double *tx, double *ty, double *tz, double *th,
-    int *perm, float4 *txf, int *pairpos, int subbase, int *leaf_at, int *lvlstat, NodeF *nodesf, int *node_list,
-    int *node_count, int *maxcnt, int *err) {
+__device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0, int level, int rootid, int subbase,
+                                 const double *mtab, const double *th, const SubOut &out, int *nnext, int *gmax,
+                                 int *lvl, int *err) {
   const unsigned FULL = 0xffffffffu;
   constexpr int NSEG = 32 / SEG;
   const int lane = lane_id(), seg = lane / SEG, sl = lane % SEG;
   const unsigned segmask = (SEG == 32) ? FULL : (((1u << SEG) - 1u) << (seg * SEG));
   const unsigned lt = (1u << lane) - 1u;
-  const int wg = blockIdx.x * SPLIT_WARPS + (threadIdx.x >> 5);
-  if (wg * NSEG >= ncur) return;  // warp-uniform
-  const int g = wg * NSEG + seg;
-  const bool valid = g < ncur;
-  GenEntry e{};
-  if (valid) e = cur[g];
-  const int s = e.start, n = valid ? e.count : 0, end = s + n;
-  double sx = 0.0, sy = 0.0, sz = 0.0;
-  if (valid) { sx = com[4 * (size_t)g]; sy = com[4 * (size_t)g + 1]; sz = com[4 * (size_t)g + 2]; }
-  const bool split = valid && n > p.minpart;  // kdtree.F90:792
-  int ax = 0;
-  if (split) {  // longest bounding-box extent (kdtree.F90:800-816)
-    const double ext0 = e.bb[3] - e.bb[0], ext1 = e.bb[4] - e.bb[1], ext2 = e.bb[5] - e.bb[2];
-    double em = ext0;
-    if (ext1 > em) { ax = 1; em = ext1; }
-    if (ext2 > em) ax = 2;
-  }
-  const double pv = ax == 0 ? sx : (ax == 1 ? sy : sz);
-  const long long pk = dkey(pv);
-  // size (kdtree.F90:734-741): FP32 separations d' obey |d' - d| <= E with
-  // E = 2^-23 (|x'| + |c'| + |d'|) per axis, which brackets each r^2; only
-  // particles whose upper bound reaches the largest lower bound can hold the
-  // maximum, and their r^2 is evaluated exactly in FP64.
-  const float cxf = (float)sx, cyf = (float)sy, czf = (float)sz;
-  const float eps23 = 1.1920929e-7f;
-  float lbmax = 0.0f;
-  long long l0 = KEY_HI, l1 = KEY_HI, l2 = KEY_HI, l3 = KEY_LO, l4 = KEY_LO, l5 = KEY_LO;
-  long long r0 = KEY_HI, r1 = KEY_HI, r2 = KEY_HI, r3 = KEY_LO, r4 = KEY_LO, r5 = KEY_LO;
-  long long hk = KEY_LO;
-  int nl = 0;
-  for (int i = s + sl; i < end; i += SEG) {
-    const float4 q = txf[i];
-    const float dx = q.x - cxf, dy = q.y - cyf, dz = q.z - czf;
-    const float ex = eps23 * (fabsf(q.x) + fabsf(cxf) + fabsf(dx));
-    const float ey = eps23 * (fabsf(q.y) + fabsf(cyf) + fabsf(dy));
-    const float ez = eps23 * (fabsf(q.z) + fabsf(czf) + fabsf(dz));
-    const float bx = fmaxf(fabsf(dx) - ex, 0.0f), by = fmaxf(fabsf(dy) - ey, 0.0f), bz = fmaxf(fabsf(dz) - ez, 0.0f);
-    lbmax = fmaxf(lbmax, bx * bx + by * by + bz * bz);
-    hk = max(hk, dkey(th[i]));  // hmax (kdtree.F90:661): a max, so lanes over particles
-    if (split) {
-      // count on the pivot's left (kdtree.F90:954-955) and both sides' boxes
-      const long long kx = dkey(tx[i]), ky = dkey(ty[i]), kz = dkey(tz[i]);
-      const long long kc = ax == 0 ? kx : (ax == 1 ? ky : kz);
-      if (kc <= pk) {
-        ++nl;
-        l0 = min(l0, kx); l1 = min(l1, ky); l2 = min(l2, kz); l3 = max(l3, kx); l4 = max(l4, ky); l5 = max(l5, kz);
-      } else {
-        r0 = min(r0, kx); r1 = min(r1, ky); r2 = min(r2, kz); r3 = max(r3, kx); r4 = max(r4, ky); r5 = max(r5, kz);
+  for (int wg = threadIdx.x >> 5; wg * NSEG < ncur; wg += SUB_WARPS) {
+    const int g = wg * NSEG + seg;
+    const bool valid = g < ncur;
+    const int s = valid ? S.cur.st[g] : 0, n = valid ? S.cur.ct[g] : 0, end = s + n;
+    const int fl = valid ? S.cur.fl[g] : 0;
+    double sx = 0.0, sy = 0.0, sz = 0.0;
+    if (valid) { sx = S.com[3 * g]; sy = S.com[3 * g + 1]; sz = S.com[3 * g + 2]; }
+    const bool split = valid && n > p.minpart;  // kdtree.F90:792
+    const int ax = fl & 3;
+    const double pv = ax == 0 ? sx : (ax == 1 ? sy : sz);
+    const long long pk = dkey(pv);
+    // size (kdtree.F90:734-741): FP32 separations d' obey |d' - d| <= E with
+    // E = 2^-23 (|x'| + |c'| + |d'|) per axis, which brackets each r^2; only
+    // particles whose upper bound reaches the largest lower bound can hold the
+    // maximum, and their r^2 is evaluated exactly in FP64.
+    const float cxf = (float)sx, cyf = (float)sy, czf = (float)sz;
+    const float eps23 = 1.1920929e-7f;
+    float lbmax = 0.0f;
+    long long l0 = KEY_HI, l1 = KEY_HI, l2 = KEY_HI, l3 = KEY_LO, l4 = KEY_LO, l5 = KEY_LO;
+    long long r0 = KEY_HI, r1 = KEY_HI, r2 = KEY_HI, r3 = KEY_LO, r4 = KEY_LO, r5 = KEY_LO;
+    long long hk = KEY_LO;
+    int nl = 0;
+    for (int i = s + sl; i < end; i += SEG) {
+      const int o = S.ix[i];
+      const float qx = S.XF[o], qy = S.YF[o], qz = S.ZF[o];
+      const float dx = qx - cxf, dy = qy - cyf, dz = qz - czf;
+      const float ex = eps23 * (fabsf(qx) + fabsf(cxf) + fabsf(dx));
+      const float ey = eps23 * (fabsf(qy) + fabsf(cyf) + fabsf(dy));
+      const float ez = eps23 * (fabsf(qz) + fabsf(czf) + fabsf(dz));
+      const float bx = fmaxf(fabsf(dx) - ex, 0.0f), by = fmaxf(fabsf(dy) - ey, 0.0f), bz = fmaxf(fabsf(dz) - ez, 0.0f);
+      lbmax = fmaxf(lbmax, bx * bx + by * by + bz * bz);
+      hk = max(hk, dkey(th[s0 + o]));  // hmax (kdtree.F90:661): a max, so lanes over particles
+      if (split) {
+        // count on the pivot's left (kdtree.F90:954-955) and both sides' boxes
+        const long long kx = dkey(S.X[o]), ky = dkey(S.Y[o]), kz = dkey(S.Z[o]);
+        const long long kc = ax == 0 ? kx : (ax == 1 ? ky : kz);
+        if (kc <= pk) {
+          ++nl;
+          l0 = min(l0, kx); l1 = min(l1, ky); l2 = min(l2, kz); l3 = max(l3, kx); l4 = max(l4, ky); l5 = max(l5, kz);
+        } else {
+          r0 = min(r0, kx); r1 = min(r1, ky); r2 = min(r2, kz); r3 = max(r3, kx); r4 = max(r4, ky); r5 = max(r5, kz);
+        }
       }
     }
-  }
-  for (int o = SEG / 2; o > 0; o >>= 1) lbmax = fmaxf(lbmax, __shfl_xor_sync(FULL, lbmax, o));
-  lbmax *= 0.999999f;
-  long long r2k = 0;
-  for (int i = s + sl; i < end; i += SEG) {
-    const float4 q = txf[i];
-    const float dx = q.x - cxf, dy = q.y - cyf, dz = q.z - czf;
-    const float ex = eps23 * (fabsf(q.x) + fabsf(cxf) + fabsf(dx));
-    const float ey = eps23 * (fabsf(q.y) + fabsf(cyf) + fabsf(dy));
-    const float ez = eps23 * (fabsf(q.z) + fabsf(czf) + fabsf(dz));
-    const float bx = fabsf(dx) + ex, by = fabsf(dy) + ey, bz = fabsf(dz) + ez;
-    if ((bx * bx + by * by + bz * bz) * 1.000001f >= lbmax) {
-      const double ddx = tx[i] - sx, ddy = ty[i] - sy, ddz = tz[i] - sz;
-      r2k = max(r2k, dkey(r2_exact(ddx, ddy, ddz)));
-    }
-  }
-  r2k = seg_max_ll<SEG>(r2k);
-  const double hm = fmax(0.0, dunkey(seg_max_ll<SEG>(hk)));
-  if (p.gravity) {
-    // quadrupoles (kdtree.F90:744-752): m sum of dx_a dx_b; lanes over
-    // particles, then a fixed-order butterfly (no tree decision reads them)
-    double q0 = 0, q1 = 0, q2 = 0, q3 = 0, q4 = 0, q5 = 0;
+    for (int o = SEG / 2; o > 0; o >>= 1) lbmax = fmaxf(lbmax, __shfl_xor_sync(FULL, lbmax, o));
+    lbmax *= 0.999999f;
+    long long r2k = 0;
     for (int i = s + sl; i < end; i += SEG) {
-      const double dx = tx[i] - sx, dy = ty[i] - sy, dz = tz[i] - sz;
-      q0 = fma(dx, dx, q0); q1 = fma(dx, dy, q1); q2 = fma(dx, dz, q2);
-      q3 = fma(dy, dy, q3); q4 = fma(dy, dz, q4); q5 = fma(dz, dz, q5);
+      const int o = S.ix[i];
+      const float qx = S.XF[o], qy = S.YF[o], qz = S.ZF[o];
+      const float dx = qx - cxf, dy = qy - cyf, dz = qz - czf;
+      const float ex = eps23 * (fabsf(qx) + fabsf(cxf) + fabsf(dx));
+      const float ey = eps23 * (fabsf(qy) + fabsf(cyf) + fabsf(dy));
+      const float ez = eps23 * (fabsf(qz) + fabsf(czf) + fabsf(dz));
+      const float bx = fabsf(dx) + ex, by = fabsf(dy) + ey, bz = fabsf(dz) + ez;
+      if ((bx * bx + by * by + bz * bz) * 1.000001f >= lbmax)
+        r2k = max(r2k, dkey(r2_exact(S.X[o] - sx, S.Y[o] - sy, S.Z[o] - sz)));
     }
-    for (int o = SEG / 2; o > 0; o >>= 1) {
-      q0 += __shfl_xor_sync(FULL, q0, o); q1 += __shfl_xor_sync(FULL, q1, o); q2 += __shfl_xor_sync(FULL, q2, o);
-      q3 += __shfl_xor_sync(FULL, q3, o); q4 += __shfl_xor_sync(FULL, q4, o); q5 += __shfl_xor_sync(FULL, q5, o);
-    }
-    if (valid && sl == 0) {
-      const double pm = p.massoftype;
-      double *qo = nquads + 6 * (size_t)e.id;
-      qo[0] = pm * q0; qo[1] = pm * q1; qo[2] = pm * q2; qo[3] = pm * q3; qo[4] = pm * q4; qo[5] = pm * q5;
-    }
-  }
-  nl = seg_sum_int<SEG>(nl);
-  const bool noswap = split && (nl == n || nl == 0);
-  if (noswap) {
-    // no split along the axis: halves by position, no swaps (kdtree.F90:856-865)
-    nl = n / 2;
-    l0 = l1 = l2 = r0 = r1 = r2 = KEY_HI;
-    l3 = l4 = l5 = r3 = r4 = r5 = KEY_LO;
-    for (int i = s + sl; i < end; i += SEG) {
-      const long long kx = dkey(tx[i]), ky = dkey(ty[i]), kz = dkey(tz[i]);
-      if (i < s + nl) {
-        l0 = min(l0, kx); l1 = min(l1, ky); l2 = min(l2, kz); l3 = max(l3, kx); l4 = max(l4, ky); l5 = max(l5, kz);
-      } else {
-        r0 = min(r0, kx); r1 = min(r1, ky); r2 = min(r2, kz); r3 = max(r3, kx); r4 = max(r4, ky); r5 = max(r5, kz);
+    r2k = seg_max_ll<SEG>(r2k);
+    const double hm = fmax(0.0, dunkey(seg_max_ll<SEG>(hk)));
+    const int id = (fl & 8) ? rootid : ((fl & 4) ? subbase + 2 * (s0 + s) + 1 : subbase + 2 * (s0 + end - 1));
+    if (p.gravity) {
+      // quadrupoles (kdtree.F90:744-752): m sum of dx_a dx_b; lanes over
+      // particles, then a fixed-order butterfly (no tree decision reads them)
+      double q0 = 0, q1 = 0, q2 = 0, q3 = 0, q4 = 0, q5 = 0;
+      for (int i = s + sl; i < end; i += SEG) {
+        const int o = S.ix[i];
+        const double dx = S.X[o] - sx, dy = S.Y[o] - sy, dz = S.Z[o] - sz;
+        q0 = fma(dx, dx, q0); q1 = fma(dx, dy, q1); q2 = fma(dx, dz, q2);
+        q3 = fma(dy, dy, q3); q4 = fma(dy, dz, q4); q5 = fma(dz, dz, q5);
+      }
+      for (int o = SEG / 2; o > 0; o >>= 1) {
+        q0 += __shfl_xor_sync(FULL, q0, o); q1 += __shfl_xor_sync(FULL, q1, o); q2 += __shfl_xor_sync(FULL, q2, o);
+        q3 += __shfl_xor_sync(FULL, q3, o); q4 += __shfl_xor_sync(FULL, q4, o); q5 += __shfl_xor_sync(FULL, q5, o);
+      }
+      if (valid && sl == 0) {
+        const double pm = p.massoftype;
+        double *qo = out.nquads + 6 * (size_t)id;
+        qo[0] = pm * q0; qo[1] = pm * q1; qo[2] = pm * q2; qo[3] = pm * q3; qo[4] = pm * q4; qo[5] = pm * q5;
       }
     }
-  }
-  l0 = seg_min_ll<SEG>(l0); l1 = seg_min_ll<SEG>(l1); l2 = seg_min_ll<SEG>(l2);
-  l3 = seg_max_ll<SEG>(l3); l4 = seg_max_ll<SEG>(l4); l5 = seg_max_ll<SEG>(l5);
-  r0 = seg_min_ll<SEG>(r0); r1 = seg_min_ll<SEG>(r1); r2 = seg_min_ll<SEG>(r2);
-  r3 = seg_max_ll<SEG>(r3); r4 = seg_max_ll<SEG>(r4); r5 = seg_max_ll<SEG>(r5);
-  // partition: the k-th element > pivot left of the boundary (counted from
-  // the left) swaps with the k-th element <= pivot right of it (counted
-  // from the right), as the two-pointer loop of the reference pairs them
-  const bool part = split && !noswap;
-  const double *cx = ax == 0 ? tx : (ax == 1 ? ty : tz);
-  const int bnd = s + nl;
-  const int tr = part ? (end - bnd + SEG - 1) / SEG : 0, tl = part ? (nl + SEG - 1) / SEG : 0;
-  const int trmax = (int)__reduce_max_sync(FULL, (unsigned)tr), tlmax = (int)__reduce_max_sync(FULL, (unsigned)tl);
-  int m2 = 0;
-  for (int t = 0; t < trmax; ++t) {
-    const int i = end - 1 - t * SEG - sl;
-    const bool f = t < tr && i >= bnd && dkey(cx[i]) <= pk;
-    const unsigned bal = __ballot_sync(FULL, f) & segmask;
-    if (f) pairpos[s + m2 + __popc(bal & lt)] = i;
-    m2 += __popc(bal);
-  }
-  __syncwarp();
-  int m = 0;
-  for (int t = 0; t < tlmax; ++t) {
-    const int i = s + t * SEG + sl;
-    const bool f = t < tl && i < bnd && dkey(cx[i]) > pk;
-    const unsigned bal = __ballot_sync(FULL, f) & segmask;
-    if (f) {
-      const int r = m + __popc(bal & lt);
-      if (r < m2) swap_rows(tx, ty, tz, th, perm, txf, i, pairpos[s + r]);
+    nl = seg_sum_int<SEG>(nl);
+    const bool noswap = split && (nl == n || nl == 0);
+    if (noswap) {
+      // no split along the axis: halves by position, no swaps (kdtree.F90:856-865)
+      nl = n / 2;
+      l0 = l1 = l2 = r0 = r1 = r2 = KEY_HI;
+      l3 = l4 = l5 = r3 = r4 = r5 = KEY_LO;
+      for (int i = s + sl; i < end; i += SEG) {
+        const int o = S.ix[i];
+        const long long kx = dkey(S.X[o]), ky = dkey(S.Y[o]), kz = dkey(S.Z[o]);
+        if (i < s + nl) {
+          l0 = min(l0, kx); l1 = min(l1, ky); l2 = min(l2, kz); l3 = max(l3, kx); l4 = max(l4, ky); l5 = max(l5, kz);
+        } else {
+          r0 = min(r0, kx); r1 = min(r1, ky); r2 = min(r2, kz); r3 = max(r3, kx); r4 = max(r4, ky); r5 = max(r5, kz);
+        }
+      }
     }
-    m += __popc(bal);
-  }
-  if (part && m != m2 && sl == 0) set_error(err, PH_ERR_TREE);
-  __syncwarp();
-  // node records, next-generation entries and statistics (segment leaders)
-  const bool lead = valid && sl == 0;
-  const double sm = valid ? mtab[n] : 0.0;
-  Node nd{};
-  nd.x = sx; nd.y = sy; nd.z = sz; nd.size = sqrt(dunkey(r2k)) + EPS_D; nd.hmax = hm;
-  nd.start = s; nd.count = n; nd.level = e.level; nd.parent = e.parent;
-  nd.left = -1; nd.right = -1;
-  const unsigned bsplit = __ballot_sync(FULL, lead && split);
-  const unsigned bleaf = __ballot_sync(FULL, lead && !split);
-  int base_list = 0, base_next = 0;
-  if (bsplit) {
-    const int first = __ffs(bsplit) - 1;
-    if (lane == first) {
-      base_list = atomicAdd(node_count, 2 * __popc(bsplit));
-      base_next = atomicAdd(nnext, 2 * __popc(bsplit));
+    if (__any_sync(FULL, split)) {
+      l0 = seg_min_ll<SEG>(l0); l1 = seg_min_ll<SEG>(l1); l2 = seg_min_ll<SEG>(l2);
+      l3 = seg_max_ll<SEG>(l3); l4 = seg_max_ll<SEG>(l4); l5 = seg_max_ll<SEG>(l5);
+      r0 = seg_min_ll<SEG>(r0); r1 = seg_min_ll<SEG>(r1); r2 = seg_min_ll<SEG>(r2);
+      r3 = seg_max_ll<SEG>(r3); r4 = seg_max_ll<SEG>(r4); r5 = seg_max_ll<SEG>(r5);
     }
-    base_list = __shfl_sync(FULL, base_list, first);
-    base_next = __shfl_sync(FULL, base_next, first);
+    // partition: the k-th element > pivot left of the boundary (counted from
+    // the left) swaps with the k-th element <= pivot right of it (counted
+    // from the right), as the two-pointer loop of the reference pairs them
+    const bool part = split && !noswap;
+    const double *cx = ax == 0 ? S.X : (ax == 1 ? S.Y : S.Z);
+    const int bnd = s + nl;
+    const int tr = part ? (end - bnd + SEG - 1) / SEG : 0, tl = part ? (nl + SEG - 1) / SEG : 0;
+    const int trmax = (int)__reduce_max_sync(FULL, (unsigned)tr), tlmax = (int)__reduce_max_sync(FULL, (unsigned)tl);
+    int m2 = 0;
+    for (int t = 0; t < trmax; ++t) {
+      const int i = end - 1 - t * SEG - sl;
+      const bool f = t < tr && i >= bnd && dkey(cx[S.ix[i]]) <= pk;
+      const unsigned bal = __ballot_sync(FULL, f) & segmask;
+      if (f) S.pr[s + m2 + __popc(bal & lt)] = (unsigned short)i;
+      m2 += __popc(bal);
+    }
+    __syncwarp();
+    int m = 0;
+    for (int t = 0; t < tlmax; ++t) {
+      const int i = s + t * SEG + sl;
+      const bool f = t < tl && i < bnd && dkey(cx[S.ix[i]]) > pk;
+      const unsigned bal = __ballot_sync(FULL, f) & segmask;
+      if (f) {
+        const int r = m + __popc(bal & lt);
+        if (r < m2) {
+          const int q = S.pr[s + r];
+          const unsigned short a = S.ix[i];
+          S.ix[i] = S.ix[q];
+          S.ix[q] = a;
+        }
+      }
+      m += __popc(bal);
+    }
+    if (part && m != m2 && sl == 0) set_error(err, PH_ERR_TREE);
+    __syncwarp();
+    // node records and next-generation entries (segment leaders)
+    const bool lead = valid && sl == 0;
+    const unsigned bsplit = __ballot_sync(FULL, lead && split);
+    int base = 0;
+    if (bsplit) {
+      const int first = __ffs(bsplit) - 1;
+      if (lane == first) base = atomicAdd(nnext, 2 * __popc(bsplit));
+      base = __shfl_sync(FULL, base, first);
+    }
+    if (!lead) continue;
+    Node nd{};
+    nd.x = sx; nd.y = sy; nd.z = sz; nd.size = sqrt(dunkey(r2k)) + EPS_D; nd.hmax = hm;
+    nd.start = s0 + s; nd.count = n; nd.level = level; nd.parent = S.cur.par[g];
+    nd.left = -1; nd.right = -1;
+    if (split) { nd.left = subbase + 2 * (s0 + bnd - 1); nd.right = subbase + 2 * (s0 + bnd) + 1; }
+    out.nodes[id] = nd;
+    out.nodesf[id] = make_nodef(nd);
+    out.nmass[id] = mtab[n];
+    if (!split) {
+      out.leaf_at[s0 + s] = id;
+      atomicMax(&lvl[0], level);
+      atomicMin(&lvl[1], level);
+      continue;
+    }
+    const int q = base + 2 * __popc(bsplit & lt);
+    S.next.st[q] = (unsigned short)s; S.next.ct[q] = (unsigned short)nl; S.next.par[q] = id;
+    S.next.fl[q] = (unsigned char)split_axis(dunkey(l3) - dunkey(l0), dunkey(l4) - dunkey(l1), dunkey(l5) - dunkey(l2));
+    S.next.st[q + 1] = (unsigned short)bnd; S.next.ct[q + 1] = (unsigned short)(n - nl); S.next.par[q + 1] = id;
+    S.next.fl[q + 1] =
+        (unsigned char)(4 | split_axis(dunkey(r3) - dunkey(r0), dunkey(r4) - dunkey(r1), dunkey(r5) - dunkey(r2)));
+    atomicMax(gmax, max(nl, n - nl));
   }
-  // deepest and shallowest leaf levels, one atomic each per warp
-  int lmax = (lead && !split) ? e.level : 0, lmin = (lead && !split) ? e.level : (1 << 30);
-  for (int o = 16; o > 0; o >>= 1) {
-    lmax = max(lmax, __shfl_xor_sync(FULL, lmax, o));
-    lmin = min(lmin, __shfl_xor_sync(FULL, lmin, o));
+}
+
+__global__ void __launch_bounds__(SUB_THREADS, 2) k_subtree(Params p, const GenEntry *gen, const double *mtab,
+                                                            double *tx, double *ty, double *tz, double *th, int *perm,
+                                                            float4 *txf, int subbase, SubOut out, int *lvlstat,
+                                                            int *err) {
+  extern __shared__ __align__(16) unsigned char dsm[];
+  __shared__ int nnext, gmax, lbase, lvl[2];
+  const GenEntry e = gen[blockIdx.x];
+  const int n = e.count, s0 = e.start, tid = threadIdx.x, cap = sub_cap(p.minpart);
+  if (n < 1 || n > SMALL) { if (tid == 0) set_error(err, PH_ERR_TREE); return; }
+  Sub S;
+  S.X = reinterpret_cast<double *>(dsm); S.Y = S.X + SMALL; S.Z = S.Y + SMALL; S.com = S.Z + SMALL;
+  S.XF = reinterpret_cast<float *>(S.com + 3 * cap); S.YF = S.XF + SMALL; S.ZF = S.YF + SMALL;
+  S.cur.par = reinterpret_cast<int *>(S.ZF + SMALL); S.next.par = S.cur.par + cap;
+  S.ix = reinterpret_cast<unsigned short *>(S.next.par + cap); S.pr = S.ix + SMALL;
+  S.cur.st = S.pr + SMALL; S.cur.ct = S.cur.st + cap; S.next.st = S.cur.ct + cap; S.next.ct = S.next.st + cap;
+  S.cur.fl = reinterpret_cast<unsigned char *>(S.next.ct + cap); S.next.fl = S.cur.fl + cap;
+  for (int i = tid; i < n; i += SUB_THREADS) {
+    S.X[i] = tx[s0 + i]; S.Y[i] = ty[s0 + i]; S.Z[i] = tz[s0 + i];
+    const float4 q = txf[s0 + i];
+    S.XF[i] = q.x; S.YF[i] = q.y; S.ZF[i] = q.z;
+    S.ix[i] = (unsigned short)i;
   }
-  // largest child count of the warp (the next generation's segment width)
-  int cmax = (lead && split) ? max(nl, n - nl) : 0;
-  for (int o = 16; o > 0; o >>= 1) cmax = max(cmax, __shfl_xor_sync(FULL, cmax, o));
-  if (lane == 0) {
-    if (bleaf) { atomicMax(&lvlstat[0], lmax); atomicMin(&lvlstat[1], lmin); }
-    if (bsplit) atomicMax(maxcnt, cmax);
+  if (tid == 0) {
+    S.cur.st[0] = 0; S.cur.ct[0] = (unsigned short)n; S.cur.par[0] = e.parent;
+    S.cur.fl[0] = (unsigned char)(8 | split_axis(e.bb[3] - e.bb[0], e.bb[4] - e.bb[1], e.bb[5] - e.bb[2]));
+    gmax = n; lvl[0] = 0; lvl[1] = 1 << 30;
   }
-  if (!lead) return;
-  if (!split) {
-    nodes[e.id] = nd;
-    nodesf[e.id] = make_nodef(nd);
-    nmass[e.id] = sm;
-    leaf_at[s] = e.id;
-    return;
+  const double pm = p.massoftype, dfac = (pm > 0.0) ? 1.0 / pm : 1.0, fac = pm * dfac;
+  const bool fac1 = fac == 1.0;
+  int ncur = 1;
+  for (int level = e.level; ncur > 0; ++level) {
+    __syncthreads();
+    const int top = gmax;  // largest node of the generation
+    __syncthreads();
+    if (tid == 0) { nnext = 0; gmax = 0; }
+    // centres of mass (kdtree.F90:639-675)
+    auto centre = [&](int g, int a, double acc) {
+      const double sm = mtab[S.cur.ct[g]], d = sm * dfac;
+      S.com[3 * g + a] = sm > 0.0 ? ddiv(acc, d) : acc;
+    };
+    if (top > SUB_SEQ)
+      for (int t = tid >> 5; t < 3 * ncur; t += SUB_WARPS) {
+        const int g = t / 3, a = t - 3 * g, c = S.cur.ct[g];
+        if (c <= SUB_SEQ) continue;
+        const double acc = warp_seq_sum(a == 0 ? S.X : (a == 1 ? S.Y : S.Z), S.ix + S.cur.st[g], c, fac, fac1);
+        if (lane_id() == 0) centre(g, a, acc);
+      }
+    for (int t = tid; t < 3 * ncur; t += SUB_THREADS) {
+      const int g = t / 3, a = t - 3 * g, c = S.cur.ct[g];
+      if (c > SUB_SEQ) continue;
+      const double *A = a == 0 ? S.X : (a == 1 ? S.Y : S.Z);
+      const unsigned short *ix = S.ix + S.cur.st[g];
+      double acc = 0.0;
+      for (int q = 0; q < c; ++q) acc = dadd(acc, fac1 ? A[ix[q]] : dmul(fac, A[ix[q]]));
+      centre(g, a, acc);
+    }
+    __syncthreads();
+    if (top > 96)
+      split_generation<32>(p, S, ncur, s0, level, e.id, subbase, mtab, th, out, &nnext, &gmax, lvl, err);
+    else if (top > 24)
+      split_generation<16>(p, S, ncur, s0, level, e.id, subbase, mtab, th, out, &nnext, &gmax, lvl, err);
+    else
+      split_generation<8>(p, S, ncur, s0, level, e.id, subbase, mtab, th, out, &nnext, &gmax, lvl, err);
+    __syncthreads();
+    const int nn = nnext;
+    if (tid == 0 && nn > 0) lbase = atomicAdd(out.node_count, nn);
+    __syncthreads();
+    for (int q = tid; q < nn; q += SUB_THREADS) {
+      const int st = S.next.st[q], ct = S.next.ct[q];
+      out.node_list[lbase + q] = (S.next.fl[q] & 4) ? subbase + 2 * (s0 + st) + 1 : subbase + 2 * (s0 + st + ct - 1);
+    }
+    const SubList t = S.cur;
+    S.cur = S.next;
+    S.next = t;
+    ncur = nn;
   }
-  const int il = subbase + 2 * (s + nl - 1), ir = subbase + 2 * (s + nl) + 1;
-  nd.left = il; nd.right = ir;
-  nodes[e.id] = nd;
-  nodesf[e.id] = make_nodef(nd);
-  nmass[e.id] = sm;
-  const int rank = 2 * __popc(bsplit & lt);
-  const int ls = base_list + rank;
-  node_list[ls] = il;
-  node_list[ls + 1] = ir;
-  const int slot = base_next + rank;
-  if (slot + 2 > next_cap) { set_error(err, PH_ERR_TREE); return; }
-  GenEntry a, b;
-  a.id = il; a.start = s; a.count = nl; a.level = e.level + 1; a.parent = e.id; a.pad = 0;
-  b.id = ir; b.start = s + nl; b.count = n - nl; b.level = e.level + 1; b.parent = e.id; b.pad = 0;
-  a.bb[0] = dunkey(l0); a.bb[1] = dunkey(l1); a.bb[2] = dunkey(l2);
-  a.bb[3] = dunkey(l3); a.bb[4] = dunkey(l4); a.bb[5] = dunkey(l5);
-  b.bb[0] = dunkey(r0); b.bb[1] = dunkey(r1); b.bb[2] = dunkey(r2);
-  b.bb[3] = dunkey(r3); b.bb[4] = dunkey(r4); b.bb[5] = dunkey(r5);
-  next[slot] = a;
-  next[slot + 1] = b;
+  // the rows in their final order: all reads before the writes
+  constexpr int PER_T = SMALL / SUB_THREADS;
+  double rh[PER_T];
+  float4 rf[PER_T];
+  int rp[PER_T];
+#pragma unroll
+  for (int q = 0; q < PER_T; ++q) {
+    const int i = tid + q * SUB_THREADS;
+    if (i < n) { const int o = s0 + S.ix[i]; rh[q] = th[o]; rf[q] = txf[o]; rp[q] = perm[o]; }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PER_T; ++q) {
+    const int i = tid + q * SUB_THREADS;
+    if (i < n) {
+      const int o = S.ix[i];
+      tx[s0 + i] = S.X[o]; ty[s0 + i] = S.Y[o]; tz[s0 + i] = S.Z[o];
+      th[s0 + i] = rh[q]; txf[s0 + i] = rf[q]; perm[s0 + i] = rp[q];
+    }
+  }
+  if (tid == 0) { atomicMax(&lvlstat[0], lvl[0]); atomicMin(&lvlstat[1], lvl[1]); }
 }
 
 // ------------------------------------------------------------------ revtree
@@ -1141,12 +1334,7 @@ int build_tree(ph_ctx *c) {
   cudaStreamSynchronize(st);
   int nb = counters[0];
   int next_id = 1;
-  // sequential sums of k equal particle masses (node masses, chunk partials)
-  if (c->mtab_pm != p.massoftype) {
-    k_mass_table<<<1, 1, 0, st>>>(p.massoftype, c->mtab);
-    count_launch(c, 1);
-    c->mtab_pm = p.massoftype;
-  }
+  mass_table(c, p.massoftype);
 
   int *lvl = c->lvl_a, *lvl_next = c->lvl_b;
   double *bb = c->lvl_bb_a, *bb_next = c->lvl_bb_b;
@@ -1189,30 +1377,18 @@ int build_tree(ph_ctx *c) {
   count_launch(c, 1);
   c->nbig_nodes = next_id;
   cudaMemsetAsync(c->counters + 12, 0, sizeof(int), st);
-  // small nodes, generation by generation
-  GenEntry *gcur = c->gen_a, *gnext = c->gen_b;
-  int ncur = counters[1];
-  int gmax = SMALL;  // largest node of the generation
-  for (int gen = 0; ncur > 0; ++gen) {
-    if (gen > 4 * SMALL) return PH_ERR_TREE;
-    cudaMemsetAsync(c->counters + 2, 0, 2 * sizeof(int), st);
-    k_small_com<<<nblk(3 * (int64_t)ncur, 32), 32, 0, st>>>(p, gcur, ncur, c->mtab, c->tx, c->ty, c->tz, c->gen_com);
-#define PH_SPLIT(SEG)                                                                                              \
-  k_small_split<SEG><<<nblk(nblk(ncur, 32 / SEG), SPLIT_WARPS), 32 * SPLIT_WARPS, 0, st>>>(                       \
-      p, gcur, ncur, c->gen_com, gnext, c->counters + 2, c->gen_cap, c->mtab, c->nodes, c->nmass, c->nquads, c->tx, \
-      c->ty, c->tz, c->th, c->perm, c->txf, c->pairpos, c->subbase, c->leaf_at, c->d_maxlevel, c->nodesf,          \
-      c->node_list, c->counters + 12, c->counters + 3, c->d_err)
-    if (gmax > 96) PH_SPLIT(32);
-    else if (gmax > 24) PH_SPLIT(16);
-    else PH_SPLIT(8);
-#undef PH_SPLIT
-    count_launch(c, 2);
-    int nv[2];
-    cudaMemcpyAsync(nv, c->counters + 2, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    ncur = nv[0];
-    gmax = nv[1];
-    std::swap(gcur, gnext);
+  // the subtrees of at most SMALL particles
+  const int nsub = counters[1];
+  if (nsub > 0) {
+    const size_t smem = sub_smem(p.minpart);
+    if (!(c->attr_done & 16u)) {
+      cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sub_smem(MINPART_LO));
+      c->attr_done |= 16u;
+    }
+    const SubOut so{c->nodes, c->nodesf, c->nmass, c->nquads, c->leaf_at, c->node_list, c->counters + 12};
+    k_subtree<<<nsub, SUB_THREADS, smem, st>>>(p, c->gen_a, c->mtab, c->tx, c->ty, c->tz, c->th, c->perm, c->txf,
+                                               c->subbase, so, c->d_maxlevel, c->d_err);
+    count_launch(c, 1);
   }
   // leaf list in ascending start order
   k_flag_leaves<<<nblk(nalive, 256), 256, 0, st>>>(c->leaf_at, nalive, c->alive);
@@ -1249,11 +1425,7 @@ int revtree(ph_ctx *c) {
   const int nt = (int)c->ntree, nbig = c->nbig_nodes, nsmall = c->nsmall_nodes;
   k_rev_gather<<<nblk(nt, 256), 256, 0, st>>>(c->xyzh, nt, c->perm, c->tx, c->ty, c->tz, c->th, c->txf);
   count_launch(c, 1);
-  if (c->mtab_pm != p.massoftype) {
-    k_mass_table<<<1, 1, 0, st>>>(p.massoftype, c->mtab);
-    count_launch(c, 1);
-    c->mtab_pm = p.massoftype;
-  }
+  mass_table(c, p.massoftype);
   // node ids [0, nbig) come from the level kernels: group those of more than
   // SMALL particles by level; the rest, with the generation-built nodes, are
   // refitted as small nodes
