@@ -741,9 +741,17 @@ __global__ void __launch_bounds__(32) k_small_com(Params p, const GenEntry *cur,
   if (valid) com[4 * (size_t)g + axis] = acc;
 }
 
+// 64-bit maxima and minima over the warp: the high words first, then the low
+// words of the lanes that hold the extreme high word
 __device__ __forceinline__ long long warp_max_ll(long long v) {
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  const int hi = __reduce_max_sync(0xffffffffu, (int)(v >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (int)(v >> 32) == hi ? (unsigned)v : 0u);
+  return ((long long)hi << 32) | lo;
+}
+__device__ __forceinline__ long long warp_min_ll(long long v) {
+  const int hi = __reduce_min_sync(0xffffffffu, (int)(v >> 32));
+  const unsigned lo = __reduce_min_sync(0xffffffffu, (int)(v >> 32) == hi ? (unsigned)v : 0xffffffffu);
+  return ((long long)hi << 32) | lo;
 }
 
 // s = x_0 + x_1 + ... in the reference's order and rounding (every partial sum
@@ -755,8 +763,8 @@ __device__ __forceinline__ long long warp_max_ll(long long v) {
 // sum before it, which is even right after another tie and otherwise follows
 // from the parities of the increments in between. A term that takes the sum out
 // of its binade is added on its own; a chunk that keeps changing binade (a node
-// across a coordinate's zero) is added term by term. 2048 terms of one sign take
-// 73 rounds instead of 2048 dependent additions of 68 cycles. x_k = fac A[ix[k]].
+// across a coordinate's zero) is added term by term. 1728 terms take about 20k
+// cycles instead of 130k of dependent additions. x_k = fac A[ix[k]].
 __device__ __forceinline__ double warp_seq_sum(const double *A, const unsigned short *ix, int n, double fac,
                                                bool fac1) {
   const unsigned FULL = 0xffffffffu;
@@ -765,9 +773,42 @@ __device__ __forceinline__ double warp_seq_sum(const double *A, const unsigned s
   constexpr long long HID = 1ll << 52, MANT = HID - 1, TOP = 1ll << 53;
   double s = 0.0;
   for (int base = 0; base < n; base += 32) {
+    // 128 terms at once (four per lane) where nothing but plain increments
+    // occurs: no tie, no term of the other sign, no change of binade
+    while (base >= 128 && base + 128 <= n) {
+      const long long sb = __double_as_longlong(s);
+      const int es = (int)(sb >> 52) & 0x7ff;
+      long long sum = 0;
+      bool plain = es != 0 && es != 0x7ff;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        double x = A[ix[base + 32 * q + lane]];
+        if (!fac1) x = dmul(fac, x);
+        const long long xb = __double_as_longlong(x);
+        const int exf = (int)(xb >> 52) & 0x7ff, ex = max(exf, 1);
+        const long long mx = (xb & MANT) | (exf ? HID : 0ll);
+        const int t = min(max(es - ex, 1), 62);
+        const long long rem = mx & ((1ll << t) - 1), half = 1ll << (t - 1);
+        plain = plain && es > ex && rem != half && ((xb ^ sb) >= 0 || mx == 0);
+        sum += (mx >> t) + (rem > half ? 1 : 0);
+      }
+      if (!__all_sync(FULL, plain)) break;
+      const unsigned lo = __reduce_add_sync(FULL, (unsigned)sum & 0x1fffffu),
+                     mi = __reduce_add_sync(FULL, (unsigned)(sum >> 21) & 0x1fffffu),
+                     hi = __reduce_add_sync(FULL, (unsigned)(sum >> 42));
+      const long long R = ((sb & MANT) | HID) + (long long)lo + ((long long)mi << 21) + ((long long)hi << 42);
+      if (R >= TOP) break;
+      s = __longlong_as_double((sb & (long long)0xfff0000000000000ull) | (R & MANT));
+      base += 128;
+    }
+    if (base >= n) break;
     const int cnt = min(32, n - base);
     double x = lane < cnt ? A[ix[base + lane]] : 0.0;
     if (!fac1) x = dmul(fac, x);
+    if (base == 0) {  // the sum doubles every few terms
+      for (int q = 0; q < cnt; ++q) s = dadd(s, __shfl_sync(FULL, x, q));
+      continue;
+    }
     const long long xb = __double_as_longlong(x);
     const int exf = (int)(xb >> 52) & 0x7ff, ex = max(exf, 1);
     const long long mx = (xb & MANT) | (exf ? HID : 0ll);
@@ -833,13 +874,21 @@ __device__ __forceinline__ double warp_seq_sum(const double *A, const unsigned s
 
 template <int SEG>
 __device__ __forceinline__ long long seg_min_ll(long long v) {
-  for (int o = SEG / 2; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  if constexpr (SEG == 32) {
+    return warp_min_ll(v);
+  } else {
+    for (int o = SEG / 2; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+  }
 }
 template <int SEG>
 __device__ __forceinline__ long long seg_max_ll(long long v) {
-  for (int o = SEG / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  if constexpr (SEG == 32) {
+    return warp_max_ll(v);
+  } else {
+    for (int o = SEG / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+  }
 }
 template <int SEG>
 __device__ __forceinline__ int seg_sum_int(int v) {
@@ -852,17 +901,19 @@ __device__ __forceinline__ int seg_sum_int(int v) {
 // generation lists (first particle, count, flags: split axis in bits 0-1, bit
 // 2 a right child, bit 3 the subtree's root; parent id)
 constexpr int SUB_THREADS = 512, SUB_WARPS = SUB_THREADS / 32;
-constexpr int SUB_SEQ = 64;  // nodes up to this size: one lane per chain
+constexpr int SUB_SEQ = 256;  // nodes up to this size: one lane per chain (all chains at once, ~70 cycles a term)
 struct SubList { unsigned short *st, *ct; unsigned char *fl; int *par; };
 struct Sub {
   double *X, *Y, *Z, *com;
+  long long *r2, *hm;   // per node of the generation: r^2 and hmax keys
   float *XF, *YF, *ZF;
   unsigned short *ix, *pr;
+  unsigned short *bnd;  // its boundary (first particle of the right child), 0: a leaf
   SubList cur, next;
 };
 __host__ __device__ __forceinline__ int sub_cap(int minpart) { return 2 * (SMALL / (minpart + 1)) + 4; }
 __host__ __device__ __forceinline__ size_t sub_smem(int minpart) {
-  return (size_t)SMALL * (3 * 8 + 3 * 4 + 2 * 2) + (size_t)sub_cap(minpart) * (3 * 8 + 2 * (4 + 2 + 2 + 1)) + 64;
+  return (size_t)SMALL * (3 * 8 + 3 * 4 + 2 * 2) + (size_t)sub_cap(minpart) * (5 * 8 + 2 + 2 * (4 + 2 + 2 + 1)) + 64;
 }
 
 // global arrays the subtree kernel reads and writes
@@ -882,15 +933,43 @@ __device__ __forceinline__ int split_axis(double e0, double e1, double e2) {
   return ax;
 }
 
+__device__ __forceinline__ int sub_id(int fl, int s, int n, int s0, int rootid, int subbase) {
+  return (fl & 8) ? rootid : ((fl & 4) ? subbase + 2 * (s0 + s) + 1 : subbase + 2 * (s0 + s + n - 1));
+}
+
+// The node records of a generation, one thread per node: the square roots and
+// conversions take the FP64 pipe with full warps (by the segments' leaders they
+// held it for most of a small build).
+__device__ __forceinline__ void finish_generation(const Sub &S, int ncur, int s0, int level, int rootid, int subbase,
+                                                  const double *mtab, const SubOut &out, int *lvl) {
+  for (int g = threadIdx.x; g < ncur; g += SUB_THREADS) {
+    const int s = S.cur.st[g], n = S.cur.ct[g], bnd = S.bnd[g], id = sub_id(S.cur.fl[g], s, n, s0, rootid, subbase);
+    Node nd{};
+    nd.x = S.com[3 * g]; nd.y = S.com[3 * g + 1]; nd.z = S.com[3 * g + 2];
+    nd.size = sqrt(dunkey(S.r2[g])) + EPS_D;
+    nd.hmax = dunkey(max(S.hm[g], 0ll));
+    nd.start = s0 + s; nd.count = n; nd.level = level; nd.parent = S.cur.par[g];
+    nd.left = -1; nd.right = -1;
+    if (bnd) { nd.left = subbase + 2 * (s0 + bnd - 1); nd.right = subbase + 2 * (s0 + bnd) + 1; }
+    out.nodes[id] = nd;
+    out.nodesf[id] = make_nodef(nd);
+    out.nmass[id] = mtab[n];
+    if (!bnd) {
+      out.leaf_at[s0 + s] = id;
+      atomicMax(&lvl[0], level);
+      atomicMin(&lvl[1], level);
+    }
+  }
+}
+
 // One generation's nodes, a segment of SEG lanes per node (32 / SEG nodes per
 // warp): size, hmax, the count on the pivot's left, both sides' bounding
 // boxes, the partition and the node record; the children go to the next list.
 // Segment reductions are xor butterflies inside the segment; the partition's
 // ballots run a warp-uniform number of rounds.
 template <int SEG>
-__device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0, int level, int rootid, int subbase,
-                                 const double *mtab, const double *th, const SubOut &out, int *nnext, int *gmax,
-                                 int *lvl, int *err) {
+__device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0, int rootid, int subbase,
+                                 const double *th, const SubOut &out, int *nnext, int *gmax, int *err) {
   const unsigned FULL = 0xffffffffu;
   constexpr int NSEG = 32 / SEG;
   const int lane = lane_id(), seg = lane / SEG, sl = lane % SEG;
@@ -911,7 +990,7 @@ __device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0
     // E = 2^-23 (|x'| + |c'| + |d'|) per axis, which brackets each r^2; only
     // particles whose upper bound reaches the largest lower bound can hold the
     // maximum, and their r^2 is evaluated exactly in FP64.
-    const float cxf = (float)sx, cyf = (float)sy, czf = (float)sz;
+    const float cxf = d2f_rn(sx), cyf = d2f_rn(sy), czf = d2f_rn(sz);
     const float eps23 = 1.1920929e-7f;
     float lbmax = 0.0f;
     long long l0 = KEY_HI, l1 = KEY_HI, l2 = KEY_HI, l3 = KEY_LO, l4 = KEY_LO, l5 = KEY_LO;
@@ -955,8 +1034,8 @@ __device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0
         r2k = max(r2k, dkey(r2_exact(S.X[o] - sx, S.Y[o] - sy, S.Z[o] - sz)));
     }
     r2k = seg_max_ll<SEG>(r2k);
-    const double hm = fmax(0.0, dunkey(seg_max_ll<SEG>(hk)));
-    const int id = (fl & 8) ? rootid : ((fl & 4) ? subbase + 2 * (s0 + s) + 1 : subbase + 2 * (s0 + end - 1));
+    hk = seg_max_ll<SEG>(hk);
+    const int id = sub_id(fl, s, n, s0, rootid, subbase);
     if (p.gravity) {
       // quadrupoles (kdtree.F90:744-752): m sum of dx_a dx_b; lanes over
       // particles, then a fixed-order butterfly (no tree decision reads them)
@@ -994,11 +1073,22 @@ __device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0
         }
       }
     }
+    // the children's split axes from their boxes: lane (side, axis) of the
+    // segment forms its extent, compared on bit patterns (extents are >= 0)
+    int axl = 0, axr = 0;
     if (__any_sync(FULL, split)) {
       l0 = seg_min_ll<SEG>(l0); l1 = seg_min_ll<SEG>(l1); l2 = seg_min_ll<SEG>(l2);
       l3 = seg_max_ll<SEG>(l3); l4 = seg_max_ll<SEG>(l4); l5 = seg_max_ll<SEG>(l5);
       r0 = seg_min_ll<SEG>(r0); r1 = seg_min_ll<SEG>(r1); r2 = seg_min_ll<SEG>(r2);
       r3 = seg_max_ll<SEG>(r3); r4 = seg_max_ll<SEG>(r4); r5 = seg_max_ll<SEG>(r5);
+      const int c = sl % 6;
+      const long long lo = c == 0 ? l0 : (c == 1 ? l1 : (c == 2 ? l2 : (c == 3 ? r0 : (c == 4 ? r1 : r2))));
+      const long long hi = c == 0 ? l3 : (c == 1 ? l4 : (c == 2 ? l5 : (c == 3 ? r3 : (c == 4 ? r4 : r5))));
+      const long long ext = split ? __double_as_longlong(dsub(dunkey(hi), dunkey(lo))) : 0ll;
+      long long x[6];
+      for (int q = 0; q < 6; ++q) x[q] = __shfl_sync(FULL, ext, seg * SEG + q);
+      axl = x[1] > x[0] ? 1 : 0; if (x[2] > max(x[0], x[1])) axl = 2;
+      axr = x[4] > x[3] ? 1 : 0; if (x[5] > max(x[3], x[4])) axr = 2;
     }
     // partition: the k-th element > pivot left of the boundary (counted from
     // the left) swaps with the k-th element <= pivot right of it (counted
@@ -1035,7 +1125,7 @@ __device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0
     }
     if (part && m != m2 && sl == 0) set_error(err, PH_ERR_TREE);
     __syncwarp();
-    // node records and next-generation entries (segment leaders)
+    // what the node records need and the next generation's entries (segment leaders)
     const bool lead = valid && sl == 0;
     const unsigned bsplit = __ballot_sync(FULL, lead && split);
     int base = 0;
@@ -1045,28 +1135,205 @@ __device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0
       base = __shfl_sync(FULL, base, first);
     }
     if (!lead) continue;
-    Node nd{};
-    nd.x = sx; nd.y = sy; nd.z = sz; nd.size = sqrt(dunkey(r2k)) + EPS_D; nd.hmax = hm;
-    nd.start = s0 + s; nd.count = n; nd.level = level; nd.parent = S.cur.par[g];
-    nd.left = -1; nd.right = -1;
-    if (split) { nd.left = subbase + 2 * (s0 + bnd - 1); nd.right = subbase + 2 * (s0 + bnd) + 1; }
-    out.nodes[id] = nd;
-    out.nodesf[id] = make_nodef(nd);
-    out.nmass[id] = mtab[n];
-    if (!split) {
-      out.leaf_at[s0 + s] = id;
-      atomicMax(&lvl[0], level);
-      atomicMin(&lvl[1], level);
-      continue;
-    }
+    S.r2[g] = r2k; S.hm[g] = hk; S.bnd[g] = (unsigned short)(split ? bnd : 0);
+    if (!split) continue;
     const int q = base + 2 * __popc(bsplit & lt);
     S.next.st[q] = (unsigned short)s; S.next.ct[q] = (unsigned short)nl; S.next.par[q] = id;
-    S.next.fl[q] = (unsigned char)split_axis(dunkey(l3) - dunkey(l0), dunkey(l4) - dunkey(l1), dunkey(l5) - dunkey(l2));
+    S.next.fl[q] = (unsigned char)axl;
     S.next.st[q + 1] = (unsigned short)bnd; S.next.ct[q + 1] = (unsigned short)(n - nl); S.next.par[q + 1] = id;
-    S.next.fl[q + 1] =
-        (unsigned char)(4 | split_axis(dunkey(r3) - dunkey(r0), dunkey(r4) - dunkey(r1), dunkey(r5) - dunkey(r2)));
+    S.next.fl[q + 1] = (unsigned char)(4 | axr);
     atomicMax(gmax, max(nl, n - nl));
   }
+}
+
+// The first generations hold fewer nodes than the block has warps: a team of
+// tw = SUB_WARPS / 2^k warps takes each node (all teams in step, block-wide
+// barriers between the phases), where one warp per node left the rest idle
+//, and
+// the sums a whole round each: a 12^3 build 303 -> 226 us, 2M particles 1.38 -> 1.02 ms. Same tests and
+// records as split_generation.
+struct SubTeam {
+  long long key[SUB_WARPS][14];  // boxes (12), hmax, r2
+  float lb[SUB_WARPS];
+  int nl[SUB_WARPS], cr[SUB_WARPS], cl[SUB_WARPS];
+  double q[SUB_WARPS][6];
+};
+
+__device__ void split_team(const Params &p, const Sub &S, SubTeam &T, int tw, int ncur, int s0, int rootid, int subbase,
+                           const double *th, const SubOut &out, int *nnext, int *gmax, int *err) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = lane_id(), w = threadIdx.x >> 5, g = w / tw, wr = w - g * tw, w0 = g * tw;
+  const unsigned lt = (1u << lane) - 1u;
+  const bool valid = g < ncur;
+  const int s = valid ? S.cur.st[g] : 0, n = valid ? S.cur.ct[g] : 0, end = s + n;
+  const int fl = valid ? S.cur.fl[g] : 0;
+  double sx = 0.0, sy = 0.0, sz = 0.0;
+  if (valid) { sx = S.com[3 * g]; sy = S.com[3 * g + 1]; sz = S.com[3 * g + 2]; }
+  const bool split = valid && n > p.minpart;  // kdtree.F90:792
+  const int ax = fl & 3;
+  const double pv = ax == 0 ? sx : (ax == 1 ? sy : sz);
+  const long long pk = dkey(pv);
+  const float cxf = d2f_rn(sx), cyf = d2f_rn(sy), czf = d2f_rn(sz);
+  const float eps23 = 1.1920929e-7f;
+  float lbmax = 0.0f;
+  long long k[13];  // left box, right box (minima, maxima), hmax
+  auto clear = [&]() {
+#pragma unroll
+    for (int q = 0; q < 12; ++q) k[q] = (q % 6) < 3 ? KEY_HI : KEY_LO;
+  };
+  auto box = [&](int b, int o) {
+    const long long kx = dkey(S.X[o]), ky = dkey(S.Y[o]), kz = dkey(S.Z[o]);
+    if (b == 0) {
+      k[0] = min(k[0], kx); k[1] = min(k[1], ky); k[2] = min(k[2], kz);
+      k[3] = max(k[3], kx); k[4] = max(k[4], ky); k[5] = max(k[5], kz);
+    } else {
+      k[6] = min(k[6], kx); k[7] = min(k[7], ky); k[8] = min(k[8], kz);
+      k[9] = max(k[9], kx); k[10] = max(k[10], ky); k[11] = max(k[11], kz);
+    }
+  };
+  auto combine = [&]() {  // the team's boxes
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      const long long v = (q % 6) < 3 ? warp_min_ll(k[q]) : warp_max_ll(k[q]);
+      if (lane == 0) T.key[w][q] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {  // lane t reads warp t's value
+      const bool mine = lane < tw;
+      if ((q % 6) < 3) k[q] = warp_min_ll(mine ? T.key[w0 + lane][q] : KEY_HI);
+      else k[q] = warp_max_ll(mine ? T.key[w0 + lane][q] : KEY_LO);
+    }
+  };
+  clear();
+  k[12] = KEY_LO;
+  int nl = 0;
+  for (int i = s + wr * 32 + lane; i < end; i += 32 * tw) {
+    const int o = S.ix[i];
+    const float qx = S.XF[o], qy = S.YF[o], qz = S.ZF[o];
+    const float dx = qx - cxf, dy = qy - cyf, dz = qz - czf;
+    const float ex = eps23 * (fabsf(qx) + fabsf(cxf) + fabsf(dx));
+    const float ey = eps23 * (fabsf(qy) + fabsf(cyf) + fabsf(dy));
+    const float ez = eps23 * (fabsf(qz) + fabsf(czf) + fabsf(dz));
+    const float bx = fmaxf(fabsf(dx) - ex, 0.0f), by = fmaxf(fabsf(dy) - ey, 0.0f), bz = fmaxf(fabsf(dz) - ez, 0.0f);
+    lbmax = fmaxf(lbmax, bx * bx + by * by + bz * bz);
+    k[12] = max(k[12], dkey(th[s0 + o]));
+    const double c = ax == 0 ? S.X[o] : (ax == 1 ? S.Y[o] : S.Z[o]);
+    const bool left = dkey(c) <= pk;
+    nl += left ? 1 : 0;
+    box(left ? 0 : 1, o);
+  }
+  for (int o = 16; o > 0; o >>= 1) lbmax = fmaxf(lbmax, __shfl_xor_sync(FULL, lbmax, o));
+  nl = warp_sum_int(nl);
+  const long long hkw = warp_max_ll(k[12]);
+  if (lane == 0) { T.lb[w] = lbmax; T.nl[w] = nl; T.key[w][12] = hkw; }
+  combine();  // (the barrier inside orders lb, nl and hmax too)
+  lbmax = 0.0f; nl = 0;
+  long long hk = KEY_LO;
+  for (int t = 0; t < tw; ++t) { lbmax = fmaxf(lbmax, T.lb[w0 + t]); nl += T.nl[w0 + t]; hk = max(hk, T.key[w0 + t][12]); }
+  lbmax *= 0.999999f;
+  long long r2k = 0;
+  for (int i = s + wr * 32 + lane; i < end; i += 32 * tw) {
+    const int o = S.ix[i];
+    const float qx = S.XF[o], qy = S.YF[o], qz = S.ZF[o];
+    const float dx = qx - cxf, dy = qy - cyf, dz = qz - czf;
+    const float ex = eps23 * (fabsf(qx) + fabsf(cxf) + fabsf(dx));
+    const float ey = eps23 * (fabsf(qy) + fabsf(cyf) + fabsf(dy));
+    const float ez = eps23 * (fabsf(qz) + fabsf(czf) + fabsf(dz));
+    const float bx = fabsf(dx) + ex, by = fabsf(dy) + ey, bz = fabsf(dz) + ez;
+    if ((bx * bx + by * by + bz * bz) * 1.000001f >= lbmax)
+      r2k = max(r2k, dkey(r2_exact(S.X[o] - sx, S.Y[o] - sy, S.Z[o] - sz)));
+  }
+  r2k = warp_max_ll(r2k);
+  if (lane == 0) T.key[w][13] = r2k;
+  const int id = sub_id(fl, s, n, s0, rootid, subbase);
+  if (p.gravity) {  // quadrupoles (kdtree.F90:744-752), fixed order
+    double q[6] = {0, 0, 0, 0, 0, 0};
+    for (int i = s + wr * 32 + lane; i < end; i += 32 * tw) {
+      const int o = S.ix[i];
+      const double dx = S.X[o] - sx, dy = S.Y[o] - sy, dz = S.Z[o] - sz;
+      q[0] = fma(dx, dx, q[0]); q[1] = fma(dx, dy, q[1]); q[2] = fma(dx, dz, q[2]);
+      q[3] = fma(dy, dy, q[3]); q[4] = fma(dy, dz, q[4]); q[5] = fma(dz, dz, q[5]);
+    }
+    for (int c = 0; c < 6; ++c) {
+      for (int o = 16; o > 0; o >>= 1) q[c] += __shfl_xor_sync(FULL, q[c], o);
+      if (lane == 0) T.q[w][c] = q[c];
+    }
+  }
+  const bool noswap = split && (nl == n || nl == 0);
+  if (__syncthreads_or(noswap ? 1 : 0)) {
+    // no split along the axis: halves by position, no swaps (kdtree.F90:856-865)
+    if (noswap) {
+      nl = n / 2;
+      clear();
+      for (int i = s + wr * 32 + lane; i < end; i += 32 * tw) box(i < s + nl ? 0 : 1, S.ix[i]);
+    }
+    __syncthreads();
+    combine();
+  }
+  // partition (split_generation): each warp takes a contiguous share of the
+  // right side, counted from the right, and of the left side
+  const bool part = split && !noswap;
+  const double *cx = ax == 0 ? S.X : (ax == 1 ? S.Y : S.Z);
+  const int bnd = s + nl, nrt = part ? end - bnd : 0, nlf = part ? nl : 0;
+  const int chr = ((nrt + tw - 1) / tw + 31) & ~31, chl = ((nlf + tw - 1) / tw + 31) & ~31;
+  const int ra = min(wr * chr, nrt), rb = min(ra + chr, nrt), la = min(wr * chl, nlf), lb = min(la + chl, nlf);
+  int cr = 0, cl = 0;
+  for (int q = ra + lane; q < rb; q += 32) cr += dkey(cx[S.ix[end - 1 - q]]) <= pk ? 1 : 0;
+  for (int q = la + lane; q < lb; q += 32) cl += dkey(cx[S.ix[s + q]]) > pk ? 1 : 0;
+  cr = warp_sum_int(cr); cl = warp_sum_int(cl);
+  if (lane == 0) { T.cr[w] = cr; T.cl[w] = cl; }
+  __syncthreads();
+  int m2 = 0, m = 0, tr = 0, tl = 0;
+  for (int t = 0; t < tw; ++t) {
+    if (t == wr) { m2 = tr; m = tl; }
+    tr += T.cr[w0 + t]; tl += T.cl[w0 + t];
+  }
+  for (int q0 = ra; q0 < rb; q0 += 32) {
+    const int q = q0 + lane, i = end - 1 - q;
+    const bool f = q < rb && dkey(cx[S.ix[i]]) <= pk;
+    const unsigned bal = __ballot_sync(FULL, f);
+    if (f) S.pr[s + m2 + __popc(bal & lt)] = (unsigned short)i;
+    m2 += __popc(bal);
+  }
+  __syncthreads();
+  for (int q0 = la; q0 < lb; q0 += 32) {
+    const int q = q0 + lane, i = s + q;
+    const bool f = q < lb && dkey(cx[S.ix[i]]) > pk;
+    const unsigned bal = __ballot_sync(FULL, f);
+    if (f) {
+      const int r = m + __popc(bal & lt);
+      if (r < tr) {
+        const int o = S.pr[s + r];
+        const unsigned short a = S.ix[i];
+        S.ix[i] = S.ix[o];
+        S.ix[o] = a;
+      }
+    }
+    m += __popc(bal);
+  }
+  if (!valid || wr != 0 || lane != 0) return;
+  if (part && tl != tr) set_error(err, PH_ERR_TREE);
+  r2k = 0;
+  for (int t = 0; t < tw; ++t) r2k = max(r2k, T.key[w0 + t][13]);
+  if (p.gravity) {
+    double *qo = out.nquads + 6 * (size_t)id;
+    for (int c = 0; c < 6; ++c) {
+      double q = T.q[w0][c];
+      for (int t = 1; t < tw; ++t) q += T.q[w0 + t][c];
+      qo[c] = p.massoftype * q;
+    }
+  }
+  S.r2[g] = r2k; S.hm[g] = hk; S.bnd[g] = (unsigned short)(split ? bnd : 0);
+  if (!split) return;
+  const int q = atomicAdd(nnext, 2);
+  S.next.st[q] = (unsigned short)s; S.next.ct[q] = (unsigned short)nl; S.next.par[q] = id;
+  S.next.fl[q] = (unsigned char)split_axis(dunkey(k[3]) - dunkey(k[0]), dunkey(k[4]) - dunkey(k[1]),
+                                           dunkey(k[5]) - dunkey(k[2]));
+  S.next.st[q + 1] = (unsigned short)bnd; S.next.ct[q + 1] = (unsigned short)(n - nl); S.next.par[q + 1] = id;
+  S.next.fl[q + 1] = (unsigned char)(4 | split_axis(dunkey(k[9]) - dunkey(k[6]), dunkey(k[10]) - dunkey(k[7]),
+                                                    dunkey(k[11]) - dunkey(k[8])));
+  atomicMax(gmax, max(nl, n - nl));
 }
 
 __global__ void __launch_bounds__(SUB_THREADS, 2) k_subtree(Params p, const GenEntry *gen, const double *mtab,
@@ -1075,16 +1342,19 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subtree(Params p, const GenE
                                                             int *err) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ int nnext, gmax, lbase, lvl[2];
+  __shared__ SubTeam team;
   const GenEntry e = gen[blockIdx.x];
   const int n = e.count, s0 = e.start, tid = threadIdx.x, cap = sub_cap(p.minpart);
   if (n < 1 || n > SMALL) { if (tid == 0) set_error(err, PH_ERR_TREE); return; }
   Sub S;
   S.X = reinterpret_cast<double *>(dsm); S.Y = S.X + SMALL; S.Z = S.Y + SMALL; S.com = S.Z + SMALL;
-  S.XF = reinterpret_cast<float *>(S.com + 3 * cap); S.YF = S.XF + SMALL; S.ZF = S.YF + SMALL;
+  S.r2 = reinterpret_cast<long long *>(S.com + 3 * cap); S.hm = S.r2 + cap;
+  S.XF = reinterpret_cast<float *>(S.hm + cap); S.YF = S.XF + SMALL; S.ZF = S.YF + SMALL;
   S.cur.par = reinterpret_cast<int *>(S.ZF + SMALL); S.next.par = S.cur.par + cap;
   S.ix = reinterpret_cast<unsigned short *>(S.next.par + cap); S.pr = S.ix + SMALL;
   S.cur.st = S.pr + SMALL; S.cur.ct = S.cur.st + cap; S.next.st = S.cur.ct + cap; S.next.ct = S.next.st + cap;
-  S.cur.fl = reinterpret_cast<unsigned char *>(S.next.ct + cap); S.next.fl = S.cur.fl + cap;
+  S.bnd = S.next.ct + cap;
+  S.cur.fl = reinterpret_cast<unsigned char *>(S.bnd + cap); S.next.fl = S.cur.fl + cap;
   for (int i = tid; i < n; i += SUB_THREADS) {
     S.X[i] = tx[s0 + i]; S.Y[i] = ty[s0 + i]; S.Z[i] = tz[s0 + i];
     const float4 q = txf[s0 + i];
@@ -1126,13 +1396,18 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subtree(Params p, const GenE
       centre(g, a, acc);
     }
     __syncthreads();
-    if (top > 96)
-      split_generation<32>(p, S, ncur, s0, level, e.id, subbase, mtab, th, out, &nnext, &gmax, lvl, err);
+    if (ncur <= SUB_WARPS / 2 && top > 64) {
+      int tw = SUB_WARPS;
+      while (tw * ncur > SUB_WARPS) tw >>= 1;
+      split_team(p, S, team, tw, ncur, s0, e.id, subbase, th, out, &nnext, &gmax, err);
+    } else if (top > 96)
+      split_generation<32>(p, S, ncur, s0, e.id, subbase, th, out, &nnext, &gmax, err);
     else if (top > 24)
-      split_generation<16>(p, S, ncur, s0, level, e.id, subbase, mtab, th, out, &nnext, &gmax, lvl, err);
+      split_generation<16>(p, S, ncur, s0, e.id, subbase, th, out, &nnext, &gmax, err);
     else
-      split_generation<8>(p, S, ncur, s0, level, e.id, subbase, mtab, th, out, &nnext, &gmax, lvl, err);
+      split_generation<8>(p, S, ncur, s0, e.id, subbase, th, out, &nnext, &gmax, err);
     __syncthreads();
+    finish_generation(S, ncur, s0, level, e.id, subbase, mtab, out, lvl);
     const int nn = nnext;
     if (tid == 0 && nn > 0) lbase = atomicAdd(out.node_count, nn);
     __syncthreads();
