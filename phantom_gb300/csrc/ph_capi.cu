@@ -70,7 +70,7 @@ int alloc_all(ph_ctx *c, int64_t cap) {
   r |= dalloc(c, &c->cbase, (size_t)c->lvl_cap + 1);
   r |= dalloc(c, &c->part_d, 16 * (size_t)std::max<int64_t>(c->chunk_cap, 2048));
   r |= dalloc(c, &c->part_i, 3 * (size_t)c->chunk_cap);
-  r |= dalloc(c, &c->counters, 64);
+  r |= dalloc(c, &c->counters, 64); r |= dalloc(c, &c->top_nodes, 32);
   r |= dalloc(c, &c->hcur, n); r |= dalloc(c, &c->hold, n); r |= dalloc(c, &c->psum, PSUM * n);
   r |= dalloc(c, &c->gradh64, n); r |= dalloc(c, &c->gsoft64, n);
   r |= dalloc(c, &c->cell_nits, n); r |= dalloc(c, &c->cell_state, n); r |= dalloc(c, &c->cell_hmax, n);

@@ -771,7 +771,7 @@ int density(ph_ctx *c, int icall) {
     for (int attempt = 0;; ++attempt) {
       cudaEventRecord(c->evk[4], st);
       launch_walk<false>(ww, nact, st,
-          p, c->nodes, c->nodesf, c->root, c->leaves, act, nact, need, c->cell_hmax, c->pool, c->pool_cap, c->pool_top,
+          p, c->nodes, c->nodesf, c->top_nodes, c->leaves, act, nact, need, c->cell_hmax, c->pool, c->pool_cap, c->pool_top,
           c->cell_off, c->cell_nleaf, c->cell_ntrial, c->d_err);
       cudaEventRecord(c->evk[5], st);
       count_launch(c, 1);

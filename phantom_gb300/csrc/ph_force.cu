@@ -1440,7 +1440,7 @@ int force_lists(ph_ctx *c) {
       const int nw = ind ? c->ncell_act : ncell;
       if (nw > 0) {
         launch_walk<true>(c->walk_warps, nw, st,
-            p, c->nodes, c->nodesf, c->root, c->leaves, ind ? c->cell_act : nullptr, nw, nullptr, nullptr, c->pool,
+            p, c->nodes, c->nodesf, c->top_nodes, c->leaves, ind ? c->cell_act : nullptr, nw, nullptr, nullptr, c->pool,
             c->pool_cap, c->pool_top, c->cell_off, c->cell_nleaf, c->cell_ntrial, c->d_err);
         count_launch(c, 1);
       }

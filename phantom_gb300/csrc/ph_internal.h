@@ -156,6 +156,7 @@ struct ph_ctx {
   float4 *mqf = nullptr;         // FP32 node mass and quadrupole (mixed form), two float4 per node id
   int *leaf_of = nullptr;        // gravity: leaf index of each tree position
   double *nmass = nullptr, *nquads = nullptr;
+  int *top_nodes = nullptr;      // the first five levels by heap index (walks)
   int node_cap = 0, subbase = 0, root = 0;
   int *leaf_at = nullptr;   // tree position -> leaf node id starting there (or -1)
   int *leaves = nullptr;    // leaf node ids in ascending start order

@@ -1148,10 +1148,10 @@ __device__ void split_generation(const Params &p, const Sub &S, int ncur, int s0
 
 // The first generations hold fewer nodes than the block has warps: a team of
 // tw = SUB_WARPS / 2^k warps takes each node (all teams in step, block-wide
-// barriers between the phases), where one warp per node left the rest idle
-//, and
-// the sums a whole round each: a 12^3 build 303 -> 226 us, 2M particles 1.38 -> 1.02 ms. Same tests and
-// records as split_generation.
+// barriers between the phases), where one warp per node left the rest idle.
+// With it and the 128-term rounds of the sums a 12^3 build takes 226 us instead
+// of 303, 2M particles 1.02 ms instead of 1.38. Same tests and records as
+// split_generation.
 struct SubTeam {
   long long key[SUB_WARPS][14];  // boxes (12), hmax, r2
   float lb[SUB_WARPS];
@@ -1574,6 +1574,16 @@ __global__ void k_compact_leaves(const int *leaf_at, const int *pos, int n, int 
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && leaf_at[i] >= 0) leaves[pos[i]] = leaf_at[i];
 }
+// the tree's first five levels by heap index (root 1, children 2 h and 2 h +
+// 1), -1 where a leaf ends the path: the walks test them in one round
+__global__ void k_top_nodes(const Node *nodes, int root, int *top) {
+  const int h = threadIdx.x;
+  int nd = h >= 1 ? root : -1;
+  for (int b = 30 - __clz(max(h, 1)); b >= 0 && nd >= 0; --b)
+    nd = ((h >> b) & 1) ? nodes[nd].right : nodes[nd].left;
+  top[h] = nd;
+}
+
 __global__ void k_iperm(const int *perm, int n, int *iperm) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) iperm[perm[i]] = i;
@@ -1670,7 +1680,8 @@ int build_tree(ph_ctx *c) {
   scan_int(c, c->alive, c->pairpos, nalive, c->counters + 4);
   k_compact_leaves<<<nblk(nalive, 256), 256, 0, st>>>(c->leaf_at, c->pairpos, nalive, c->leaves);
   k_iperm<<<nblk(nalive, 256), 256, 0, st>>>(c->perm, nalive, c->iperm);
-  count_launch(c, 3);
+  k_top_nodes<<<1, 32, 0, st>>>(c->nodes, 0, c->top_nodes);
+  count_launch(c, 4);
   int hostv[4];
   cudaMemcpyAsync(hostv, c->counters + 4, sizeof(int), cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(hostv + 3, c->counters + 12, sizeof(int), cudaMemcpyDeviceToHost, st);
