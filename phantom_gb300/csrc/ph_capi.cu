@@ -121,6 +121,23 @@ int grow_pool(ph_ctx *c) {
   return 0;
 }
 
+// Room for a pair record of `rows` rows, kept with the context. Taken only
+// where it leaves three quarters of the free device memory; false: no record.
+bool grow_record(ph_ctx *c, int64_t rows) {
+  if (c->rec_cap >= rows) return true;
+  if (rows > INT32_MAX) return false;
+  size_t avail = 0, total = 0;
+  const size_t bytes = 128 * (size_t)rows + (c->rec_cell ? 0 : sizeof(int) * (size_t)c->cap);
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 4 < bytes) return false;
+  if (c->rec_rows) dfree(c, c->rec_rows);
+  c->rec_rows = nullptr;
+  c->rec_cap = 0;
+  if (!c->rec_cell && dalloc(c, &c->rec_cell, (size_t)c->cap) != 0) return false;
+  if (dalloc(c, &c->rec_rows, 32 * (size_t)rows) != 0) return false;
+  c->rec_cap = rows;
+  return true;
+}
+
 int alloc_sym(ph_ctx *c, int64_t jbuf_stride, int nj) {
   int r = 0;
   if (!c->cell_at) {

@@ -767,8 +767,8 @@ __device__ __forceinline__ bool pair_cell(PairCell &c, const Node *nodes, const 
 // totals of a cell -> psum: value k of particle il at idx = k np + il; the
 // particle mass, left out of the pair terms, applied to every sum but
 // d(rho)/dt's (which the finish multiplies) and the maxima
-template <bool MHD, int NR>
-__device__ __forceinline__ void store_totals(const ListBase &sm, int nv, int np, double pm, const double (&tot)[NR],
+template <bool MHD, int NR, class S>
+__device__ __forceinline__ void store_totals(const S &sm, int nv, int np, double pm, const double (&tot)[NR],
                                              double *psum, int64_t ps) {
   for (int r = 0; r < NR; ++r) {
     const int idx = lane_id() + 32 * r;
@@ -1278,12 +1278,26 @@ __device__ __forceinline__ void force_pair_mixed(const Params &p, const IMix<MHD
 // register allocation left alone (108 registers, 16 warps) takes 0.513 ms (MHD
 // 0.75), this bound 0.47 (0.62), one more block 0.49 (0.70); self-gravity at
 // 300001 particles 2.77 -> 2.39 ms.
-template <bool MHD, bool IND>
+//
+// A velocity iteration evaluates the force again with the same positions and
+// smoothing lengths, so its pairs, and their lanes, are those of the evaluation
+// before. With REC the kernel writes each drain's pairs as the lanes take them:
+// a row of the lanes' particles, a row with the number of pair rows, whether
+// code rows follow and the cell's next drain, then a row of 32 trial particles
+// per step (-1: idle lane), then as many of their offset codes where any is not
+// 0. The rows are counted on past the buffer's end; the host then takes no
+// part of the record.
+struct PairRec {
+  int *rows, *cell;  // rows of 32, first row of every cell
+  int cap, *top;     // rows there are, rows taken (counted on past cap)
+};
+template <bool MHD, bool IND, bool REC>
 __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
     Params p, const Node *nodes, const int *leaves, int ncell, const LeafEntry *pool, const int *cell_off,
     const int *cell_nleaf, const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl,
     const float *jrecf, const float *jmhdf, ForceOut out, double *psum, int64_t ps, const int *cells,
-    const unsigned char *actf, const int8_t *ibin_old_t, unsigned char *wakemark, int *err) {
+    const unsigned char *actf, const int8_t *ibin_old_t, unsigned char *wakemark, PairRec rec,
+    int *err) {
   constexpr int NV = NJS<MHD>::n + (IND ? 1 : 0), NR = (NV * MAXCELL + 31) / 32, VS = NJS<MHD>::n - 1;
   PairCell c;
   if (!pair_cell<IND>(c, nodes, leaves, ncell, cells, cell_off, cell_nleaf, actf, out, err)) return;
@@ -1304,12 +1318,40 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
   ListPos pos;
   __syncwarp();
   bool more = true;
+  int prev = -1;
   while (more) {
     int myc;
     more = SWEEP_END != sweep_list<false>(p, c.cc, np, pool, c.off, c.nleaf, txf, sm, qstride, pos, myc,
                                               [&](float h1) { return __fdividef(q2lim, h1 * h1); });
     const QueueLanes ql = balance_queues(np, myc, sm);
     const int il = max(ql.il, 0);
+    if constexpr (REC) {
+      const int nst = ql.c > ql.m0 ? (ql.c - ql.m0 + ql.step - 1) / ql.step : 0;
+      const int nit = (int)__reduce_max_sync(0xffffffffu, (unsigned)nst);
+      bool coded = false;
+      if (p.periodic)
+        for (int t = 0; t < nst; ++t) coded = coded || sm.qc[il * qstride + ql.m0 + t * ql.step] != 0;
+      coded = __any_sync(0xffffffffu, coded);
+      const int need = 2 + nit * (coded ? 2 : 1);
+      int row = 0;
+      if (lane == 0) row = atomicAdd(rec.top, need);
+      row = __shfl_sync(0xffffffffu, row, 0);
+      if (row >= 0 && row <= rec.cap - need) {
+        int *d = rec.rows + 32 * (size_t)row + lane;
+        d[0] = ql.il;
+        d[32] = lane == 0 ? nit : (lane == 1 ? (coded ? 1 : 0) : -1);
+        for (int t = 0; t < nit; ++t) {
+          const int m = il * qstride + ql.m0 + t * ql.step;
+          d[64 + 32 * t] = t < nst ? sm.qj[m] : -1;
+          if (coded) d[64 + 32 * (nit + t)] = t < nst ? sm.qc[m] & 63 : 0;
+        }
+        if (lane == 0) {
+          if (prev < 0) rec.cell[c.cell] = row;
+          else rec.rows[32 * (size_t)prev + 34] = row;
+        }
+        prev = row;
+      }
+    }
     const IMix<MHD> I = imix_init<MHD>(sm.ipos[il], txf, txl, jrecf, jmhdf);
     Kahan f[NF];
     float vsigmax = 0.0f;
@@ -1320,6 +1362,62 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
     static_assert(32 * NV <= LQ / 2, "lane sums staged in the queues' space");
     flush_lanes<NV>(np, sm, sm.red, tot,
         [&](int k) -> double { return k < VS ? f[njs_slot(k, MHD)].value() : (k == VS ? (double)vsigmax : (double)nbi); },
+        [](int k, double s, double v) -> double { return k < VS ? s + v : fmax_pos(s, v); });
+  }
+  store_totals<MHD>(sm, NV, np, p.massoftype, tot, psum, ps);
+}
+
+// The evaluations after a recorded one: same pairs, same lanes, same sums in the
+// same order (bit-identical results) without the sweep, which is half of the
+// kernel above (189 of 395 us at 64^3); what remains waits for the gathers of
+// the trial particles' records. Three Sedov steps of 128^3 particles, five
+// evaluations each: 99.5 -> 88.1 ms, with the Cullen-Dehnen switch at 96^3
+// 58.3 -> 49.6 ms.
+template <int NV>
+struct ReplaySmem {
+  double red[32 * NV];
+  int ipos[MAXCELL];
+  unsigned char first[MAXCELL], lanes[MAXCELL];
+};
+template <bool MHD>
+__global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_replay(
+    Params p, const Node *nodes, const int *leaves, int ncell, const int *cell_off, const int *cell_nleaf,
+    const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl, const float *jrecf,
+    const float *jmhdf, ForceOut out, double *psum, int64_t ps, PairRec rec, int *err) {
+  constexpr int NV = NJS<MHD>::n, NR = (NV * MAXCELL + 31) / 32, VS = NV - 1;
+  __shared__ ReplaySmem<NV> smem[MAX_WARPS];
+  ReplaySmem<NV> &sm = smem[threadIdx.x >> 5];
+  PairCell c;
+  if (!pair_cell<false>(c, nodes, leaves, ncell, nullptr, cell_off, cell_nleaf, nullptr, out, err)) return;
+  const int lane = lane_id(), np = c.np;
+  if (lane < np) { sm.ipos[lane] = c.s0 + lane; sm.lanes[lane] = 0; sm.first[lane] = 0; }
+  double tot[NR];
+  for (int r = 0; r < NR; ++r) tot[r] = 0.0;
+  __syncwarp();
+  for (int row = rec.cell[c.cell]; row >= 0;) {
+    const int *d = rec.rows + 32 * (size_t)row + lane;
+    const int own = d[0], head = d[32], il = max(own, 0);
+    const int nit = __shfl_sync(0xffffffffu, head, 0), coded = __shfl_sync(0xffffffffu, head, 1);
+    row = __shfl_sync(0xffffffffu, head, 2);
+    const unsigned g = __match_any_sync(0xffffffffu, own);
+    if (lane < np) sm.lanes[lane] = 0;
+    __syncwarp();
+    if (own >= 0 && lane == __ffs(g) - 1) { sm.first[il] = (unsigned char)lane; sm.lanes[il] = (unsigned char)__popc(g); }
+    const IMix<MHD> I = imix_init<MHD>(sm.ipos[il], txf, txl, jrecf, jmhdf);
+    Kahan f[NF];
+    float vsigmax = 0.0f;
+    int nbi = 0;
+    d += 64;
+    int jn = nit > 0 ? d[0] : -1;
+    for (int t = 0; t < nit; ++t) {
+      const int j = jn, code = coded ? d[32 * (nit + t)] : 0;
+      jn = t + 1 < nit ? d[32 * (t + 1)] : -1;
+      if (j >= 0)
+        force_pair_mixed<MHD, false, false>(p, I, j, code, txf, txl, tx, ty, tz, jrecf, jmhdf, nullptr, nullptr, f,
+                                            vsigmax, nbi);
+    }
+    flush_lanes<NV>(np, sm, sm.red, tot,
+        [&](int k) -> double { return k < VS ? f[njs_slot(k, MHD)].value() : (double)vsigmax; },
         [](int k, double s, double v) -> double { return k < VS ? s + v : fmax_pos(s, v); });
   }
   store_totals<MHD>(sm, NV, np, p.massoftype, tot, psum, ps);
@@ -1378,6 +1476,12 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed_gra
   store_pair_sums<IND>(sm, lane, np, S, c.s0, c.am, psum, ps, p.massoftype, [&](int q) -> double {
     return q < NF ? f[q].value() : (q == NF ? (double)vsigmax : (double)nbi);
   });
+}
+
+// whether force evaluations of this context can be recorded and replayed
+bool pairs_recordable(const ph_ctx *c) {
+  const Params &p = c->dp;
+  return p.precision == PH_PREC_MIXED && !p.gravity && !p.ind && !c->keep_order;
 }
 
 static inline int nblk(int64_t n, int b) { return (int)((n + b - 1) / b); }
@@ -1503,12 +1607,14 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   if (!(c->attr_done & 2u)) {
     const int lb = MAX_WARPS * (int)sizeof(ListSmem), pb = MAX_WARPS * (int)sizeof(PairSmem);
 #define PH_FORCE_ATTR(M, I)                                                                                  \
-  cudaFuncSetAttribute(k_force_mixed<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);                \
+  cudaFuncSetAttribute(k_force_mixed<M, I, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);         \
   cudaFuncSetAttribute(k_force<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);                      \
   cudaFuncSetAttribute(k_force_mixed_grav<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb);           \
   cudaFuncSetAttribute(k_force_grav<M, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, pb)
     PH_FORCE_ATTR(false, false); PH_FORCE_ATTR(true, false); PH_FORCE_ATTR(false, true); PH_FORCE_ATTR(true, true);
 #undef PH_FORCE_ATTR
+    cudaFuncSetAttribute(k_force_mixed<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
+    cudaFuncSetAttribute(k_force_mixed<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb);
     cudaFuncSetAttribute(k_force_sym<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          sym_smem_bytes<NJS<false>::n>(MAXCELL));
     cudaFuncSetAttribute(k_force_sym<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1535,20 +1641,35 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
     ro_force(c);
   } else if (mixed) {
     cudaEventRecord(c->evk[0], st);
-#define PH_FORCE_MIXED(K, M, I, SM)                                                                            \
-  K<M, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(SM), st>>>(                                                    \
-      p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl,   \
-      c->jrecf, jmhdf, out, c->psum, c->cap, cells, actf, ibo, wake, c->d_err)
-#define PH_FORCE_MIXED_I(K, M, SM) do { if (ind) PH_FORCE_MIXED(K, M, true, SM); else PH_FORCE_MIXED(K, M, false, SM); } while (0)
+    const int mode = pairs_recordable(c) ? c->rec_mode : PAIRS_SWEEP;
+    const PairRec rec{c->rec_rows, c->rec_cell, (int)c->rec_cap, c->counters + REC_ROWS};
+    if (mode == PAIRS_RECORD) cudaMemsetAsync(c->counters + REC_ROWS, 0, sizeof(int), st);
+#define PH_FORCE_ARGS                                                                                          \
+  p, c->nodes, c->leaves, nfc, c->pool, c->cell_off, c->cell_nleaf, c->tx, c->ty, c->tz, c->txf, c->txl,       \
+      c->jrecf, jmhdf, out, c->psum, c->cap, cells, actf, ibo, wake
+#define PH_FORCE_MIXED(M, I, R)                                                                                \
+  k_force_mixed<M, I, R><<<nblk(nfc, fw), 32 * fw, fw * sizeof(ListSmem), st>>>(PH_FORCE_ARGS, rec, c->d_err)
+#define PH_FORCE_GRAV(M, I)                                                                                    \
+  k_force_mixed_grav<M, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(PairSmem), st>>>(PH_FORCE_ARGS, c->d_err)
+#define PH_FORCE_REPLAY(M)                                                                                     \
+  k_force_replay<M><<<nblk(nfc, fw), 32 * fw, 0, st>>>(p, c->nodes, c->leaves, nfc, c->cell_off, c->cell_nleaf, \
+                                                       c->tx, c->ty, c->tz, c->txf, c->txl, c->jrecf, jmhdf,   \
+                                                       out, c->psum, c->cap, rec, c->d_err)
     if (p.gravity) {
-      if (p.mhd) PH_FORCE_MIXED_I(k_force_mixed_grav, true, PairSmem);
-      else PH_FORCE_MIXED_I(k_force_mixed_grav, false, PairSmem);
+      if (p.mhd) { if (ind) PH_FORCE_GRAV(true, true); else PH_FORCE_GRAV(true, false); }
+      else { if (ind) PH_FORCE_GRAV(false, true); else PH_FORCE_GRAV(false, false); }
+    } else if (mode == PAIRS_REPLAY) {
+      if (p.mhd) PH_FORCE_REPLAY(true); else PH_FORCE_REPLAY(false);
+    } else if (mode == PAIRS_RECORD) {
+      if (p.mhd) PH_FORCE_MIXED(true, false, true); else PH_FORCE_MIXED(false, false, true);
     } else {
-      if (p.mhd) PH_FORCE_MIXED_I(k_force_mixed, true, ListSmem);
-      else PH_FORCE_MIXED_I(k_force_mixed, false, ListSmem);
+      if (p.mhd) { if (ind) PH_FORCE_MIXED(true, true, false); else PH_FORCE_MIXED(true, false, false); }
+      else { if (ind) PH_FORCE_MIXED(false, true, false); else PH_FORCE_MIXED(false, false, false); }
     }
+#undef PH_FORCE_ARGS
+#undef PH_FORCE_GRAV
+#undef PH_FORCE_REPLAY
 #undef PH_FORCE_MIXED
-#undef PH_FORCE_MIXED_I
   } else if (use_sym(c)) {
     cudaEventRecord(c->evk[0], st);
     if (p.mhd) {

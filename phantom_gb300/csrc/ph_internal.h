@@ -49,6 +49,10 @@ int get_nodes(ph_ctx *c, int64_t *nnodes, int32_t *range, double *xcen, double *
 int ref_ncells(ph_ctx *c, int64_t *ncells);
 int density(ph_ctx *c, int icall);
 int force_dev(ph_ctx *c, const double *vel, const double *Bv);
+enum { PAIRS_SWEEP = 0, PAIRS_RECORD, PAIRS_REPLAY };
+constexpr int REC_ROWS = 24;  // slot of ph_ctx::counters: rows of the pair record
+bool pairs_recordable(const ph_ctx *c);
+bool grow_record(ph_ctx *c, int64_t rows);
 // hydro evaluations of the precision form's rollouts (ph_rollout_pairs.cu)
 void ro_density(ph_ctx *c, const int *act, int nact);
 void ro_force_prologue(ph_ctx *c, const double *vel);
@@ -208,6 +212,14 @@ struct ph_ctx {
   // within a precision-form hydro rollout: evaluations keep the pair order of
   // ph_rollout_pairs.cu
   bool keep_order = false;
+
+  // pair record of the precision form's force (ph_step's velocity iterations):
+  // what the next evaluation does, the recorded rows of 32 ints, the buffer's
+  // rows and the first row of every cell; iterations of the last step
+  int rec_mode = 0;  // PAIRS_SWEEP, PAIRS_RECORD or PAIRS_REPLAY
+  int rec_its = 0;
+  int *rec_rows = nullptr, *rec_cell = nullptr;
+  int64_t rec_cap = 0;
   double *ro_buf = nullptr;  // rollout adjoint buffer (ph_rollout_adjoint)
   size_t ro_cap = 0;
 

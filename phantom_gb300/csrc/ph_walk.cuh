@@ -505,8 +505,8 @@ __device__ __forceinline__ QueueLanes balance_queues(int np, int c, ListBase &sm
 // values pass through shared memory at red (32 RW doubles, free when every lane
 // is done with the queues) and are added in lane order, so totals are
 // deterministic.
-template <int RW, int NR, class T, class Get, class Add>
-__device__ __forceinline__ void flush_lanes(int np, const ListBase &sm, T *red, T (&tot)[NR], Get get, Add add) {
+template <int RW, int NR, class S, class T, class Get, class Add>
+__device__ __forceinline__ void flush_lanes(int np, const S &sm, T *red, T (&tot)[NR], Get get, Add add) {
   static_assert(RW * MAXCELL <= 32 * NR, "totals per lane");
   const int lane = lane_id();
   __syncwarp();
