@@ -601,7 +601,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
           const float hf = (float)hmax_new;
           nodesf[leaf].hmax = hf;
           int pa = nodes[leaf].parent;
-          while (pa >= 0) {
+          // an ancestor that holds as much already was, or is being, raised
+          // with all of its own ancestors: the climb ends there. (Climbing to
+          // the root each time, the growing cells queued for its one address:
+          // 885k particles, a pass 589 -> 223 us.)
+          while (pa >= 0 && *(volatile double *)&nodes_w[pa].hmax < hmax_new) {
             atomic_max_pos(&nodes_w[pa].hmax, hmax_new);
             atomicMax(reinterpret_cast<int *>(&nodesf[pa].hmax), __float_as_int(hf));
             pa = nodes[pa].parent;
