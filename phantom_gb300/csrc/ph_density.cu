@@ -510,7 +510,7 @@ __global__ void k_dv_finish(int n, const double *dvsum, int64_t ps, const double
 // dens.F90:1486-1500, finish_cell dens.F90:1425-1462). FP64 throughout, without
 // its divisions: 1/h by rcp_fast, rho(h) = m (hfact/h)^3, dh/drho = -h^4 /
 // (3 m hfact^3), the convergence test multiplied out. The FP64 pipe bounds the
-// finish; per pass over 2M particles 0.96 -> 0.37 ms.
+// finish; per pass over 2M particles 0.97 -> 0.45 ms.
 struct DensNR {
   double rhoi, dhdrhoi, omega1, hmine;  // omega1 = 1/Omega
   bool conv;
