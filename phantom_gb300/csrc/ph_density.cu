@@ -2,16 +2,15 @@
 // with get_density_sums (dens.F90:578-857), finish_cell (dens.F90:1382-1466),
 // compute_hmax (dens.F90:1275-1289) and store_results (dens.F90:1511-1681).
 //
-// Work decomposition: k_density_pairs takes one warp per active leaf cell. A
-// cell holds np <= 10 particles; the warp's lanes are split into np groups of
-// S = 32/np lanes. Lane (i, s) tests the trial-list entries s, s+S, ... of each
-// staged window for particle i and queues the ones that pass the distance
-// pre-filter; the queued pairs are then summed with every lane busy. The sums
-// of each particle go to a per-particle array, and k_density_finish (one thread
-// per cell) takes the Newton-Raphson update, the cell-wide convergence test,
-// the neighbour-list redo decision and store_results. Cells iterate in
-// device-wide passes; a cell whose hmax grew is re-walked before its next
-// pass, as the reference does per cell.
+// Work decomposition: k_density_pairs takes one warp per active leaf cell. The
+// warp sweeps the cell's trial list with one trial particle per lane, queues
+// for each of the cell's particles the ones that pass the distance pre-filter,
+// and sums the queued pairs with its lanes dealt out by queue length (list
+// sweep and balanced drain). The sums of each particle go to a per-particle
+// array, and k_density_finish (16 lanes per cell) takes the Newton-Raphson
+// update, the cell-wide convergence test, the neighbour-list redo decision and
+// store_results. Cells iterate in device-wide passes; a cell whose hmax grew is
+// re-walked before its next pass, as the reference does per cell.
 //
 // Neighbour decisions are exact: an FP32 pre-filter with a 1e-3 margin in q^2
 // only discards pairs that are provably outside the kernel, and every other
@@ -537,11 +536,15 @@ __device__ __forceinline__ DensNR dens_nr(const Params &p, double r0, double r1,
 
 // finish_cell + compute_hmax (dens.F90:1275-1289) + the redo decision and,
 // for converged cells, store_results (dens.F90:1561-1677). A cell takes a
-// 16-lane segment of a warp, lane q its particle q: the cell-wide convergence
-// test and hmax are segment shuffles, the cell's own decisions are taken by
-// lane 0 of the segment, and the global maxima and statistics are reduced
-// per block before one atomic each (a per-particle atomic on rhomax would
-// serialise 2M updates on one address).
+// 16-lane segment of a warp for its decisions: lane q holds its particle q, the
+// cell-wide convergence test and hmax are segment shuffles, and lane 0 acts for
+// the cell. The particles' FP64 work, which bounds the kernel, is done between
+// by threads packed over the block's particles: in the segments half of the
+// lanes would be idle and an FP64 instruction takes as long for one lane as
+// for 32 (885k particles, the last pass 220 -> 119 us, passes that mostly raise
+// hmax 220 -> 183). Global maxima and statistics are reduced per block before one atomic
+// each (a per-particle atomic on rhomax would serialise 2M updates on one
+// address).
 constexpr int FIN_SEG = 16;  // lanes per cell, >= MAXCELL
 constexpr int FIN_THREADS = 256;
 static_assert(MAXCELL <= FIN_SEG, "a finish segment holds a whole cell");
@@ -552,10 +555,14 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
     double *cell_hmax, int *cell_nits, int *need_walk, int *next_act, int *nnext, DensOut out, NodeF *nodesf,
     const unsigned char *actf, int *err) {
   __shared__ unsigned long long bst[8];  // stats 0..6, rhomax bits
+  constexpr int CELLS = FIN_THREADS / FIN_SEG;
+  __shared__ double pnh[FIN_THREADS];    // per packed particle: new h, tree position, cell, converged
+  __shared__ int pi[FIN_THREADS];
+  __shared__ unsigned char pc[FIN_THREADS], pconv[FIN_THREADS];
+  __shared__ int cnp[CELLS], cnits[CELLS], ctry[CELLS];  // per cell; iterations 0: not converged
   if (threadIdx.x < 8) bst[threadIdx.x] = 0ull;
-  __syncthreads();
   const unsigned FULL = 0xffffffffu;
-  const int lane = lane_id(), q = lane & (FIN_SEG - 1);
+  const int lane = lane_id(), q = lane & (FIN_SEG - 1), seg = threadIdx.x / FIN_SEG;
   const long long a = ((long long)blockIdx.x * FIN_THREADS + threadIdx.x) / FIN_SEG;
   bool cell_ok = a < nact;
   int cell = 0, leaf = 0, np = 0, s0 = 0;
@@ -573,10 +580,27 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
   const bool mine = cell_ok && q < np;
   const size_t ip = (size_t)(s0 + (mine ? (int)__fns(segm, 0, q + 1) : q));
   const double pm = p.massoftype;
+  if (q == 0) { cnp[seg] = cell_ok ? np : 0; cnits[seg] = 0; }
+  __syncthreads();
+  int first_p = 0, total = 0;
+  for (int k = 0; k < CELLS; ++k) {
+    first_p += k < seg ? cnp[k] : 0;
+    total += cnp[k];
+  }
+  if (mine) { pi[first_p + q] = (int)ip; pc[first_p + q] = (unsigned char)seg; }
+  __syncthreads();
+  const bool packed = (int)threadIdx.x < total;
+  const size_t jp = packed ? (size_t)pi[threadIdx.x] : 0;
   DensNR o{};
-  if (mine) o = dens_nr(p, psum[ip], psum[ps + ip], hcur[ip], hold[ip]);
-  int conv = (!mine || o.conv) ? 1 : 0;
-  double hm = mine ? o.hmine : 0.0;
+  if (packed) {
+    o = dens_nr(p, psum[jp], psum[ps + jp], hcur[jp], hold[jp]);
+    pnh[threadIdx.x] = o.hmine;
+    pconv[threadIdx.x] = o.conv ? 1 : 0;
+  }
+  __syncthreads();
+  int conv = !mine || pconv[first_p + q] ? 1 : 0;
+  const double hmine = mine ? pnh[first_p + q] : 0.0;
+  double hm = hmine;
   for (int m = 1; m < FIN_SEG; m <<= 1) {
     conv &= __shfl_xor_sync(FULL, conv, m);
     hm = fmax_pos(hm, __shfl_xor_sync(FULL, hm, m));
@@ -590,7 +614,7 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
     if (nits >= MAXDENSITS) {
       if (lead) set_error(err, PH_ERR_DENS_NOCONV);
     } else {
-      if (mine) hcur[ip] = o.hmine;
+      if (mine) hcur[ip] = hmine;
       if (lead) {
         redo = hmax_new > cell_hmax[cell];
         cell_nits[cell] = nits;
@@ -627,12 +651,18 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
   }
   unsigned long long sv[5] = {0ull, 0ull, 0ull, 0ull, 0ull}, mx[2] = {0ull, 0ull};
   double rhoi_max = 0.0;
-  if (cell_ok && conv) {
-    if (lead) { cell_hmax[cell] = hmax_new; cell_nits[cell] = nits; need_walk[cell] = 0; }
-    const double hme = mine ? hcur[ip] : 0.0;
-    if (mine && hme < 0.0) set_error(err, PH_ERR_NEG_H);
-    if (mine && hme >= 0.0) {
-      const int ntry = cell_ntrial[cell];
+  if (lead && conv) {
+    cell_hmax[cell] = hmax_new; cell_nits[cell] = nits; need_walk[cell] = 0;
+    cnits[seg] = nits;
+    ctry[seg] = cell_ntrial[cell];
+  }
+  __syncthreads();
+  if (packed && cnits[pc[threadIdx.x]] > 0) {
+    const size_t ip = jp;
+    const int nits = cnits[pc[threadIdx.x]], ntry = ctry[pc[threadIdx.x]];
+    const double hme = hcur[ip];
+    if (hme < 0.0) set_error(err, PH_ERR_NEG_H);
+    if (hme >= 0.0) {
       const int pid = perm[ip];
       const double grad = o.omega1;
       const double hfin = p.hfact * cbrt_fast(pm * rcp_fast(o.rhoi));  // hrho (part.F90:845-850)
