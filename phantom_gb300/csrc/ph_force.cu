@@ -5,11 +5,13 @@
 // (anisotropic Lorentz stress, artificial resistivity, div B cleaning) and the
 // self-gravity near field; global Courant/force timestep minima.
 //
-// Decomposition mirrors the density: one warp per leaf cell, lanes split into
-// (particle i, stripe s) pairs over the trial list; pairs that pass the
-// distance pre-filter are queued per particle and evaluated with every lane
-// busy, and the per-particle sums go to k_force_finish (one thread per
-// particle) for finish_cell_and_store_results. The j-side quantities that
+// Decomposition mirrors the density: one warp per leaf cell sweeps the trial
+// list, pairs that pass the distance pre-filter are queued per particle and
+// evaluated with the lanes dealt out by queue length, and the per-particle sums
+// go to k_force_finish (one thread per particle) for
+// finish_cell_and_store_results. With self-gravity every trial pair has a
+// term: those kernels keep lanes of (particle i, stripe s), which evaluate the
+// far pairs where they test them and queue the near ones. The j-side quantities that
 // compute_forces recomputes for every pair (rho_j, P_j/rho_j^2, v_wave,j, the
 // magnetic stress, ...) are computed once per particle by k_force_prologue and
 // read per pair. The neighbour test q_i^2 < 4 .or. q_j^2 < 4 is evaluated with
