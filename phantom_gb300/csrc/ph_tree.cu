@@ -509,21 +509,25 @@ __global__ void __launch_bounds__(256) k_big_pairs(const int *lvl, int nb, const
 
 __device__ __forceinline__ void swap_rows(double *tx, double *ty, double *tz, double *th, int *perm, float4 *txf,
                                           int a, int b) {
-  double t;
-  t = tx[a]; tx[a] = tx[b]; tx[b] = t;
-  t = ty[a]; ty[a] = ty[b]; ty[b] = t;
-  t = tz[a]; tz[a] = tz[b]; tz[b] = t;
-  t = th[a]; th[a] = th[b]; th[b] = t;
-  int u = perm[a]; perm[a] = perm[b]; perm[b] = u;
-  float4 f = txf[a]; txf[a] = txf[b]; txf[b] = f;
+  // all loads before the stores, which may alias to the compiler
+  const double xa = tx[a], ya = ty[a], za = tz[a], ha = th[a], xb = tx[b], yb = ty[b], zb = tz[b], hb = th[b];
+  const int ua = perm[a], ub = perm[b];
+  const float4 fa = txf[a], fb = txf[b];
+  tx[a] = xb; ty[a] = yb; tz[a] = zb; th[a] = hb; perm[a] = ub; txf[a] = fb;
+  tx[b] = xa; ty[b] = ya; tz[b] = za; th[b] = ha; perm[b] = ua; txf[b] = fa;
 }
 
-// swap each left-region big with its paired right-region small (kdtree.F90:969-977)
+// swap each left-region big with its paired right-region small (kdtree.F90:969-977).
+// The chunk's bigs are listed in shared memory and dealt to the threads one by
+// one: a thread that swapped its own eight in turn waited for up to eight
+// rounds of loads, 64 bytes apart between lanes (885k particles, a level 64 ->
+// 19 us).
 __global__ void __launch_bounds__(256) k_big_swap(const int *lvl, int nb, const int *cbase, const Node *nodes,
                                                   double *tx, double *ty, double *tz, double *th, int *perm,
                                                   float4 *txf, const int *misc, const double *pivot,
                                                   const int *bl, const int *pairpos) {
   __shared__ int s[16];
+  __shared__ unsigned short bigs[CHUNK];
   int c = blockIdx.x;
   if (c >= cbase[nb]) return;
   int k = find_chunk_node(cbase, nb, c);
@@ -531,6 +535,7 @@ __global__ void __launch_bounds__(256) k_big_swap(const int *lvl, int nb, const 
   if (misc[4 * k + 2]) return;
   int b = nd.start + (c - cbase[k]) * CHUNK, e = min(b + CHUNK, nd.start + nd.count);
   int ax = misc[4 * k], bnd = nd.start + misc[4 * k + 1];
+  if (b >= bnd) return;
   const long long pk = dkey(pivot[k]);
   const double *cx = ax == 0 ? tx : (ax == 1 ? ty : tz);
   int i0 = b + threadIdx.x * 8;
@@ -542,14 +547,11 @@ __global__ void __launch_bounds__(256) k_big_swap(const int *lvl, int nb, const 
   }
   int total;
   int pre = block_excl_scan(cntl, s, total);
-  int r = bl[c] + pre;
-  for (int q = 0; q < 8; ++q) {
-    if (flags & (1 << q)) {
-      int partner = pairpos[nd.start + r];
-      swap_rows(tx, ty, tz, th, perm, txf, i0 + q, partner);
-      ++r;
-    }
-  }
+  for (int q = 0; q < 8; ++q)
+    if (flags & (1 << q)) bigs[pre++] = (unsigned short)(threadIdx.x * 8 + q);
+  __syncthreads();
+  const int *partner = pairpos + nd.start + bl[c];
+  for (int m = threadIdx.x; m < total; m += 256) swap_rows(tx, ty, tz, th, perm, txf, b + bigs[m], partner[m]);
 }
 
 // child bounding boxes (kdtree.F90:868-896): partial min/max per chunk and
