@@ -67,7 +67,7 @@ int alloc_all(ph_ctx *c, int64_t cap) {
   r |= dalloc(c, &c->lvl_bb_a, 6 * (size_t)c->lvl_cap); r |= dalloc(c, &c->lvl_bb_b, 6 * (size_t)c->lvl_cap);
   r |= dalloc(c, &c->lvl_misc, 4 * (size_t)c->lvl_cap); r |= dalloc(c, &c->lvl_pivot, (size_t)c->lvl_cap);
   c->chunk_cap = (int)(n / CHUNK + c->lvl_cap + 8);
-  r |= dalloc(c, &c->cbase, (size_t)c->lvl_cap + 1);
+  r |= dalloc(c, &c->cbase, (size_t)c->lvl_cap + 1 + (size_t)c->chunk_cap);
   r |= dalloc(c, &c->part_d, 16 * (size_t)std::max<int64_t>(c->chunk_cap, 2048));
   r |= dalloc(c, &c->part_i, 3 * (size_t)c->chunk_cap);
   r |= dalloc(c, &c->counters, 64); r |= dalloc(c, &c->top_nodes, 32);
