@@ -127,7 +127,7 @@ bool grow_record(ph_ctx *c, int64_t rows) {
   if (c->rec_cap >= rows) return true;
   if (rows > INT32_MAX) return false;
   size_t avail = 0, total = 0;
-  const size_t bytes = 128 * (size_t)rows + (c->rec_cell ? 0 : sizeof(int) * (size_t)c->cap);
+  const size_t bytes = 512 * (size_t)rows + (c->rec_cell ? 0 : sizeof(int) * (size_t)c->cap);
   if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 4 < bytes) return false;
   if (c->rec_rows) dfree(c, c->rec_rows);
   c->rec_rows = nullptr;

@@ -1184,20 +1184,28 @@ __device__ __forceinline__ void far_pair_mixed(float dx, float dy, float dz, flo
   f[3].add(-y);
 }
 
+// The trial particle's FP32 record. Loaded after the separation, whose
+// registers are free by then (cloud of 2M particles 91.6 -> 90.1 ms); with MHD
+// before it, to have the longer pair's operands under way (force of 128^3
+// particles 4.54 -> 4.52 ms).
+struct MixRec {
+  float4 a, b, c, d;
+  __device__ __forceinline__ void load(const float *jrecf, int j) {
+    const float4 *r4 = reinterpret_cast<const float4 *>(jrecf + JRECF * (size_t)j);
+    a = r4[0]; b = r4[1]; c = r4[2]; d = r4[3];
+  }
+};
+
 // One trial pair of compute_forces (force.F90:914-2060) in FP32 (sums without
 // the particle mass)
 template <bool MHD, bool GRAV, bool IND>
-__device__ __forceinline__ void force_pair_mixed(const Params &p, const IMix<MHD> &I, int j, int code,
-                                                 const float4 *txf, const float4 *txl, const double *tx,
-                                                 const double *ty, const double *tz, const float *jrecf,
-                                                 const float *jmhdf, const int8_t *ibin_old_t,
+__device__ __forceinline__ void force_pair_mixed(const Params &p, const IMix<MHD> &I, int j, float dx, float dy,
+                                                 float dz, float rij2, const MixRec &jr, const float *jmhdf,
+                                                 const int8_t *ibin_old_t,
                                                  unsigned char *wakemark, Kahan (&f)[NF], float &vsigmax, int &nbi) {
   const bool adiab = !p.isothermal;
   const float beta = (float)p.beta;
-  const float4 *r4 = reinterpret_cast<const float4 *>(jrecf + JRECF * (size_t)j);
-  const float4 ra = r4[0], rb = r4[1], rc = r4[2], rd = r4[3];
-  float dx, dy, dz, rij2;
-  separation_2f(p, I.s, j, code, txf[j], txl[j], tx, ty, tz, dx, dy, dz, rij2);
+  const float4 ra = jr.a, rb = jr.b, rc = jr.c, rd = jr.d;
   const float hj1 = ra.x;
   const float q2i = rij2 * (I.h1 * I.h1), q2j = rij2 * (hj1 * hj1);
   const bool qi_in = q2i < 4.0f, qj_in = q2j < 4.0f;
@@ -1285,16 +1293,16 @@ __device__ __forceinline__ void force_pair_mixed(const Params &p, const IMix<MHD
 // 300001 particles 2.77 -> 2.39 ms.
 //
 // A velocity iteration evaluates the force again with the same positions and
-// smoothing lengths, so its pairs, and their lanes, are those of the evaluation
-// before. With REC the kernel writes each drain's pairs as the lanes take them:
-// a row of the lanes' particles, a row with the number of pair rows, whether
-// code rows follow and the cell's next drain, then a row of 32 trial particles
-// per step (-1: idle lane), then as many of their offset codes where any is not
-// 0. The rows are counted on past the buffer's end; the host then takes no
+// smoothing lengths, so its pairs, their separations and their lanes are those
+// of the evaluation before. With REC the kernel writes each drain's pairs as the
+// lanes take them: a row with every lane's particle, the number of pair rows and
+// the cell's next drain, then rows of 32 (separation, trial particle; -1: idle
+// lane). The rows are counted on past the buffer's end; the host then takes no
 // part of the record.
 struct PairRec {
-  int *rows, *cell;  // rows of 32, first row of every cell
-  int cap, *top;     // rows there are, rows taken (counted on past cap)
+  float4 *rows;    // rows of 32
+  int *cell;       // first row of every cell
+  int cap, *top;   // rows there are, rows taken
 };
 template <bool MHD, bool IND, bool REC>
 __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
@@ -1330,40 +1338,40 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
                                               [&](float h1) { return __fdividef(q2lim, h1 * h1); });
     const QueueLanes ql = balance_queues(np, myc, sm);
     const int il = max(ql.il, 0);
+    float4 *rd = nullptr;  // the lane's next record slot
+    int nit = 0;
     if constexpr (REC) {
       const int nst = ql.c > ql.m0 ? (ql.c - ql.m0 + ql.step - 1) / ql.step : 0;
-      const int nit = (int)__reduce_max_sync(0xffffffffu, (unsigned)nst);
-      bool coded = false;
-      if (p.periodic)
-        for (int t = 0; t < nst; ++t) coded = coded || sm.qc[il * qstride + ql.m0 + t * ql.step] != 0;
-      coded = __any_sync(0xffffffffu, coded);
-      const int need = 2 + nit * (coded ? 2 : 1);
+      nit = (int)__reduce_max_sync(0xffffffffu, (unsigned)nst);
       int row = 0;
-      if (lane == 0) row = atomicAdd(rec.top, need);
+      if (lane == 0) row = atomicAdd(rec.top, 1 + nit);
       row = __shfl_sync(0xffffffffu, row, 0);
-      if (row >= 0 && row <= rec.cap - need) {
-        int *d = rec.rows + 32 * (size_t)row + lane;
-        d[0] = ql.il;
-        d[32] = lane == 0 ? nit : (lane == 1 ? (coded ? 1 : 0) : -1);
-        for (int t = 0; t < nit; ++t) {
-          const int m = il * qstride + ql.m0 + t * ql.step;
-          d[64 + 32 * t] = t < nst ? sm.qj[m] : -1;
-          if (coded) d[64 + 32 * (nit + t)] = t < nst ? sm.qc[m] & 63 : 0;
-        }
-        if (lane == 0) {
-          if (prev < 0) rec.cell[c.cell] = row;
-          else rec.rows[32 * (size_t)prev + 34] = row;
-        }
+      if (row >= 0 && row <= rec.cap - (1 + nit)) {
+        rd = rec.rows + 32 * (size_t)row + lane;
+        *rd = make_float4(__int_as_float(ql.il), __int_as_float(nit), __int_as_float(-1), 0.0f);
+        __syncwarp();
+        if (lane == 0 && prev < 0) rec.cell[c.cell] = row;
+        if (prev >= 0) rec.rows[32 * (size_t)prev + lane].z = __int_as_float(row);
         prev = row;
+        rd += 32;
       }
     }
     const IMix<MHD> I = imix_init<MHD>(sm.ipos[il], txf, txl, jrecf, jmhdf);
     Kahan f[NF];
     float vsigmax = 0.0f;
     int nbi = 0;
-    for (int m = ql.m0; m < ql.c; m += ql.step)
-      force_pair_mixed<MHD, false, IND>(p, I, sm.qj[il * qstride + m], sm.qc[il * qstride + m] & 63, txf, txl, tx, ty,
-                                        tz, jrecf, jmhdf, ibin_old_t, wakemark, f, vsigmax, nbi);
+    for (int m = ql.m0; m < ql.c; m += ql.step) {
+      const int j = sm.qj[il * qstride + m];
+      MixRec jr;
+      if (MHD) jr.load(jrecf, j);
+      float dx, dy, dz, r2;
+      separation_2f(p, I.s, j, sm.qc[il * qstride + m] & 63, txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
+      if (!MHD) jr.load(jrecf, j);
+      if (REC && rd) { *rd = make_float4(dx, dy, dz, __int_as_float(j)); rd += 32; --nit; }
+      force_pair_mixed<MHD, false, IND>(p, I, j, dx, dy, dz, r2, jr, jmhdf, ibin_old_t, wakemark, f, vsigmax, nbi);
+    }
+    if (REC && rd)
+      for (; nit > 0; --nit, rd += 32) *rd = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
     static_assert(32 * NV <= LQ / 2, "lane sums staged in the queues' space");
     flush_lanes<NV>(np, sm, sm.red, tot,
         [&](int k) -> double { return k < VS ? f[njs_slot(k, MHD)].value() : (k == VS ? (double)vsigmax : (double)nbi); },
@@ -1373,11 +1381,13 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
 }
 
 // The evaluations after a recorded one: same pairs, same lanes, same sums in the
-// same order (bit-identical results) without the sweep, which is half of the
-// kernel above (189 of 395 us at 64^3); what remains waits for the gathers of
-// the trial particles' records. Three Sedov steps of 128^3 particles, five
-// evaluations each: 99.5 -> 88.1 ms, with the Cullen-Dehnen switch at 96^3
-// 58.3 -> 49.6 ms.
+// same order (bit-identical results) without the sweep, half of the kernel above
+// (189 of 395 us at 64^3), and without the separations and their two gathers
+// per pair; what remains waits for the trial particles' records. Three Sedov
+// steps of 128^3 particles, five evaluations each: swept 99.5, with only the
+// trial particles recorded 88.1 ms; and, the tree faster since, 82.7 against
+// 77.7 ms with separations; with the Cullen-Dehnen switch at 96^3 58.3, 47.2 and 45.1 ms. 24
+// warps per SM: with 20 or 28 the Sedov steps take 2 % longer, with 32 14 %.
 template <int NV>
 struct ReplaySmem {
   double red[32 * NV];
@@ -1387,8 +1397,8 @@ struct ReplaySmem {
 template <bool MHD>
 __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_replay(
     Params p, const Node *nodes, const int *leaves, int ncell, const int *cell_off, const int *cell_nleaf,
-    const double *tx, const double *ty, const double *tz, const float4 *txf, const float4 *txl, const float *jrecf,
-    const float *jmhdf, ForceOut out, double *psum, int64_t ps, PairRec rec, int *err) {
+    const float4 *txf, const float4 *txl, const float *jrecf, const float *jmhdf, ForceOut out, double *psum, int64_t ps,
+    PairRec rec, int *err) {
   constexpr int NV = NJS<MHD>::n, NR = (NV * MAXCELL + 31) / 32, VS = NV - 1;
   __shared__ ReplaySmem<NV> smem[MAX_WARPS];
   ReplaySmem<NV> &sm = smem[threadIdx.x >> 5];
@@ -1400,10 +1410,10 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_replay(
   for (int r = 0; r < NR; ++r) tot[r] = 0.0;
   __syncwarp();
   for (int row = rec.cell[c.cell]; row >= 0;) {
-    const int *d = rec.rows + 32 * (size_t)row + lane;
-    const int own = d[0], head = d[32], il = max(own, 0);
-    const int nit = __shfl_sync(0xffffffffu, head, 0), coded = __shfl_sync(0xffffffffu, head, 1);
-    row = __shfl_sync(0xffffffffu, head, 2);
+    const float4 *d = rec.rows + 32 * (size_t)row + lane;
+    const float4 head = d[0];
+    const int own = __float_as_int(head.x), nit = __float_as_int(head.y), il = max(own, 0);
+    row = __float_as_int(head.z);
     const unsigned g = __match_any_sync(0xffffffffu, own);
     if (lane < np) sm.lanes[lane] = 0;
     __syncwarp();
@@ -1412,14 +1422,20 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_replay(
     Kahan f[NF];
     float vsigmax = 0.0f;
     int nbi = 0;
-    d += 64;
-    int jn = nit > 0 ? d[0] : -1;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+    d += 32;
+    float4 next = nit > 0 ? d[0] : none;
     for (int t = 0; t < nit; ++t) {
-      const int j = jn, code = coded ? d[32 * (nit + t)] : 0;
-      jn = t + 1 < nit ? d[32 * (t + 1)] : -1;
-      if (j >= 0)
-        force_pair_mixed<MHD, false, false>(p, I, j, code, txf, txl, tx, ty, tz, jrecf, jmhdf, nullptr, nullptr, f,
-                                            vsigmax, nbi);
+      const float4 a = next;
+      d += 32;
+      next = t + 1 < nit ? d[0] : none;
+      const int j = __float_as_int(a.w);
+      if (j >= 0) {
+        MixRec jr;
+        jr.load(jrecf, j);
+        force_pair_mixed<MHD, false, false>(p, I, j, a.x, a.y, a.z, a.x * a.x + a.y * a.y + a.z * a.z, jr, jmhdf,
+                                            nullptr, nullptr, f, vsigmax, nbi);
+      }
     }
     flush_lanes<NV>(np, sm, sm.red, tot,
         [&](int k) -> double { return k < VS ? f[njs_slot(k, MHD)].value() : (double)vsigmax; },
@@ -1474,8 +1490,13 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed_gra
       return false;
     };
     queue_window(cnt, S, act, il, stripe, sm.q, test, [&](int k) {
-      force_pair_mixed<MHD, true, IND>(p, I, stg.jidx[k], stg.code[k], txf, txl, tx, ty, tz, jrecf, jmhdf, ibin_old_t,
-                                       wakemark, f, vsigmax, nbi);
+      const int j = stg.jidx[k];
+      MixRec jr;
+      if (MHD) jr.load(jrecf, j);
+      float dx, dy, dz, r2;
+      separation_2f(p, I.s, j, stg.code[k], txf[j], txl[j], tx, ty, tz, dx, dy, dz, r2);
+      if (!MHD) jr.load(jrecf, j);
+      force_pair_mixed<MHD, true, IND>(p, I, j, dx, dy, dz, r2, jr, jmhdf, ibin_old_t, wakemark, f, vsigmax, nbi);
     });
   }
   store_pair_sums<IND>(sm, lane, np, S, c.s0, c.am, psum, ps, p.massoftype, [&](int q) -> double {
@@ -1658,7 +1679,7 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   k_force_mixed_grav<M, I><<<nblk(nfc, fw), 32 * fw, fw * sizeof(PairSmem), st>>>(PH_FORCE_ARGS, c->d_err)
 #define PH_FORCE_REPLAY(M)                                                                                     \
   k_force_replay<M><<<nblk(nfc, fw), 32 * fw, 0, st>>>(p, c->nodes, c->leaves, nfc, c->cell_off, c->cell_nleaf, \
-                                                       c->tx, c->ty, c->tz, c->txf, c->txl, c->jrecf, jmhdf,   \
+                                                       c->txf, c->txl, c->jrecf, jmhdf,                        \
                                                        out, c->psum, c->cap, rec, c->d_err)
     if (p.gravity) {
       if (p.mhd) { if (ind) PH_FORCE_GRAV(true, true); else PH_FORCE_GRAV(true, false); }

@@ -214,11 +214,12 @@ struct ph_ctx {
   bool keep_order = false;
 
   // pair record of the precision form's force (ph_step's velocity iterations):
-  // what the next evaluation does, the recorded rows of 32 ints, the buffer's
-  // rows and the first row of every cell; iterations of the last step
+  // what the next evaluation does, the recorded rows of 32 float4, the
+  // buffer's rows and the first row of every cell; iterations of the last step
   int rec_mode = 0;  // PAIRS_SWEEP, PAIRS_RECORD or PAIRS_REPLAY
   int rec_its = 0;
-  int *rec_rows = nullptr, *rec_cell = nullptr;
+  float4 *rec_rows = nullptr;
+  int *rec_cell = nullptr;
   int64_t rec_cap = 0;
   double *ro_buf = nullptr;  // rollout adjoint buffer (ph_rollout_adjoint)
   size_t ro_cap = 0;

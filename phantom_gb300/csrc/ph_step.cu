@@ -325,7 +325,7 @@ int ph_step(ph_ctx *c, double t, double dtsph, double *dtnew, int32_t *its_out, 
   // evaluation: the predictor's where the last step iterated twice or more,
   // else the first iteration's. A record that did not fit is taken again with
   // room for it (a context's first record only counts its rows). Recording adds
-  // about 7 % to an evaluation and a replay saves 45 %, so an evaluation that
+  // about a tenth to an evaluation and a replay saves more than half, so an evaluation that
   // nothing is known to follow (one iteration per step) is not recorded.
   struct RecordMode {
     ph_ctx *c;
