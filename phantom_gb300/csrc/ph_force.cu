@@ -1386,8 +1386,9 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_mixed(
 // per pair; what remains waits for the trial particles' records. Three Sedov
 // steps of 128^3 particles, five evaluations each: swept 99.5, with only the
 // trial particles recorded 88.1 ms; and, the tree faster since, 82.7 against
-// 77.7 ms with separations; with the Cullen-Dehnen switch at 96^3 58.3, 47.2 and 45.1 ms. 24
-// warps per SM: with 20 or 28 the Sedov steps take 2 % longer, with 32 14 %.
+// 77.7 ms with separations. With the Cullen-Dehnen switch at 96^3: 58.3, 47.2
+// and 45.1 ms. 24 warps per SM: 20 or 28 make the Sedov steps 2 % longer, 32
+// 14 %.
 template <int NV>
 struct ReplaySmem {
   double red[32 * NV];
