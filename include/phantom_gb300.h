@@ -36,7 +36,8 @@ enum {
   PH_ERR_NEG_H = 8,        /* negative smoothing length (dens.F90:1566,1598; force.F90:2271) */
   PH_ERR_DT = 9,           /* invalid Courant timestep (force.F90:3214) */
   PH_ERR_TOLV = 10,        /* leapfrog velocity iterations not converged (step_leapfrog.f90:753-756) */
-  PH_ERR_LIST = 11,        /* neighbour list pool exhausted (retried internally) */
+  PH_ERR_LIST = 11,        /* neighbour list pool exhausted (retried internally), or a pair record
+                              whose rows do not follow one another */
   PH_ERR_CAPACITY = 12,    /* npart exceeds the context capacity */
   PH_ERR_STATE = 13,       /* call order: e.g. force before density */
   PH_ERR_NOT_BUILT = 14,   /* feature not compiled into this library */

@@ -10,12 +10,14 @@ using namespace ph;
 
 namespace {
 
+// A cleared device buffer of the context. Cleared on the context's stream, which
+// does not wait for the default stream: the launches that follow write into it.
 template <typename T>
 int dalloc(ph_ctx *c, T **p, size_t count) {
   size_t bytes = sizeof(T) * (count > 0 ? count : 1);
   void *q = nullptr;
   if (cudaMalloc(&q, bytes) != cudaSuccess) return PH_ERR_CUDA;
-  cudaMemset(q, 0, bytes);
+  cudaMemsetAsync(q, 0, bytes, c->stream);
   c->allocs.push_back(DeviceBuf{q, bytes});
   *p = static_cast<T *>(q);
   return 0;

@@ -1410,11 +1410,16 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MHD ? 5 : 6) k_force_replay(
   double tot[NR];
   for (int r = 0; r < NR; ++r) tot[r] = 0.0;
   __syncwarp();
-  for (int row = rec.cell[c.cell]; row >= 0;) {
+  for (int row = rec.cell[c.cell], last = -1; row >= 0;) {
+    // a cell's drains took their rows one after the other, each inside the
+    // buffer: anything else is not a record, and following it need not end
+    if (row <= last || row >= rec.cap) { if (lane == 0) set_error(err, PH_ERR_LIST); break; }
     const float4 *d = rec.rows + 32 * (size_t)row + lane;
     const float4 head = d[0];
-    const int own = __float_as_int(head.x), nit = __float_as_int(head.y), il = max(own, 0);
-    row = __float_as_int(head.z);
+    const int own = __float_as_int(head.x), il = max(own, 0);
+    const int nit = min(__shfl_sync(0xffffffffu, __float_as_int(head.y), 0), rec.cap - 1 - row);
+    last = row;
+    row = __shfl_sync(0xffffffffu, __float_as_int(head.z), 0);
     const unsigned g = __match_any_sync(0xffffffffu, own);
     if (lane < np) sm.lanes[lane] = 0;
     __syncwarp();
