@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "ph_internal.h"
+#include "ph_jbuf.h"
 
 using namespace ph;
 
@@ -140,29 +141,28 @@ bool grow_record(ph_ctx *c, int64_t rows) {
   return true;
 }
 
-int alloc_sym(ph_ctx *c, int64_t jbuf_stride, int nj) {
-  int r = 0;
-  if (!c->cell_at) {
-    r |= dalloc(c, &c->cell_at, (size_t)c->cap);
-    r |= dalloc(c, &c->cell_tbase, (size_t)c->cap + 1);
+int alloc_sym(ph_ctx *c, int64_t rows, int nj) {
+  if (!c->cell_tbase) {
+    if (!c->cell_at && dalloc(c, &c->cell_at, (size_t)c->cap) != 0) return PH_ERR_CUDA;
+    if (dalloc(c, &c->cell_tbase, (size_t)c->cap + 1) != 0) return PH_ERR_CUDA;
   }
   if (c->toff_cap < c->pool_cap) {
     if (c->toff) dfree(c, c->toff);
     c->toff = nullptr;
-    r |= dalloc(c, &c->toff, (size_t)c->pool_cap);
+    c->toff_cap = 0;
+    if (dalloc(c, &c->toff, (size_t)c->pool_cap) != 0) return PH_ERR_CUDA;
     c->toff_cap = c->pool_cap;
   }
-  const int64_t bytes = (int64_t)sizeof(double) * nj * jbuf_stride;
-  if (c->jbuf_bytes < bytes || c->jbuf_stride < jbuf_stride) {
+  const JbufPlan jp = jbuf_plan(c->jbuf_stride, c->jbuf_doubles, rows, nj);
+  if (!jp.keep) {
     if (c->jbuf) dfree(c, c->jbuf);
     c->jbuf = nullptr;
-    // room for 25 % more trial entries than this build has
-    const int64_t stride = jbuf_stride + jbuf_stride / 4 + 1024;
-    r |= dalloc(c, &c->jbuf, (size_t)nj * (size_t)stride);
-    c->jbuf_stride = stride;
-    c->jbuf_bytes = (int64_t)sizeof(double) * nj * stride;
+    c->jbuf_stride = c->jbuf_doubles = 0;
+    if (dalloc(c, &c->jbuf, (size_t)jp.doubles) != 0) return PH_ERR_CUDA;
+    c->jbuf_stride = jp.stride;
+    c->jbuf_doubles = jp.doubles;
   }
-  return r ? PH_ERR_CUDA : 0;
+  return 0;
 }
 
 int alloc_rollout(ph_ctx *c, size_t doubles) {

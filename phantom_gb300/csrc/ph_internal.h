@@ -62,7 +62,7 @@ int force_lists(ph_ctx *c);
 // symmetric FP64 pair loop: cell_at / cell_tbase (per position / cell), the
 // flattened trial offsets toff (pool capacity) and the j-side buffer jbuf
 // (nj values x stride doubles), grown to the sizes asked for
-int alloc_sym(ph_ctx *c, int64_t jbuf_stride, int nj);
+int alloc_sym(ph_ctx *c, int64_t rows, int nj);
 // device buffer of the rollout adjoint (checkpoints, segment states, cotangents), grown to `doubles`
 int alloc_rollout(ph_ctx *c, size_t doubles);
 int gravity_far(ph_ctx *c);
@@ -206,7 +206,7 @@ struct ph_ctx {
   int *cell_at = nullptr, *cell_tbase = nullptr, *toff = nullptr;
   int64_t toff_cap = 0;
   double *jbuf = nullptr;
-  int64_t jbuf_stride = 0, jbuf_bytes = 0;
+  int64_t jbuf_stride = 0, jbuf_doubles = 0;
   int64_t sym_total = 0;  // owned trial entries of the current lists (jbuf rows in use)
 
   // within a precision-form hydro rollout: evaluations keep the pair order of
