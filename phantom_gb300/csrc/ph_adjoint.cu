@@ -1378,6 +1378,7 @@ int adjoint_dev(ph_ctx *c, const double *w_dev, const double *wB_dev, double *gx
   // records' space, which the next force call rebuilds); FP64 on the symmetric
   // force lists, each pair once
   const bool hydro = !p.mhd && !p.gravity && !c->keep_order;
+  if (hydro && mixed) low_words(c);
   const bool sym = hydro && !mixed && c->force_sym && c->toff && c->sym_total > 0;
   double *hrec = sym ? c->jrec : nullptr;
   float *hrecf = hydro && mixed ? c->jrecf : nullptr;

@@ -57,6 +57,18 @@ __global__ void k_dens_bprep(Params p, int n, const int *perm, const double *Bev
   }
 }
 
+// the low parts of position i
+__device__ __forceinline__ float4 low_parts(const double *tx, const double *ty, const double *tz, const float4 *txf,
+                                            int i) {
+  const float4 f = txf[i];
+  return make_float4(d2f_rn(tx[i] - (double)f.x), d2f_rn(ty[i] - (double)f.y), d2f_rn(tz[i] - (double)f.z), 0.0f);
+}
+__global__ void k_low_words(int n, const double *tx, const double *ty, const double *tz, const float4 *txf,
+                            float4 *txl) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) txl[i] = low_parts(tx, ty, tz, txf, i);
+}
+
 // gather per-particle tree-order inputs: h, and for the mixed form the low
 // parts of the positions (txf holds the high parts, set by the tree build)
 __global__ void k_dens_gather(int n, const int *perm, const double *xyzh, const double *tx, const double *ty,
@@ -65,10 +77,7 @@ __global__ void k_dens_gather(int n, const int *perm, const double *xyzh, const 
   if (i >= n) return;
   double h = xyzh[4 * (size_t)perm[i] + 3];
   hcur[i] = h; hold[i] = h;
-  if (txl) {
-    const float4 f = txf[i];
-    txl[i] = make_float4(d2f_rn(tx[i] - (double)f.x), d2f_rn(ty[i] - (double)f.y), d2f_rn(tz[i] - (double)f.z), 0.0f);
-  }
+  if (txl) txl[i] = low_parts(tx, ty, tz, txf, i);
 }
 
 __global__ void k_dens_init_cells(int ncell, const int *leaves, const Node *nodes, double *cell_hmax,
@@ -741,6 +750,16 @@ __global__ void __launch_bounds__(FIN_THREADS) k_density_finish(
 
 static inline int nblk(int64_t n, int b) { return (int)((n + b - 1) / b); }
 
+// The low parts for the precision form's force and adjoint, where the density
+// before them was the plain form's (else its gather has written them)
+void low_words(ph_ctx *c) {
+  if (c->have_low) return;
+  const int nt = (int)c->ntree;
+  k_low_words<<<nblk(nt, 256), 256, 0, c->stream>>>(nt, c->tx, c->ty, c->tz, c->txf, c->txl);
+  count_launch(c, 1);
+  c->have_low = true;
+}
+
 // densityiterate driver
 int density(ph_ctx *c, int icall) {
   if (!c->have_tree) return PH_ERR_STATE;
@@ -750,6 +769,7 @@ int density(ph_ctx *c, int icall) {
   const Params p = c->dp;
   k_dens_gather<<<nblk(nt, 256), 256, 0, st>>>(nt, c->perm, c->xyzh, c->tx, c->ty, c->tz, c->hcur, c->hold, c->txf,
                                               p.precision == PH_PREC_MIXED ? c->txl : nullptr);
+  c->have_low = c->have_low || p.precision == PH_PREC_MIXED;
   k_dens_init_cells<<<nblk(ncell, 256), 256, 0, st>>>(ncell, c->leaves, c->nodes, c->cell_hmax, c->cell_nits, c->act_a);
   cudaMemsetAsync(c->stats, 0, 8 * sizeof(unsigned long long), st);
   cudaMemsetAsync(c->red, 0, 8 * sizeof(double), st);

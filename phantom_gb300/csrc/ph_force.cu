@@ -1618,6 +1618,7 @@ int force_dev(ph_ctx *c, const double *vel, const double *Bv) {
   double *jmhd = c->jrec + JREC * (size_t)c->cap;
   const bool mixed = p.precision == PH_PREC_MIXED;
   float *jmhdf = c->jrecf + JRECF * (size_t)c->cap;
+  if (mixed) low_words(c);
   if (c->keep_order)
     ro_force_prologue(c, vel);
   else if (mixed)

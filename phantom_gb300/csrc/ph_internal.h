@@ -59,6 +59,7 @@ void ro_force_prologue(ph_ctx *c, const double *vel);
 void ro_force(ph_ctx *c);
 int derivs_dev(ph_ctx *c, int icall, const double *vel, const double *Bv, double *dtnew);
 int force_lists(ph_ctx *c);
+void low_words(ph_ctx *c);
 // symmetric FP64 pair loop: cell_at / cell_tbase (per position / cell), the
 // flattened trial offsets toff (pool capacity) and the j-side buffer jbuf
 // (nj values x stride doubles), grown to the sizes asked for
@@ -235,6 +236,7 @@ struct ph_ctx {
   float *jrecf = nullptr;    // FP32 copy of the j records (mixed precision form)
   float4 *txf = nullptr;     // float x,y,z (high parts of tx, ty, tz); w: 1/h for the force
   float4 *txl = nullptr;     // low parts: tx - (double)txf.x, ... (mixed form)
+  bool have_low = false;     // txl belongs to the present positions (low_words)
   float4 *bjf = nullptr;     // FP32 B rho per tree position (mixed MHD density)
   double pf_hmin = 0.0;      // below this h the FP32 prefilter is bypassed
   double *red = nullptr;     // reductions: dtcourant, dtforce, rhomax, ...

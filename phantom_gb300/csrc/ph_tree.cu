@@ -1613,6 +1613,7 @@ int build_tree(ph_ctx *c) {
   cudaStream_t st = c->stream;
   const int n = (int)c->n;
   const Params p = c->dp;
+  c->have_low = false;
   k_root_wrap<<<nblk(n, 256), 256, 0, st>>>(p, c->xyzh, n, c->alive, c->d_err);
   scan_int(c, c->alive, c->pairpos, n, c->counters + 4);
   int nalive = 0;
@@ -1726,6 +1727,7 @@ int revtree(ph_ctx *c) {
   cudaStream_t st = c->stream;
   const Params p = c->dp;
   const int nt = (int)c->ntree, nbig = c->nbig_nodes, nsmall = c->nsmall_nodes;
+  c->have_low = false;
   k_rev_gather<<<nblk(nt, 256), 256, 0, st>>>(c->xyzh, nt, c->perm, c->tx, c->ty, c->tz, c->th, c->txf);
   count_launch(c, 1);
   mass_table(c, p.massoftype);
