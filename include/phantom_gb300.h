@@ -99,6 +99,11 @@ typedef struct ph_ctx ph_ctx;
  * Replaces the allocation done by allocate_neigh/allocate_kdtree
  * (neigh_kdtree.f90:56-72, kdtree.F90:75-87). */
 int ph_init(const ph_params *params, int64_t maxp, ph_ctx **ctx);
+/* Change the parameters of a context. The tree and density of the present
+ * particles stay usable by the calls that follow (a force in the other precision
+ * form included; trial lists are made again where a parameter they depend on
+ * changed), except that a new minpart, or self-gravity switched on, needs a
+ * new tree and density (PH_ERR_STATE until then). */
 int ph_set_params(ph_ctx *ctx, const ph_params *params);
 void ph_finalize(ph_ctx *ctx);
 const char *ph_strerror(int code);

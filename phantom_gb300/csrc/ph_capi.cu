@@ -363,8 +363,20 @@ int ph_init(const ph_params *params, int64_t maxp, ph_ctx **out) {
   return 0;
 }
 
+// whether the force's trial lists, with the symmetric pass's offsets and the far
+// field that are made with them, differ between two parameter sets
+static bool lists_differ(const ph_params &a, const ph_params &b) {
+  return a.precision != b.precision || a.gravity != b.gravity || a.mhd != b.mhd || a.periodic != b.periodic ||
+         a.ind_timesteps != b.ind_timesteps || a.tree_accuracy != b.tree_accuracy || a.massoftype != b.massoftype ||
+         a.xmin != b.xmin || a.xmax != b.xmax || a.ymin != b.ymin || a.ymax != b.ymax || a.zmin != b.zmin ||
+         a.zmax != b.zmax;
+}
+
 int ph_set_params(ph_ctx *c, const ph_params *params) {
   if (!c || !params || !params_ok(params)) return PH_ERR_ARG;
+  if (lists_differ(c->hp, *params)) c->have_force_lists = false;
+  if (params->gravity && !c->hp.gravity)  // no quadrupoles, no softening sums
+    c->have_tree = c->have_density = c->have_force = c->have_force_lists = false;
   if ((params->minpart > 0 ? params->minpart : MINPART) != c->dp.minpart)
     c->have_tree = c->have_density = c->have_force = c->have_force_lists = false;  // a new leaf size needs a new tree
   c->hp = *params;
