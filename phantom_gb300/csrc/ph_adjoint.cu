@@ -686,7 +686,10 @@ struct HConst {
   bool cond, pdv, shock;
 };
 
-// the record of tree position i from its adjoint record
+// the record of tree position i from its adjoint record. The HR_KR* are
+// derivatives with respect to rho times drho/dh = -3 rho/h (HR_KH), which leaves
+// no power of 1/rho above the first: u/rho^2 would leave the FP32 range with the
+// pair's own factors from rho = 1e-17 down
 template <typename T>
 __device__ __forceinline__ void hydro_record(const Params &p, const double *r, T *o) {
   const double h1 = r[AR_H1], rho = r[AR_RHO], rho1 = r[AR_RHO1], cs = r[AR_CS0], u = r[AR_U];
@@ -696,17 +699,15 @@ __device__ __forceinline__ void hydro_record(const Params &p, const double *r, T
   const double au = 0.5 * p.alphau * rho1;
   const double v[HR_A3] = {h1, (double)hs1_fac<T>() * h4 * r[AR_G], 1.5 * h4 * h1 * r[AR_G], rho, r[AR_PRO2],
                            r[AR_ALPHA] * cs, -0.5 * rho1, r[AR_P], u, au, r[AR_S], r[AR_WX], r[AR_WY], r[AR_WZ],
-                           r[AR_VX], r[AR_VY], r[AR_VZ], -r[AR_PRO2] * rho1, gm1 * rho1, pon, gm1 * rho,
-                           0.5 * rho1 * rho1, -au * rho1, cs > 0.0 ? r[AR_ALPHA] * p.gamma * gm1 / (2.0 * cs) : 0.0,
-                           -3.0 * rho * h1};
+                           r[AR_VX], r[AR_VY], r[AR_VZ], 3.0 * r[AR_PRO2] * h1, gm1 * rho1, -3.0 * pon * rho * h1,
+                           gm1 * rho, -1.5 * rho1 * h1, 3.0 * au * h1,
+                           cs > 0.0 ? r[AR_ALPHA] * p.gamma * gm1 / (2.0 * cs) : 0.0, -3.0 * rho * h1};
   for (int k = 0; k < HR_A3; ++k) o[k] = (T)v[k];
   if (p.ieos == 1) o[HR_KUC] = T(0.0);
 }
 
 __device__ __forceinline__ double inv_r(double r2) { return rsqrt_fast(r2); }
 __device__ __forceinline__ float inv_r(float r2) { return r2 > TINY_F ? rsqrt_nr(r2) : 0.0f; }
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt_fast(x); }
-__device__ __forceinline__ float rsqrt_t(float x) { return x >= TINY_F ? rsqrt_nr(x) : 0.0f; }
 
 // kernel shape at r h1: q, hs1, hs2 = w''/1.5 and the bracket 12 w + 8 q w' + q^2 w''
 __device__ __forceinline__ void hshape(double r, double h1, double &q, double &hs1, double &hs2, double &d2) {
@@ -731,6 +732,31 @@ __device__ __forceinline__ void hshape(float r, float h1, float &q, float &hs1, 
     hs2 = t;
     d2 = t * (6.0f + t * (10.5f * t - 18.0f));
   }
+}
+
+// The conductivity's signal speed vsu = sqrt(2 |dP| / rs), rs = rho_i + rho_j, and
+// its derivatives with respect to u (pa, pb: without j's sign) and h (ra, rb) of
+// both sides. FP64: by y = (|dP| rs)^(-1/2), three instructions fewer than with
+// the quotient. FP32: by the quotient, since y^2 with the pair's own factors
+// leaves the range from rho = 1e-12 down (and |dP| rs itself at 1e-17), and each
+// factor 1/rs meets a rho before anything else.
+__device__ __forceinline__ void cond_factors(double dP, double rs, const double *a, const double *b, double &vsu,
+                                             double &pa, double &pb, double &ra, double &rb) {
+  const double dPa = fabs(dP), y = rsqrt_fast(dPa * rs);
+  vsu = 1.4142135623730951 * dPa * y;
+  const double dv = y * (dP > 0.0 ? 0.70710678118654752 : -0.70710678118654752);  // dvsu/dP
+  const double dr = -0.5 * vsu * (y * y) * dPa;                                     // dvsu/drs
+  pa = dv * a[HR_KUPP]; pb = dv * b[HR_KUPP];
+  ra = fma(dv, a[HR_KRPP], dr * a[HR_KH]); rb = fma(-dv, b[HR_KRPP], dr * b[HR_KH]);
+}
+__device__ __forceinline__ void cond_factors(float dP, float rs, const float *a, const float *b, float &vsu, float &pa,
+                                             float &pb, float &ra, float &rb) {
+  const float i = 1.0f / rs, t = 2.0f * fabsf(dP) * i;
+  const float y = t >= TINY_F ? rsqrt_nr(t) : 0.0f;
+  vsu = t * y;
+  const float dv = dP > 0.0f ? y : -y, dr = -0.5f * vsu;  // rs dvsu/dP, rs dvsu/drs
+  pa = dv * (a[HR_KUPP] * i); pb = dv * (b[HR_KUPP] * i);
+  ra = dv * (a[HR_KRPP] * i) + dr * (a[HR_KH] * i); rb = dr * (b[HR_KH] * i) - dv * (b[HR_KRPP] * i);
 }
 
 // Reverse of C: the gradient gd with respect to d = x_i - x_j and gv to dv =
@@ -775,22 +801,19 @@ __device__ __forceinline__ void hydro_pair_rev(const HConst &k, T dx, T dy, T dz
     Ua += vab * a[HR_KUC]; Ub += vbb * b[HR_KUC];
   }
   if (k.cond) {
-    // vsu = sqrt(2 |dP| / rs) = sqrt(2) |dP| yc, yc = (|dP| rs)^(-1/2), rs = rho_i + rho_j
-    const T dP = a[HR_P] - b[HR_P], dPa = fabs(dP);
-    const T yc = rsqrt_t(dPa * (a[HR_RHO] + b[HR_RHO]));
-    const T vsu = T(1.4142135623730951) * dPa * yc;
+    const T dP = a[HR_P] - b[HR_P], rs = a[HR_RHO] + b[HR_RHO];
+    T vsu, pa_, pb_, ra_, rb_;
+    cond_factors(dP, rs, a, b, vsu, pa_, pb_, ra_, rb_);
     const T Sd = sa - sb, Du = a[HR_U] - b[HR_U];
     const T SD = Sd * Du, cu = SD * vsu;
     const T E = a[HR_AU] * ga + b[HR_AU] * gb;
     gab += cu * a[HR_AU]; gbb += cu * b[HR_AU];
     const T du = Sd * vsu * E;
     const T vsb = SD * E;
-    const T Pb_ = vsb * yc * (dP > T(0.0) ? T(0.70710678118654752) : T(-0.70710678118654752));
-    const T rX = T(-0.5) * vsb * vsu * (yc * yc) * dPa;
-    Ra += (cu * ga) * a[HR_KRA] + Pb_ * a[HR_KRPP] + rX;
-    Rb += (cu * gb) * b[HR_KRA] - Pb_ * b[HR_KRPP] + rX;
-    Ua += Pb_ * a[HR_KUPP] + du;
-    Ub -= Pb_ * b[HR_KUPP] + du;
+    Ra += (cu * ga) * a[HR_KRA] + vsb * ra_;
+    Rb += (cu * gb) * b[HR_KRA] + vsb * rb_;
+    Ua += vsb * pa_ + du;
+    Ub -= vsb * pb_ + du;
   }
   const T Gs = Xa * ga + Xb * gb;
   const T nbx = pvb * dvx - Gs * wx, nby = pvb * dvy - Gs * wy, nbz = pvb * dvz - Gs * wz;
@@ -801,8 +824,8 @@ __device__ __forceinline__ void hydro_pair_rev(const HConst &k, T dx, T dy, T dz
   const T pvy = pvb * y;
   gv[0] = pvy * dx; gv[1] = pvy * dy; gv[2] = pvy * dz;
   oa[1] = gab * ga; ob[1] = gbb * gb;
-  oa[0] = Ra * a[HR_KH] - (za * qa_ + T(4.0) * a[HR_H1] * oa[1]);
-  ob[0] = Rb * b[HR_KH] - (zb * qb_ + T(4.0) * b[HR_H1] * ob[1]);
+  oa[0] = Ra - (za * qa_ + T(4.0) * a[HR_H1] * oa[1]);
+  ob[0] = Rb - (zb * qb_ + T(4.0) * b[HR_H1] * ob[1]);
   oa[2] = Ua; ob[2] = Ub;
   oa[3] = d2a; ob[3] = d2b;
 }
