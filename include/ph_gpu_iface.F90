@@ -106,6 +106,9 @@ module ph_gpu_iface
   integer(c_int) function ph_set_params(ctx, p) bind(c, name="ph_set_params")
     import; type(c_ptr), value :: ctx; type(ph_params), intent(in) :: p
   end function
+  integer(c_int) function ph_set_record_limit(ctx, bytes) bind(c, name="ph_set_record_limit")
+    import; type(c_ptr), value :: ctx; integer(c_int64_t), value :: bytes
+  end function
   subroutine ph_finalize(ctx) bind(c, name="ph_finalize")
     import; type(c_ptr), value :: ctx
   end subroutine

@@ -105,6 +105,16 @@ int ph_init(const ph_params *params, int64_t maxp, ph_ctx **ctx);
  * changed), except that a new minpart, or self-gravity switched on, needs a
  * new tree and density (PH_ERR_STATE until then). */
 int ph_set_params(ph_ctx *ctx, const ph_params *params);
+/* Bound on the device memory that ph_step may take for its pair record, in
+ * bytes (negative, the default: none of its own; 0: no record). In the precision
+ * form without self-gravity, a step of three or more velocity iterations records
+ * its pairs (about 1.1 kB per particle at 58 neighbours, 512 bytes per 32
+ * pairs) and replays them in the iterations that follow; results are the same
+ * bit for bit with and without it. The record takes a quarter of the free device
+ * memory at most, stays with the context, and is given up where another
+ * buffer of the context finds no memory. A record above a new bound is freed
+ * at once. No counterpart in the reference. */
+int ph_set_record_limit(ph_ctx *ctx, int64_t bytes);
 void ph_finalize(ph_ctx *ctx);
 const char *ph_strerror(int code);
 

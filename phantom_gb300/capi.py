@@ -69,6 +69,7 @@ _vp = C.c_void_p
 _SIGS = {
     "ph_init": (C.c_int, [C.POINTER(PhParams), C.c_int64, C.POINTER(_vp)]),
     "ph_set_params": (C.c_int, [_vp, C.POINTER(PhParams)]),
+    "ph_set_record_limit": (C.c_int, [_vp, C.c_int64]),
     "ph_finalize": (None, [_vp]),
     "ph_strerror": (C.c_char_p, [C.c_int]),
     "ph_upload": (C.c_int, [_vp, C.c_int64, _vp, _vp, _vp]),
@@ -190,6 +191,10 @@ class Context:
         prec = self.params.precision if precision is None else precision
         self.params = make_params(self.cfg, prec)
         self._chk(self.L.ph_set_params(self.h, C.byref(self.params)), "ph_set_params")
+
+    def set_record_limit(self, nbytes: int):
+        """ph_set_record_limit: bound on the step's pair record (negative: none, 0: no record)."""
+        self._chk(self.L.ph_set_record_limit(self.h, nbytes), "ph_set_record_limit")
 
     def upload(self, xyzh, vxyzu, Bevol=None):
         xyzh = np.ascontiguousarray(xyzh, np.float64)

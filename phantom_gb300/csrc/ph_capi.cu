@@ -11,13 +11,34 @@ using namespace ph;
 
 namespace {
 
+void dfree(ph_ctx *c, void *p);
+
+void drop_record(ph_ctx *c) {
+  if (c->rec_rows) dfree(c, c->rec_rows);
+  c->rec_rows = nullptr;
+  c->rec_cap = 0;
+}
+
+// Device memory for a context. Where there is none left, the pair record, which
+// only saves time, is given up for it (unless the evaluation under way replays
+// it). A failure is the caller's status, not an error of the launches after it.
+cudaError_t device_alloc(ph_ctx *c, void **q, size_t bytes) {
+  cudaError_t e = cudaMalloc(q, bytes);
+  if (e != cudaSuccess && c->rec_rows && c->rec_mode != PAIRS_REPLAY) {
+    drop_record(c);
+    e = cudaMalloc(q, bytes);
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 // A cleared device buffer of the context. Cleared on the context's stream, which
 // does not wait for the default stream: the launches that follow write into it.
 template <typename T>
 int dalloc(ph_ctx *c, T **p, size_t count) {
   size_t bytes = sizeof(T) * (count > 0 ? count : 1);
   void *q = nullptr;
-  if (cudaMalloc(&q, bytes) != cudaSuccess) return PH_ERR_CUDA;
+  if (device_alloc(c, &q, bytes) != cudaSuccess) return PH_ERR_CUDA;
   cudaMemsetAsync(q, 0, bytes, c->stream);
   c->allocs.push_back(DeviceBuf{q, bytes});
   *p = static_cast<T *>(q);
@@ -113,8 +134,9 @@ namespace ph {
 
 int grow_pool(ph_ctx *c) {
   int64_t ncap = c->pool_cap * 2;
-  LeafEntry *np_ = nullptr;
-  if (cudaMalloc(&np_, sizeof(LeafEntry) * (size_t)ncap) != cudaSuccess) return PH_ERR_CUDA;
+  void *q = nullptr;
+  if (device_alloc(c, &q, sizeof(LeafEntry) * (size_t)ncap) != cudaSuccess) return PH_ERR_CUDA;
+  LeafEntry *np_ = static_cast<LeafEntry *>(q);
   cudaMemcpyAsync(np_, c->pool, sizeof(LeafEntry) * (size_t)c->pool_cap, cudaMemcpyDeviceToDevice, c->stream);
   cudaStreamSynchronize(c->stream);
   dfree(c, c->pool);
@@ -125,16 +147,16 @@ int grow_pool(ph_ctx *c) {
 }
 
 // Room for a pair record of `rows` rows, kept with the context. Taken only
-// where it leaves three quarters of the free device memory; false: no record.
+// where it leaves three quarters of the free device memory and within the
+// caller's limit; false: no record.
 bool grow_record(ph_ctx *c, int64_t rows) {
   if (c->rec_cap >= rows) return true;
   if (rows > INT32_MAX) return false;
   size_t avail = 0, total = 0;
-  const size_t bytes = 512 * (size_t)rows + (c->rec_cell ? 0 : sizeof(int) * (size_t)c->cap);
+  const size_t cells = sizeof(int) * (size_t)c->cap, bytes = 512 * (size_t)rows + (c->rec_cell ? 0 : cells);
+  if (c->rec_limit >= 0 && 512 * (size_t)rows + cells > (size_t)c->rec_limit) return false;
   if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 4 < bytes) return false;
-  if (c->rec_rows) dfree(c, c->rec_rows);
-  c->rec_rows = nullptr;
-  c->rec_cap = 0;
+  drop_record(c);
   if (!c->rec_cell && dalloc(c, &c->rec_cell, (size_t)c->cap) != 0) return false;
   if (dalloc(c, &c->rec_rows, 32 * (size_t)rows) != 0) return false;
   c->rec_cap = rows;
@@ -384,6 +406,14 @@ int ph_set_params(ph_ctx *c, const ph_params *params) {
   return 0;
 }
 
+int ph_set_record_limit(ph_ctx *c, int64_t bytes) {
+  if (!c) return PH_ERR_ARG;
+  c->rec_limit = bytes;
+  c->rec_refused = false;
+  if (bytes >= 0 && 512 * (size_t)c->rec_cap + sizeof(int) * (size_t)c->cap > (size_t)bytes) drop_record(c);
+  return 0;
+}
+
 void ph_finalize(ph_ctx *c) {
   if (!c) return;
   cudaStreamSynchronize(c->stream);
@@ -426,6 +456,7 @@ int ph_upload(ph_ctx *c, int64_t npart, const double *xyzh, const double *vxyzu,
   }
   cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
   c->have_tree = c->have_density = c->have_force = c->have_force_lists = false;
+  c->rec_refused = false;
   // FP32 pre-filter guard: h must exceed 4e-4 of the coordinate scale
   double xs = 0.0;
   const double b[6] = {c->hp.xmin, c->hp.xmax, c->hp.ymin, c->hp.ymax, c->hp.zmin, c->hp.zmax};

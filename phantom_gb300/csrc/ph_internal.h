@@ -222,6 +222,8 @@ struct ph_ctx {
   float4 *rec_rows = nullptr;
   int *rec_cell = nullptr;
   int64_t rec_cap = 0;
+  int64_t rec_limit = -1;    // the caller's bound on its bytes (negative: none)
+  bool rec_refused = false;  // did not fit: not tried again before the next upload
   double *ro_buf = nullptr;  // rollout adjoint buffer (ph_rollout_adjoint)
   size_t ro_cap = 0;
 

@@ -326,12 +326,13 @@ int ph_step(ph_ctx *c, double t, double dtsph, double *dtnew, int32_t *its_out, 
   // else the first iteration's. A record that did not fit is taken again with
   // room for it (a context's first record only counts its rows). Recording adds
   // about a tenth to an evaluation and a replay saves more than half, so an evaluation that
-  // nothing is known to follow (one iteration per step) is not recorded.
+  // nothing is known to follow (one iteration per step) is not recorded, nor
+  // one of a particle set whose record was found not to fit.
   struct RecordMode {
     ph_ctx *c;
     ~RecordMode() { c->rec_mode = PAIRS_SWEEP; }
   } record_mode{c};
-  const bool recordable = pairs_recordable(c);
+  const bool recordable = pairs_recordable(c) && c->rec_limit != 0 && !c->rec_refused;
   bool norecord = !recordable;
   c->rec_mode = recordable && c->rec_its > 1 ? PAIRS_RECORD : PAIRS_SWEEP;
   int r = derivs_dev(c, 1, c->vpred, Bv, &dtn);
@@ -381,7 +382,10 @@ int ph_step(ph_ctx *c, double t, double dtsph, double *dtnew, int32_t *its_out, 
       count_launch(c);
       if (c->rec_mode == PAIRS_RECORD) {
         if (rows <= c->rec_cap) c->rec_mode = PAIRS_REPLAY;
-        else if (!grow_record(c, (int64_t)rows + rows / 16 + 64)) { c->rec_mode = PAIRS_SWEEP; norecord = true; }
+        else if (!grow_record(c, (int64_t)rows + rows / 16 + 64)) {
+          c->rec_mode = PAIRS_SWEEP;
+          c->rec_refused = norecord = true;
+        }
       } else if (c->rec_mode == PAIRS_SWEEP && !norecord) {
         c->rec_mode = PAIRS_RECORD;
       }

@@ -37,3 +37,27 @@ def test_record_grows(n1d, mk):
         assert got[0] == want[0] and got[0][1] >= 3
         for a, b in zip(got[1], want[1]):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("mk", [S.hydro_lattice, S.mhd_vortex])
+def test_record_limits(mk):
+    """No record, one that does not fit, one given up between steps and one that
+    is bounded but fits: the same steps, bit for bit."""
+    cfg, x, v, B = mk(16, jitter=0.2, seed=3)
+    cfg = dict(cfg, tolv=1.0e-8)
+    n = len(x)
+    runs = []
+    for limits in ((-1, -1, -1), (0, 0, 0), (4096, 4096, 4096), (-1, 4096, -1), (0, 1 << 30, 1 << 30)):
+        ctx = capi.Context(cfg, precision=capi.PH_PREC_MIXED)
+        ctx.upload(x, v, B)
+        dt, out = ctx.derivs(1, 0.0), []
+        for lim in limits:
+            ctx.set_record_limit(lim)
+            r = ctx.step(0.0, dt)
+            assert r[1] >= 3
+            out.append(r)
+        out += list(ctx.download())
+        runs.append(out)
+    for run in runs[1:]:
+        for a, b in zip(run, runs[0]):
+            assert np.array_equal(a, b)
