@@ -1118,10 +1118,11 @@ __global__ void k_cell_at(const Node *nodes, const int *leaves, int ncell, int *
 }
 
 // ------------------------------------------------------------------ mixed precision
-// Precision form: the pair separation is formed in FP64 (positions stay FP64)
-// and rounded to FP32; W, grad W and every pair term are evaluated in FP32
-// and accumulated per particle in FP32 with compensated (Kahan) summation. The
-// per-particle finish (accelerations, du/dt, dB/dt, timesteps) is FP64.
+// Precision form: positions stay FP64, and a pair's separation is their
+// difference rounded to FP32, formed from high and low FP32 parts (separation_2f;
+// in FP64 for the closest pairs and those across a periodic image); W, grad W and
+// every pair term are evaluated in FP32 and accumulated per particle in FP32 with
+// compensated (Kahan) summation.
 
 __device__ __forceinline__ float grkernf(float q) {
   if (q < 1.0f) return q * (2.25f * q - 3.0f);
