@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 4) k_density_dv(
         if (r2 * hi21f < 4.0f) {
           const float rij = sqrt_nr(r2), q = rij * hi1f;
           const float grk = q < 1.0f ? q * (2.25f * q - 3.0f) : -0.75f * (q - 2.0f) * (q - 2.0f);
-          const float r1g = __fdividef(grk, rij + 1.0e-30f);
+          const float r1g = grk / (rij + 1.0e-30f);
           const float rux = dx * r1g * pmf, ruy = dy * r1g * pmf, ruz = dz * r1g * pmf;
           const float2 *v2 = reinterpret_cast<const float2 *>(vff + 6 * (size_t)j);
           const float2 va = v2[0], vb = v2[1], vc = v2[2];
