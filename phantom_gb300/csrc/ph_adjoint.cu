@@ -38,6 +38,8 @@
 //     (with self-gravity also C_k dphi_h(r,h_k)/dr + C_j dphi_h(r,h_j)/dr,
 //     C the coefficient on the gradsoft sum).
 //  4. With self-gravity, the far field's reverse (gravity_adjoint_far).
+#include <type_traits>
+
 #include "ph_internal.h"
 #include "ph_walk.cuh"
 
@@ -735,28 +737,36 @@ __device__ __forceinline__ void hshape(float r, float h1, float &q, float &hs1, 
 }
 
 // The conductivity's signal speed vsu = sqrt(2 |dP| / rs), rs = rho_i + rho_j, and
-// its derivatives with respect to u (pa, pb: without j's sign) and h (ra, rb) of
-// both sides. FP64: by y = (|dP| rs)^(-1/2), three instructions fewer than with
-// the quotient. FP32: by the quotient, since y^2 with the pair's own factors
-// leaves the range from rho = 1e-12 down (and |dP| rs itself at 1e-17), and each
-// factor 1/rs meets a rho before anything else.
-__device__ __forceinline__ void cond_factors(double dP, double rs, const double *a, const double *b, double &vsu,
-                                             double &pa, double &pb, double &ra, double &rb) {
-  const double dPa = fabs(dP), y = rsqrt_fast(dPa * rs);
-  vsu = 1.4142135623730951 * dPa * y;
-  const double dv = y * (dP > 0.0 ? 0.70710678118654752 : -0.70710678118654752);  // dvsu/dP
-  const double dr = -0.5 * vsu * (y * y) * dPa;                                     // dvsu/drs
-  pa = dv * a[HR_KUPP]; pb = dv * b[HR_KUPP];
-  ra = fma(dv, a[HR_KRPP], dr * a[HR_KH]); rb = fma(-dv, b[HR_KRPP], dr * b[HR_KH]);
+// the share of its cotangent vsb in h (Ra, Rb) and u (Ua, Ub) of both sides. FP64:
+// from y = (|dP| rs)^(-1/2). FP32: from the quotient, since y^2 with the pair's
+// own factors leaves the range from rho = 1e-12 down (and |dP| rs itself at
+// 1e-17), and each factor 1/rs meets a rho before anything else.
+struct CondD { double y, t; };
+struct CondF { float y, i; };
+__device__ __forceinline__ double cond_speed(double dP, double rs, CondD &c) {
+  const double dPa = fabs(dP);
+  c.y = rsqrt_fast(dPa * rs);
+  c.t = dPa * c.y;
+  return 1.4142135623730951 * c.t;
 }
-__device__ __forceinline__ void cond_factors(float dP, float rs, const float *a, const float *b, float &vsu, float &pa,
-                                             float &pb, float &ra, float &rb) {
-  const float i = 1.0f / rs, t = 2.0f * fabsf(dP) * i;
-  const float y = t >= TINY_F ? rsqrt_nr(t) : 0.0f;
-  vsu = t * y;
-  const float dv = dP > 0.0f ? y : -y, dr = -0.5f * vsu;  // rs dvsu/dP, rs dvsu/drs
-  pa = dv * (a[HR_KUPP] * i); pb = dv * (b[HR_KUPP] * i);
-  ra = dv * (a[HR_KRPP] * i) + dr * (a[HR_KH] * i); rb = dr * (b[HR_KH] * i) - dv * (b[HR_KRPP] * i);
+__device__ __forceinline__ void cond_rev(const CondD &c, double dP, double vsu, double vsb, const double *a,
+                                         const double *b, double &Ra, double &Rb, double &Ua, double &Ub) {
+  const double w = 0.70710678118654752 * (vsb * c.y), rX = -w * (c.t * c.t);  // vsb dvsu/d|dP|, vsb dvsu/drs
+  const double P = dP > 0.0 ? w : -w;
+  Ra = fma(P, a[HR_KRPP], fma(rX, a[HR_KH], Ra)); Rb = fma(-P, b[HR_KRPP], fma(rX, b[HR_KH], Rb));
+  Ua = fma(P, a[HR_KUPP], Ua); Ub = fma(-P, b[HR_KUPP], Ub);
+}
+__device__ __forceinline__ float cond_speed(float dP, float rs, CondF &c) {
+  c.i = 1.0f / rs;
+  const float t = 2.0f * fabsf(dP) * c.i;
+  c.y = t >= TINY_F ? rsqrt_nr(t) : 0.0f;
+  return t * c.y;
+}
+__device__ __forceinline__ void cond_rev(const CondF &c, float dP, float vsu, float vsb, const float *a, const float *b,
+                                         float &Ra, float &Rb, float &Ua, float &Ub) {
+  const float P = vsb * (dP > 0.0f ? c.y : -c.y), rX = -0.5f * vsb * vsu;  // each times rs
+  Ra += P * (a[HR_KRPP] * c.i) + rX * (a[HR_KH] * c.i); Rb += rX * (b[HR_KH] * c.i) - P * (b[HR_KRPP] * c.i);
+  Ua += P * (a[HR_KUPP] * c.i); Ub -= P * (b[HR_KUPP] * c.i);
 }
 
 // Reverse of C: the gradient gd with respect to d = x_i - x_j and gv to dv =
@@ -802,18 +812,19 @@ __device__ __forceinline__ void hydro_pair_rev(const HConst &k, T dx, T dy, T dz
   }
   if (k.cond) {
     const T dP = a[HR_P] - b[HR_P], rs = a[HR_RHO] + b[HR_RHO];
-    T vsu, pa_, pb_, ra_, rb_;
-    cond_factors(dP, rs, a, b, vsu, pa_, pb_, ra_, rb_);
+    typename std::conditional<sizeof(T) == 8, CondD, CondF>::type cd;
+    const T vsu = cond_speed(dP, rs, cd);
     const T Sd = sa - sb, Du = a[HR_U] - b[HR_U];
     const T SD = Sd * Du, cu = SD * vsu;
     const T E = a[HR_AU] * ga + b[HR_AU] * gb;
     gab += cu * a[HR_AU]; gbb += cu * b[HR_AU];
     const T du = Sd * vsu * E;
     const T vsb = SD * E;
-    Ra += (cu * ga) * a[HR_KRA] + vsb * ra_;
-    Rb += (cu * gb) * b[HR_KRA] + vsb * rb_;
-    Ua += vsb * pa_ + du;
-    Ub -= vsb * pb_ + du;
+    Ra += (cu * ga) * a[HR_KRA];
+    Rb += (cu * gb) * b[HR_KRA];
+    Ua += du;
+    Ub -= du;
+    cond_rev(cd, dP, vsu, vsb, a, b, Ra, Rb, Ua, Ub);
   }
   const T Gs = Xa * ga + Xb * gb;
   const T nbx = pvb * dvx - Gs * wx, nby = pvb * dvy - Gs * wy, nbz = pvb * dvz - Gs * wz;
