@@ -49,53 +49,94 @@ sys.path.insert(0, ROOT)
 
 METRIC = "particle-steps/s, 1 GB300: mixed vs FP64 at stated error; adjoint/forward ratio"
 UNIT = "particle-steps/s"
-# force pair loop, leaf-staged gather model (bytes): neighbour record read once
-# per leaf trial entry, own record read + results written per particle
-R_NB_FORCE = 72
-R_OWN_FORCE = 72 + 40
-# mixed form: positions FP64 (24 B), the rest of the neighbour record FP32
-R_NB_FORCE_MIXED = 24 + 24
-R_OWN_FORCE_MIXED = 24 + 64 + 40
-# DRAM bytes (read + write) per particle of one k_force_mixed launch, from the
-# ncu capture of the Sedov 96^3 case (profiles/pair_kernels_sedov96.md),
-# scaled to the launch by the particle count
-TRAFFIC_PER_PARTICLE_MIXED = (203.11e6 + 71.06e6) / 884736
-TRAFFIC_SOURCE = ("scaled: ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_force_mixed launch on "
-                  "Sedov 96^3 (profiles/pair_kernels_sedov96.md) x npart / 884,736")
-# floating-point operations per particle of one force launch: thread-level
-# SASS counts from ncu on the Sedov 96^3 case (profiles/flop_counts_sedov96.md;
-# FP32 fadd + fmul + 2 ffma, FP64 dadd + dmul + 2 dfma), scaled to a launch by
-# the particle count (the neighbours per particle do not depend on it)
-FLOPS_PER_PARTICLE = {
-    "k_force_mixed": {"fp32": (3759926183 + 3865459352 + 2 * 1511419870) / 884736, "fp64": 242924786 / 884736},
-    "k_force": {"fp64": (1451552236 + 2536837906 + 2 * 1784275018) / 884736,
-                "fp32": (1537615966 + 2704518873 + 2 * 948633950) / 884736},
+# Force launches: what one launch has to move and what it did on the Sedov 96^3
+# set (884,736 particles; ncu, profiles/pair_kernels_sedov96.md), per particle.
+# bytes: the model - positions (mixed: two FP32 parts; FP64 and their FP32 copy),
+# particle record and pair sums once per particle, and the pair record that is written
+# or read (mixed) or the j-side buffer, written and read back (FP64);
+# dram: dram__bytes_read + dram__bytes_write; fp32, fp64: thread-level operations
+# (add + mul + 2 fma); pipes: active share of the pipes and issue slots (an FP64
+# warp instruction holds its pipe whatever its active lanes, so the thread-level
+# fraction understates the pipe's use).
+N96 = 884736
+R_PAIR_RECORD = (1066.49e6 - 38.48e6) / N96  # B per particle at 58 neighbours
+R_OWN_MIXED, R_OWN_FP64 = 32 + 64 + 64, 24 + 16 + 128 + 64
+LAUNCHES = {
+    "swept": {"kernel": "k_force_mixed", "bytes": R_OWN_MIXED, "dram": (199.75e6 + 37.92e6) / N96,
+              "fp32": (5.061e9 + 3.006e9 + 2 * 1.773e9) / N96, "fp64": (5.882e7 + 6.19e6) / N96,
+              "pipes": {"fp64_pipe_active": 0.217, "fma_pipe_active": 0.254, "issue_active": 0.615}},
+    "recorded": {"kernel": "k_force_mixed, recording", "bytes": R_OWN_MIXED + R_PAIR_RECORD,
+                 "dram": (226.84e6 + 1066.49e6) / N96, "fp32": (5.061e9 + 2.79e9 + 2 * 1.957e9) / N96,
+                 "fp64": (5.882e7 + 6.19e6) / N96,
+                 "pipes": {"fp64_pipe_active": 0.188, "fma_pipe_active": 0.231, "issue_active": 0.555}},
+    "replayed": {"kernel": "k_force_replay", "bytes": R_OWN_MIXED + R_PAIR_RECORD,
+                 "dram": (1157.12e6 + 48.42e6) / N96, "fp32": (1.971e9 + 1.974e9 + 2 * 5.628e8) / N96,
+                 "fp64": (4.904e7 + 6.19e6) / N96,
+                 "pipes": {"fp64_pipe_active": 0.412, "fma_pipe_active": 0.268, "issue_active": 0.468}},
+    "symmetric": {"kernel": "k_force_sym + k_force_gather", "bytes": R_OWN_FP64,
+                  "dram": (292.94e6 + 1882.51e6 + 2823.84e6 + 51.57e6) / N96,
+                  "fp64": (9.955e8 + 7.479e8 + 2 * 6.543e8 + 1.974e8 + 2 * 4.424e6) / N96,
+                  "fp32": (9.418e8 + 3.572e8 + 2 * 6.197e8) / N96,
+                  "pipes": {"fp64_pipe_active": 0.691, "fma_pipe_active": 0.032, "issue_active": 0.173}},
 }
+KINDS = ("swept", "recorded", "replayed", "symmetric")
 # pipe peaks of one GB300 at its 2.07 GHz maximum SM clock: 152 SMs x 128 FP32
 # or 2 FP64 lanes x 2 flops (an FMA-chain probe reaches 86 % and 95 % of them)
 PEAK_TFLOPS = {"fp32": 152 * 128 * 2 * 2.07e9 / 1e12, "fp64": 152 * 2 * 2 * 2.07e9 / 1e12}
-# the binding pipe of each force kernel as ncu sees it on the Sedov 96^3 case
-# (profiles/flop_counts_sedov96.md, profiles/pair_kernels_sedov96.md): an FP64
-# warp instruction holds the FP64 pipe whatever its active lanes, so the
-# thread-level flop fraction understates the plain kernel's use of it
-NCU_PIPES = {"k_force": {"fp64_pipe_active": 0.853, "issue_active": 0.117},
-             "k_force_mixed": {"fp64_pipe_active": 0.326, "fma_pipe_active": 0.213, "issue_active": 0.541}}
 
 
-def flop_roofline(kernel: str, n: int, ms_per_launch: float) -> dict:
-    """Flop roofline of one force launch: the kernel's arithmetic pipe (FP32
-    for the mixed form, FP64 for the plain path) against its peak."""
-    fl = FLOPS_PER_PARTICLE[kernel]
-    pipe = "fp32" if kernel == "k_force_mixed" else "fp64"
-    out = {"kernel": kernel, "pipe": pipe, "unit": "TFLOP/s", "peak_source": "nominal (SM count x lanes x clock)"}
-    for k, per in fl.items():
-        out[k] = {"flops_per_launch": per * n, "achieved": per * n / (ms_per_launch / 1e3) / 1e12,
-                  "peak": PEAK_TFLOPS[k]}
-        out[k]["frac"] = out[k]["achieved"] / PEAK_TFLOPS[k]
-    out["frac"] = out[pipe]["frac"]
-    out["ncu_pipes"] = dict(NCU_PIPES[kernel], source="ncu, Sedov 96^3 launch (profiles/)")
-    out["scaled_from"] = "ncu thread-level op counts of one Sedov 96^3 launch (profiles/), x npart / 884,736"
-    return out
+def launch_kinds(cfg: dict, mixed: bool, its: int, last_its: int) -> list:
+    """Force launches of a step of `its` evaluations, per entry of KINDS. The
+    precision form without self-gravity records the predictor's pairs where the
+    step before iterated (else the first iteration's) and replays them."""
+    if not mixed:
+        return [0, 0, 0, its]
+    if cfg["gravity"] or its == 0:
+        return [its, 0, 0, 0]
+    if last_its > 1:
+        return [0, 1, its - 1, 0]
+    return [1, min(its - 1, 1), max(its - 2, 0), 0]
+
+
+def force_rooflines(arm: dict, cfg: dict, n: int, peak_hbm: float, hbm_source: str) -> tuple:
+    """(roofline, flop_roofline) of an arm's force launches, summed over the
+    kinds of launch it made, over their device time (pair loop and finish). The
+    per-launch counts are those of a hydro set of 58 neighbours without
+    self-gravity: None for other sets."""
+    if cfg["gravity"] or cfg["mhd"] or arm["its"] == 0:
+        return None, None
+    count = np.asarray(arm["kinds"], float)
+    tot, ms = count.sum(0), float(np.sum(arm["step_force_ms"]))
+    used = [k for k in range(len(KINDS)) if tot[k] > 0]
+    fit, _, rank, _ = np.linalg.lstsq(count[:, used], np.asarray(arm["step_force_ms"]), rcond=None)
+    launches = {KINDS[k]: {"kernel": LAUNCHES[KINDS[k]]["kernel"], "launches": int(tot[k]),
+                           "ms_per_launch": float(fit[q]) if rank == len(used) else None,
+                           "ncu_pipes": LAUNCHES[KINDS[k]]["pipes"]} for q, k in enumerate(used)}
+    jbuf = 2 * 56 * arm["trial_sum"] / 2 if tot[3] else 0.0  # owned half of the trial entries, written and read
+    nbytes = sum(tot[k] * LAUNCHES[KINDS[k]]["bytes"] * n for k in used) + jbuf
+    nl = arm["its"]
+    roof = {"bound": "hbm", "kernel": " / ".join(v["kernel"] for v in launches.values()),
+            "achieved": nbytes / (ms / 1e3) / 1e9, "peak": peak_hbm, "unit": "GB/s",
+            "frac": nbytes / (ms / 1e3) / 1e9 / peak_hbm,
+            "traffic": sum(tot[k] * LAUNCHES[KINDS[k]]["dram"] * n for k in used) / nl,
+            "traffic_source": "ncu dram bytes of one launch of each kind on Sedov 96^3 "
+                              "(profiles/pair_kernels_sedov96.md), scaled by the particle count",
+            "peak_source": hbm_source,
+            "model": f"per particle {R_OWN_MIXED} B (mixed) or {R_OWN_FP64} B (FP64) of positions, record and sums, "
+                     f"{R_PAIR_RECORD:.0f} B of pair record recorded or replayed, 112 B per owned trial entry of the "
+                     "symmetric loop's buffer; the kernels are bound by the FP64 pipe or by issue and latency",
+            "algorithmic_bytes_per_launch": nbytes / nl, "ms_per_launch": ms / nl, "launches": launches}
+    fl = {k: sum(tot[q] * LAUNCHES[KINDS[q]][k] * n for q in used) for k in ("fp32", "fp64")}
+    pipe = "fp64" if tot[3] else "fp32"
+    flop = {"kernel": roof["kernel"], "pipe": pipe, "unit": "TFLOP/s",
+            "peak_source": "nominal (SM count x lanes x clock)",
+            "scaled_from": "ncu thread-level op counts of one launch of each kind on Sedov 96^3 (profiles/), "
+                           "x npart / 884,736"}
+    for k, v in fl.items():
+        flop[k] = {"flops_per_launch": v / nl, "achieved": v / (ms / 1e3) / 1e12, "peak": PEAK_TFLOPS[k],
+                   "frac": v / (ms / 1e3) / 1e12 / PEAK_TFLOPS[k]}
+    flop["frac"] = flop[pipe]["frac"]
+    return roof, flop
 
 
 def workload(name: str):
@@ -308,9 +349,9 @@ def time_arm(args, dist, ws, cfg, x, v, B, prec, local, e2e=True, steps=None, wa
     dt = ctx.derivs(1, 0.0)
     if cfg.get("nalpha", 0):
         ctx.alpha_initial()  # initial.F90:736-742
-    t = 0.0
+    t, last_its = 0.0, 0
     for _ in range(warmup):
-        dtn, _, dterr = ctx.step(t, dt); t += dt; dt = min(dtn, dterr)
+        dtn, last_its, dterr = ctx.step(t, dt); t += dt; dt = min(dtn, dterr)
 
     def pinned(shape, dtype):
         return torch.empty(shape, dtype=dtype, pin_memory=True).numpy()
@@ -324,16 +365,20 @@ def time_arm(args, dist, ws, cfg, x, v, B, prec, local, e2e=True, steps=None, wa
     p0 = sum_m_abs_v(ctx, cfg)
     torch.cuda.synchronize(); barrier(dist)
     l0 = ctx.launches()
-    dev_ms, kforce_ms, ktotal = 0.0, 0.0, np.zeros(8)
+    dev_ms, ktotal = 0.0, np.zeros(8)
     trial_sum, pairs, its_tot = 0, 0, 0
+    kinds, step_force_ms = [], []
     with ClockSampler(local) as clk:
         w0 = time.perf_counter()
         for _ in range(steps):
             dtn, its, dterr = ctx.step(t, dt)
             tm = ctx.timings()
             wc = ctx.work_counters()
-            dev_ms += tm[7]; ktotal += tm; kforce_ms += tm[4]
+            dev_ms += tm[7]; ktotal += tm
             trial_sum += int(wc[0]); pairs += int(wc[2]); its_tot += its
+            kinds.append(launch_kinds(cfg, prec == capi.PH_PREC_MIXED, its, last_its))
+            step_force_ms.append(float(tm[4]))
+            last_its = its
             t += dt; dt = min(dtn, dterr)
         torch.cuda.synchronize()
         wall = time.perf_counter() - w0
@@ -345,8 +390,9 @@ def time_arm(args, dist, ws, cfg, x, v, B, prec, local, e2e=True, steps=None, wa
     dev_s = reduce_max(dist, dev_ms / 1e3)
     out = {"value": n * ws * steps / dev_s, "ms_per_step": dev_s * 1e3 / steps,
            "wall_ms_per_step": 1e3 * wall / steps, "launches": launches, "clocks": clk.summary(),
-           "phases": (ktotal / steps).tolist(), "kforce_ms": kforce_ms, "its": its_tot,
-           "trial_sum": trial_sum, "pairs": pairs, "tune": tuned, "conservation": cons}
+           "phases": (ktotal / steps).tolist(), "its": its_tot,
+           "trial_sum": trial_sum, "pairs": pairs, "tune": tuned, "conservation": cons,
+           "kinds": kinds, "step_force_ms": step_force_ms}
     if e2e:
         host = [None if a is None else torch.from_numpy(a.copy()).pin_memory().numpy() for a in snap]
         # per step: xyzh, vxyzu, fxyzu (+ Bevol, dBevol) as (4,N) float64 and div v float32, each way
@@ -699,23 +745,10 @@ def run_ours(args, dist, rank, ws):
     hp = precs[-1]
     h = arms[hp]
     mixed = hp == capi.PH_PREC_MIXED
-    # ---- roofline of the dominant kernel (force pair loop), hbm model
+    # ---- rooflines of the force launches, the dominant kernels
     peaks = measured_peaks()
-    peak = peaks["hbm_gbs"] if peaks else 6800.0
-    nlaunch = max(h["its"], 1)  # one force evaluation per velocity iteration
-    kf_per = h["kforce_ms"] / nlaunch / 1e3
-    rnb, rown = (R_NB_FORCE_MIXED, R_OWN_FORCE_MIXED) if mixed else (R_NB_FORCE, R_OWN_FORCE)
-    bytes_per_launch = (h["trial_sum"] / nlaunch) * rnb + n * rown
-    achieved = bytes_per_launch / max(kf_per, 1e-12) / 1e9
-    traffic = TRAFFIC_PER_PARTICLE_MIXED * n if (mixed and args.workload.startswith("sedov")) else None
-    roof = {"bound": "hbm", "kernel": "k_force_mixed" if mixed else "k_force", "achieved": achieved, "peak": peak,
-            "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
-            "traffic_source": TRAFFIC_SOURCE if traffic is not None else None,
-            "peak_source": "measured" if peaks else "fallback",
-            "model": f"leaf-staged gather: {rnb} B x trial entries + {rown} B x particles per launch",
-            "algorithmic_bytes_per_launch": bytes_per_launch,
-            "ms_per_launch": kf_per * 1e3, "launches_per_step": h["its"] / args.steps}
-    flop_roof = flop_roofline("k_force_mixed" if mixed else "k_force", n, kf_per * 1e3)
+    peak, source = (peaks["hbm_gbs"], "measured") if peaks else (6800.0, "fallback")
+    roof, flop_roof = force_rooflines(h, cfg, n, peak, source)
     nth = os.cpu_count() or 1
     # ---- CPU baseline: oracle port on the host cores, a bounded sample of the
     # timed steps (the same warm-up, then the first steps the GPU arm times)
@@ -766,14 +799,14 @@ def run_ours(args, dist, rank, ws):
         line["adjoint_rollout"] = ro
     if len(precs) == 2:
         f = arms[capi.PH_PREC_FP64]
-        f_per_ms = f["kforce_ms"] / max(f["its"], 1)
+        froof, fflop = force_rooflines(f, cfg, n, peak, source)
         line["fp64"] = {"value": f["value"], "ms_per_step": f["ms_per_step"], "gpu_launches": f["launches"],
                         "clocks": f["clocks"], "k_force_ms_per_step": f["phases"][4],
                         "e2e": {"value": f["e2e"], "unit": UNIT, "h2d_bytes_per_step": f["h2d"],
                                 "d2h_bytes_per_step": f["d2h"]},
                         "conservation": f["conservation"],
                         "velocity_iterations_per_step": f["its"] / args.steps,
-                        "flop_roofline": flop_roofline("k_force", n, f_per_ms)}
+                        "roofline": froof, "flop_roofline": fflop}
         if cpu:
             line["vs_cpu"]["fp64_device"] = f["value"] / cpu["value"]
             line["vs_cpu"]["fp64_e2e"] = f["e2e"] / cpu["value"]

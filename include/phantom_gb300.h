@@ -259,8 +259,15 @@ int ph_adjoint_full(ph_ctx *ctx, const double *w_fxyzu, const double *w_dBevol, 
  * recomputes, ms8[7] the whole call. With self-gravity each adjoint starts
  * from the h its forward evaluation started from (the predicted h of the
  * step, the uploaded h for the first), so its tree, node hmax and walk are
- * the forward's; otherwise from the converged h. The Cullen-Dehnen switch and individual timesteps return
- * PH_ERR_NOT_BUILT. */
+ * the forward's; otherwise from the converged h. In the precision form a hydro
+ * rollout evaluates with pair sums of its own order, so its trajectory and loss are
+ * those of ph_step to rounding, not bit for bit. With viscosity or conductivity
+ * on, the gradient passes through their switches (v.r = 0, P_i = P_j) at
+ * every step, and FP32 sums leave single components of it undetermined: over 8
+ * steps of 64000 particles the median component is within 2e-6 of the FP64 form's,
+ * 99 % within 2e-3, the norm of the difference 2e-3 to 6e-3, but the largest
+ * difference is of the size of the largest component. The Cullen-Dehnen switch
+ * and individual timesteps return PH_ERR_NOT_BUILT. */
 int ph_rollout_adjoint(ph_ctx *ctx, int32_t nsteps, const double *dts, int32_t ckpt, const double *w_fxyzu,
                        double *loss, double *g_xyzh, double *g_vxyzu);
 

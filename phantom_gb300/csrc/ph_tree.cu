@@ -918,7 +918,10 @@ __device__ __forceinline__ int seg_sum_int(int v) {
 // generation lists (first particle, count, flags: split axis in bits 0-1, bit
 // 2 a right child, bit 3 the subtree's root; parent id)
 constexpr int SUB_THREADS = 512, SUB_WARPS = SUB_THREADS / 32;
-constexpr int SUB_SEQ = 256;  // nodes up to this size: one lane per chain (all chains at once, ~70 cycles a term)
+// nodes up to this size: one lane per chain (all chains at once, ~70 cycles a
+// term). Builds of 12^3, 40^3, 128^3 particles with 64: +8, +5, +6 %; 128: +3, +1,
+// +2 %; 512: +2, +1, +1 %; 1024: +8, +4, +4 %.
+constexpr int SUB_SEQ = 256;
 struct SubList { unsigned short *st, *ct; unsigned char *fl; int *par; };
 struct Sub {
   double *X, *Y, *Z, *com;
@@ -1413,6 +1416,12 @@ __global__ void __launch_bounds__(SUB_THREADS, 2) k_subtree(Params p, const GenE
       centre(g, a, acc);
     }
     __syncthreads();
+    // Which form takes a generation, by its largest node. Teams leave warps of
+    // their own to nodes of up to two particles per lane; segments keep two to
+    // six particles per lane. The lines are flat: builds of 12^3 to 128^3
+    // particles (0.36, 0.81, 1.04, 3.00 ms at 12^3, 40^3, 64^3, 128^3) change
+    // by less than 1 % with 16 to 256 in place of 64, or 48 to 384 of 96, and with 24
+    // at 12 and 96 by +1 % and -1 %.
     if (ncur <= SUB_WARPS / 2 && top > 64) {
       int tw = SUB_WARPS;
       while (tw * ncur > SUB_WARPS) tw >>= 1;
