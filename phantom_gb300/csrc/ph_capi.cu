@@ -9,11 +9,18 @@
 
 using namespace ph;
 
-namespace {
+namespace ph {
 
-void dfree(ph_ctx *c, void *p);
+static void dfree(ph_ctx *c, void *p) {
+  for (size_t k = 0; k < c->allocs.size(); ++k)
+    if (c->allocs[k].p == p) {
+      cudaFree(p);
+      c->allocs.erase(c->allocs.begin() + k);
+      return;
+    }
+}
 
-void drop_record(ph_ctx *c) {
+static void drop_record(ph_ctx *c) {
   if (c->rec_rows) dfree(c, c->rec_rows);
   c->rec_rows = nullptr;
   c->rec_cap = 0;
@@ -22,6 +29,7 @@ void drop_record(ph_ctx *c) {
 // Device memory for a context. Where there is none left, the pair record, which
 // only saves time, is given up for it (unless the evaluation under way replays
 // it). A failure is the caller's status, not an error of the launches after it.
+// Freed with cudaFree, or with the context where it is kept in allocs.
 cudaError_t device_alloc(ph_ctx *c, void **q, size_t bytes) {
   cudaError_t e = cudaMalloc(q, bytes);
   if (e != cudaSuccess && c->rec_rows && c->rec_mode != PAIRS_REPLAY) {
@@ -31,6 +39,10 @@ cudaError_t device_alloc(ph_ctx *c, void **q, size_t bytes) {
   if (e != cudaSuccess) cudaGetLastError();
   return e;
 }
+
+}  // namespace ph
+
+namespace {
 
 // A cleared device buffer of the context. Cleared on the context's stream, which
 // does not wait for the default stream: the launches that follow write into it.
@@ -45,13 +57,11 @@ int dalloc(ph_ctx *c, T **p, size_t count) {
   return 0;
 }
 
-void dfree(ph_ctx *c, void *p) {
-  for (size_t k = 0; k < c->allocs.size(); ++k)
-    if (c->allocs[k].p == p) {
-      cudaFree(p);
-      c->allocs.erase(c->allocs.begin() + k);
-      return;
-    }
+// the same where the buffer is not there yet: an allocation that failed half way
+// is taken up again by the next call
+template <typename T>
+int dneed(ph_ctx *c, T **p, size_t count) {
+  return *p ? 0 : dalloc(c, p, count);
 }
 
 int alloc_all(ph_ctx *c, int64_t cap) {
@@ -157,17 +167,15 @@ bool grow_record(ph_ctx *c, int64_t rows) {
   if (c->rec_limit >= 0 && 512 * (size_t)rows + cells > (size_t)c->rec_limit) return false;
   if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail / 4 < bytes) return false;
   drop_record(c);
-  if (!c->rec_cell && dalloc(c, &c->rec_cell, (size_t)c->cap) != 0) return false;
+  if (dneed(c, &c->rec_cell, (size_t)c->cap) != 0) return false;
   if (dalloc(c, &c->rec_rows, 32 * (size_t)rows) != 0) return false;
   c->rec_cap = rows;
   return true;
 }
 
 int alloc_sym(ph_ctx *c, int64_t rows, int nj) {
-  if (!c->cell_tbase) {
-    if (!c->cell_at && dalloc(c, &c->cell_at, (size_t)c->cap) != 0) return PH_ERR_CUDA;
-    if (dalloc(c, &c->cell_tbase, (size_t)c->cap + 1) != 0) return PH_ERR_CUDA;
-  }
+  if (dneed(c, &c->cell_at, (size_t)c->cap) != 0 || dneed(c, &c->cell_tbase, (size_t)c->cap + 1) != 0)
+    return PH_ERR_CUDA;
   if (c->toff_cap < c->pool_cap) {
     if (c->toff) dfree(c, c->toff);
     c->toff = nullptr;
@@ -200,26 +208,23 @@ int alloc_rollout(ph_ctx *c, size_t doubles) {
 // gravity far-field buffers, allocated on the first force evaluation with
 // self-gravity (about 160 bytes per node id)
 int alloc_gravity(ph_ctx *c) {
-  if (c->fb) return 0;
   int r = 0;
-  r |= dalloc(c, &c->fb, (size_t)LENFG * (size_t)c->node_cap);
-  r |= dalloc(c, &c->gleaf, (size_t)LENFG * (size_t)c->cap);
-  r |= dalloc(c, &c->leaf_of, (size_t)c->cap);
+  r |= dneed(c, &c->fb, (size_t)LENFG * (size_t)c->node_cap);
+  r |= dneed(c, &c->gleaf, (size_t)LENFG * (size_t)c->cap);
+  r |= dneed(c, &c->leaf_of, (size_t)c->cap);
   return r ? PH_ERR_CUDA : 0;
 }
 
 // level-by-level far field: per-node arrays once, the opened-list pool
 // (re)allocated to at least `need` entries
 int alloc_levels(ph_ctx *c, int64_t need) {
-  if (!c->lv_nodes) {
-    const size_t nc = (size_t)c->node_cap;
-    int r = 0;
-    r |= dalloc(c, &c->lv_nodes, nc); r |= dalloc(c, &c->lv_depth, nc);
-    r |= dalloc(c, &c->o_off, nc); r |= dalloc(c, &c->o_len, nc); r |= dalloc(c, &c->cell_of_node, nc);
-    r |= dalloc(c, &c->lv_hist, 2 * (size_t)(LV_MAXDEPTH + 1)); r |= dalloc(c, &c->lv_flag, 4);
-    r |= dalloc(c, &c->mqf, 2 * nc);
-    if (r) return PH_ERR_CUDA;
-  }
+  const size_t nc = (size_t)c->node_cap;
+  int r = 0;
+  r |= dneed(c, &c->lv_nodes, nc); r |= dneed(c, &c->lv_depth, nc);
+  r |= dneed(c, &c->o_off, nc); r |= dneed(c, &c->o_len, nc); r |= dneed(c, &c->cell_of_node, nc);
+  r |= dneed(c, &c->lv_hist, 2 * (size_t)(LV_MAXDEPTH + 1)); r |= dneed(c, &c->lv_flag, 4);
+  r |= dneed(c, &c->mqf, 2 * nc);
+  if (r) return PH_ERR_CUDA;
   if (c->opool_cap < need) {
     if (c->opool) dfree(c, c->opool);
     c->opool = nullptr;
@@ -232,13 +237,13 @@ int alloc_levels(ph_ctx *c, int64_t need) {
 
 // individual-timestep state (allocated for contexts with ind_timesteps)
 int alloc_ind(ph_ctx *c) {
-  if (c->ibin) return 0;
   const size_t n = (size_t)c->cap;
   int r = 0;
-  r |= dalloc(c, &c->ibin, n); r |= dalloc(c, &c->ibin_old, n); r |= dalloc(c, &c->ibin_wake, n);
-  r |= dalloc(c, &c->ibin_old_t, n); r |= dalloc(c, &c->twas, n);
-  r |= dalloc(c, &c->actf, n); r |= dalloc(c, &c->actf_t, n); r |= dalloc(c, &c->wakemark, n);
-  r |= dalloc(c, &c->cell_act, n); r |= dalloc(c, &c->d_ind, 8);
+  r |= dneed(c, &c->ibin_old, n); r |= dneed(c, &c->ibin_wake, n);
+  r |= dneed(c, &c->ibin_old_t, n); r |= dneed(c, &c->twas, n);
+  r |= dneed(c, &c->actf, n); r |= dneed(c, &c->actf_t, n); r |= dneed(c, &c->wakemark, n);
+  r |= dneed(c, &c->cell_act, n); r |= dneed(c, &c->d_ind, 8);
+  if (r == 0) r = dneed(c, &c->ibin, n);  // last: stands for the others elsewhere
   return r ? PH_ERR_CUDA : 0;
 }
 
@@ -251,9 +256,8 @@ int alloc_dvsum(ph_ctx *c) {
 // curl v (3 rows per particle, caller order) and the staging array of the
 // caller's divcurlv(4,N), allocated on first use
 int alloc_curlv(ph_ctx *c) {
-  if (c->curl3) return 0;
-  int r = dalloc(c, &c->curl3, 3 * (size_t)c->cap);
-  r |= dalloc(c, &c->dcv_stage, 4 * (size_t)c->cap);
+  int r = dneed(c, &c->dcv_stage, 4 * (size_t)c->cap);
+  if (r == 0) r = dneed(c, &c->curl3, 3 * (size_t)c->cap);
   return r ? PH_ERR_CUDA : 0;
 }
 

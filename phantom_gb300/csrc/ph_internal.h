@@ -53,6 +53,7 @@ enum { PAIRS_SWEEP = 0, PAIRS_RECORD, PAIRS_REPLAY };
 constexpr int REC_ROWS = 24;  // slot of ph_ctx::counters: rows of the pair record
 bool pairs_recordable(const ph_ctx *c);
 bool grow_record(ph_ctx *c, int64_t rows);
+cudaError_t device_alloc(ph_ctx *c, void **q, size_t bytes);
 // hydro evaluations of the precision form's rollouts (ph_rollout_pairs.cu)
 void ro_density(ph_ctx *c, const int *act, int nact);
 void ro_force_prologue(ph_ctx *c, const double *vel);

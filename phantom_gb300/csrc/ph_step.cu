@@ -275,12 +275,13 @@ int ph_get_alpha(ph_ctx *c, float *alphaind, float *dvdx) {
   if (!c) return PH_ERR_ARG;
   const int n = (int)c->n;
   if (n <= 0 || (!alphaind && !dvdx)) return 0;
-  float *da = nullptr, *dd = nullptr;
-  if (cudaMalloc(&da, sizeof(float) * 3 * (size_t)n) != cudaSuccess ||
-      cudaMalloc(&dd, sizeof(float) * 9 * (size_t)n) != cudaSuccess) {
-    if (da) cudaFree(da);
+  void *qa = nullptr, *qd = nullptr;
+  if (device_alloc(c, &qa, sizeof(float) * 3 * (size_t)n) != cudaSuccess ||
+      device_alloc(c, &qd, sizeof(float) * 9 * (size_t)n) != cudaSuccess) {
+    if (qa) cudaFree(qa);
     return PH_ERR_CUDA;
   }
+  float *da = static_cast<float *>(qa), *dd = static_cast<float *>(qd);
   k_alpha_gather<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->alpha1, c->alphaloc_t, c->ddivvdt_c, c->dvdx_c,
                                                       c->have_tree ? c->iperm : nullptr, da, dd);
   count_launch(c);

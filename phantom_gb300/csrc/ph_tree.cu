@@ -1822,16 +1822,16 @@ int get_nodes(ph_ctx *c, int64_t *nnodes, int32_t *range, double *xcen, double *
   cudaStream_t st = c->stream;
   std::vector<int> iota((size_t)nbig);
   for (int k = 0; k < nbig; ++k) iota[(size_t)k] = k;
-  int *ids = nullptr, *dr = nullptr, *dl = nullptr;
-  double *dx = nullptr, *ds = nullptr, *dh = nullptr, *dm = nullptr;
-  bool ok = cudaMalloc(&ids, sizeof(int) * (size_t)m) == cudaSuccess &&
-            cudaMalloc(&dr, sizeof(int) * 2 * (size_t)m) == cudaSuccess &&
-            cudaMalloc(&dl, sizeof(int) * (size_t)m) == cudaSuccess &&
-            cudaMalloc(&dx, sizeof(double) * 3 * (size_t)m) == cudaSuccess &&
-            cudaMalloc(&ds, sizeof(double) * (size_t)m) == cudaSuccess &&
-            cudaMalloc(&dh, sizeof(double) * (size_t)m) == cudaSuccess &&
-            cudaMalloc(&dm, sizeof(double) * (size_t)m) == cudaSuccess;
+  const size_t sz[7] = {sizeof(int) * (size_t)m,        sizeof(int) * 2 * (size_t)m, sizeof(int) * (size_t)m,
+                        sizeof(double) * 3 * (size_t)m, sizeof(double) * (size_t)m,  sizeof(double) * (size_t)m,
+                        sizeof(double) * (size_t)m};
+  void *buf[7] = {};
+  bool ok = true;
+  for (int k = 0; k < 7; ++k) ok = ok && device_alloc(c, &buf[k], sz[k]) == cudaSuccess;
   if (ok) {
+    int *ids = static_cast<int *>(buf[0]), *dr = static_cast<int *>(buf[1]), *dl = static_cast<int *>(buf[2]);
+    double *dx = static_cast<double *>(buf[3]), *ds = static_cast<double *>(buf[4]), *dh = static_cast<double *>(buf[5]),
+           *dm = static_cast<double *>(buf[6]);
     cudaMemcpyAsync(ids, iota.data(), sizeof(int) * (size_t)nbig, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(ids + nbig, c->node_list, sizeof(int) * (size_t)c->nsmall_nodes, cudaMemcpyDeviceToDevice, st);
     k_get_nodes<<<nblk(m, 256), 256, 0, st>>>(ids, m, c->nodes, c->nmass, dr, dx, ds, dh, dm, dl);
@@ -1844,7 +1844,7 @@ int get_nodes(ph_ctx *c, int64_t *nnodes, int32_t *range, double *xcen, double *
     cudaMemcpyAsync(mass, dm, sizeof(double) * (size_t)m, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
   }
-  for (void *q : {(void *)ids, (void *)dr, (void *)dl, (void *)dx, (void *)ds, (void *)dh, (void *)dm})
+  for (void *q : buf)
     if (q) cudaFree(q);
   return ok ? 0 : PH_ERR_CUDA;
 }

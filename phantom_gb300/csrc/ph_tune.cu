@@ -19,9 +19,11 @@ struct Snapshot {
 
 int take(ph_ctx *c, Snapshot &s) {
   const size_t b4 = sizeof(double) * 4 * (size_t)c->n;
-  if (cudaMalloc(&s.x, b4) != cudaSuccess || cudaMalloc(&s.v, b4) != cudaSuccess ||
-      cudaMalloc(&s.b, b4) != cudaSuccess)
-    return PH_ERR_CUDA;
+  for (double **q : {&s.x, &s.v, &s.b}) {
+    void *m = nullptr;
+    if (ph::device_alloc(c, &m, b4) != cudaSuccess) return PH_ERR_CUDA;
+    *q = static_cast<double *>(m);
+  }
   cudaMemcpyAsync(s.x, c->xyzh, b4, cudaMemcpyDeviceToDevice, c->stream);
   cudaMemcpyAsync(s.v, c->vxyzu, b4, cudaMemcpyDeviceToDevice, c->stream);
   cudaMemcpyAsync(s.b, c->Bevol, b4, cudaMemcpyDeviceToDevice, c->stream);
