@@ -103,7 +103,8 @@ int ph_init(const ph_params *params, int64_t maxp, ph_ctx **ctx);
  * particles stay usable by the calls that follow (a force in the other precision
  * form included; trial lists are made again where a parameter they depend on
  * changed), except that a new minpart, or self-gravity switched on, needs a
- * new tree and density (PH_ERR_STATE until then). */
+ * new tree and density before ph_density and ph_force (PH_ERR_STATE until then;
+ * ph_derivs, ph_step and the adjoints make their own). */
 int ph_set_params(ph_ctx *ctx, const ph_params *params);
 /* Bound on the device memory that ph_step may take for its pair record, in
  * bytes (negative, the default: none of its own; 0: no record). In the precision

@@ -1396,7 +1396,7 @@ int adjoint_dev(ph_ctx *c, const double *w_dev, const double *wB_dev, double *gx
   cudaEventRecord(c->ev[0], st);
   // forward state at the uploaded positions: tree, density, force lists
   int r = 0;
-  if (!c->have_tree) { r = build_tree(c); if (r) return r; }
+  if (!c->have_tree || (p.gravity && !c->tree_grav)) { r = build_tree(c); if (r) return r; }
   if (!c->have_density) { r = density(c, 1); if (r) return r; }
   r = force_lists(c);
   if (r) return r;

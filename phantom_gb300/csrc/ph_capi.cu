@@ -401,8 +401,7 @@ static bool lists_differ(const ph_params &a, const ph_params &b) {
 int ph_set_params(ph_ctx *c, const ph_params *params) {
   if (!c || !params || !params_ok(params)) return PH_ERR_ARG;
   if (lists_differ(c->hp, *params)) c->have_force_lists = false;
-  if (params->gravity && !c->hp.gravity)  // no quadrupoles, no softening sums
-    c->have_tree = c->have_density = c->have_force = c->have_force_lists = false;
+  if (params->gravity && !c->hp.gravity) c->have_density = c->have_force_lists = false;  // no softening sums
   if ((params->minpart > 0 ? params->minpart : MINPART) != c->dp.minpart)
     c->have_tree = c->have_density = c->have_force = c->have_force_lists = false;  // a new leaf size needs a new tree
   c->hp = *params;

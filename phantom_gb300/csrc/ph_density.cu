@@ -768,7 +768,7 @@ void low_words(ph_ctx *c) {
 
 // densityiterate driver
 int density(ph_ctx *c, int icall) {
-  if (!c->have_tree) return PH_ERR_STATE;
+  if (!c->have_tree || (c->dp.gravity && !c->tree_grav)) return PH_ERR_STATE;
   c->have_force_lists = false;  // the density walks reuse the list pool
   cudaStream_t st = c->stream;
   const int nt = (int)c->ntree, ncell = c->nleaves;

@@ -95,6 +95,7 @@ struct ph_ctx {
   int64_t cap = 0;  // particle capacity
   int64_t n = 0;    // live particle count (caller order)
   int64_t launches = 0;
+  bool tree_grav = false;  // the tree's nodes hold quadrupoles
   bool have_tree = false, have_density = false, have_force = false, have_force_lists = false;
   // kernel attributes (dynamic shared memory) set on this context's device:
   // bit 0 density pair kernels, bit 1 force pair kernels, bit 2 adjoint, bit 3

@@ -1725,6 +1725,7 @@ int build_tree(ph_ctx *c) {
   c->minlevel = hostv[2];
   c->root = 0;
   c->have_tree = true;
+  c->tree_grav = p.gravity != 0;
   c->have_density = c->have_force_lists = false;
   if (p.ind && c->ibin) return ind_after_tree(c);  // active flags and cells in the new tree order
   return 0;
@@ -1808,6 +1809,7 @@ int revtree(ph_ctx *c) {
   cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost);
   if (herr) return herr;
   // positions changed: density, force lists and far field follow the refit
+  c->tree_grav = p.gravity != 0;
   c->have_density = c->have_force = c->have_force_lists = false;
   return 0;
 }

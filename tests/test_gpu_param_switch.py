@@ -84,8 +84,29 @@ def test_self_gravity_needs_its_own_tree():
     with pytest.raises(capi.PhantomError) as e:
         ctx.force(1, 0.0)
     assert e.value.code == 13
+    with pytest.raises(capi.PhantomError) as e:
+        ctx.densityiterate(1)
+    assert e.value.code == 13
     ctx.upload(x, v, B)  # the given h again: the tree's hmax, hence its opening, depends on it
     ctx.build_tree()
     ctx.densityiterate(1)
     got = ctx.force(1, 0.0)["fxyzu"]
     close(got[:, :3], solved(cfg, x, v, B, FP64).force(1, 0.0)["fxyzu"][:, :3], 1.0e-9)
+
+
+def test_self_gravity_switched_on_before_a_step():
+    """The step kicks with the forces it has and evaluates with its own tree: as
+    from the same state uploaded into a context with self-gravity."""
+    cfg, x, v, B = case("cloud")
+    ctx = capi.Context(dict(cfg, gravity=0))
+    ctx.upload(x, v, B)
+    dt = ctx.derivs(1, 0.0)
+    n = len(x)
+    st = [np.zeros((n, 4)) for _ in range(5)] + [np.zeros(n, np.float32)]
+    ctx.download_state(*st)
+    ctx.set_params(dict(gravity=1))
+    want = capi.Context(cfg)
+    want.upload_state(*st)
+    assert ctx.step(0.0, dt) == want.step(0.0, dt)
+    for a, b in zip(ctx.download(), want.download()):
+        assert np.array_equal(a, b)
